@@ -8,14 +8,16 @@
 //
 //  * div_rn(x, d, r): x / d rounded to nearest for a divisor d > 0 whose
 //    reciprocal r = RN(1/d) was computed beforehand.  q0 = RN(x * r) is
-//    within 1.5 ulp of x / d; one exact FMA remainder e0 = q0 * d - x,
-//    compared as an integer with half an ulp of q0 times d, picks the
-//    correctly rounded quotient among q0 and its two neighbours.  1 DMUL +
-//    1 DFMA.  When q0 is a power of two (the spacing changes below it) the
-//    quotient takes Markstein's two refinements instead (Markstein,
-//    "Computation of elementary functions on the IBM RISC System/6000
-//    processor", IBM J. Res. Dev. 34(1), 1990; Muller et al., Handbook of
-//    Floating-Point Arithmetic, 2nd ed., Sec. 4.7), 1 DMUL + 4 DFMA.
+//    within 1.5 ulp of x / d; the exact remainder q0 * d - x, formed from
+//    the significands in 64-bit integers and compared with half an ulp of q0
+//    times d, picks the correctly rounded quotient among q0 and its two
+//    neighbours.  1 DMUL and about 20 integer instructions (the remainder by
+//    FMA cost one DFMA more, 64 issue slots of a scheduler against ~10).
+//    When q0 is a power of two (the spacing changes below it) the quotient
+//    takes Markstein's two refinements instead (Markstein, "Computation of
+//    elementary functions on the IBM RISC System/6000 processor", IBM J.
+//    Res. Dev. 34(1), 1990; Muller et al., Handbook of Floating-Point
+//    Arithmetic, 2nd ed., Sec. 4.7), 1 DMUL + 4 DFMA.
 //    x = +-0 returns x.  Dividends whose magnitude is tiny (below 2^-899,
 //    other than zero), huge (2^900 and above) or not finite use the IEEE
 //    divide, so no intermediate underflows or overflows; divisors are
@@ -69,26 +71,33 @@ static __device__ __noinline__ double div_markstein(double x, double d, double r
 }
 
 __device__ __forceinline__ double div_rn(double x, double d, double r) {
-  const long long xb = bits(x);
-  if ((xb & 0x7fffffffffffffffLL) == 0) return x;  // +-0 / d keeps the sign for d > 0
-  const int ex = (int)((xb >> 52) & 0x7ff);
-  if (ex < 124 || ex > 1922) return div_ieee(x, d);
+  const unsigned long long xb = (unsigned long long)bits(x);
+  const unsigned xh = (unsigned)(xb >> 32);
+  const int ex = (int)((xh >> 20) & 0x7ff);
+  if (ex < 124 || ex > 1922) {
+    if ((xb & 0x7fffffffffffffffULL) == 0) return x;  // +-0 / d keeps the sign for d > 0
+    return div_ieee(x, d);
+  }
   const double q0 = x * r;
-  const long long qb = bits(q0);
-  if ((qb & 0xfffffffffffffLL) == 0) return div_markstein(x, d, r);
+  const unsigned long long qb = (unsigned long long)bits(q0), db = (unsigned long long)bits(d);
+  constexpr unsigned long long kFrac = 0xfffffffffffffULL, kOne = 1ULL << 52;
+  if ((qb & kFrac) == 0) return div_markstein(x, d, r);
   // q0 is not a power of two, so q = x / d lies in q0's binade and within
-  // 1.5 ulp of it: RN(q) is q0 - ulp, q0 or q0 + ulp.  The remainder
-  // e0 = q0 * d - x = d * (q0 - q) is exact wherever it decides (|e0| <
-  // 2^53 units of its grid), and RN(q) moves off q0 exactly when |e0| >
-  // h = d * ulp(q0) / 2 (a quotient is never a midpoint).  h is d with
-  // its exponent shifted, compared as a bit pattern.
-  const double e0 = fma(q0, d, -x);
-  const long long eb = bits(e0);
-  const int eq = (int)((qb >> 52) & 0x7ff);
-  const long long hb = bits(d) + ((long long)(eq - 1076) << 52);
-  long long k = 0;  // +1: one ulp up in value, -1: one ulp down
-  if ((eb & 0x7fffffffffffffffLL) > hb) k = (eb < 0) ? 1 : -1;
-  return from_bits(qb + (qb < 0 ? -k : k));
+  // 1.5 ulp of it: RN(q) is q0 - ulp, q0 or q0 + ulp.  With the significands
+  // mq, md, mx as integers, q0 * d - x = 2^t (mq md - mx 2^s) for the s of
+  // the three exponents (52 or 53 here), and RN(q) moves off q0 exactly when
+  // |mq md - mx 2^s| > md / 2 (a quotient is never a midpoint).  That
+  // difference is below 1.5 md + 1 < 2^55 in size, so its low 64 bits are
+  // all of it: of mx 2^s only the low bits of x count.
+  const unsigned long long mq = (qb & kFrac) | kOne, md = (db & kFrac) | kOne;
+  const unsigned sh = ((xh >> 20) - ((unsigned)(qb >> 32) >> 20) - (unsigned)(db >> 52) +
+                       (1075u - 32u)) & 31u;  // s - 32
+  const unsigned long long rem =
+      mq * md - ((unsigned long long)((unsigned)xb << sh) << 32);
+  // +1: one ulp up in magnitude (the remainder is negative), -1: one down
+  long long k = 0;
+  if (rem + (md >> 1) > (md & ~1ULL)) k = (long long)rem < 0 ? 1 : -1;
+  return from_bits((long long)qb + k);
 }
 
 __device__ __forceinline__ double half(double x) {
