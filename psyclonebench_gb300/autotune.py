@@ -5,13 +5,13 @@ nl2d_ens_tile):
 
 * FP64 form: persistent CTAs per SM (1 or 2), tile assignment (contiguous
   cost-balanced chunks, longest processing time first, or one tile per CTA
-  left to the hardware block scheduler), the cost weight given to the edge
-  cells of boundary tiles (which take the general per-cell path), and the
-  tile shape (32 x 16, 32 x 8, 16 x 16, 64 x 8, 32 x 32).  The reference's
+  left to the hardware block scheduler), the cost weight given to the
+  domains' ring cells (which take the general per-cell path), and the tile
+  shape (32 x 16, 32 x 8, 16 x 16, 64 x 8, 32 x 32).  The reference's
   tiled OpenMP layer (psykal_omp/time_step_mod.f90:587-1182) takes its tile
   size as a run parameter; here it is searched.  The search has two stages:
   every schedule at the default shape, then every shape under the best
-  schedule and under one-tile-per-CTA.
+  schedule and under one-tile-per-CTA (the runner-up where that is the best).
 * Mixed and FP64-equivalent ("df") forms: the column march's strip height
   (8, 16, 32 or 64 rows), under the FP64 knobs already applied.
 
@@ -83,15 +83,14 @@ def _time(ens, c, steps):
     return ms / steps
 
 
-def _fp64_candidates(best_schedule=None):
-    if best_schedule is None:
+def _fp64_candidates(schedules=None):
+    if schedules is None:
         return [{"ctas_per_sm": cps, "policy": pol, "boundary_weight": bw,
                  "tile": list(DEFAULT_SHAPE), "march_rows": DEFAULT_MARCH_ROWS}
                 for cps, pol, bw in SCHEDULES]
     out = []
     for shape in SHAPES[1:]:
-        for sched in sorted({best_schedule, (2, 2, 0.0)}):
-            cps, pol, bw = sched
+        for cps, pol, bw in schedules:
             out.append({"ctas_per_sm": cps, "policy": pol, "boundary_weight": bw,
                         "tile": list(shape), "march_rows": DEFAULT_MARCH_ROWS})
     return out
@@ -120,9 +119,11 @@ def tune(ens, steps=4, precision="fp64", use_cache=True, base=None):
     else:
         for c in _fp64_candidates():
             timings.append((_time(ens, c, steps), c))
-        first = min(timings, key=lambda t: t[0])[1]
-        sched = (first["ctas_per_sm"], first["policy"], first["boundary_weight"])
-        for c in _fp64_candidates(sched):
+        order = [(c["ctas_per_sm"], c["policy"], c["boundary_weight"])
+                 for _, c in sorted(timings, key=lambda t: t[0])]
+        # the best schedule and one tile per CTA (the runner-up where that is the best)
+        scheds = [order[0], order[1] if order[0][1] == 2 else (2, 2, 0.0)]
+        for c in _fp64_candidates(scheds):
             timings.append((_time(ens, c, steps), c))
     ms, best = min(timings, key=lambda t: t[0])
     choice = dict(best, ms_per_step=ms,

@@ -565,12 +565,12 @@ bool do_register(void* const* ptrs, int xs, int xe, int ys, int ye, int width, i
   const size_t n = (size_t)width * height;
   s.registered = true;  // so free_device releases partial allocations
   s.h2d_bytes = s.d2h_bytes = 0;
-  // One allocation carved into the registration's 32 arrays (256-byte
+  // One allocation carved into the registration's 34 arrays (256-byte
   // aligned): 34 separate cudaMalloc calls took 1.7-2.9 ms on the GB300
   // box, one of the same total 0.18 ms, and the first call waits for them
   // before its first copy.
   const size_t a8 = (n * 8 + 255) & ~(size_t)255, a4 = (n * 4 + 255) & ~(size_t)255;
-  if (!CK(cudaMalloc(&s.slab, (size_t)(kNumFields + kNumGrid - 1 + 4 + 3) * a8 + a4)))
+  if (!CK(cudaMalloc(&s.slab, (size_t)(kNumFields + kNumGrid - 1 + 6 + 3) * a8 + a4)))
     return false;
   char* cut = static_cast<char*>(s.slab);
   auto take = [&cut](size_t bytes) {
@@ -583,6 +583,8 @@ bool do_register(void* const* ptrs, int xs, int xe, int ys, int ye, int width, i
   for (int k = 1; k < kNumGrid; k++) *grid_slot(s.dev, k) = (double*)take(a8);
   s.dev.sin_u = (double*)take(a8);
   s.dev.sin_v = (double*)take(a8);
+  s.dev.d_hu = (double*)take(a8);
+  s.dev.d_hv = (double*)take(a8);
   s.dev.r_hu = (double*)take(a8);
   s.dev.r_hv = (double*)take(a8);
   for (double*& p : s.shadow) p = (double*)take(a8);
@@ -609,12 +611,12 @@ bool do_register(void* const* ptrs, int xs, int xe, int ys, int ye, int width, i
     if (!s.backups_done &&
         !CK(cudaEventCreateWithFlags(&s.backups_done, cudaEventDisableTiming)))
       return false;
-    int th = 0;
-    const int ntr = fused_step_tile_rows(dims(), &th);
+    const int ntr = fused_step_tile_rows(dims());
     s.nbands = std::min(State::kMaxBands, ntr);
     for (int b = 0; b <= s.nbands; b++) {
       s.band_tile[b] = (int)((long long)ntr * b / s.nbands);
-      s.band_row[b] = b == 0 ? 0 : (b == s.nbands ? height : ys - 1 + s.band_tile[b] * th);
+      s.band_row[b] =
+          b == 0 ? 0 : (b == s.nbands ? height : fused_step_first_row(dims(), s.band_tile[b]));
     }
     for (int b = 0; b < s.nbands; b++) {
       for (int k : kStepArrays)

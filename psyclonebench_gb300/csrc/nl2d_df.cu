@@ -14,8 +14,8 @@
 // every face they read takes next_ssh's two-sided formula and no momentum
 // mask, bc_ssh, solid-wall or Flather rule applies.  Every other cell of the
 // copy region (the exact cells) is computed in exact FP64 by the fused
-// step's general per-cell code reading global memory (general_cell with a
-// GlobalCtx, nl2d_fused_tile.cuh), one thread each, by blocks of the same
+// step's general per-cell code reading global memory (general_part with a
+// GlobalCtx, nl2d_fused_tile.cuh), three threads each, by blocks of the same
 // launch spread evenly among the march's blocks.
 //
 // Loads split each FP64 state value into a pair from its bit pattern
@@ -33,8 +33,8 @@ namespace {
 using namespace dfm;
 constexpr int MR = 32;
 
-// One step.  Of the grid's blocks, nring take the exact cells (128 each,
-// one per thread; block b is one when floor((b+1) nring / grid) >
+// One step.  Of the grid's blocks, nring take the exact cells' parts (all
+// cells' v, then u, then ssh; 128 each, one per thread; block b is one when floor((b+1) nring / grid) >
 // floor(b nring / grid)), so that they spread evenly among the march's
 // blocks and share the SMs with them: the march issues on the FP32 and
 // integer pipes, the exact cells wait on the FP64 pipe.  The others march
@@ -50,14 +50,15 @@ __global__ void __launch_bounds__(32 * WARPS, 3)
   const int q0 = (int)(b * nring / grid), q1 = (int)((b + 1) * nring / grid);
   if (q1 > q0) {  // exact-cell block q0
     const int g = q0 * (32 * WARPS) + (int)threadIdx.x;
-    if (g < ff.n_ring) {
-      const int c = ff.ring[g];
+    const int part = g / ff.n_ring;
+    if (part < kParts) {
+      const int c = ff.ring[g - part * ff.n_ring];
       const int j = c / d.width, i = c - j * d.width;
       const GlobalCtx x{fs.sshn_in, fs.un_in,    fs.vn_in, f.hu,      f.hv,
                         f.ht,       f.ssha_u,    f.ssha_v, f.r_hu,    f.r_hv,
                         f.tmask,    f.sshn_u,    f.sshn_v, d.width,   d,
                         fk};
-      general_cell(x, f, fs, p, tide_table ? tide_table[tide_index] : tide, i, j);
+      general_part(x, f, fs, p, tide_table ? tide_table[tide_index] : tide, part, i, j);
     }
     return;
   }
@@ -185,7 +186,7 @@ void launch_df_step(const Fields& f, const FusedState& fs, const Dims& d, const 
   int mr = MR;
   while (mr > 8 && (long long)ncol * ((ny + mr - 1) / mr) < 2 * 152 * 2 * WARPS) mr /= 2;
   const int nrow = (ny + mr - 1) / mr, nwarps = ncol * nrow;
-  const int nring = (ff.n_ring + 32 * WARPS - 1) / (32 * WARPS);
+  const int nring = (kParts * ff.n_ring + 32 * WARPS - 1) / (32 * WARPS);
   k_df_step<<<(nwarps + WARPS - 1) / WARPS + nring, 32 * WARPS, 0, st>>>(
       fs, ff, d, make_df_const(s, um), ncol, nwarps, mr, f, s, make_fast_const(s, um),
       tide_table, tide_index, tide, nring);

@@ -78,9 +78,10 @@ __global__ void k_mixed_statics(const double* __restrict__ ht, const double* __r
   }
 }
 
-// Ensemble: a persistent grid walks a tile list spanning many independent
-// domains; CTA b takes tiles [first[b], first[b+1]).  `tides` holds this
-// step's bc_ssh value per domain.
+// Ensemble: a persistent grid walks a list spanning many independent
+// domains; CTA b takes entries [first[b], first[b+1]).  An entry (domain, i0,
+// j0, -1) is a tile, (domain, -, -, g) parts g .. g + NTHREADS - 1 of the
+// domain's ring cells.  `tides` holds this step's bc_ssh value per domain.
 template <class T>
 __global__ void __launch_bounds__(NTHREADS, T::kMinBlocks)
     k_ensemble_step(const EnsDomain* __restrict__ doms, const int4* __restrict__ tiles,
@@ -91,8 +92,19 @@ __global__ void __launch_bounds__(NTHREADS, T::kMinBlocks)
   for (int t = first[blockIdx.x]; t < t1; t++) {
     const int4 tl = tiles[t];
     const EnsDomain& D = doms[tl.x];
+    if (tl.w >= 0) {
+      const int tid = threadIdx.y * T::TX + threadIdx.x, g = tl.w + tid;
+      const int ja = D.d.ys - 1, jb = D.d.ye + 1, n = ring_count(D.d, ja, jb);
+      const int part = g / n;
+      if (part < kParts) {
+        int i, j;
+        ring_pos(D.d, ja, jb, g - part * n, i, j);
+        general_at(D.f, D.fs[parity], D.d, D.p, D.k, tides[tl.x], part, i, j);
+      }
+      continue;
+    }
     __syncthreads();  // the previous tile's last readers are done with smem
-    fused_tile<T>(D.f, D.fs[parity], D.d, D.p, D.um, D.k, tides[tl.x], tl.y, tl.z, smem);
+    fused_tile<T>(D.f, D.fs[parity], D.d, D.p, D.k, tides[tl.x], tl.y, tl.z, smem);
   }
 }
 
@@ -101,21 +113,22 @@ __global__ void __launch_bounds__(NTHREADS, T::kMinBlocks)
 // and cells beside land), given as (domain, cell index), by the fused step's
 // general per-cell code reading the domain's arrays in global memory.  The
 // result is the FP64 step's, bit for bit, with that domain's tide.
-__device__ __forceinline__ void ring_cell(const EnsDomain* __restrict__ doms, int2 e, int parity,
-                                          const double* __restrict__ tides) {
+__device__ __forceinline__ void ring_cell(const EnsDomain* __restrict__ doms, int2 e, int part,
+                                          int parity, const double* __restrict__ tides) {
   const EnsDomain& D = doms[e.x];
   const FusedState& st = D.fs[parity];
   const GlobalCtx x{st.sshn_in, st.un_in,   st.vn_in, D.f.hu,    D.f.hv,    D.f.ht,
                     D.f.ssha_u, D.f.ssha_v, D.f.r_hu, D.f.r_hv,  D.f.tmask, D.f.sshn_u,
                     D.f.sshn_v, D.d.width,  D.d,      D.k};
   const int j = e.y / D.d.width, i = e.y - j * D.d.width;
-  general_cell(x, D.f, st, D.p, tides[e.x], i, j);
+  general_part(x, D.f, st, D.p, tides[e.x], part, i, j);
 }
 
 // One launch per step of the FP64-equivalent form.  A block takes one of two
 // roles: a march block runs four warps' (domain, i0, j0) units of the
-// double-float column march (nl2d_df_march.cuh); a ring block runs 128 exact
-// cells, one per thread.  The nring ring blocks are spread evenly through the
+// double-float column march (nl2d_df_march.cuh); a ring block runs 128 parts
+// of exact cells (all cells' v, then u, then ssh), one per thread.  The nring
+// ring blocks are spread evenly through the
 // grid (block b is one when floor((b+1) nring / grid) > floor(b nring /
 // grid)), so both kinds share every SM: the march issues on the FP32 and
 // integer pipes while the exact cells wait on the FP64 pipe.  Both read the
@@ -135,7 +148,8 @@ __global__ void __launch_bounds__(32 * dfm::WARPS, 3)
   const int q0 = (int)(b * nring / grid), q1 = (int)((b + 1) * nring / grid);
   if (q1 > q0) {  // ring block q0
     const int g = q0 * (32 * dfm::WARPS) + (int)threadIdx.x;
-    if (g < ncells) ring_cell(doms, cells[g], parity, tides);
+    const int part = g / ncells;
+    if (part < kParts) ring_cell(doms, cells[g - part * ncells], part, parity, tides);
     return;
   }
   // march block b - q0: q0 ring blocks precede it
@@ -445,27 +459,28 @@ double tide_at(const DomainHost& D, int istep, double rdt) {
   return D.amp * std::sin(omega_tide * rtime);
 }
 
-// Tile list and static schedule.
+// Tile list and static schedule.  A domain's ring units come before its
+// tiles; a ring cell's general code is worth boundary_weight regular cells.
 bool build_schedule(int TXv, int TYv) {
   Ens& e = g_ens;
   struct T {
-    int dom, i0, j0;
+    int dom, i0, j0, g;
     double cost;
   };
   std::vector<T> tiles;
   for (int k = 0; k < e.ndom; k++) {
     const DomainHost& D = e.dom[k];
-    const int nx = D.xe - D.xs + 3, ny = D.ye - D.ys + 2;
+    const Dims d{D.xs, D.xe, D.ys, D.ye, D.W, D.H};
+    const int nr = kParts * ring_count(d, D.ys - 1, D.ye + 1);
+    for (int g = 0; g < nr; g += NTHREADS)
+      tiles.push_back({k, 0, 0, g, e.boundary_weight * std::min(NTHREADS, nr - g) / kParts});
+    const int nx = D.xe - D.xs - 1, ny = D.ye - D.ys - 1;
+    if (nx < 1 || ny < 1) continue;
     const int ntx = (nx + TXv - 1) / TXv, nty = (ny + TYv - 1) / TYv;
     for (int by = 0; by < nty; by++)
       for (int bx = 0; bx < ntx; bx++) {
         const int cx = std::min(TXv, nx - bx * TXv), cy = std::min(TYv, ny - by * TYv);
-        // boundary tiles run the general per-cell path on their edge cells
-        double edge = 0.0;
-        if (bx == 0 || bx == ntx - 1) edge += cy;
-        if (by == 0 || by == nty - 1) edge += cx;
-        tiles.push_back({k, D.xs - 1 + bx * TXv, D.ys - 1 + by * TYv,
-                         (double)(cx * cy) + e.boundary_weight * edge});
+        tiles.push_back({k, D.xs + 1 + bx * TXv, D.ys + 1 + by * TYv, -1, (double)(cx * cy)});
       }
   }
   int dev = 0, sms = 0;
@@ -478,7 +493,7 @@ bool build_schedule(int TXv, int TYv) {
     // one tile per CTA, in domain order: the hardware block scheduler
     // balances the load and keeps as many CTAs per SM as fit
     for (size_t t = 0; t < tiles.size(); t++) {
-      order.push_back(make_int4(tiles[t].dom, tiles[t].i0, tiles[t].j0, 0));
+      order.push_back(make_int4(tiles[t].dom, tiles[t].i0, tiles[t].j0, tiles[t].g));
       first[t + 1] = (int)t + 1;
     }
   } else if (e.policy == 1) {
@@ -497,7 +512,7 @@ bool build_schedule(int TXv, int TYv) {
     for (int b = 0; b < e.nctas; b++) {
       std::sort(bins[b].begin(), bins[b].end());  // keep each CTA's tiles in memory order
       first[b + 1] = first[b] + (int)bins[b].size();
-      for (int t : bins[b]) order.push_back(make_int4(tiles[t].dom, tiles[t].i0, tiles[t].j0, 0));
+      for (int t : bins[b]) order.push_back(make_int4(tiles[t].dom, tiles[t].i0, tiles[t].j0, tiles[t].g));
     }
   } else {
     // contiguous chunks of (nearly) equal cost, in domain order
@@ -508,7 +523,7 @@ bool build_schedule(int TXv, int TYv) {
     for (size_t t = 0; t < tiles.size(); t++) {
       while (b < e.nctas - 1 && acc >= total * (b + 1) / e.nctas) first[++b] = (int)t;
       acc += tiles[t].cost;
-      order.push_back(make_int4(tiles[t].dom, tiles[t].i0, tiles[t].j0, 0));
+      order.push_back(make_int4(tiles[t].dom, tiles[t].i0, tiles[t].j0, tiles[t].g));
     }
     while (b < e.nctas) first[++b] = (int)tiles.size();
   }
@@ -545,6 +560,8 @@ bool build_descriptors() {
     // rest start: sshn_u / sshn_v, ua / va and ssha_u / ssha_v are zero where
     // no step writes them
     x.f.sshn_u = x.f.sshn_v = x.f.ua = x.f.va = x.f.ssha_u = x.f.ssha_v = e.zero + o;
+    x.f.d_hu = e.hu + o;  // + ssha_u = 0
+    x.f.d_hv = e.hv + o;
     x.f.r_hu = e.r_hu + o;
     x.f.r_hv = e.r_hv + o;
     for (int p = 0; p < 2; p++) {
@@ -1054,7 +1071,7 @@ int nl2d_ens_run(int istep0, int nsteps, int checksum_every, double* checksums_o
                                                                             sums);
       } else if (e.precision == 2) {
         constexpr int B = 32 * dfm::WARPS;
-        const int nring = (e.ndfring + B - 1) / B;
+        const int nring = (kParts * e.ndfring + B - 1) / B;
         const int nmarch = (e.ndfunits + dfm::WARPS - 1) / dfm::WARPS;
         const double* tq = e.d_tides + (size_t)q * e.ndom;
         if (e.d_dks)

@@ -11,8 +11,8 @@
 // (time_update_kern.c:90-155): those kernels are their only writers, so the
 // recomputed values are bit-identical to the stored ones; faces outside
 // their range keep their stored (never-updated) value and are read from the
-// sshn_u / sshn_v arrays.  The recomputed face values of a tile and its
-// 2-cell halo are staged in shared memory once and shared by the
+// sshn_u / sshn_v arrays.  The recomputed face values of a tile and of the
+// faces around it are staged in shared memory once and shared by the
 // continuity and both momentum updates.
 //
 // Preconditions, checked on the host before this path is used:
@@ -38,33 +38,63 @@ using T = DefaultTile;
 // arithmetic does not depend on the shape).
 using SmallTile = Tile<16, 16>;
 
+// One step of copy-region rows [ja, jb).  The first nring blocks take the
+// ring's cells in those rows, rc parts of them each (one per thread: their
+// long FP64 chains start first and run beside the tiles); the others one tile
+// each of the ntx per row of tiles, from tile row row0.
 template <class TT>
 __global__ void __launch_bounds__(NTHREADS, TT::kMinBlocks)
-    k_fused_step(Fields f, FusedState fs, Dims d, Scalars p, UniformMetrics um, FastConst k,
-                 const double* __restrict__ tide_table, int tide_index, double tide, int row0) {
+    k_fused_step(const __grid_constant__ Fields f, const __grid_constant__ FusedState fs,
+                 const __grid_constant__ Dims d, const __grid_constant__ Scalars p,
+                 const __grid_constant__ FastConst k, const double* __restrict__ tide_table,
+                 int tide_index, double tide, int row0, int ntx, int ja, int jb, int nring,
+                 int rc) {
   extern __shared__ double smem[];
-  // Tiles cover the copy region [xs-1, xe+1] x [ys-1, ye]; this launch takes
-  // tile rows row0 .. row0 + gridDim.y - 1.
-  fused_tile<TT>(f, fs, d, p, um, k, tide_table ? tide_table[tide_index] : tide,
-                 d.xs - 1 + blockIdx.x * TT::TX, d.ys - 1 + (row0 + blockIdx.y) * TT::TY,
+  const double td = tide_table ? tide_table[tide_index] : tide;
+  if ((int)blockIdx.x < nring) {
+    const int tid = threadIdx.y * TT::TX + threadIdx.x, g = blockIdx.x * rc + tid;
+    const int n = ring_count(d, ja, jb);
+    if (tid < rc && g < kParts * n) {
+      const int part = g / n;
+      int i, j;
+      ring_pos(d, ja, jb, g - part * n, i, j);
+      general_at(f, fs, d, p, k, td, part, i, j);
+    }
+    return;
+  }
+  const int t = blockIdx.x - nring, by = t / ntx, bx = t - by * ntx;
+  fused_tile<TT>(f, fs, d, p, k, td, d.xs + 1 + bx * TT::TX, d.ys + 1 + (row0 + by) * TT::TY,
                  smem);
 }
 
+int tiles_over(int n, int t) { return n > 0 ? (n + t - 1) / t : 0; }
+int interior_x(const Dims& d) { return d.xe - d.xs - 1; }
+int interior_y(const Dims& d) { return d.ye - d.ys - 1; }
+
 // Domains too small for four 32 x 16 tiles per SM take 16 x 16 tiles.
 bool small_tiles(const Dims& d) {
-  const int nx = d.xe - d.xs + 3, ny = d.ye - d.ys + 2;
-  return (long long)((nx + T::TX - 1) / T::TX) * ((ny + T::TY - 1) / T::TY) < 4LL * 152;
+  return (long long)tiles_over(interior_x(d), T::TX) * tiles_over(interior_y(d), T::TY) <
+         4LL * 152;
 }
+int tile_height(const Dims& d) { return small_tiles(d) ? SmallTile::TY : T::TY; }
 
 template <class TT>
 void launch_rows(const Fields& f, const FusedState& fs, const Dims& d, const Scalars& s,
                  const UniformMetrics& um, double tide, const double* tide_table, int tide_index,
                  int row0, int row1, cudaStream_t st) {
-  const int nx = d.xe - d.xs + 3;
   if (row1 <= row0) return;
-  const dim3 grid((nx + TT::TX - 1) / TT::TX, row1 - row0);
-  k_fused_step<TT><<<grid, dim3(TT::TX, TT::RPP), TT::kSmemBytes, st>>>(
-      f, fs, d, s, um, make_fast_const(s, um), tide_table, tide_index, tide, row0);
+  const int ja = fused_step_first_row(d, row0), jb = fused_step_first_row(d, row1);
+  const int ntx = tiles_over(interior_x(d), TT::TX);
+  const int nty = interior_y(d) > 0 ? row1 - row0 : 0;
+  // One warp of the ring's parts per block until that would be more than a
+  // block per SM: each is ~100 dependent FP64 operations.
+  const int nr = kParts * ring_count(d, ja, jb);
+  int rc = 32;
+  while (rc < NTHREADS && nr > rc * 152) rc *= 2;
+  const int nring = (nr + rc - 1) / rc;
+  k_fused_step<TT><<<nring + ntx * nty, dim3(TT::TX, TT::RPP), TT::kSmemBytes, st>>>(
+      f, fs, d, s, make_fast_const(s, um), tide_table, tide_index, tide, row0, ntx, ja, jb,
+      nring, rc);
 }
 
 void set_step_attrs() {
@@ -80,10 +110,15 @@ void set_step_attrs() {
 
 }  // namespace
 
-int fused_step_tile_rows(const Dims& d, int* tile_height) {
-  const int ty = small_tiles(d) ? SmallTile::TY : T::TY;
-  if (tile_height) *tile_height = ty;
-  return (d.ye - d.ys + 2 + ty - 1) / ty;
+int fused_step_tile_rows(const Dims& d) {
+  const int n = interior_x(d) > 0 ? tiles_over(interior_y(d), tile_height(d)) : 0;
+  return n > 0 ? n : 1;  // without an interior: the ring alone
+}
+
+int fused_step_first_row(const Dims& d, int row) {
+  if (row <= 0) return d.ys - 1;
+  if (row >= fused_step_tile_rows(d)) return d.ye + 1;
+  return d.ys + 1 + row * tile_height(d);
 }
 
 void launch_fused_step_rows(const Fields& f, const FusedState& fs, const Dims& d,
@@ -100,7 +135,7 @@ void launch_fused_step(const Fields& f, const FusedState& fs, const Dims& d,
                        const Scalars& s, const UniformMetrics& um, double tide,
                        const double* tide_table, int tide_index, cudaStream_t st) {
   set_step_attrs();
-  const int rows = fused_step_tile_rows(d, nullptr);
+  const int rows = fused_step_tile_rows(d);
   if (small_tiles(d))
     launch_rows<SmallTile>(f, fs, d, s, um, tide, tide_table, tide_index, 0, rows, st);
   else
@@ -109,14 +144,15 @@ void launch_fused_step(const Fields& f, const FusedState& fs, const Dims& d,
 
 namespace {
 
-// Reciprocals RN(1 / (h + ssha)) of the momentum denominators, or 0 where
-// the depth lies outside [2^-100, 2^100] (the kernel then divides).
+// The momentum denominators h + ssha and their reciprocals, 0 where the
+// depth lies outside [2^-100, 2^100] (the kernel then divides).
 __global__ void k_depth_reciprocal(const double* __restrict__ h,
-                                   const double* __restrict__ ssha, double* __restrict__ r,
-                                   long long n) {
+                                   const double* __restrict__ ssha, double* __restrict__ dh,
+                                   double* __restrict__ r, long long n) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     const double dd = h[t] + ssha[t];
+    dh[t] = dd;
     r[t] = (dd >= 0x1p-100 && dd <= 0x1p100) ? 1.0 / dd : 0.0;
   }
 }
@@ -129,8 +165,8 @@ void launch_depth_reciprocals(const Fields& f, const Dims& d, cudaStream_t st, i
   const size_t o = (size_t)row0 * d.width;
   const long long n = (long long)(row1 - row0) * d.width;
   if (n <= 0) return;
-  k_depth_reciprocal<<<152 * 8, 256, 0, st>>>(f.hu + o, f.ssha_u + o, f.r_hu + o, n);
-  k_depth_reciprocal<<<152 * 8, 256, 0, st>>>(f.hv + o, f.ssha_v + o, f.r_hv + o, n);
+  k_depth_reciprocal<<<152 * 8, 256, 0, st>>>(f.hu + o, f.ssha_u + o, f.d_hu + o, f.r_hu + o, n);
+  k_depth_reciprocal<<<152 * 8, 256, 0, st>>>(f.hv + o, f.ssha_v + o, f.d_hv + o, f.r_hv + o, n);
 }
 
 }  // namespace nl2d

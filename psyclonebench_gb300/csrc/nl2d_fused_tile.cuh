@@ -10,12 +10,16 @@ namespace nl2d {
 namespace {
 
 
-// A tile is TX x TY cells, worked on by 256 threads laid out TX x
-// (256 / TX); in the last phase each thread updates TY / (256 / TX) cells
-// of one column.  Tile<TX, TY> holds a shape's constants; the ensemble
-// instantiates several shapes (its autotuner picks one), the single-domain
-// kernel uses DefaultTile.  The arithmetic does not depend on the shape.
-constexpr int HALO = 2, NTHREADS = 256;
+// The copy region splits into interior cells, [xs+1, xe-1] x [ys+1, ye-1],
+// and the ring around them (ring_pos).  A tile is TX x TY interior cells,
+// worked on by 256 threads laid out TX x (256 / TX); each thread updates TY /
+// (256 / TX) cells of one column.  Tile<TX, TY> holds a shape's constants;
+// the ensemble instantiates several shapes (its autotuner picks one), the
+// single-domain kernel picks by domain size.  Ring cells need the general
+// per-cell code, a long FP64 chain, and are taken one per thread by blocks of
+// their own that run beside the tiles.  The arithmetic does not depend on
+// the split.
+constexpr int NTHREADS = 256;
 
 // Step-invariant constants of the fast path, evaluated on the host with the
 // operations the reference performs per point (e.g. dx_v[c] + dx_v[e] on a
@@ -43,81 +47,17 @@ struct EnsDomain {
 // Division by a step constant: the Markstein form when the constants allow
 // it, otherwise the IEEE divide.  Both give the same bits.
 __device__ __forceinline__ double dvc(double x, double d, double r, int fast) {
-  return fast ? div_rn(x, d, r) : x / d;
+  return fast ? div_rn(x, d, r) : div_ieee(x, d);
 }
 // Division by a per-face depth with a precomputed reciprocal; r == 0 marks
 // a depth outside [2^-100, 2^100] (IEEE divide).
 __device__ __forceinline__ double dvf(double x, double d, double r) {
-  return bits(r) != 0 ? div_rn(x, d, r) : x / d;
+  return bits(r) != 0 ? div_rn(x, d, r) : div_ieee(x, d);
 }
 
-template <int SX>
-struct Ctx {
-  const double *__restrict__ sn, *__restrict__ un, *__restrict__ vn;
-  const double *__restrict__ hu, *__restrict__ hv, *__restrict__ ht;
-  const double *__restrict__ ssha_u, *__restrict__ ssha_v;
-  const double *__restrict__ r_hu, *__restrict__ r_hv;
-  const int* __restrict__ m;
-  const double* su_tile;  // shared: sshn_u seen by this step
-  const double* sv_tile;  // shared: sshn_v seen by this step
-  int W, i0, j0;          // tile origin (cell coordinates of su_tile[0] + HALO)
-  Dims d;
-  FastConst k;
-
-  // Shared-memory slot of cell (i,j); the caller keeps (i,j) within the
-  // tile plus its halo.
-  __device__ __forceinline__ int slot(int i, int j) const {
-    return (j - j0 + HALO) * SX + (i - i0 + HALO);
-  }
-  __device__ __forceinline__ bool in_copy(int i, int j) const {
-    return i >= d.xs - 1 && i <= d.xe + 1 && j >= d.ys - 1 && j <= d.ye;
-  }
-  // sshn_u / sshn_v this step sees at face (i,j)
-  __device__ __forceinline__ double su(int i, int j) const { return su_tile[slot(i, j)]; }
-  __device__ __forceinline__ double sv(int i, int j) const { return sv_tile[slot(i, j)]; }
-};
-
-// next_sshu_code / next_sshv_code (time_update_kern.c:90-155) at face
-// (i,j) over their loop ranges; faces outside them keep the stored value.
-// The tile stages these in shared memory (phase 0 of fused_tile); the
-// general pass without a tile computes them where it reads them.
-__device__ __forceinline__ bool next_sshu_at(const int* __restrict__ m,
-                                             const double* __restrict__ sn, const Dims& d,
-                                             const FastConst& k, int i, int j, double& su) {
-  if (!(j >= d.ys && j <= d.ye && i >= d.xs && i <= d.xe - 1)) return false;
-  const int c = j * d.width + i, n = c + 1, mm = m[c], mn = m[n];
-  if (mm + mn <= 0) return false;
-  if (mm * mn > 0) {
-    double rtmp1 = k.area_t * sn[c] + k.area_t * sn[n];
-    su = dvc(half(rtmp1), k.area_u, k.r_area_u, k.fast_div);
-  } else if (mm <= 0) {
-    su = sn[n];
-  } else {
-    su = sn[c];
-  }
-  return true;
-}
-__device__ __forceinline__ bool next_sshv_at(const int* __restrict__ m,
-                                             const double* __restrict__ sn, const Dims& d,
-                                             const FastConst& k, int i, int j, double& sv) {
-  if (!(j >= d.ys && j <= d.ye - 1 && i >= d.xs && i <= d.xe)) return false;
-  const int c = j * d.width + i, n = c + d.width, mm = m[c], mn = m[n];
-  if (mm + mn <= 0) return false;
-  if (mm * mn > 0) {
-    double rtmp1 = k.area_t * sn[c] + k.area_t * sn[n];
-    sv = dvc(half(rtmp1), k.area_v, k.r_area_v, k.fast_div);
-  } else if (mm <= 0) {
-    sv = sn[n];
-  } else {
-    sv = sn[c];
-  }
-  return true;
-}
-
-// The general pass's context without a tile: every input read from the
-// domain's arrays in global memory (the members refer to the domain's
-// descriptor, so no thread holds a copy of it), sshn_u / sshn_v computed
-// where they are read.  Valid for the faces a copy-region cell's general
+// The general code's context: every input read from the domain's arrays in
+// global memory (the members refer to the domain's descriptor, so no thread
+// holds a copy of it).  Valid for the faces a copy-region cell's general
 // update reads, all of which lie inside the array.
 struct GlobalCtx {
   const double* const& sn;  // the state buffers read this step
@@ -140,13 +80,34 @@ struct GlobalCtx {
   __device__ __forceinline__ bool in_copy(int i, int j) const {
     return i >= d.xs - 1 && i <= d.xe + 1 && j >= d.ys - 1 && j <= d.ye;
   }
+  // next_sshu_code / next_sshv_code (time_update_kern.c:90-155) at face (i,j)
+  // from the mask and sshn_t of its two cells and (pa, pb) area_t * sshn_t of
+  // them, over the kernels' loop ranges; faces outside them keep the stored
+  // value.  Everything a caller needs is loaded before any of it is used, and
+  // nothing is loaded behind a mask test: the general code is a chain of
+  // dependent loads and FP64 operations, and its length is what it costs.
+  __device__ __forceinline__ double face_u(int i, int j, int mm, int mn, double a, double b,
+                                           double pa, double pb, double stored) const {
+    const double both = dvc(half(pa + pb), k.area_u, k.r_area_u, k.fast_div);
+    const bool in = j >= d.ys && j <= d.ye && i >= d.xs && i <= d.xe - 1 && mm + mn > 0;
+    return !in ? stored : (mm * mn > 0 ? both : (mm <= 0 ? b : a));
+  }
+  __device__ __forceinline__ double face_v(int i, int j, int mm, int mn, double a, double b,
+                                           double pa, double pb, double stored) const {
+    const double both = dvc(half(pa + pb), k.area_v, k.r_area_v, k.fast_div);
+    const bool in = j >= d.ys && j <= d.ye - 1 && i >= d.xs && i <= d.xe && mm + mn > 0;
+    return !in ? stored : (mm * mn > 0 ? both : (mm <= 0 ? b : a));
+  }
+  // sshn_u / sshn_v this step sees at one face
   __device__ __forceinline__ double su(int i, int j) const {
-    double v;
-    return next_sshu_at(m, sn, d, k, i, j, v) ? v : sshn_u[j * W + i];
+    const int c = j * W + i, n = min(c + 1, W * d.height - 1);
+    const double a = sn[c], b = sn[n];
+    return face_u(i, j, m[c], m[n], a, b, k.area_t * a, k.area_t * b, sshn_u[c]);
   }
   __device__ __forceinline__ double sv(int i, int j) const {
-    double v;
-    return next_sshv_at(m, sn, d, k, i, j, v) ? v : sshn_v[j * W + i];
+    const int c = j * W + i, n = j + 1 < d.height ? c + W : c;
+    const double a = sn[c], b = sn[n];
+    return face_v(i, j, m[c], m[n], a, b, k.area_t * a, k.area_t * b, sshn_v[c]);
   }
 };
 
@@ -175,51 +136,68 @@ template <class X>
 __device__ __forceinline__ bool mom_u(const X& x, int i, int j, double& out) {
   const int W = x.W, c = j * W + i, e = c + 1, wst = c - 1, s = c - W, n = c + W,
             se = s + 1, ne = n + 1;
-  const int* m = x.m;
-  if (m[c] + m[e] <= 0) return false;
-  if (m[c] <= 0 || m[e] <= 0) return false;
-  const double *un = x.un, *vn = x.vn, *hu = x.hu, *hv = x.hv, *ht = x.ht, *sn = x.sn;
   const FastConst& k = x.k;
-  const double su_c = x.su(i, j), su_s = x.su(i, j - 1), su_n = x.su(i, j + 1);
-  const double sv_s = x.sv(i, j - 1), sv_se = x.sv(i + 1, j - 1), sv_c = x.sv(i, j),
-               sv_e = x.sv(i + 1, j);
+  // the masks, heights and stored face values of the six cells around
+  const int m_c = x.m[c], m_e = x.m[e], m_s = x.m[s], m_se = x.m[se], m_n = x.m[n],
+            m_ne = x.m[ne];
+  const double sn_c = x.sn[c], sn_e = x.sn[e], sn_s = x.sn[s], sn_se = x.sn[se],
+               sn_n = x.sn[n], sn_ne = x.sn[ne];
+  const double su0_c = x.sshn_u[c], su0_s = x.sshn_u[s], su0_n = x.sshn_u[n];
+  const double sv0_c = x.sshn_v[c], sv0_e = x.sshn_v[e], sv0_s = x.sshn_v[s],
+               sv0_se = x.sshn_v[se];
+  const double u_c = x.un[c], u_E = x.un[e], u_W = x.un[wst], u_S = x.un[s], u_N = x.un[n];
+  const double v_C = x.vn[c], v_E = x.vn[e], v_S = x.vn[s], v_SE = x.vn[se];
+  const double hu_c = x.hu[c], hu_s = x.hu[s], hu_n = x.hu[n];
+  const double hv_c = x.hv[c], hv_e = x.hv[e], hv_s = x.hv[s], hv_se = x.hv[se];
+  const double ht_c = x.ht[c], ht_e = x.ht[e], ssha = x.ssha_u[c], rhu = x.r_hu[c];
+  if (m_c + m_e <= 0) return false;
+  if (m_c <= 0 || m_e <= 0) return false;
+  const double p_c = k.area_t * sn_c, p_e = k.area_t * sn_e, p_s = k.area_t * sn_s,
+               p_se = k.area_t * sn_se, p_n = k.area_t * sn_n, p_ne = k.area_t * sn_ne;
+  const double su_c = x.face_u(i, j, m_c, m_e, sn_c, sn_e, p_c, p_e, su0_c),
+               su_s = x.face_u(i, j - 1, m_s, m_se, sn_s, sn_se, p_s, p_se, su0_s),
+               su_n = x.face_u(i, j + 1, m_n, m_ne, sn_n, sn_ne, p_n, p_ne, su0_n);
+  const double sv_s = x.face_v(i, j - 1, m_s, m_c, sn_s, sn_c, p_s, p_c, sv0_s),
+               sv_se = x.face_v(i + 1, j - 1, m_se, m_e, sn_se, sn_e, p_se, p_e, sv0_se),
+               sv_c = x.face_v(i, j, m_c, m_n, sn_c, sn_n, p_c, p_n, sv0_c),
+               sv_e = x.face_v(i + 1, j, m_e, m_ne, sn_e, sn_ne, p_e, p_ne, sv0_e);
 
-  double u_e = half(un[c] + un[e]) * k.dy_t;
-  double depe = ht[e] + sn[e];
-  double u_w = half(un[c] + un[wst]) * k.dy_t;
-  double depw = ht[c] + sn[c];
-  double v_sc = half(vn[s] + vn[se]);
+  double u_e = half(u_c + u_E) * k.dy_t;
+  double depe = ht_e + sn_e;
+  double u_w = half(u_c + u_W) * k.dy_t;
+  double depw = ht_c + sn_c;
+  double v_sc = half(v_S + v_SE);
   double v_s = half(v_sc) * k.dxv2;
-  double deps = half(hv[s] + sv_s + hv[se] + sv_se);
-  double v_nc = half(vn[c] + vn[e]);
+  double deps = half(hv_s + sv_s + hv_se + sv_se);
+  double v_nc = half(v_C + v_E);
   double v_n = half(v_nc) * k.dxv2;
-  double depn = half(hv[c] + sv_c + hv[e] + sv_e);
+  double depn = half(hv_c + sv_c + hv_e + sv_e);
 
-  double uu_w = upwind(u_w, un[c], un[wst]);
-  double uu_e = upwind(u_e, un[e], un[c]);
-  const bool south_dry = m[s] <= 0 || m[se] <= 0;
-  const bool north_dry = m[n] <= 0 || m[ne] <= 0;
-  double uu_s = south_dry ? lo_only(v_s, un[c]) : upwind(v_s, un[c], un[s]);
-  double uu_n = north_dry ? hi_only(v_n, un[c]) : upwind(v_n, un[n], un[c]);
+  double uu_w = upwind(u_w, u_c, u_W);
+  double uu_e = upwind(u_e, u_E, u_c);
+  const bool south_dry = m_s <= 0 || m_se <= 0;
+  const bool north_dry = m_n <= 0 || m_ne <= 0;
+  double uu_s = south_dry ? lo_only(v_s, u_c) : upwind(v_s, u_c, u_S);
+  double uu_n = north_dry ? hi_only(v_n, u_c) : upwind(v_n, u_N, u_c);
   double adv = uu_w * u_w * depw - uu_e * u_e * depe + uu_s * v_s * deps -
                uu_n * v_n * depn;
 
-  double dudx_e = dvc(un[e] - un[c], k.dx_t, k.r_dx_t, k.fast_div) * (ht[e] + sn[e]);
-  double dudx_w = dvc(un[c] - un[wst], k.dx_t, k.r_dx_t, k.fast_div) * (ht[c] + sn[c]);
+  double dudx_e = dvc(u_E - u_c, k.dx_t, k.r_dx_t, k.fast_div) * depe;
+  double dudx_w = dvc(u_c - u_W, k.dx_t, k.r_dx_t, k.fast_div) * depw;
   double dudy_s = south_dry ? 0.0
-                            : dvc(un[c] - un[s], k.dyu2, k.r_dyu2, k.fast_div) *
-                                  (hu[c] + su_c + hu[s] + su_s);
+                            : dvc(u_c - u_S, k.dyu2, k.r_dyu2, k.fast_div) *
+                                  (hu_c + su_c + hu_s + su_s);
   double dudy_n = north_dry ? 0.0
-                            : dvc(un[n] - un[c], k.dyu2, k.r_dyu2, k.fast_div) *
-                                  (hu[c] + su_c + hu[n] + su_n);
+                            : dvc(u_N - u_c, k.dyu2, k.r_dyu2, k.fast_div) *
+                                  (hu_c + su_c + hu_n + su_n);
   double vis = (dudx_e - dudx_w) * k.dy_u + half((dudy_n - dudy_s) * k.dx_u);
   vis = k.visc * vis;
-  double cor = half(k.cor_u * (v_sc + v_nc)) * k.area_u * (hu[c] + su_c);
-  double hpg = k.neg_g * (hu[c] + su_c) * k.dy_u * (sn[e] - sn[c]);
+  double cor = half(k.cor_u * (v_sc + v_nc)) * k.area_u * (hu_c + su_c);
+  double hpg = k.neg_g * (hu_c + su_c) * k.dy_u * (sn_e - sn_c);
   const double num =
-      un[c] * (hu[c] + su_c) + dvc(k.rdt * (adv + vis + cor + hpg), k.area_u, k.r_area_u,
-                                   k.fast_div);
-  out = dvc(dvf(num, hu[c] + x.ssha_u[c], x.r_hu[c]), k.fric, k.r_fric, k.fast_div);
+      u_c * (hu_c + su_c) + dvc(k.rdt * (adv + vis + cor + hpg), k.area_u, k.r_area_u,
+                                k.fast_div);
+  out = dvc(dvf(num, hu_c + ssha, rhu), k.fric, k.r_fric, k.fast_div);
   return true;
 }
 
@@ -228,51 +206,67 @@ template <class X>
 __device__ __forceinline__ bool mom_v(const X& x, int i, int j, double& out) {
   const int W = x.W, c = j * W + i, e = c + 1, wst = c - 1, s = c - W, n = c + W,
             nw = n - 1, ne = n + 1;
-  const int* m = x.m;
-  if (m[c] + m[e] <= 0) return false;
-  if (m[c] <= 0 || m[n] <= 0) return false;
-  const double *un = x.un, *vn = x.vn, *hu = x.hu, *hv = x.hv, *ht = x.ht, *sn = x.sn;
   const FastConst& k = x.k;
-  const double su_w = x.su(i - 1, j), su_nw = x.su(i - 1, j + 1), su_c = x.su(i, j),
-               su_n = x.su(i, j + 1);
-  const double sv_c = x.sv(i, j), sv_w = x.sv(i - 1, j), sv_e = x.sv(i + 1, j);
+  const int m_c = x.m[c], m_e = x.m[e], m_w = x.m[wst], m_n = x.m[n], m_nw = x.m[nw],
+            m_ne = x.m[ne];
+  const double sn_c = x.sn[c], sn_e = x.sn[e], sn_w = x.sn[wst], sn_n = x.sn[n],
+               sn_nw = x.sn[nw], sn_ne = x.sn[ne];
+  const double su0_c = x.sshn_u[c], su0_w = x.sshn_u[wst], su0_n = x.sshn_u[n],
+               su0_nw = x.sshn_u[nw];
+  const double sv0_c = x.sshn_v[c], sv0_w = x.sshn_v[wst], sv0_e = x.sshn_v[e];
+  const double v_c = x.vn[c], v_E = x.vn[e], v_W = x.vn[wst], v_S = x.vn[s], v_N = x.vn[n];
+  const double u_C = x.un[c], u_N = x.un[n], u_W = x.un[wst], u_NW = x.un[nw];
+  const double hv_c = x.hv[c], hv_w = x.hv[wst], hv_e = x.hv[e];
+  const double hu_c = x.hu[c], hu_n = x.hu[n], hu_w = x.hu[wst], hu_nw = x.hu[nw];
+  const double ht_c = x.ht[c], ht_n = x.ht[n], ssha = x.ssha_v[c], rhv = x.r_hv[c];
+  if (m_c + m_e <= 0) return false;
+  if (m_c <= 0 || m_n <= 0) return false;
+  const double p_c = k.area_t * sn_c, p_e = k.area_t * sn_e, p_w = k.area_t * sn_w,
+               p_n = k.area_t * sn_n, p_nw = k.area_t * sn_nw, p_ne = k.area_t * sn_ne;
+  const double su_w = x.face_u(i - 1, j, m_w, m_c, sn_w, sn_c, p_w, p_c, su0_w),
+               su_nw = x.face_u(i - 1, j + 1, m_nw, m_n, sn_nw, sn_n, p_nw, p_n, su0_nw),
+               su_c = x.face_u(i, j, m_c, m_e, sn_c, sn_e, p_c, p_e, su0_c),
+               su_n = x.face_u(i, j + 1, m_n, m_ne, sn_n, sn_ne, p_n, p_ne, su0_n);
+  const double sv_c = x.face_v(i, j, m_c, m_n, sn_c, sn_n, p_c, p_n, sv0_c),
+               sv_w = x.face_v(i - 1, j, m_w, m_nw, sn_w, sn_nw, p_w, p_nw, sv0_w),
+               sv_e = x.face_v(i + 1, j, m_e, m_ne, sn_e, sn_ne, p_e, p_ne, sv0_e);
 
-  double v_n = half(vn[c] + vn[n]) * k.dx_t;
-  double depn = ht[n] + sn[n];
-  double v_s = half(vn[c] + vn[s]) * k.dx_t;
-  double deps = ht[c] + sn[c];
-  double u_wc = half(un[wst] + un[nw]);
+  double v_n = half(v_c + v_N) * k.dx_t;
+  double depn = ht_n + sn_n;
+  double v_s = half(v_c + v_S) * k.dx_t;
+  double deps = ht_c + sn_c;
+  double u_wc = half(u_W + u_NW);
   double u_w = half(u_wc) * k.dyu2;
-  double depw = half(hu[wst] + su_w + hu[nw] + su_nw);
-  double u_ec = half(un[c] + un[n]);
+  double depw = half(hu_w + su_w + hu_nw + su_nw);
+  double u_ec = half(u_C + u_N);
   double u_e = half(u_ec) * k.dyu2;
-  double depe = half(hu[c] + su_c + hu[n] + su_n);
+  double depe = half(hu_c + su_c + hu_n + su_n);
 
-  double vv_s = upwind(v_s, vn[c], vn[s]);
-  double vv_n = upwind(v_n, vn[n], vn[c]);
-  const bool west_dry = m[wst] <= 0 || m[nw] <= 0;
-  const bool east_dry = m[e] <= 0 || m[ne] <= 0;
-  double vv_w = west_dry ? lo_only(u_w, vn[c]) : upwind(u_w, vn[c], vn[wst]);
-  double vv_e = east_dry ? hi_only(u_e, vn[c]) : upwind(u_e, vn[e], vn[c]);
+  double vv_s = upwind(v_s, v_c, v_S);
+  double vv_n = upwind(v_n, v_N, v_c);
+  const bool west_dry = m_w <= 0 || m_nw <= 0;
+  const bool east_dry = m_e <= 0 || m_ne <= 0;
+  double vv_w = west_dry ? lo_only(u_w, v_c) : upwind(u_w, v_c, v_W);
+  double vv_e = east_dry ? hi_only(u_e, v_c) : upwind(u_e, v_E, v_c);
   double adv = vv_w * u_w * depw - vv_e * u_e * depe + vv_s * v_s * deps -
                vv_n * v_n * depn;
 
-  double dvdy_n = dvc(vn[n] - vn[c], k.dy_t, k.r_dy_t, k.fast_div) * (ht[n] + sn[n]);
-  double dvdy_s = dvc(vn[c] - vn[s], k.dy_t, k.r_dy_t, k.fast_div) * (ht[c] + sn[c]);
+  double dvdy_n = dvc(v_N - v_c, k.dy_t, k.r_dy_t, k.fast_div) * depn;
+  double dvdy_s = dvc(v_c - v_S, k.dy_t, k.r_dy_t, k.fast_div) * deps;
   double dvdx_w = west_dry ? 0.0
-                           : dvc(vn[c] - vn[wst], k.dxv2, k.r_dxv2, k.fast_div) *
-                                 (hv[c] + sv_c + hv[wst] + sv_w);
+                           : dvc(v_c - v_W, k.dxv2, k.r_dxv2, k.fast_div) *
+                                 (hv_c + sv_c + hv_w + sv_w);
   double dvdx_e = east_dry ? 0.0
-                           : dvc(vn[e] - vn[c], k.dxv2, k.r_dxv2, k.fast_div) *
-                                 (hv[c] + sv_c + hv[e] + sv_e);
+                           : dvc(v_E - v_c, k.dxv2, k.r_dxv2, k.fast_div) *
+                                 (hv_c + sv_c + hv_e + sv_e);
   double vis = (dvdy_n - dvdy_s) * k.dx_v + half((dvdx_e - dvdx_w) * k.dy_v);
   vis = k.visc * vis;
-  double cor = -half(k.cor_v * (u_ec + u_wc)) * k.area_v * (hv[c] + sv_c);
-  double hpg = k.neg_g * (hv[c] + sv_c) * k.dx_v * (sn[n] - sn[c]);
+  double cor = -half(k.cor_v * (u_ec + u_wc)) * k.area_v * (hv_c + sv_c);
+  double hpg = k.neg_g * (hv_c + sv_c) * k.dx_v * (sn_n - sn_c);
   const double num =
-      vn[c] * (hv[c] + sv_c) + dvc(k.rdt * (adv + vis + cor + hpg), k.area_v, k.r_area_v,
-                                   k.fast_div);
-  out = dvc(dvf(num, hv[c] + x.ssha_v[c], x.r_hv[c]), k.fric, k.r_fric, k.fast_div);
+      v_c * (hv_c + sv_c) + dvc(k.rdt * (adv + vis + cor + hpg), k.area_v, k.r_area_v,
+                                k.fast_div);
+  out = dvc(dvf(num, hv_c + ssha, rhv), k.fric, k.r_fric, k.fast_div);
   return true;
 }
 
@@ -309,70 +303,124 @@ __device__ __forceinline__ double va_pre_flather(const X& x, const double* va_ar
   return va;
 }
 
-// A copy-region cell's update by the reference's per-point code, in its
-// order: sea-surface height (continuity_kern.c:90-117, then bc_ssh), u at
-// the east face (momentum_u, bc_solid_u, bc_flather_u), v at the north face
-// (momentum_v, bc_solid_v, bc_flather_v).  x supplies the fields and the
-// sshn_u / sshn_v this step sees (a tile's shared memory, or global memory).
+// A copy-region cell's update by the reference's per-point code, in three
+// independent parts (each reads the old state only), so that three threads
+// share what would be one long chain: v at the north face (momentum_v,
+// bc_solid_v, bc_flather_v), u at the east face (momentum_u, bc_solid_u,
+// bc_flather_u), sea-surface height (continuity_kern.c:90-117, then bc_ssh).
+// A Flather face takes the momentum of the face next to it instead of its
+// own (bc_flather replaces it), so each part evaluates one momentum update.
+enum { kPartV, kPartU, kPartSsh, kParts };
 template <class X>
-__device__ __forceinline__ void general_cell(const X& x, const Fields& f, const FusedState& fs,
-                                             const Scalars& p, double tide, int i, int j) {
+__device__ __forceinline__ void general_part(const X& x, const Fields& f, const FusedState& fs,
+                                             const Scalars& p, double tide, int part, int i,
+                                             int j) {
   const int W = x.W;
   const Dims& d = x.d;
   const FastConst& k = x.k;
   const int* __restrict__ m = x.m;
-  const double* __restrict__ sn = x.sn;
-  const double* __restrict__ un = x.un;
-  const double* __restrict__ vn = x.vn;
   const int c = j * W + i;
 
-  double ssh = sn[c];
-  if (i >= d.xs && i <= d.xe && j >= d.ys && j <= d.ye) {
-    const int w = c - 1, s = c - W;
-    double r1 = (x.su(i, j) + f.hu[c]) * un[c];
-    double r2 = (x.su(i - 1, j) + f.hu[w]) * un[w];
-    double r3 = (x.sv(i, j) + f.hv[c]) * vn[c];
-    double r4 = (x.sv(i, j - 1) + f.hv[s]) * vn[s];
-    ssh = sn[c] + dvc((r2 - r1 + r4 - r3) * k.rdt, k.area_t, k.r_area_t, k.fast_div);
-    if (m[c] > 0 && (m[c - W] < 0 || m[c + W] < 0 || m[c + 1] < 0 || m[c - 1] < 0))
-      ssh = tide;
-  }
-  fs.sshn_out[c] = ssh;
-
-  double ua = un[c];
-  if (i <= d.xe) {  // u whole range [xs-1, xe] x [ys-1, ye+1] (tiling gives the rest)
-    ua = ua_pre_flather(x, f.ua, i, j);
-    if (m[c] + m[c + 1] > -1) {
-      if (m[c] < 0) {
-        ua = ua_pre_flather(x, f.ua, i + 1, j) +
-             sqrt(p.g / f.hu[c]) * (x.su(i, j) - x.su(i + 1, j));
-      } else if (m[c + 1] < 0 && i >= 1) {  // i == 0 would read outside the array
-        ua = ua_pre_flather(x, f.ua, i - 1, j) +
-             sqrt(p.g / f.hu[c]) * (x.su(i, j) - x.su(i - 1, j));
+  if (part == kPartSsh) {
+    double ssh = x.sn[c];
+    if (i >= d.xs && i <= d.xe && j >= d.ys && j <= d.ye) {
+      const int w = c - 1, s = c - W;
+      double r1 = (x.su(i, j) + f.hu[c]) * x.un[c];
+      double r2 = (x.su(i - 1, j) + f.hu[w]) * x.un[w];
+      double r3 = (x.sv(i, j) + f.hv[c]) * x.vn[c];
+      double r4 = (x.sv(i, j - 1) + f.hv[s]) * x.vn[s];
+      ssh = x.sn[c] + dvc((r2 - r1 + r4 - r3) * k.rdt, k.area_t, k.r_area_t, k.fast_div);
+      if (m[c] > 0 && (m[c - W] < 0 || m[c + W] < 0 || m[c + 1] < 0 || m[c - 1] < 0))
+        ssh = tide;
+    }
+    fs.sshn_out[c] = ssh;
+  } else if (part == kPartU) {
+    double ua;
+    if (i <= d.xe) {  // u whole range [xs-1, xe] x [ys-1, ye+1] (the copy region gives the rest)
+      const int mc = m[c], me = m[c + 1];
+      int fi = i;  // the face whose momentum this face takes
+      if (mc + me > -1) {
+        if (mc < 0)
+          fi = i + 1;
+        else if (me < 0 && i >= 1)  // i == 0 would read outside the array
+          fi = i - 1;
       }
+      ua = ua_pre_flather(x, f.ua, fi, j);
+      if (fi != i) ua = ua + sqrt(p.g / f.hu[c]) * (x.su(i, j) - x.su(fi, j));
+    } else {
+      ua = x.un[c];
     }
-  }
-  fs.un_out[c] = ua;
-
-  // the copy region is exactly the v whole range [xs-1, xe+1] x [ys-1, ye]
-  double va = va_pre_flather(x, f.va, i, j);
-  if (m[c] + m[c + W] > -1) {
-    if (m[c] < 0) {
-      va = va_pre_flather(x, f.va, i, j + 1) +
-           sqrt(p.g / f.hv[c]) * (x.sv(i, j) - x.sv(i, j + 1));
-    } else if (m[c + W] < 0 && j >= 1) {
-      va = va_pre_flather(x, f.va, i, j - 1) +
-           sqrt(p.g / f.hv[c]) * (x.sv(i, j) - x.sv(i, j - 1));
+    fs.un_out[c] = ua;
+  } else {
+    // the copy region is exactly the v whole range [xs-1, xe+1] x [ys-1, ye]
+    const int mc = m[c], mn = m[c + W];
+    int fj = j;
+    if (mc + mn > -1) {
+      if (mc < 0)
+        fj = j + 1;
+      else if (mn < 0 && j >= 1)
+        fj = j - 1;
     }
+    double va = va_pre_flather(x, f.va, i, fj);
+    if (fj != j) va = va + sqrt(p.g / f.hv[c]) * (x.sv(i, j) - x.sv(i, fj));
+    fs.vn_out[c] = va;
   }
-  fs.vn_out[c] = va;
 }
 
-// Shared-memory layout of one tile.  Phase 0 (halo 2) holds the loaded
-// fields and the sshn_u / sshn_v values this step sees; phase 1 (halo 1)
-// holds the terms that two neighbouring updates share.
+// general_part on the domain's arrays, out of line: the tiles' registers are
+// sized by the regular update, and the few land-side cells of a tile and the
+// ring's cells share one copy of the code.
+static __device__ __noinline__ void general_at(const Fields& f, const FusedState& fs,
+                                               const Dims& d, const Scalars& p,
+                                               const FastConst& k, double tide, int part, int i,
+                                               int j) {
+  const GlobalCtx x{fs.sshn_in, fs.un_in, fs.vn_in, f.hu,     f.hv,     f.ht,
+                    f.ssha_u,   f.ssha_v, f.r_hu,   f.r_hv,   f.tmask,  f.sshn_u,
+                    f.sshn_v,   d.width,  d,        k};
+  general_part(x, f, fs, p, tide, part, i, j);
+}
+
+// The ring: the copy region's cells outside the interior, rows ys-1, ys, ye
+// and columns xs-1, xs, xe, xe+1 (the whole copy region when it has no
+// interior).  ring_count: its cells in copy-region rows [ja, jb); ring_pos:
+// the g-th of them, the full rows first.
+struct RingRows {
+  int nfull, npart, part0;  // full rows; the others, from row part0
+};
+__host__ __device__ __forceinline__ RingRows ring_rows(const Dims& d, int ja, int jb) {
+  if (d.xe - d.xs < 2 || d.ye - d.ys < 2) return RingRows{jb - ja, 0, 0};
+  const int p0 = ja > d.ys + 1 ? ja : d.ys + 1, p1 = jb < d.ye ? jb : d.ye;
+  const int np = p1 > p0 ? p1 - p0 : 0;
+  return RingRows{jb - ja - np, np, p0};
+}
+__host__ __device__ __forceinline__ int ring_count(const Dims& d, int ja, int jb) {
+  const RingRows r = ring_rows(d, ja, jb);
+  return r.nfull * (d.xe - d.xs + 3) + r.npart * 4;
+}
+__host__ __device__ __forceinline__ void ring_pos(const Dims& d, int ja, int jb, int g, int& i,
+                                                  int& j) {
+  const RingRows r = ring_rows(d, ja, jb);
+  const int nx = d.xe - d.xs + 3;
+  if (g < r.nfull * nx) {
+    const int q = g / nx;
+    i = d.xs - 1 + (g - q * nx);
+    j = ja + q;  // rows below the partial ones, then those above
+    if (r.npart > 0 && j >= r.part0) j += r.npart;
+  } else {
+    const int h = g - r.nfull * nx, c = h & 3;
+    j = r.part0 + (h >> 2);
+    i = c < 2 ? d.xs - 1 + c : d.xe + c - 2;
+  }
+}
+
+// Shared-memory layout of one tile, all on the tile plus one cell on each
+// side: the loaded fields and the sshn_u / sshn_v this step sees, then the
+// terms that two neighbouring updates share.
 enum { A_SN, A_UN, A_VN, A_HU, A_HV, A_SU, A_SV, A_HUS, A_HVS, N_A0 };
 enum { B_FLXU, B_FLXV, B_GX, B_GY, B_FXU, B_FYV, B_VSC, B_FYU, B_QY, B_UWC, B_FXV, B_QX, N_B1 };
+// area_t * sshn_t, needed until the face values are formed, shares the slot
+// of a term that is formed after them
+constexpr int B_AREA_SSH = B_QX;
 
 template <int TX_, int TY_>
 struct Tile {
@@ -381,205 +429,261 @@ struct Tile {
   static constexpr int RPT = TY / RPP;       // cells per thread in the update phase
   static_assert(NTHREADS % TX == 0 && TY % RPP == 0 && (RPT == 1 || RPT == 2 || RPT == 4),
                 "tile shape");
-  static constexpr int SX = TX + 2 * HALO, SY = TY + 2 * HALO;
-  static constexpr int S0 = SX * SY;  // phase-0 positions (36 x 20 for 32 x 16)
-  static constexpr int P1X = TX + 2, P1Y = TY + 2;
-  static constexpr int S1 = P1X * P1Y;  // phase-1 positions (34 x 18 for 32 x 16)
+  static constexpr int SX = TX + 2, SY = TY + 2;
+  static constexpr int S0 = SX * SY;  // staged positions (34 x 18 for 32 x 16)
   // + the mask, and the list of the tile's general (non-regular) cells
   static constexpr size_t kSmemBytes =
-      sizeof(double) * (N_A0 * S0 + N_B1 * S1) + sizeof(int) * (S0 + TX * TY + 1);
-  // two CTAs of 256 threads per SM when their shared memory fits
-  static constexpr int kMinBlocks = 2 * kSmemBytes <= 227 * 1024 ? 2 : 1;
+      sizeof(double) * (N_A0 + N_B1) * S0 + sizeof(int) * (S0 + TX * TY + 1);
+  // two CTAs of 256 threads per SM when their shared memory (with the 1 KB
+  // the driver reserves per CTA) fits the SM's 228 KB
+  static constexpr int kMinBlocks = 2 * (kSmemBytes + 1024) <= 228 * 1024 ? 2 : 1;
+  // Items along the tile's edges are handled by whole warps: an edge's items
+  // start at a multiple of 32 of the thread index.
+  static constexpr int RX = (TX + 31) / 32 * 32, RY = (TY + 31) / 32 * 32,
+                       RY1 = (TY + 32) / 32 * 32;
 };
 using DefaultTile = Tile<32, 16>;
 
 // A regular cell's new (sshn_t, un, vn) from the tile's staged fields (a0)
-// and shared terms (b1) at its slots q (phase 0) and r (phase 1): continuity
-// (continuity_kern.c:90-117) and unmasked momentum
-// (momentum_u_kern.c:184-261, momentum_v_kern.c:159-239) in the
-// reference's operation order.  sau, rhu, sav, rhv: ssha_u, RN(1 / (hu +
-// ssha_u)), ssha_v, RN(1 / (hv + ssha_v)) at the cell.
+// and shared terms (b1) at its slot q: continuity (continuity_kern.c:90-117)
+// and unmasked momentum (momentum_u_kern.c:184-261,
+// momentum_v_kern.c:159-239) in the reference's operation order.  dhu, rhu,
+// dhv, rhv: hu + ssha_u and hv + ssha_v at the cell and their reciprocals.
 struct RegOut {
   double ssh, u, v;
 };
 template <class T>
-__device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b1, int q, int r,
-                                               double sau, double rhu, double sav, double rhv,
+__device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b1, int q,
+                                               double dhu, double rhu, double dhv, double rhv,
                                                const FastConst& k) {
-  constexpr int S0 = T::S0, S1 = T::S1, SX = T::SX, P1X = T::P1X;
+  constexpr int S0 = T::S0, SX = T::SX;
 #define A(qq, t) a0[(qq) * S0 + (t)]
-#define B(qq, t) b1[(qq) * S1 + (t)]
+#define B(qq, t) b1[(qq) * S0 + (t)]
   RegOut o;
   const double snc = A(A_SN, q), Hu = A(A_HUS, q), Hv = A(A_HVS, q);
-  const double ssh = (((B(B_FLXU, r - 1) - B(B_FLXU, r)) + B(B_FLXV, r - P1X)) - B(B_FLXV, r)) *
+  const double ssh = (((B(B_FLXU, q - 1) - B(B_FLXU, q)) + B(B_FLXV, q - SX)) - B(B_FLXV, q)) *
                      k.rdt;
   o.ssh = snc + dvc(ssh, k.area_t, k.r_area_t, k.fast_div);
   {
-    const double adv = ((B(B_FXU, r) - B(B_FXU, r + 1)) + B(B_FYU, r)) - B(B_FYU, r + P1X);
-    const double dudy_s = B(B_QY, r) * ((Hu + A(A_HU, q - SX)) + A(A_SU, q - SX));
-    const double dudy_n = B(B_QY, r + P1X) * ((Hu + A(A_HU, q + SX)) + A(A_SU, q + SX));
-    double vis = (B(B_GX, r + 1) - B(B_GX, r)) * k.dy_u + half((dudy_n - dudy_s) * k.dx_u);
+    const double adv = ((B(B_FXU, q) - B(B_FXU, q + 1)) + B(B_FYU, q)) - B(B_FYU, q + SX);
+    const double dudy_s = B(B_QY, q) * ((Hu + A(A_HU, q - SX)) + A(A_SU, q - SX));
+    const double dudy_n = B(B_QY, q + SX) * ((Hu + A(A_HU, q + SX)) + A(A_SU, q + SX));
+    double vis = (B(B_GX, q + 1) - B(B_GX, q)) * k.dy_u + half((dudy_n - dudy_s) * k.dx_u);
     vis = k.visc * vis;
-    const double cor = (half(k.cor_u * (B(B_VSC, r) + B(B_VSC, r + P1X))) * k.area_u) * Hu;
+    const double cor = (half(k.cor_u * (B(B_VSC, q) + B(B_VSC, q + SX))) * k.area_u) * Hu;
     const double hpg = ((k.neg_g * Hu) * k.dy_u) * (A(A_SN, q + 1) - snc);
     const double num =
         A(A_UN, q) * Hu +
         dvc(k.rdt * (((adv + vis) + cor) + hpg), k.area_u, k.r_area_u, k.fast_div);
-    const double t1 = dvf(num, A(A_HU, q) + sau, rhu);
+    const double t1 = dvf(num, dhu, rhu);
     o.u = dvc(t1, k.fric, k.r_fric, k.fast_div);
   }
   {
-    const double adv = ((B(B_FXV, r) - B(B_FXV, r + 1)) + B(B_FYV, r)) - B(B_FYV, r + P1X);
-    const double dvdx_w = B(B_QX, r) * ((Hv + A(A_HV, q - 1)) + A(A_SV, q - 1));
-    const double dvdx_e = B(B_QX, r + 1) * ((Hv + A(A_HV, q + 1)) + A(A_SV, q + 1));
-    double vis = (B(B_GY, r + P1X) - B(B_GY, r)) * k.dx_v + half((dvdx_e - dvdx_w) * k.dy_v);
+    const double adv = ((B(B_FXV, q) - B(B_FXV, q + 1)) + B(B_FYV, q)) - B(B_FYV, q + SX);
+    const double dvdx_w = B(B_QX, q) * ((Hv + A(A_HV, q - 1)) + A(A_SV, q - 1));
+    const double dvdx_e = B(B_QX, q + 1) * ((Hv + A(A_HV, q + 1)) + A(A_SV, q + 1));
+    double vis = (B(B_GY, q + SX) - B(B_GY, q)) * k.dx_v + half((dvdx_e - dvdx_w) * k.dy_v);
     vis = k.visc * vis;
-    const double cor = (-half(k.cor_v * (B(B_UWC, r + 1) + B(B_UWC, r))) * k.area_v) * Hv;
+    const double cor = (-half(k.cor_v * (B(B_UWC, q + 1) + B(B_UWC, q))) * k.area_v) * Hv;
     const double hpg = ((k.neg_g * Hv) * k.dx_v) * (A(A_SN, q + SX) - snc);
     const double num =
         A(A_VN, q) * Hv +
         dvc(k.rdt * (((adv + vis) + cor) + hpg), k.area_v, k.r_area_v, k.fast_div);
-    const double t1 = dvf(num, A(A_HV, q) + sav, rhv);
+    const double t1 = dvf(num, dhv, rhv);
     o.v = dvc(t1, k.fric, k.r_fric, k.fast_div);
   }
-#undef A
-#undef B
   return o;
 }
 
-// One tile of the fused step: cells [i0, i0+TX) x [j0, j0+TY) of the copy
-// region of one domain.  `tide` is this step's bc_ssh value.
-template <class T>
-__device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs, const Dims& d,
-                                           const Scalars& p, const UniformMetrics& um,
-                                           const FastConst& k, double tide, int i0, int j0,
-                                           double* smem) {
-  constexpr int TX = T::TX, SX = T::SX, S0 = T::S0, S1 = T::S1, P1X = T::P1X;
-  constexpr int ROWS_PER_PASS = T::RPP;
-  double* a0 = smem;                 // [N_A0][S0]
-  double* b1 = smem + N_A0 * S0;     // [N_B1][S1]
-  int* mk = (int*)(b1 + N_B1 * S1);  // [S0]
-  int* glist = mk + S0;              // [TX * TY] general cells of this tile
-  int* gcount = glist + TX * T::TY;
-#define A(q, t) a0[(q) * S0 + (t)]
-#define B(q, t) b1[(q) * S1 + (t)]
-
-  const int W = d.width, H = d.height;
-  const int* __restrict__ m = f.tmask;
-  const double* __restrict__ sn = fs.sshn_in;
-  const double* __restrict__ un = fs.un_in;
-  const double* __restrict__ vn = fs.vn_in;
-  const int tid = threadIdx.y * TX + threadIdx.x;
-
-  if (tid == 0) *gcount = 0;
-  // ---- phase 0: fields and the sshn_u / sshn_v this step reads ----
-  for (int t = tid; t < S0; t += NTHREADS) {
-    const int i = i0 - HALO + t % SX, j = j0 - HALO + t / SX;
-    double vsn = 0.0, vun = 0.0, vvn = 0.0, vhu = 0.0, vhv = 0.0, su = 0.0, sv = 0.0;
-    int mm = 0;
-    if (i >= 0 && i < W && j >= 0 && j < H) {
-      const int c = j * W + i;
-      vsn = sn[c];
-      vun = un[c];
-      vvn = vn[c];
-      vhu = f.hu[c];
-      vhv = f.hv[c];
-      mm = m[c];
-      // next_sshu_code / next_sshv_code (time_update_kern.c:90-155) over
-      // their loop ranges; other faces keep the stored value, which is read
-      // only for them.
-      bool su_stored = true, sv_stored = true;
-      if (j >= d.ys && j <= d.ye && i >= d.xs && i <= d.xe - 1) {
-        const int n = c + 1, mn = m[n];
-        if (mm + mn > 0) {
-          su_stored = false;
-          if (mm * mn > 0) {
-            double rtmp1 = k.area_t * vsn + k.area_t * sn[n];
-            su = dvc(half(rtmp1), k.area_u, k.r_area_u, k.fast_div);
-          } else if (mm <= 0) {
-            su = sn[n];
-          } else {
-            su = vsn;
-          }
-        }
-      }
-      if (j >= d.ys && j <= d.ye - 1 && i >= d.xs && i <= d.xe) {
-        const int n = c + W, mn = m[n];
-        if (mm + mn > 0) {
-          sv_stored = false;
-          if (mm * mn > 0) {
-            double rtmp1 = k.area_t * vsn + k.area_t * sn[n];
-            sv = dvc(half(rtmp1), k.area_v, k.r_area_v, k.fast_div);
-          } else if (mm <= 0) {
-            sv = sn[n];
-          } else {
-            sv = vsn;
-          }
-        }
-      }
-      if (su_stored) su = f.sshn_u[c];
-      if (sv_stored) sv = f.sshn_v[c];
-    }
-    A(A_SN, t) = vsn;
-    A(A_UN, t) = vun;
-    A(A_VN, t) = vvn;
-    A(A_HU, t) = vhu;
-    A(A_HV, t) = vhv;
-    A(A_SU, t) = su;
-    A(A_SV, t) = sv;
-    A(A_HUS, t) = vhu + su;
-    A(A_HVS, t) = vhv + sv;
-    mk[t] = mm;
+// The terms at slot q (cell (i, j)) that neighbouring updates share.  X: the
+// terms of the cell's west side, Y: of its south side (a tile's east and
+// north neighbours need one of the two only).  Every term is the exact
+// operation sequence of momentum_{u,v}_kern.c / continuity_kern.c for one of
+// the two updates that use it; for the other update the reference evaluates
+// the same operations on the same operands (addition commuted), so the bits
+// agree.  ht: the T depth at the cell.
+template <class T, bool X, bool Y>
+__device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q, double ht,
+                                             const FastConst& k) {
+  constexpr int S0 = T::S0, SX = T::SX;
+  const int qw = q - 1, qs = q - SX, qse = qs + 1, qwn = qw + SX;
+  const double D = ht + A(A_SN, q);  // ht + sshn at T(i,j)
+  const double u_c = A(A_UN, q), v_c = A(A_VN, q);
+  if (X && Y) {  // continuity fluxes (sshn_u + hu) * un and (sshn_v + hv) * vn
+    B(B_FLXU, q) = A(A_HUS, q) * u_c;
+    B(B_FLXV, q) = A(A_HVS, q) * v_c;
   }
-  __syncthreads();
-
-  // ---- phase 1: terms shared by neighbouring updates ----
-  // Every term is the exact operation sequence of momentum_{u,v}_kern.c /
-  // continuity_kern.c for one of the two updates that use it; for the other
-  // update the reference evaluates the same operations on the same operands
-  // (addition commuted), so the bits agree.
-  for (int t = tid; t < S1; t += NTHREADS) {
-    const int ti = t % P1X, tj = t / P1X;
-    const int i = i0 - 1 + ti, j = j0 - 1 + tj;
-    const int q = (tj + 1) * SX + (ti + 1);  // phase-0 slot of (i,j)
-    const int qw = q - 1, qs = q - SX, qse = qs + 1, qwn = qw + SX;
-    const double ht = (i >= 0 && i < W && j >= 0 && j < H) ? f.ht[j * W + i] : 0.0;
-    const double D = ht + A(A_SN, q);  // ht + sshn at T(i,j)
-    const double u_c = A(A_UN, q), u_w = A(A_UN, qw), u_s = A(A_UN, qs), u_wn = A(A_UN, qwn);
-    const double v_c = A(A_VN, q), v_w = A(A_VN, qw), v_s = A(A_VN, qs), v_se = A(A_VN, qse);
-    // continuity fluxes (sshn_u + hu) * un and (sshn_v + hv) * vn
-    B(B_FLXU, t) = A(A_HUS, q) * u_c;
-    B(B_FLXV, t) = A(A_HVS, q) * v_c;
-    // dudx at T(i,j) (dudx_w of u face i, dudx_e of face i-1); dvdy likewise
-    B(B_GX, t) = dvc(u_c - u_w, k.dx_t, k.r_dx_t, k.fast_div) * D;
-    B(B_GY, t) = dvc(v_c - v_s, k.dy_t, k.r_dy_t, k.fast_div) * D;
+  if (X) {
+    const double u_w = A(A_UN, qw), v_w = A(A_VN, qw);
+    // dudx at T(i,j): dudx_w of u face i, dudx_e of face i-1
+    B(B_GX, q) = dvc(u_c - u_w, k.dx_t, k.r_dx_t, k.fast_div) * D;
     // x-advective flux of u through T(i,j): uu_w * u_w * depw of face i
     const double U = half(u_c + u_w) * k.dy_t;
-    B(B_FXU, t) = (upwind(U, u_c, u_w) * U) * D;
-    // y-advective flux of v through T(i,j): vv_s * v_s * deps of face j
-    const double V = half(v_c + v_s) * k.dx_t;
-    B(B_FYV, t) = (upwind(V, v_c, v_s) * V) * D;
-    // south edge of u face (i,j): v_sc, v_s, deps, uu_s (unmasked form)
-    const double vsc = half(v_s + v_se);
-    B(B_VSC, t) = vsc;
-    const double Vs = half(vsc) * k.dxv2;
-    const double deps = half((A(A_HVS, qs) + A(A_HV, qse)) + A(A_SV, qse));
-    B(B_FYU, t) = (upwind(Vs, u_c, u_s) * Vs) * deps;
-    B(B_QY, t) = dvc(u_c - u_s, k.dyu2, k.r_dyu2, k.fast_div);
+    B(B_FXU, q) = (upwind(U, u_c, u_w) * U) * D;
     // west edge of v face (i,j): u_wc, u_w, depw, vv_w (unmasked form)
-    const double uwc = half(u_w + u_wn);
-    B(B_UWC, t) = uwc;
+    const double uwc = half(u_w + A(A_UN, qwn));
+    B(B_UWC, q) = uwc;
     const double Uw = half(uwc) * k.dyu2;
     const double depw = half((A(A_HUS, qw) + A(A_HU, qwn)) + A(A_SU, qwn));
-    B(B_FXV, t) = (upwind(Uw, v_c, v_w) * Uw) * depw;
-    B(B_QX, t) = dvc(v_c - v_w, k.dxv2, k.r_dxv2, k.fast_div);
+    B(B_FXV, q) = (upwind(Uw, v_c, v_w) * Uw) * depw;
+    B(B_QX, q) = dvc(v_c - v_w, k.dxv2, k.r_dxv2, k.fast_div);
+  }
+  if (Y) {
+    const double u_s = A(A_UN, qs), v_s = A(A_VN, qs);
+    // dvdy at T(i,j): dvdy_s of v face j, dvdy_n of face j-1
+    B(B_GY, q) = dvc(v_c - v_s, k.dy_t, k.r_dy_t, k.fast_div) * D;
+    // y-advective flux of v through T(i,j): vv_s * v_s * deps of face j
+    const double V = half(v_c + v_s) * k.dx_t;
+    B(B_FYV, q) = (upwind(V, v_c, v_s) * V) * D;
+    // south edge of u face (i,j): v_sc, v_s, deps, uu_s (unmasked form)
+    const double vsc = half(v_s + A(A_VN, qse));
+    B(B_VSC, q) = vsc;
+    const double Vs = half(vsc) * k.dxv2;
+    const double deps = half((A(A_HVS, qs) + A(A_HV, qse)) + A(A_SV, qse));
+    B(B_FYU, q) = (upwind(Vs, u_c, u_s) * Vs) * deps;
+    B(B_QY, q) = dvc(u_c - u_s, k.dyu2, k.r_dyu2, k.fast_div);
+  }
+}
+
+// One tile of the fused step: interior cells [i0, i0+TX) x [j0, j0+TY) of one
+// domain.  `tide` is this step's bc_ssh value (general cells).
+//
+// The FP64 pipe bounds the step (about 1.7 instructions per clock per SM;
+// each holds a scheduler's share of it for 64 issue slots), so every phase
+// forms a value on exactly the positions that are read: a full warp per row
+// of the tile, and the edges' extra values (next column, next row) packed
+// into warps of their own.  140 -> 123 FP64 instructions per cell against the
+// form that formed everything on a 2- and a 1-cell halo.
+template <class T>
+__device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs, const Dims& d,
+                                           const Scalars& p, const FastConst& k, double tide,
+                                           int i0, int j0, double* smem) {
+  constexpr int TX = T::TX, TY = T::TY, SX = T::SX, S0 = T::S0;
+  constexpr int RX = T::RX, RY = T::RY, RY1 = T::RY1;
+  double* a0 = smem;                 // [N_A0][S0]
+  double* b1 = smem + N_A0 * S0;     // [N_B1][S0]
+  int* mk = (int*)(b1 + N_B1 * S0);  // [S0]
+  int* glist = mk + S0;              // [TX * TY] general cells of this tile
+  int* gcount = glist + TX * TY;
+
+  const int W = d.width, H = d.height;
+  const int tid = threadIdx.y * TX + threadIdx.x;
+  const int i = i0 + threadIdx.x;
+
+  if (tid == 0) *gcount = 0;
+  // ---- the fields (positions past the array's end hold what the last
+  // column or row does; no cell that is written reads them) ----
+  for (int t = tid; t < S0; t += NTHREADS) {
+    const int c = min(j0 - 1 + t / SX, H - 1) * W + min(i0 - 1 + t % SX, W - 1);
+    const double sn = fs.sshn_in[c];
+    A(A_SN, t) = sn;
+    A(A_UN, t) = fs.un_in[c];
+    A(A_VN, t) = fs.vn_in[c];
+    A(A_HU, t) = f.hu[c];
+    A(A_HV, t) = f.hv[c];
+    mk[t] = f.tmask[c];
+    B(B_AREA_SSH, t) = k.area_t * sn;
+  }
+  double ht[T::RPT];  // of this thread's own cells, for the shared terms
+#pragma unroll
+  for (int e = 0; e < T::RPT; e++)
+    ht[e] = f.ht[min(j0 + (int)threadIdx.y + e * T::RPP, H - 1) * W + min(i, W - 1)];
+  __syncthreads();
+
+  // ---- the sshn_u / sshn_v this step reads: next_sshu_code /
+  // next_sshv_code (time_update_kern.c:90-155) over their loop ranges; other
+  // faces keep the stored value, which is read only for them ----
+  auto face_u = [&](int tx, int ty, bool sum) {
+    const int q = (ty + 1) * SX + tx + 1, fi = i0 + tx, fj = j0 + ty;
+    double su;
+    const int mm = mk[q], mn = mk[q + 1];
+    if (fj <= d.ye && fi <= d.xe - 1 && mm + mn > 0) {
+      if (mm * mn > 0)
+        su = dvc(half(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + 1)), k.area_u, k.r_area_u,
+                 k.fast_div);
+      else
+        su = mm <= 0 ? A(A_SN, q + 1) : A(A_SN, q);
+    } else {
+      su = f.sshn_u[min(fj, H - 1) * W + min(fi, W - 1)];
+    }
+    A(A_SU, q) = su;
+    if (sum) A(A_HUS, q) = A(A_HU, q) + su;
+  };
+  auto face_v = [&](int tx, int ty, bool sum) {
+    const int q = (ty + 1) * SX + tx + 1, fi = i0 + tx, fj = j0 + ty;
+    double sv;
+    const int mm = mk[q], mn = mk[q + SX];
+    if (fj <= d.ye - 1 && fi <= d.xe && mm + mn > 0) {
+      if (mm * mn > 0)
+        sv = dvc(half(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + SX)), k.area_v, k.r_area_v,
+                 k.fast_div);
+      else
+        sv = mm <= 0 ? A(A_SN, q + SX) : A(A_SN, q);
+    } else {
+      sv = f.sshn_v[min(fj, H - 1) * W + min(fi, W - 1)];
+    }
+    A(A_SV, q) = sv;
+    if (sum) A(A_HVS, q) = A(A_HV, q) + sv;
+  };
+#pragma unroll
+  for (int e = 0; e < T::RPT; e++) {
+    face_u(threadIdx.x, threadIdx.y + e * T::RPP, true);
+    face_v(threadIdx.x, threadIdx.y + e * T::RPP, true);
+  }
+  // u faces: rows -1 and TY, column -1 (rows 0 .. TY); v faces: row -1,
+  // columns -1 and TX (rows -1 .. TY-1)
+  for (int t = tid; t < 3 * RX + RY + 2 * RY1; t += NTHREADS) {
+    int e = t;
+    if (e < RX) {
+      if (e < TX) face_u(e, -1, false);
+    } else if ((e -= RX) < RX) {
+      if (e < TX) face_u(e, TY, false);
+    } else if ((e -= RX) < RX) {
+      if (e < TX) face_v(e, -1, true);
+    } else if ((e -= RX) < RY1) {
+      if (e <= TY) face_u(-1, e, true);
+    } else if ((e -= RY1) < RY1) {
+      if (e <= TY) face_v(TX, e - 1, false);
+    } else {
+      e -= RY1;
+      if (e < TY) face_v(-1, e, false);
+    }
   }
   __syncthreads();
 
+  // ---- the terms shared by neighbouring updates ----
+#pragma unroll
+  for (int e = 0; e < T::RPT; e++)
+    shared_terms<T, true, true>(a0, b1, (threadIdx.y + e * T::RPP + 1) * SX + threadIdx.x + 1,
+                                ht[e], k);
+  // the south terms of row TY, the west terms of column TX, and the fluxes
+  // through the tile's west and south edges
+  for (int t = tid; t < 2 * RX + 2 * RY; t += NTHREADS) {
+    int e = t;
+    if (e < RX) {
+      if (e < TX)
+        shared_terms<T, false, true>(a0, b1, (TY + 1) * SX + e + 1,
+                                     f.ht[min(j0 + TY, H - 1) * W + min(i0 + e, W - 1)], k);
+    } else if ((e -= RX) < RY) {
+      if (e < TY)
+        shared_terms<T, true, false>(a0, b1, (e + 1) * SX + TX + 1,
+                                     f.ht[min(j0 + e, H - 1) * W + min(i0 + TX, W - 1)], k);
+    } else if ((e -= RY) < RY) {
+      const int q = (e + 1) * SX;
+      if (e < TY) B(B_FLXU, q) = A(A_HUS, q) * A(A_UN, q);
+    } else {
+      e -= RY;
+      const int q = e + 1;
+      if (e < TX) B(B_FLXV, q) = A(A_HVS, q) * A(A_VN, q);
+    }
+  }
+  __syncthreads();
+
+  // ---- the update ----
   // Each thread owns the cells (i, j0 + row) of its rows.  Regular cells
   // (wet 3x3 neighbourhood: continuity without bc_ssh, unmasked momentum, no
   // solid-wall or Flather change) are computed here; the others are queued
-  // for the packed general pass below, so that a warp holding a few boundary
+  // for the packed general pass below, so that a warp holding a few land-side
   // cells does not run both paths.  When both of a thread's cells are
   // regular they are computed in one straight-line block, so the compiler
   // can interleave two independent FP64 chains; the per-face global inputs
@@ -588,45 +692,40 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
 #pragma unroll
   for (int pb = 0; pb < T::RPT; pb += 2) {
     constexpr int NP = T::RPT >= 2 ? 2 : 1;  // rows taken together
-    const int i = i0 + threadIdx.x;
-    int c[NP], q[NP], r[NP];
+    int c[NP], q[NP];
     bool reg[NP];
 #pragma unroll
     for (int e = 0; e < NP; e++) {
-      const int row = threadIdx.y + (pb + e) * ROWS_PER_PASS, j = j0 + row;
+      const int row = threadIdx.y + (pb + e) * T::RPP, j = j0 + row;
       c[e] = j * W + i;
-      q[e] = (row + HALO) * SX + (threadIdx.x + HALO);
-      r[e] = (row + 1) * P1X + (threadIdx.x + 1);
-      const bool live = i <= d.xe + 1 && j <= d.ye;
-      bool regular = live && i >= d.xs && i <= d.xe - 1 && j >= d.ys && j <= d.ye - 1;
-      if (regular) {
+      q[e] = (row + 1) * SX + (threadIdx.x + 1);
+      const bool live = i <= d.xe - 1 && j <= d.ye - 1;
+      bool regular = live;
 #pragma unroll
-        for (int dj = -1; dj <= 1; dj++)
+      for (int dj = -1; dj <= 1; dj++)
 #pragma unroll
-          for (int di = -1; di <= 1; di++) regular &= mk[q[e] + dj * SX + di] > 0;
-      }
+        for (int di = -1; di <= 1; di++) regular &= mk[q[e] + dj * SX + di] > 0;
       reg[e] = regular;
       if (live && !regular) glist[atomicAdd(gcount, 1)] = row * TX + threadIdx.x;
     }
-    double sau[NP], rhu[NP], sav[NP], rhv[NP];
+    double dhu[NP], rhu[NP], dhv[NP], rhv[NP];
 #pragma unroll
     for (int e = 0; e < NP; e++)
       if (reg[e]) {
-        sau[e] = f.ssha_u[c[e]];
+        dhu[e] = f.d_hu[c[e]];
         rhu[e] = f.r_hu[c[e]];
-        sav[e] = f.ssha_v[c[e]];
+        dhv[e] = f.d_hv[c[e]];
         rhv[e] = f.r_hv[c[e]];
       }
     RegOut o[NP];
     if (NP == 2 && reg[0] && reg[NP - 1]) {
-      o[0] = regular_cell<T>(a0, b1, q[0], r[0], sau[0], rhu[0], sav[0], rhv[0], k);
-      o[NP - 1] = regular_cell<T>(a0, b1, q[NP - 1], r[NP - 1], sau[NP - 1], rhu[NP - 1],
-                                  sav[NP - 1], rhv[NP - 1], k);
+      o[0] = regular_cell<T>(a0, b1, q[0], dhu[0], rhu[0], dhv[0], rhv[0], k);
+      o[NP - 1] = regular_cell<T>(a0, b1, q[NP - 1], dhu[NP - 1], rhu[NP - 1], dhv[NP - 1],
+                                  rhv[NP - 1], k);
     } else {
 #pragma unroll
       for (int e = 0; e < NP; e++)
-        if (reg[e])
-          o[e] = regular_cell<T>(a0, b1, q[e], r[e], sau[e], rhu[e], sav[e], rhv[e], k);
+        if (reg[e]) o[e] = regular_cell<T>(a0, b1, q[e], dhu[e], rhu[e], dhv[e], rhv[e], k);
     }
 #pragma unroll
     for (int e = 0; e < NP; e++)
@@ -640,29 +739,11 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
 
   // ---- general cells: the reference's per-point code, in its order ----
   const int ngen = *gcount;
-  for (int g = tid; g < ngen; g += NTHREADS) {
-    const int row = glist[g] / TX, col = glist[g] - (glist[g] / TX) * TX;
-    Ctx<SX> x;
-    x.sn = sn;
-    x.un = un;
-    x.vn = vn;
-    x.hu = f.hu;
-    x.hv = f.hv;
-    x.ht = f.ht;
-    x.ssha_u = f.ssha_u;
-    x.ssha_v = f.ssha_v;
-    x.r_hu = f.r_hu;
-    x.r_hv = f.r_hv;
-    x.m = m;
-    x.su_tile = &A(A_SU, 0);
-    x.sv_tile = &A(A_SV, 0);
-    x.W = W;
-    x.i0 = i0;
-    x.j0 = j0;
-    x.d = d;
-    x.k = k;
-    general_cell(x, f, fs, p, tide, i0 + col, j0 + row);
-  }  // general cells
+  for (int g = tid; g < kParts * ngen; g += NTHREADS) {
+    const int part = g / ngen, cell = glist[g - part * ngen];
+    const int row = cell / TX, col = cell - row * TX;
+    general_at(f, fs, d, p, k, tide, part, i0 + col, j0 + row);
+  }
 #undef A
 #undef B
 }

@@ -33,9 +33,10 @@ struct Fields {
   double *area_t, *area_u, *area_v, *dx_u, *dx_v, *dx_t, *dy_u, *dy_v, *dy_t,
       *gphiu, *gphiv;
   double *sin_u, *sin_v;
-  // RN(1 / (hu + ssha_u)) and RN(1 / (hv + ssha_v)) (0 where out of the
-  // range the exact reciprocal division needs), for the fused step.
-  double *r_hu, *r_hv;
+  // hu + ssha_u and hv + ssha_v (no step writes either operand) and RN(1 /
+  // them) (0 where out of the range the exact reciprocal division needs), for
+  // the fused step's regular cells.
+  double *d_hu, *d_hv, *r_hu, *r_hv;
 };
 
 struct Dims {
@@ -85,9 +86,10 @@ void launch_fused_step(const Fields& f, const FusedState& fs, const Dims& d,
                        const Scalars& s, const UniformMetrics& um, double tide,
                        const double* tide_table, int tide_index,
                        cudaStream_t st);
-// The rows of tiles the fused step's grid has for this domain, and the
-// tile's height in cells (its tile rows start at row ys - 1).
-int fused_step_tile_rows(const Dims& d, int* tile_height);
+// The rows of tiles the fused step's grid has for this domain, and the first
+// copy-region row that tile row `row` updates (0 .. the number of rows).
+int fused_step_tile_rows(const Dims& d);
+int fused_step_first_row(const Dims& d, int row);
 // The fused step on tile rows [row0, row1) of that grid only.
 void launch_fused_step_rows(const Fields& f, const FusedState& fs, const Dims& d,
                             const Scalars& s, const UniformMetrics& um, double tide, int row0,
@@ -134,7 +136,7 @@ void launch_df_step(const Fields& f, const FusedState& fs, const Dims& d, const 
 void launch_df_split(const double* a, float2* out, long long n, cudaStream_t st);
 void launch_df_flags(const int* tmask, const Dims& d, unsigned char* reg, cudaStream_t st);
 
-// Recomputes Fields::r_hu / r_hv from hu, ssha_u, hv, ssha_v (array rows
+// Recomputes Fields::d_hu / r_hu / d_hv / r_hv from hu, ssha_u, hv, ssha_v (array rows
 // [row0, row1) only, when given).
 void launch_depth_reciprocals(const Fields& f, const Dims& d, cudaStream_t st, int row0 = 0,
                               int row1 = -1);

@@ -134,7 +134,7 @@ class Ensemble:
     def schedule(self, ctas_per_sm=2, policy=0, boundary_weight=4.0, tile=(32, 16),
                  march_rows=32):
         """Schedule and tile knobs (nl2d_ens_schedule, nl2d_ens_tile): CTAs
-        per SM, tile assignment policy, boundary-edge cost weight, the FP64
+        per SM, tile assignment policy, ring-cell cost weight, the FP64
         tile shape and the mixed form's march strip height."""
         self._check(self.lib.nl2d_ens_schedule(ctas_per_sm, policy, boundary_weight),
                     "nl2d_ens_schedule")
