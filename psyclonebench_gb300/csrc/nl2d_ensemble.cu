@@ -82,7 +82,7 @@ __global__ void k_mixed_statics(const double* __restrict__ ht, const double* __r
 // domains; CTA b takes entries [first[b], first[b+1]).  An entry (domain, i0,
 // j0, -1) is a tile, (domain, -, -, g) parts g .. g + NTHREADS - 1 of the
 // domain's ring cells.  `tides` holds this step's bc_ssh value per domain.
-template <class T>
+template <class T, bool IC>
 __global__ void __launch_bounds__(NTHREADS, T::kMinBlocks)
     k_ensemble_step(const EnsDomain* __restrict__ doms, const int4* __restrict__ tiles,
                     const int* __restrict__ first, int parity,
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(NTHREADS, T::kMinBlocks)
       continue;
     }
     __syncthreads();  // the previous tile's last readers are done with smem
-    fused_tile<T>(D.f, D.fs[parity], D.d, D.p, D.k, tides[tl.x], tl.y, tl.z, smem);
+    fused_tile<T, IC>(D.f, D.fs[parity], D.d, D.p, D.k, tides[tl.x], tl.y, tl.z, smem);
   }
 }
 
@@ -184,7 +184,11 @@ template <class T>
 bool set_ens_attr() {
   static bool attr = false;
   if (!attr)
-    attr = cudaFuncSetAttribute(k_ensemble_step<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    attr = cudaFuncSetAttribute(k_ensemble_step<T, false>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)T::kSmemBytes) == cudaSuccess &&
+           cudaFuncSetAttribute(k_ensemble_step<T, true>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)T::kSmemBytes) == cudaSuccess;
   return attr;
 }
@@ -202,21 +206,25 @@ bool prepare_ens_step(int shape) {
 }
 
 template <class T>
-void launch_ens_step_shape(int nctas, const EnsDomain* doms, const int4* tiles, const int* first,
+void launch_ens_step_shape(bool int_mul, int nctas, const EnsDomain* doms, const int4* tiles, const int* first,
                            int parity, const double* tides, cudaStream_t st) {
-  k_ensemble_step<T><<<nctas, dim3(T::TX, T::RPP), T::kSmemBytes, st>>>(doms, tiles, first,
-                                                                         parity, tides);
+  auto step = int_mul ? k_ensemble_step<T, true> : k_ensemble_step<T, false>;
+  step<<<nctas, dim3(T::TX, T::RPP), T::kSmemBytes, st>>>(doms, tiles, first, parity, tides);
 }
 
-void launch_ens_step(int shape, int nctas, const EnsDomain* doms, const int4* tiles,
-                     const int* first, int parity, const double* tides, cudaStream_t st) {
+// int_mul: every domain's constants have the integer form (FastConst).
+void launch_ens_step(int shape, bool int_mul, int nctas, const EnsDomain* doms,
+                     const int4* tiles, const int* first, int parity, const double* tides,
+                     cudaStream_t st) {
+  auto launch = launch_ens_step_shape<DefaultTile>;
   switch (shape) {
-    case 1: launch_ens_step_shape<Tile<32, 8>>(nctas, doms, tiles, first, parity, tides, st); break;
-    case 2: launch_ens_step_shape<Tile<16, 16>>(nctas, doms, tiles, first, parity, tides, st); break;
-    case 3: launch_ens_step_shape<Tile<64, 8>>(nctas, doms, tiles, first, parity, tides, st); break;
-    case 4: launch_ens_step_shape<Tile<32, 32>>(nctas, doms, tiles, first, parity, tides, st); break;
-    default: launch_ens_step_shape<DefaultTile>(nctas, doms, tiles, first, parity, tides, st);
+    case 1: launch = launch_ens_step_shape<Tile<32, 8>>; break;
+    case 2: launch = launch_ens_step_shape<Tile<16, 16>>; break;
+    case 3: launch = launch_ens_step_shape<Tile<64, 8>>; break;
+    case 4: launch = launch_ens_step_shape<Tile<32, 32>>; break;
+    default: break;
   }
+  launch(int_mul, nctas, doms, tiles, first, parity, tides, st);
 }
 
 // Per-domain checksums: block (dom, field) sums |f| over the domain's
@@ -313,6 +321,7 @@ struct Ens {
   cudaGraphExec_t graph = nullptr;
   int graph_key[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
   bool built = false;
+  bool int_mul = false;  // every domain's constants have the integer form
   int shape = 0;        // index into kShapes: the FP64 kernel's tile
   int march_rows = kDefaultMarchRows;  // strip height of the column marches
   // mixed-precision form
@@ -548,6 +557,7 @@ bool build_schedule(int TXv, int TYv) {
 bool build_descriptors() {
   Ens& e = g_ens;
   std::vector<EnsDomain> desc(e.ndom);
+  e.int_mul = true;
   for (int k = 0; k < e.ndom; k++) {
     const DomainHost& D = e.dom[k];
     EnsDomain& x = desc[k];
@@ -581,6 +591,7 @@ bool build_descriptors() {
     um.sin_u = um.sin_v = std::sin(D.gphi * e.sc.d2r);
     x.um = um;
     x.k = make_fast_const(e.sc, um);
+    e.int_mul = e.int_mul && x.k.int_mul;
   }
   cudaFree(e.d_desc);
   e.d_desc = nullptr;
@@ -1087,7 +1098,7 @@ int nl2d_ens_run(int istep0, int nsteps, int checksum_every, double* checksums_o
           k_ensemble_checksums<<<dim3(e.ndom, 3), 256, 0, e.stream>>>(e.d_desc, par, e.ndom,
                                                                       sums);
       } else {
-        launch_ens_step(e.shape, e.nctas, e.d_desc, e.d_tiles, e.d_first, par,
+        launch_ens_step(e.shape, e.int_mul, e.nctas, e.d_desc, e.d_tiles, e.d_first, par,
                         e.d_tides + (size_t)q * e.ndom, e.stream);
         par = 1 - par;
         if (want_sums)

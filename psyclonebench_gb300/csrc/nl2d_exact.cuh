@@ -22,6 +22,8 @@
 //    other than zero), huge (2^900 and above) or not finite use the IEEE
 //    divide, so no intermediate underflows or overflows; divisors are
 //    checked on the host to lie in [2^-100, 2^100].
+//  * mul_const(x, f, c): x * c for a step constant c of at most 32
+//    significant bits, in integers.
 //  * half(x): 0.5 * x.  For normal x with a biased exponent >= 2 this is
 //    exact, i.e. the exponent minus one, done in integer arithmetic; zero
 //    keeps its bits; subnormal, smallest-normal and non-finite x use DMUL.
@@ -98,6 +100,40 @@ __device__ __forceinline__ double div_rn(double x, double d, double r) {
   long long k = 0;
   if (rem + (md >> 1) > (md & ~1ULL)) k = (long long)rem < 0 ? 1 : -1;
   return from_bits((long long)qb + k);
+}
+
+// A constant factor c > 0 in [2^-100, 2^100] of at most 32 significant bits
+// (grid spacings and time steps in whole or simply fractional units), as
+// mul_const takes it: co 2^e with co in [2^31, 2^32), and what the product's
+// exponent field gains.  co = 0: c is not of that kind.
+struct IntFactor {
+  unsigned co, add;
+};
+
+// RN(x * c) in integers: the product of the significands (85 bits) is exact
+// in three words, normalised by its leading bit and rounded to nearest even.
+// Magnitudes of x below 2^-899 or from 2^900 take the IEEE product, +-0
+// itself.  About 20 instructions on the integer pipes, where the DMUL holds
+// a scheduler's share of the FP64 pipe for 64 issue slots.
+static __device__ __noinline__ double mul_ieee(double x, double c) { return x * c; }
+__device__ __forceinline__ double mul_const(double x, IntFactor f, double c) {
+  const unsigned long long b = (unsigned long long)bits(x);
+  const unsigned xl = (unsigned)b, xh = (unsigned)(b >> 32);
+  if (((xh >> 20) & 0x7ffu) - 124u > 1798u) {
+    if ((b & 0x7fffffffffffffffULL) == 0) return x;
+    return mul_ieee(x, c);
+  }
+  const unsigned long long p = (unsigned long long)xl * f.co;
+  const unsigned long long t =
+      (unsigned long long)((xh & 0xfffffu) | 0x100000u) * f.co + (p >> 32);
+  const unsigned w0 = (unsigned)p, w1 = (unsigned)t, w2 = (unsigned)(t >> 32);
+  const unsigned top = w2 >> 20, s = top ^ 1u;  // the leading bit is bit 84 or 83
+  const unsigned qh = __funnelshift_l(w1, w2, s), ql = __funnelshift_l(w0, w1, s);
+  const unsigned frac = w0 << s;
+  unsigned long long q = ((unsigned long long)qh << 32) | ql;
+  if (frac > 0x80000000u - (ql & 1u)) q++;  // above half, or half and odd
+  const unsigned eh = (xh & 0xfff00000u) + f.add + (top << 20);
+  return from_bits((long long)(q + ((unsigned long long)eh << 32)));
 }
 
 __device__ __forceinline__ double half(double x) {

@@ -42,7 +42,7 @@ using SmallTile = Tile<16, 16>;
 // ring's cells in those rows, rc parts of them each (one per thread: their
 // long FP64 chains start first and run beside the tiles); the others one tile
 // each of the ntx per row of tiles, from tile row row0.
-template <class TT>
+template <class TT, bool IC>
 __global__ void __launch_bounds__(NTHREADS, TT::kMinBlocks)
     k_fused_step(const __grid_constant__ Fields f, const __grid_constant__ FusedState fs,
                  const __grid_constant__ Dims d, const __grid_constant__ Scalars p,
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(NTHREADS, TT::kMinBlocks)
     return;
   }
   const int t = blockIdx.x - nring, by = t / ntx, bx = t - by * ntx;
-  fused_tile<TT>(f, fs, d, p, k, td, d.xs + 1 + bx * TT::TX, d.ys + 1 + (row0 + by) * TT::TY,
+  fused_tile<TT, IC>(f, fs, d, p, k, td, d.xs + 1 + bx * TT::TX, d.ys + 1 + (row0 + by) * TT::TY,
                  smem);
 }
 
@@ -92,18 +92,20 @@ void launch_rows(const Fields& f, const FusedState& fs, const Dims& d, const Sca
   int rc = 32;
   while (rc < NTHREADS && nr > rc * 152) rc *= 2;
   const int nring = (nr + rc - 1) / rc;
-  k_fused_step<TT><<<nring + ntx * nty, dim3(TT::TX, TT::RPP), TT::kSmemBytes, st>>>(
-      f, fs, d, s, make_fast_const(s, um), tide_table, tide_index, tide, row0, ntx, ja, jb,
-      nring, rc);
+  const FastConst k = make_fast_const(s, um);
+  auto step = k.int_mul ? k_fused_step<TT, true> : k_fused_step<TT, false>;
+  step<<<nring + ntx * nty, dim3(TT::TX, TT::RPP), TT::kSmemBytes, st>>>(
+      f, fs, d, s, k, tide_table, tide_index, tide, row0, ntx, ja, jb, nring, rc);
 }
 
 void set_step_attrs() {
   static bool attr_set = false;
   if (!attr_set) {
-    cudaFuncSetAttribute(k_fused_step<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)T::kSmemBytes);
-    cudaFuncSetAttribute(k_fused_step<SmallTile>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)SmallTile::kSmemBytes);
+    for (auto* fn : {k_fused_step<T, false>, k_fused_step<T, true>})
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmemBytes);
+    for (auto* fn : {k_fused_step<SmallTile, false>, k_fused_step<SmallTile, true>})
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)SmallTile::kSmemBytes);
     attr_set = true;
   }
 }

@@ -3,6 +3,8 @@
 // (nl2d_ensemble.cu).  See nl2d_fused.cu for what a step computes and why it
 // is bit-identical to the reference.
 #pragma once
+#include <cstring>
+
 #include "nl2d_exact.cuh"
 #include "nl2d_internal.h"
 
@@ -32,6 +34,11 @@ struct FastConst {
   double cor_u, cor_v;                                  // 2. * omega * sin(gphi * d2r)
   double neg_g, rdt, visc, g;
   int fast_div;  // every constant divisor lies in [2^-100, 2^100]
+  // the grid's and the time step's constants as integer factors (mul_const),
+  // and whether all of them have that form
+  IntFactor i_area_t, i_area_u, i_area_v, i_dx_u, i_dx_v, i_dx_t, i_dy_u, i_dy_v, i_dy_t;
+  IntFactor i_dxv2, i_dyu2, i_rdt;
+  int int_mul;
 };
 
 // One domain of an ensemble (device-resident descriptor).
@@ -43,6 +50,13 @@ struct EnsDomain {
   UniformMetrics um;
   FastConst k;
 };
+
+// Multiplication by a step constant, `kc` and its integer form `ic` (IC), the
+// same bits either way.
+template <bool IC>
+__device__ __forceinline__ double mlc(double x, double kc, IntFactor ic) {
+  return IC ? mul_const(x, ic, kc) : x * kc;
+}
 
 // Division by a step constant: the Markstein form when the constants allow
 // it, otherwise the IEEE divide.  Both give the same bits.
@@ -452,7 +466,7 @@ using DefaultTile = Tile<32, 16>;
 struct RegOut {
   double ssh, u, v;
 };
-template <class T>
+template <class T, bool IC>
 __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b1, int q,
                                                double dhu, double rhu, double dhv, double rhv,
                                                const FastConst& k) {
@@ -461,20 +475,24 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
 #define B(qq, t) b1[(qq) * S0 + (t)]
   RegOut o;
   const double snc = A(A_SN, q), Hu = A(A_HUS, q), Hv = A(A_HVS, q);
-  const double ssh = (((B(B_FLXU, q - 1) - B(B_FLXU, q)) + B(B_FLXV, q - SX)) - B(B_FLXV, q)) *
-                     k.rdt;
+  const double ssh = mlc<IC>(
+      ((B(B_FLXU, q - 1) - B(B_FLXU, q)) + B(B_FLXV, q - SX)) - B(B_FLXV, q), k.rdt, k.i_rdt);
   o.ssh = snc + dvc(ssh, k.area_t, k.r_area_t, k.fast_div);
   {
     const double adv = ((B(B_FXU, q) - B(B_FXU, q + 1)) + B(B_FYU, q)) - B(B_FYU, q + SX);
     const double dudy_s = B(B_QY, q) * ((Hu + A(A_HU, q - SX)) + A(A_SU, q - SX));
     const double dudy_n = B(B_QY, q + SX) * ((Hu + A(A_HU, q + SX)) + A(A_SU, q + SX));
-    double vis = (B(B_GX, q + 1) - B(B_GX, q)) * k.dy_u + half((dudy_n - dudy_s) * k.dx_u);
+    double vis = mlc<IC>(B(B_GX, q + 1) - B(B_GX, q), k.dy_u, k.i_dy_u) +
+                 half(mlc<IC>(dudy_n - dudy_s, k.dx_u, k.i_dx_u));
     vis = k.visc * vis;
-    const double cor = (half(k.cor_u * (B(B_VSC, q) + B(B_VSC, q + SX))) * k.area_u) * Hu;
-    const double hpg = ((k.neg_g * Hu) * k.dy_u) * (A(A_SN, q + 1) - snc);
+    const double cor = mlc<IC>(half(k.cor_u * (B(B_VSC, q) + B(B_VSC, q + SX))), k.area_u,
+                               k.i_area_u) *
+                       Hu;
+    const double hpg = mlc<IC>(k.neg_g * Hu, k.dy_u, k.i_dy_u) * (A(A_SN, q + 1) - snc);
     const double num =
         A(A_UN, q) * Hu +
-        dvc(k.rdt * (((adv + vis) + cor) + hpg), k.area_u, k.r_area_u, k.fast_div);
+        dvc(mlc<IC>(((adv + vis) + cor) + hpg, k.rdt, k.i_rdt), k.area_u, k.r_area_u,
+            k.fast_div);
     const double t1 = dvf(num, dhu, rhu);
     o.u = dvc(t1, k.fric, k.r_fric, k.fast_div);
   }
@@ -482,13 +500,17 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
     const double adv = ((B(B_FXV, q) - B(B_FXV, q + 1)) + B(B_FYV, q)) - B(B_FYV, q + SX);
     const double dvdx_w = B(B_QX, q) * ((Hv + A(A_HV, q - 1)) + A(A_SV, q - 1));
     const double dvdx_e = B(B_QX, q + 1) * ((Hv + A(A_HV, q + 1)) + A(A_SV, q + 1));
-    double vis = (B(B_GY, q + SX) - B(B_GY, q)) * k.dx_v + half((dvdx_e - dvdx_w) * k.dy_v);
+    double vis = mlc<IC>(B(B_GY, q + SX) - B(B_GY, q), k.dx_v, k.i_dx_v) +
+                 half(mlc<IC>(dvdx_e - dvdx_w, k.dy_v, k.i_dy_v));
     vis = k.visc * vis;
-    const double cor = (-half(k.cor_v * (B(B_UWC, q + 1) + B(B_UWC, q))) * k.area_v) * Hv;
-    const double hpg = ((k.neg_g * Hv) * k.dx_v) * (A(A_SN, q + SX) - snc);
+    const double cor = mlc<IC>(-half(k.cor_v * (B(B_UWC, q + 1) + B(B_UWC, q))), k.area_v,
+                               k.i_area_v) *
+                       Hv;
+    const double hpg = mlc<IC>(k.neg_g * Hv, k.dx_v, k.i_dx_v) * (A(A_SN, q + SX) - snc);
     const double num =
         A(A_VN, q) * Hv +
-        dvc(k.rdt * (((adv + vis) + cor) + hpg), k.area_v, k.r_area_v, k.fast_div);
+        dvc(mlc<IC>(((adv + vis) + cor) + hpg, k.rdt, k.i_rdt), k.area_v, k.r_area_v,
+            k.fast_div);
     const double t1 = dvf(num, dhv, rhv);
     o.v = dvc(t1, k.fric, k.r_fric, k.fast_div);
   }
@@ -502,7 +524,7 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
 // the two updates that use it; for the other update the reference evaluates
 // the same operations on the same operands (addition commuted), so the bits
 // agree.  ht: the T depth at the cell.
-template <class T, bool X, bool Y>
+template <class T, bool IC, bool X, bool Y>
 __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q, double ht,
                                              const FastConst& k) {
   constexpr int S0 = T::S0, SX = T::SX;
@@ -518,12 +540,12 @@ __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q
     // dudx at T(i,j): dudx_w of u face i, dudx_e of face i-1
     B(B_GX, q) = dvc(u_c - u_w, k.dx_t, k.r_dx_t, k.fast_div) * D;
     // x-advective flux of u through T(i,j): uu_w * u_w * depw of face i
-    const double U = half(u_c + u_w) * k.dy_t;
+    const double U = mlc<IC>(half(u_c + u_w), k.dy_t, k.i_dy_t);
     B(B_FXU, q) = (upwind(U, u_c, u_w) * U) * D;
     // west edge of v face (i,j): u_wc, u_w, depw, vv_w (unmasked form)
     const double uwc = half(u_w + A(A_UN, qwn));
     B(B_UWC, q) = uwc;
-    const double Uw = half(uwc) * k.dyu2;
+    const double Uw = mlc<IC>(half(uwc), k.dyu2, k.i_dyu2);
     const double depw = half((A(A_HUS, qw) + A(A_HU, qwn)) + A(A_SU, qwn));
     B(B_FXV, q) = (upwind(Uw, v_c, v_w) * Uw) * depw;
     B(B_QX, q) = dvc(v_c - v_w, k.dxv2, k.r_dxv2, k.fast_div);
@@ -533,12 +555,12 @@ __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q
     // dvdy at T(i,j): dvdy_s of v face j, dvdy_n of face j-1
     B(B_GY, q) = dvc(v_c - v_s, k.dy_t, k.r_dy_t, k.fast_div) * D;
     // y-advective flux of v through T(i,j): vv_s * v_s * deps of face j
-    const double V = half(v_c + v_s) * k.dx_t;
+    const double V = mlc<IC>(half(v_c + v_s), k.dx_t, k.i_dx_t);
     B(B_FYV, q) = (upwind(V, v_c, v_s) * V) * D;
     // south edge of u face (i,j): v_sc, v_s, deps, uu_s (unmasked form)
     const double vsc = half(v_s + A(A_VN, qse));
     B(B_VSC, q) = vsc;
-    const double Vs = half(vsc) * k.dxv2;
+    const double Vs = mlc<IC>(half(vsc), k.dxv2, k.i_dxv2);
     const double deps = half((A(A_HVS, qs) + A(A_HV, qse)) + A(A_SV, qse));
     B(B_FYU, q) = (upwind(Vs, u_c, u_s) * Vs) * deps;
     B(B_QY, q) = dvc(u_c - u_s, k.dyu2, k.r_dyu2, k.fast_div);
@@ -554,7 +576,7 @@ __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q
 // of the tile, and the edges' extra values (next column, next row) packed
 // into warps of their own.  140 -> 123 FP64 instructions per cell against the
 // form that formed everything on a 2- and a 1-cell halo.
-template <class T>
+template <class T, bool IC>
 __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs, const Dims& d,
                                            const Scalars& p, const FastConst& k, double tide,
                                            int i0, int j0, double* smem) {
@@ -582,7 +604,7 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
     A(A_HU, t) = f.hu[c];
     A(A_HV, t) = f.hv[c];
     mk[t] = f.tmask[c];
-    B(B_AREA_SSH, t) = k.area_t * sn;
+    B(B_AREA_SSH, t) = mlc<IC>(sn, k.area_t, k.i_area_t);
   }
   double ht[T::RPT];  // of this thread's own cells, for the shared terms
 #pragma unroll
@@ -654,7 +676,7 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
   // ---- the terms shared by neighbouring updates ----
 #pragma unroll
   for (int e = 0; e < T::RPT; e++)
-    shared_terms<T, true, true>(a0, b1, (threadIdx.y + e * T::RPP + 1) * SX + threadIdx.x + 1,
+    shared_terms<T, IC, true, true>(a0, b1, (threadIdx.y + e * T::RPP + 1) * SX + threadIdx.x + 1,
                                 ht[e], k);
   // the south terms of row TY, the west terms of column TX, and the fluxes
   // through the tile's west and south edges
@@ -662,11 +684,11 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
     int e = t;
     if (e < RX) {
       if (e < TX)
-        shared_terms<T, false, true>(a0, b1, (TY + 1) * SX + e + 1,
+        shared_terms<T, IC, false, true>(a0, b1, (TY + 1) * SX + e + 1,
                                      f.ht[min(j0 + TY, H - 1) * W + min(i0 + e, W - 1)], k);
     } else if ((e -= RX) < RY) {
       if (e < TY)
-        shared_terms<T, true, false>(a0, b1, (e + 1) * SX + TX + 1,
+        shared_terms<T, IC, true, false>(a0, b1, (e + 1) * SX + TX + 1,
                                      f.ht[min(j0 + e, H - 1) * W + min(i0 + TX, W - 1)], k);
     } else if ((e -= RY) < RY) {
       const int q = (e + 1) * SX;
@@ -719,13 +741,13 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
       }
     RegOut o[NP];
     if (NP == 2 && reg[0] && reg[NP - 1]) {
-      o[0] = regular_cell<T>(a0, b1, q[0], dhu[0], rhu[0], dhv[0], rhv[0], k);
-      o[NP - 1] = regular_cell<T>(a0, b1, q[NP - 1], dhu[NP - 1], rhu[NP - 1], dhv[NP - 1],
+      o[0] = regular_cell<T, IC>(a0, b1, q[0], dhu[0], rhu[0], dhv[0], rhv[0], k);
+      o[NP - 1] = regular_cell<T, IC>(a0, b1, q[NP - 1], dhu[NP - 1], rhu[NP - 1], dhv[NP - 1],
                                   rhv[NP - 1], k);
     } else {
 #pragma unroll
       for (int e = 0; e < NP; e++)
-        if (reg[e]) o[e] = regular_cell<T>(a0, b1, q[e], dhu[e], rhu[e], dhv[e], rhv[e], k);
+        if (reg[e]) o[e] = regular_cell<T, IC>(a0, b1, q[e], dhu[e], rhu[e], dhv[e], rhv[e], k);
     }
 #pragma unroll
     for (int e = 0; e < NP; e++)
@@ -752,6 +774,18 @@ bool in_fast_range(double d) {
   return d > 0.0 && d >= 0x1p-100 && d <= 0x1p100;
 }
 
+// c as mul_const's factor (host side).
+inline IntFactor int_factor(double c) {
+  if (!in_fast_range(c)) return IntFactor{0, 0};
+  unsigned long long b;
+  memcpy(&b, &c, sizeof b);
+  const unsigned long long m = (b & 0xfffffffffffffULL) | (1ULL << 52);
+  if (m & ((1ULL << 21) - 1)) return IntFactor{0, 0};  // more than 32 significant bits
+  // the product's exponent field: x's plus c's unbiased exponent (plus the
+  // leading bit, added there); minus one for q's own leading bit
+  return IntFactor{(unsigned)(m >> 21), ((unsigned)((int)(b >> 52) - 1023) - 1u) << 20};
+}
+
 // The fast path's constants for one domain (host side).
 inline FastConst make_fast_const(const Scalars& s, const UniformMetrics& um) {
   FastConst k;
@@ -776,6 +810,16 @@ inline FastConst make_fast_const(const Scalars& s, const UniformMetrics& um) {
   k.r_dx_t = 1.0 / k.dx_t, k.r_dy_t = 1.0 / k.dy_t;
   k.r_dxv2 = 1.0 / k.dxv2, k.r_dyu2 = 1.0 / k.dyu2;
   k.r_fric = 1.0 / k.fric;
+  k.i_area_t = int_factor(k.area_t), k.i_area_u = int_factor(k.area_u);
+  k.i_area_v = int_factor(k.area_v), k.i_dx_u = int_factor(k.dx_u);
+  k.i_dx_v = int_factor(k.dx_v), k.i_dx_t = int_factor(k.dx_t);
+  k.i_dy_u = int_factor(k.dy_u), k.i_dy_v = int_factor(k.dy_v);
+  k.i_dy_t = int_factor(k.dy_t), k.i_dxv2 = int_factor(k.dxv2);
+  k.i_dyu2 = int_factor(k.dyu2), k.i_rdt = int_factor(k.rdt);
+  const IntFactor all[12] = {k.i_area_t, k.i_area_u, k.i_area_v, k.i_dx_u, k.i_dx_v, k.i_dx_t,
+                             k.i_dy_u,   k.i_dy_v,   k.i_dy_t,   k.i_dxv2, k.i_dyu2, k.i_rdt};
+  k.int_mul = 1;
+  for (const IntFactor& q : all) k.int_mul &= q.co != 0;
   return k;
 }
 
