@@ -585,8 +585,8 @@ bool do_register(void* const* ptrs, int xs, int xe, int ys, int ye, int width, i
   s.dev.sin_v = (double*)take(a8);
   s.dev.d_hu = (double*)take(a8);
   s.dev.d_hv = (double*)take(a8);
-  s.dev.r_hu = (double*)take(a8);
-  s.dev.r_hv = (double*)take(a8);
+  s.dev.r_hu = (unsigned long long*)take(a8);
+  s.dev.r_hv = (unsigned long long*)take(a8);
   for (double*& p : s.shadow) p = (double*)take(a8);
   if (!s.partials &&
       !CK(cudaMalloc(&s.partials, sizeof(double) * checksum_partials_needed())))

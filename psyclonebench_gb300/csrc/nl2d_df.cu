@@ -69,11 +69,15 @@ __global__ void __launch_bounds__(32 * WARPS, 3)
   df_march(fs, ff, d, k, d.xs - 1 + gx * MW, d.ys - 1 + gy * mr, mr);
 }
 
-// FP64 arrays split into pairs once per set-up.
+// FP64 arrays, or their elements' reciprocals (0 for depths outside the range
+// in which the step takes reciprocals), split into pairs once per set-up.
+template <bool RECIPROCAL>
 __global__ void k_split(const double* __restrict__ a, float2* __restrict__ out, long long n) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
-    const df p = from_double(a[t]);
+    double x = a[t];
+    if (RECIPROCAL) x = (x >= 0x1p-100 && x <= 0x1p100) ? 1.0 / x : 0.0;
+    const df p = from_double(x);
     out[t] = make_float2(p.hi, p.lo);
   }
 }
@@ -163,11 +167,11 @@ DfConst make_df_const(const Scalars& s, const UniformMetrics& um) {
 
 void launch_df_setup(const Fields& f, const Dims& d, const DfFields& ff, cudaStream_t st) {
   const long long n = (long long)d.width * d.height;
-  k_split<<<152 * 8, 256, 0, st>>>(f.ht, ff.ht, n);
-  k_split<<<152 * 8, 256, 0, st>>>(f.hu, ff.hu, n);
-  k_split<<<152 * 8, 256, 0, st>>>(f.hv, ff.hv, n);
-  k_split<<<152 * 8, 256, 0, st>>>(f.r_hu, ff.rhu, n);
-  k_split<<<152 * 8, 256, 0, st>>>(f.r_hv, ff.rhv, n);
+  k_split<false><<<152 * 8, 256, 0, st>>>(f.ht, ff.ht, n);
+  k_split<false><<<152 * 8, 256, 0, st>>>(f.hu, ff.hu, n);
+  k_split<false><<<152 * 8, 256, 0, st>>>(f.hv, ff.hv, n);
+  k_split<true><<<152 * 8, 256, 0, st>>>(f.d_hu, ff.rhu, n);
+  k_split<true><<<152 * 8, 256, 0, st>>>(f.d_hv, ff.rhv, n);
   k_df_flags<<<152 * 8, 256, 0, st>>>(f.tmask, d, ff.reg);
 }
 
@@ -222,8 +226,10 @@ extern "C" int nl2d_selftest_df(const double* x, long long n, float* hi, float* 
 
 namespace nl2d {
 
-void launch_df_split(const double* a, float2* out, long long n, cudaStream_t st) {
-  k_split<<<152 * 8, 256, 0, st>>>(a, out, n);
+void launch_df_split(const double* a, float2* out, long long n, bool reciprocal,
+                     cudaStream_t st) {
+  auto split = reciprocal ? k_split<true> : k_split<false>;
+  split<<<152 * 8, 256, 0, st>>>(a, out, n);
 }
 
 void launch_df_flags(const int* tmask, const Dims& d, unsigned char* reg, cudaStream_t st) {

@@ -301,7 +301,7 @@ struct Ens {
   size_t total = 0;  // packed elements
   double *sn[2] = {}, *un[2] = {}, *vn[2] = {};
   double *ht = nullptr, *hu = nullptr, *hv = nullptr, *zero = nullptr;
-  double *r_hu = nullptr, *r_hv = nullptr;
+  unsigned long long *r_hu = nullptr, *r_hv = nullptr;  // as Fields::r_hu, r_hv
   int* tmask = nullptr;
   EnsDomain* d_desc = nullptr;
   int4* d_tiles = nullptr;
@@ -368,7 +368,11 @@ void ens_free() {
     cudaFree(e.vn[b]);
     e.sn[b] = e.un[b] = e.vn[b] = nullptr;
   }
-  for (double** p : {&e.ht, &e.hu, &e.hv, &e.zero, &e.r_hu, &e.r_hv, &e.d_tides, &e.d_sums}) {
+  for (double** p : {&e.ht, &e.hu, &e.hv, &e.zero, &e.d_tides, &e.d_sums}) {
+    cudaFree(*p);
+    *p = nullptr;
+  }
+  for (unsigned long long** p : {&e.r_hu, &e.r_hv}) {
     cudaFree(*p);
     *p = nullptr;
   }
@@ -741,8 +745,8 @@ bool build_df() {
   if (!e.dfs && (!ck(cudaMalloc(&e.dfs, 5 * n * sizeof(float2))) || !ck(cudaMalloc(&e.dfreg, n))))
     return false;
   float2* pr[5] = {e.dfs, e.dfs + n, e.dfs + 2 * n, e.dfs + 3 * n, e.dfs + 4 * n};
-  const double* src[5] = {e.ht, e.hu, e.hv, e.r_hu, e.r_hv};
-  for (int a = 0; a < 5; a++) launch_df_split(src[a], pr[a], (long long)n, st);
+  const double* src[5] = {e.ht, e.hu, e.hv, e.hu, e.hv};  // the last two: 1 / (hu + ssha_u = 0)
+  for (int a = 0; a < 5; a++) launch_df_split(src[a], pr[a], (long long)n, a >= 3, st);
   if (!ck(cudaMemsetAsync(e.dfreg, 0, n, st))) return false;
   std::vector<EnsDfDomain> desc(e.ndom);
   std::vector<int4> units;
@@ -887,12 +891,11 @@ __global__ void k_import_interior(const EnsDomain* __restrict__ doms, int ndom, 
   }
 }
 
-__global__ void k_recip(const double* __restrict__ h, double* __restrict__ r, size_t n) {
+__global__ void k_recip(const double* __restrict__ h, unsigned long long* __restrict__ r,
+                        size_t n) {
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n;
-       t += (size_t)gridDim.x * blockDim.x) {
-    const double dd = h[t] + 0.0;  // ssha_u / ssha_v are zero at rest
-    r[t] = (dd >= 0x1p-100 && dd <= 0x1p100) ? 1.0 / dd : 0.0;
-  }
+       t += (size_t)gridDim.x * blockDim.x)
+    r[t] = recip64_of(h[t] + 0.0);  // ssha_u / ssha_v are zero at rest
 }
 
 }  // namespace
@@ -939,8 +942,9 @@ int nl2d_ens_create(int ndom, const int* dims6, const double* geo3, const double
     if (!ck(cudaMalloc(&e.sn[b], bytes)) || !ck(cudaMalloc(&e.un[b], bytes)) ||
         !ck(cudaMalloc(&e.vn[b], bytes)))
       return NL2D_ERR_CUDA;
-  for (double** p : {&e.ht, &e.hu, &e.hv, &e.zero, &e.r_hu, &e.r_hv})
+  for (double** p : {&e.ht, &e.hu, &e.hv, &e.zero})
     if (!ck(cudaMalloc(p, bytes))) return NL2D_ERR_CUDA;
+  if (!ck(cudaMalloc(&e.r_hu, bytes)) || !ck(cudaMalloc(&e.r_hv, bytes))) return NL2D_ERR_CUDA;
   if (!ck(cudaMalloc(&e.tmask, off * sizeof(int)))) return NL2D_ERR_CUDA;
   for (double* p : {e.sn[0], e.sn[1], e.un[0], e.un[1], e.vn[0], e.vn[1], e.zero})
     if (!ck(cudaMemset(p, 0, bytes))) return NL2D_ERR_CUDA;

@@ -6,22 +6,17 @@
 // IEEE expression it replaces, for every input, but spends fewer FP64
 // instructions:
 //
-//  * div_rn(x, d, r): x / d rounded to nearest for a divisor d > 0 whose
-//    reciprocal r = RN(1/d) was computed beforehand.  q0 = RN(x * r) is
-//    within 1.5 ulp of x / d; the exact remainder q0 * d - x, formed from
-//    the significands in 64-bit integers and compared with half an ulp of q0
-//    times d, picks the correctly rounded quotient among q0 and its two
-//    neighbours.  1 DMUL and about 20 integer instructions (the remainder by
-//    FMA cost one DFMA more, 64 issue slots of a scheduler against ~10).
-//    When q0 is a power of two (the spacing changes below it) the quotient
-//    takes Markstein's two refinements instead (Markstein, "Computation of
-//    elementary functions on the IBM RISC System/6000 processor", IBM J.
-//    Res. Dev. 34(1), 1990; Muller et al., Handbook of Floating-Point
-//    Arithmetic, 2nd ed., Sec. 4.7), 1 DMUL + 4 DFMA.
+//  * div_core / div_const / div_depth: x / d rounded to nearest for a divisor
+//    d in [2^-100, 2^100] whose 64-bit reciprocal was computed beforehand,
+//    entirely in integers (about 32 instructions, no FP64): the quotient's
+//    leading 53 bits by a multiply with the reciprocal, never above the true
+//    quotient and less than 1.01 units below it, then the exact remainder
+//    decides whether it rounds up.  (An FP64 multiply by RN(1/d) with the
+//    remainder by FMA held the FP64 pipe for two instructions, with the
+//    remainder in integers for one; IEEE division takes ~15.)
 //    x = +-0 returns x.  Dividends whose magnitude is tiny (below 2^-899,
 //    other than zero), huge (2^900 and above) or not finite use the IEEE
-//    divide, so no intermediate underflows or overflows; divisors are
-//    checked on the host to lie in [2^-100, 2^100].
+//    divide, so no result leaves the normal range.
 //  * mul_const(x, f, c): x * c for a step constant c of at most 32
 //    significant bits, in integers.
 //  * half(x): 0.5 * x.  For normal x with a biased exponent >= 2 this is
@@ -35,6 +30,8 @@
 //    non-finite partner takes the IEEE expression.
 #pragma once
 #include <cuda_runtime.h>
+
+#include <cstring>
 
 namespace nl2d {
 
@@ -62,44 +59,67 @@ static __device__ __noinline__ double div_ieee(double x, double d) { return x / 
 static __device__ __noinline__ double half_ieee(double x) { return 0.5 * x; }
 static __device__ __noinline__ double pick_ieee(double a, double z) { return a + 0.0 * z; }
 
-// Markstein's two refinements: a faithful quotient, then the correctly
-// rounded one.  Out of line: taken only when x * r lands on a power of two.
-static __device__ __noinline__ double div_markstein(double x, double d, double r) {
-  const double q0 = x * r;
-  const double e0 = fma(q0, d, -x);
-  const double q1 = fma(-e0, r, q0);
-  const double e1 = fma(q1, d, -x);
-  return fma(-e1, r, q1);
+// floor((2^116 - 1) / md) for md in [2^52, 2^53): the 64-bit reciprocal of
+// the divisor whose significand md is.
+__host__ __device__ __forceinline__ unsigned long long recip64(unsigned long long md) {
+  const unsigned __int128 n = ((unsigned __int128)1 << 116) - 1;
+  return (unsigned long long)(n / md);
 }
 
-__device__ __forceinline__ double div_rn(double x, double d, double r) {
+__host__ __device__ __forceinline__ unsigned long long recip64_of(double d) {
+  if (!(d >= 0x1p-100 && d <= 0x1p100)) return 0;
+  unsigned long long b;
+  memcpy(&b, &d, sizeof b);
+  return recip64((b & 0xfffffffffffffULL) | (1ULL << 52));
+}
+
+// The quotient's bits for a dividend of biased exponent 124 .. 1922 (bits
+// xb), the divisor's significand md, its reciprocal rc and what the
+// quotient's exponent field gains, `add` = (1023 - the divisor's biased
+// exponent - 2) << 20.  With mx the dividend's significand, t = hi64(2^11 mx
+// rc) is mx / md 2^63 to within 4 units below (the low partial product is
+// left out): its leading bit says whether mx >= md, and q, its top 53 bits,
+// is less than 1.01 below the quotient mx 2^s / md (s = 52 or 53).  The
+// remainder mx 2^s - q md is below 2^54, so its low 64 bits are all of it,
+// and q rounds up exactly when it is above md / 2 (a quotient of two
+// significands is never a midpoint).
+__device__ __forceinline__ double div_core(unsigned long long xb, unsigned long long md,
+                                           unsigned long long rc, unsigned add) {
+  const unsigned xl = (unsigned)xb, xh = (unsigned)(xb >> 32);
+  const unsigned rl = (unsigned)rc, rh = (unsigned)(rc >> 32);
+  const unsigned ah = __funnelshift_l(xl, xh, 11) | 0x80000000u, al = xl << 11;
+  const unsigned long long t = (unsigned long long)ah * rh + __umulhi(ah, rl) + __umulhi(al, rh);
+  const unsigned top = (unsigned)(t >> 32) >> 31;
+  unsigned long long q = t >> (10 + top);
+  const unsigned long long rem = ((unsigned long long)(xl << (21 - top)) << 32) - q * md;
+  if ((long long)rem > (long long)(md >> 1)) q++;
+  const unsigned eh = (xh & 0xfff00000u) + add + (top << 20);
+  return from_bits((long long)(q + ((unsigned long long)eh << 32)));
+}
+
+// A step constant as a divisor.
+struct IntDivisor {
+  double d;
+  unsigned long long md, rc;
+  unsigned add;
+};
+__device__ __forceinline__ double div_const(double x, const IntDivisor& v) {
   const unsigned long long xb = (unsigned long long)bits(x);
-  const unsigned xh = (unsigned)(xb >> 32);
-  const int ex = (int)((xh >> 20) & 0x7ff);
-  if (ex < 124 || ex > 1922) {
+  if (((unsigned)(xb >> 52) & 0x7ffu) - 124u > 1798u) {
     if ((xb & 0x7fffffffffffffffULL) == 0) return x;  // +-0 / d keeps the sign for d > 0
+    return div_ieee(x, v.d);
+  }
+  return div_core(xb, v.md, v.rc, v.add);
+}
+// The same for a divisor from an array, with its reciprocal rc (not 0).
+__device__ __forceinline__ double div_depth(double x, double d, unsigned long long rc) {
+  const unsigned long long xb = (unsigned long long)bits(x), db = (unsigned long long)bits(d);
+  if (((unsigned)(xb >> 52) & 0x7ffu) - 124u > 1798u) {
+    if ((xb & 0x7fffffffffffffffULL) == 0) return x;
     return div_ieee(x, d);
   }
-  const double q0 = x * r;
-  const unsigned long long qb = (unsigned long long)bits(q0), db = (unsigned long long)bits(d);
-  constexpr unsigned long long kFrac = 0xfffffffffffffULL, kOne = 1ULL << 52;
-  if ((qb & kFrac) == 0) return div_markstein(x, d, r);
-  // q0 is not a power of two, so q = x / d lies in q0's binade and within
-  // 1.5 ulp of it: RN(q) is q0 - ulp, q0 or q0 + ulp.  With the significands
-  // mq, md, mx as integers, q0 * d - x = 2^t (mq md - mx 2^s) for the s of
-  // the three exponents (52 or 53 here), and RN(q) moves off q0 exactly when
-  // |mq md - mx 2^s| > md / 2 (a quotient is never a midpoint).  That
-  // difference is below 1.5 md + 1 < 2^55 in size, so its low 64 bits are
-  // all of it: of mx 2^s only the low bits of x count.
-  const unsigned long long mq = (qb & kFrac) | kOne, md = (db & kFrac) | kOne;
-  const unsigned sh = ((xh >> 20) - ((unsigned)(qb >> 32) >> 20) - (unsigned)(db >> 52) +
-                       (1075u - 32u)) & 31u;  // s - 32
-  const unsigned long long rem =
-      mq * md - ((unsigned long long)((unsigned)xb << sh) << 32);
-  // +1: one ulp up in magnitude (the remainder is negative), -1: one down
-  long long k = 0;
-  if (rem + (md >> 1) > (md & ~1ULL)) k = (long long)rem < 0 ? 1 : -1;
-  return from_bits((long long)qb + k);
+  return div_core(xb, (db & 0xfffffffffffffULL) | (1ULL << 52), rc,
+                  (1021u << 20) - ((unsigned)(db >> 32) & 0x7ff00000u));
 }
 
 // A constant factor c > 0 in [2^-100, 2^100] of at most 32 significant bits

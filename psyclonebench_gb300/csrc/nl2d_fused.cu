@@ -146,16 +146,16 @@ void launch_fused_step(const Fields& f, const FusedState& fs, const Dims& d,
 
 namespace {
 
-// The momentum denominators h + ssha and their reciprocals, 0 where the
-// depth lies outside [2^-100, 2^100] (the kernel then divides).
+// The momentum denominators h + ssha and their 64-bit reciprocals, 0 where
+// the depth lies outside [2^-100, 2^100] (the kernel then divides).
 __global__ void k_depth_reciprocal(const double* __restrict__ h,
                                    const double* __restrict__ ssha, double* __restrict__ dh,
-                                   double* __restrict__ r, long long n) {
+                                   unsigned long long* __restrict__ r, long long n) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     const double dd = h[t] + ssha[t];
     dh[t] = dd;
-    r[t] = (dd >= 0x1p-100 && dd <= 0x1p100) ? 1.0 / dd : 0.0;
+    r[t] = recip64_of(dd);
   }
 }
 
@@ -196,16 +196,23 @@ __device__ __forceinline__ double sample(unsigned long long z) {
   return from_bits(b | (ex << 52));
 }
 
-__global__ void k_selftest_exact(long long n, unsigned long long seed, double d, double r,
-                                 unsigned long long* bad) {
+__global__ void k_selftest_exact(long long n, unsigned long long seed, IntDivisor v,
+                                 IntFactor fac, unsigned long long* bad) {
+  const double d = v.d;
   unsigned long long nd = 0, nh = 0, nu = 0;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     const unsigned long long z = mix64(seed ^ (unsigned long long)t);
     const double x = sample(z);
     // division: finite quotients must agree bit for bit
-    const double q_ref = x / d, q = div_rn(x, d, r);
-    if (bits(q_ref) != bits(q) && !(q_ref != q_ref && q != q)) nd++;
+    const double q_ref = x / d;
+    for (const double q : {div_const(x, v), div_depth(x, d, v.rc)})
+      if (bits(q_ref) != bits(q) && !(q_ref != q_ref && q != q)) nd++;
+    // the product with d (counted with the quotients), where d has that form
+    if (fac.co != 0) {
+      const double p_ref = x * d, p = mul_const(x, fac, d);
+      if (bits(p_ref) != bits(p) && !(p_ref != p_ref && p != p)) nd++;
+    }
     // Quotients within ~2^-53 ulp of a midpoint: RN((Q + ulp(Q)/2) * d) and
     // its neighbours; quotients at and next to a power of two.
     {
@@ -219,8 +226,9 @@ __global__ void k_selftest_exact(long long n, unsigned long long seed, double d,
       const long long nudge = (long long)((y >> 32) & 7) - 3;
       const double cand[3] = {xm, from_bits(bits(xm) + nudge), from_bits(bits(Q * d) + nudge)};
       for (int c = 0; c < 3; c++) {
-        const double xr = cand[c] / d, xq = div_rn(cand[c], d, r);
-        if (bits(xr) != bits(xq)) nd++;
+        const double xr = cand[c] / d;
+        if (bits(xr) != bits(div_const(cand[c], v))) nd++;
+        if (bits(xr) != bits(div_depth(cand[c], d, v.rc))) nd++;
       }
     }
     const double h_ref = 0.5 * x, h = half(x);
@@ -306,7 +314,8 @@ extern "C" int nl2d_selftest_intfp(long long n, unsigned long long seed, long lo
 
 // Test hook (no reference counterpart): counts, over n sampled doubles x,
 // the inputs where the exact helpers of the fused step differ from the IEEE
-// expressions they replace: x / d, 0.5 * x and the upwind pick.  d must be
+// expressions they replace: x / d (and x * d, for a d of at most 32
+// significant bits), 0.5 * x and the upwind pick.  d must be
 // in [2^-100, 2^100].  out[3] receives the three mismatch counts.
 extern "C" int nl2d_selftest_exact(long long n, unsigned long long seed, double d,
                                    long long* out) {
@@ -314,7 +323,8 @@ extern "C" int nl2d_selftest_exact(long long n, unsigned long long seed, double 
   if (!(d >= 0x1p-100 && d <= 0x1p100)) return 2;
   if (cudaMalloc(&bad, 3 * sizeof(unsigned long long)) != cudaSuccess) return 1;
   cudaMemset(bad, 0, 3 * sizeof(unsigned long long));
-  nl2d::k_selftest_exact<<<152 * 16, 256>>>(n, seed, d, 1.0 / d, bad);
+  nl2d::k_selftest_exact<<<152 * 16, 256>>>(n, seed, nl2d::int_divisor(d), nl2d::int_factor(d),
+                                             bad);
   unsigned long long h[3] = {0, 0, 0};
   const cudaError_t e = cudaMemcpy(h, bad, sizeof h, cudaMemcpyDeviceToHost);
   cudaFree(bad);

@@ -28,12 +28,13 @@ constexpr int NTHREADS = 256;
 // uniform grid is one add of two equal values), so they are bit-identical.
 struct FastConst {
   double area_t, area_u, area_v, dx_u, dx_v, dx_t, dy_u, dy_v, dy_t;
-  double r_area_t, r_area_u, r_area_v, r_dx_t, r_dy_t;  // RN(1/d)
-  double dxv2, dyu2, r_dxv2, r_dyu2;                    // dx_v + dx_v, dy_u + dy_u
-  double fric, r_fric;                                  // 1.0 + cbfr * rdt
-  double cor_u, cor_v;                                  // 2. * omega * sin(gphi * d2r)
+  double dxv2, dyu2;                       // dx_v + dx_v, dy_u + dy_u
+  double cor_u, cor_v;                     // 2. * omega * sin(gphi * d2r)
   double neg_g, rdt, visc, g;
-  int fast_div;  // every constant divisor lies in [2^-100, 2^100]
+  // the constant divisors (fric: 1.0 + cbfr * rdt), and whether every one
+  // lies in [2^-100, 2^100]
+  IntDivisor q_area_t, q_area_u, q_area_v, q_dx_t, q_dy_t, q_dxv2, q_dyu2, q_fric;
+  int fast_div;
   // the grid's and the time step's constants as integer factors (mul_const),
   // and whether all of them have that form
   IntFactor i_area_t, i_area_u, i_area_v, i_dx_u, i_dx_v, i_dx_t, i_dy_u, i_dy_v, i_dy_t;
@@ -58,15 +59,15 @@ __device__ __forceinline__ double mlc(double x, double kc, IntFactor ic) {
   return IC ? mul_const(x, ic, kc) : x * kc;
 }
 
-// Division by a step constant: the Markstein form when the constants allow
-// it, otherwise the IEEE divide.  Both give the same bits.
-__device__ __forceinline__ double dvc(double x, double d, double r, int fast) {
-  return fast ? div_rn(x, d, r) : div_ieee(x, d);
+// Division by a step constant: in integers when the constants allow it,
+// otherwise the IEEE divide.  Both give the same bits.
+__device__ __forceinline__ double dvc(double x, const IntDivisor& v, int fast) {
+  return fast ? div_const(x, v) : div_ieee(x, v.d);
 }
-// Division by a per-face depth with a precomputed reciprocal; r == 0 marks
-// a depth outside [2^-100, 2^100] (IEEE divide).
-__device__ __forceinline__ double dvf(double x, double d, double r) {
-  return bits(r) != 0 ? div_rn(x, d, r) : div_ieee(x, d);
+// Division by a per-face depth with its 64-bit reciprocal; 0 marks a depth
+// outside [2^-100, 2^100] (IEEE divide).
+__device__ __forceinline__ double dvf(double x, double d, unsigned long long rc) {
+  return rc != 0 ? div_depth(x, d, rc) : div_ieee(x, d);
 }
 
 // The general code's context: every input read from the domain's arrays in
@@ -82,8 +83,8 @@ struct GlobalCtx {
   double* const& ht;
   double* const& ssha_u;
   double* const& ssha_v;
-  double* const& r_hu;
-  double* const& r_hv;
+  unsigned long long* const& r_hu;
+  unsigned long long* const& r_hv;
   int* const& m;
   double* const& sshn_u;
   double* const& sshn_v;
@@ -102,13 +103,13 @@ struct GlobalCtx {
   // dependent loads and FP64 operations, and its length is what it costs.
   __device__ __forceinline__ double face_u(int i, int j, int mm, int mn, double a, double b,
                                            double pa, double pb, double stored) const {
-    const double both = dvc(half(pa + pb), k.area_u, k.r_area_u, k.fast_div);
+    const double both = dvc(half(pa + pb), k.q_area_u, k.fast_div);
     const bool in = j >= d.ys && j <= d.ye && i >= d.xs && i <= d.xe - 1 && mm + mn > 0;
     return !in ? stored : (mm * mn > 0 ? both : (mm <= 0 ? b : a));
   }
   __device__ __forceinline__ double face_v(int i, int j, int mm, int mn, double a, double b,
                                            double pa, double pb, double stored) const {
-    const double both = dvc(half(pa + pb), k.area_v, k.r_area_v, k.fast_div);
+    const double both = dvc(half(pa + pb), k.q_area_v, k.fast_div);
     const bool in = j >= d.ys && j <= d.ye - 1 && i >= d.xs && i <= d.xe && mm + mn > 0;
     return !in ? stored : (mm * mn > 0 ? both : (mm <= 0 ? b : a));
   }
@@ -163,7 +164,8 @@ __device__ __forceinline__ bool mom_u(const X& x, int i, int j, double& out) {
   const double v_C = x.vn[c], v_E = x.vn[e], v_S = x.vn[s], v_SE = x.vn[se];
   const double hu_c = x.hu[c], hu_s = x.hu[s], hu_n = x.hu[n];
   const double hv_c = x.hv[c], hv_e = x.hv[e], hv_s = x.hv[s], hv_se = x.hv[se];
-  const double ht_c = x.ht[c], ht_e = x.ht[e], ssha = x.ssha_u[c], rhu = x.r_hu[c];
+  const double ht_c = x.ht[c], ht_e = x.ht[e], ssha = x.ssha_u[c];
+  const unsigned long long rhu = x.r_hu[c];
   if (m_c + m_e <= 0) return false;
   if (m_c <= 0 || m_e <= 0) return false;
   const double p_c = k.area_t * sn_c, p_e = k.area_t * sn_e, p_s = k.area_t * sn_s,
@@ -196,22 +198,21 @@ __device__ __forceinline__ bool mom_u(const X& x, int i, int j, double& out) {
   double adv = uu_w * u_w * depw - uu_e * u_e * depe + uu_s * v_s * deps -
                uu_n * v_n * depn;
 
-  double dudx_e = dvc(u_E - u_c, k.dx_t, k.r_dx_t, k.fast_div) * depe;
-  double dudx_w = dvc(u_c - u_W, k.dx_t, k.r_dx_t, k.fast_div) * depw;
+  double dudx_e = dvc(u_E - u_c, k.q_dx_t, k.fast_div) * depe;
+  double dudx_w = dvc(u_c - u_W, k.q_dx_t, k.fast_div) * depw;
   double dudy_s = south_dry ? 0.0
-                            : dvc(u_c - u_S, k.dyu2, k.r_dyu2, k.fast_div) *
+                            : dvc(u_c - u_S, k.q_dyu2, k.fast_div) *
                                   (hu_c + su_c + hu_s + su_s);
   double dudy_n = north_dry ? 0.0
-                            : dvc(u_N - u_c, k.dyu2, k.r_dyu2, k.fast_div) *
+                            : dvc(u_N - u_c, k.q_dyu2, k.fast_div) *
                                   (hu_c + su_c + hu_n + su_n);
   double vis = (dudx_e - dudx_w) * k.dy_u + half((dudy_n - dudy_s) * k.dx_u);
   vis = k.visc * vis;
   double cor = half(k.cor_u * (v_sc + v_nc)) * k.area_u * (hu_c + su_c);
   double hpg = k.neg_g * (hu_c + su_c) * k.dy_u * (sn_e - sn_c);
   const double num =
-      u_c * (hu_c + su_c) + dvc(k.rdt * (adv + vis + cor + hpg), k.area_u, k.r_area_u,
-                                k.fast_div);
-  out = dvc(dvf(num, hu_c + ssha, rhu), k.fric, k.r_fric, k.fast_div);
+      u_c * (hu_c + su_c) + dvc(k.rdt * (adv + vis + cor + hpg), k.q_area_u, k.fast_div);
+  out = dvc(dvf(num, hu_c + ssha, rhu), k.q_fric, k.fast_div);
   return true;
 }
 
@@ -232,7 +233,8 @@ __device__ __forceinline__ bool mom_v(const X& x, int i, int j, double& out) {
   const double u_C = x.un[c], u_N = x.un[n], u_W = x.un[wst], u_NW = x.un[nw];
   const double hv_c = x.hv[c], hv_w = x.hv[wst], hv_e = x.hv[e];
   const double hu_c = x.hu[c], hu_n = x.hu[n], hu_w = x.hu[wst], hu_nw = x.hu[nw];
-  const double ht_c = x.ht[c], ht_n = x.ht[n], ssha = x.ssha_v[c], rhv = x.r_hv[c];
+  const double ht_c = x.ht[c], ht_n = x.ht[n], ssha = x.ssha_v[c];
+  const unsigned long long rhv = x.r_hv[c];
   if (m_c + m_e <= 0) return false;
   if (m_c <= 0 || m_n <= 0) return false;
   const double p_c = k.area_t * sn_c, p_e = k.area_t * sn_e, p_w = k.area_t * sn_w,
@@ -265,22 +267,21 @@ __device__ __forceinline__ bool mom_v(const X& x, int i, int j, double& out) {
   double adv = vv_w * u_w * depw - vv_e * u_e * depe + vv_s * v_s * deps -
                vv_n * v_n * depn;
 
-  double dvdy_n = dvc(v_N - v_c, k.dy_t, k.r_dy_t, k.fast_div) * depn;
-  double dvdy_s = dvc(v_c - v_S, k.dy_t, k.r_dy_t, k.fast_div) * deps;
+  double dvdy_n = dvc(v_N - v_c, k.q_dy_t, k.fast_div) * depn;
+  double dvdy_s = dvc(v_c - v_S, k.q_dy_t, k.fast_div) * deps;
   double dvdx_w = west_dry ? 0.0
-                           : dvc(v_c - v_W, k.dxv2, k.r_dxv2, k.fast_div) *
+                           : dvc(v_c - v_W, k.q_dxv2, k.fast_div) *
                                  (hv_c + sv_c + hv_w + sv_w);
   double dvdx_e = east_dry ? 0.0
-                           : dvc(v_E - v_c, k.dxv2, k.r_dxv2, k.fast_div) *
+                           : dvc(v_E - v_c, k.q_dxv2, k.fast_div) *
                                  (hv_c + sv_c + hv_e + sv_e);
   double vis = (dvdy_n - dvdy_s) * k.dx_v + half((dvdx_e - dvdx_w) * k.dy_v);
   vis = k.visc * vis;
   double cor = -half(k.cor_v * (u_ec + u_wc)) * k.area_v * (hv_c + sv_c);
   double hpg = k.neg_g * (hv_c + sv_c) * k.dx_v * (sn_n - sn_c);
   const double num =
-      v_c * (hv_c + sv_c) + dvc(k.rdt * (adv + vis + cor + hpg), k.area_v, k.r_area_v,
-                                k.fast_div);
-  out = dvc(dvf(num, hv_c + ssha, rhv), k.fric, k.r_fric, k.fast_div);
+      v_c * (hv_c + sv_c) + dvc(k.rdt * (adv + vis + cor + hpg), k.q_area_v, k.fast_div);
+  out = dvc(dvf(num, hv_c + ssha, rhv), k.q_fric, k.fast_div);
   return true;
 }
 
@@ -343,7 +344,7 @@ __device__ __forceinline__ void general_part(const X& x, const Fields& f, const 
       double r2 = (x.su(i - 1, j) + f.hu[w]) * x.un[w];
       double r3 = (x.sv(i, j) + f.hv[c]) * x.vn[c];
       double r4 = (x.sv(i, j - 1) + f.hv[s]) * x.vn[s];
-      ssh = x.sn[c] + dvc((r2 - r1 + r4 - r3) * k.rdt, k.area_t, k.r_area_t, k.fast_div);
+      ssh = x.sn[c] + dvc((r2 - r1 + r4 - r3) * k.rdt, k.q_area_t, k.fast_div);
       if (m[c] > 0 && (m[c - W] < 0 || m[c + W] < 0 || m[c + 1] < 0 || m[c - 1] < 0))
         ssh = tide;
     }
@@ -462,14 +463,14 @@ using DefaultTile = Tile<32, 16>;
 // and shared terms (b1) at its slot q: continuity (continuity_kern.c:90-117)
 // and unmasked momentum (momentum_u_kern.c:184-261,
 // momentum_v_kern.c:159-239) in the reference's operation order.  dhu, rhu,
-// dhv, rhv: hu + ssha_u and hv + ssha_v at the cell and their reciprocals.
+// dhv, rhv: hu + ssha_u and hv + ssha_v at the cell and their reciprocals (dvf).
 struct RegOut {
   double ssh, u, v;
 };
 template <class T, bool IC>
 __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b1, int q,
-                                               double dhu, double rhu, double dhv, double rhv,
-                                               const FastConst& k) {
+                                               double dhu, unsigned long long rhu, double dhv,
+                                               unsigned long long rhv, const FastConst& k) {
   constexpr int S0 = T::S0, SX = T::SX;
 #define A(qq, t) a0[(qq) * S0 + (t)]
 #define B(qq, t) b1[(qq) * S0 + (t)]
@@ -477,7 +478,7 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
   const double snc = A(A_SN, q), Hu = A(A_HUS, q), Hv = A(A_HVS, q);
   const double ssh = mlc<IC>(
       ((B(B_FLXU, q - 1) - B(B_FLXU, q)) + B(B_FLXV, q - SX)) - B(B_FLXV, q), k.rdt, k.i_rdt);
-  o.ssh = snc + dvc(ssh, k.area_t, k.r_area_t, k.fast_div);
+  o.ssh = snc + dvc(ssh, k.q_area_t, k.fast_div);
   {
     const double adv = ((B(B_FXU, q) - B(B_FXU, q + 1)) + B(B_FYU, q)) - B(B_FYU, q + SX);
     const double dudy_s = B(B_QY, q) * ((Hu + A(A_HU, q - SX)) + A(A_SU, q - SX));
@@ -491,10 +492,9 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
     const double hpg = mlc<IC>(k.neg_g * Hu, k.dy_u, k.i_dy_u) * (A(A_SN, q + 1) - snc);
     const double num =
         A(A_UN, q) * Hu +
-        dvc(mlc<IC>(((adv + vis) + cor) + hpg, k.rdt, k.i_rdt), k.area_u, k.r_area_u,
-            k.fast_div);
+        dvc(mlc<IC>(((adv + vis) + cor) + hpg, k.rdt, k.i_rdt), k.q_area_u, k.fast_div);
     const double t1 = dvf(num, dhu, rhu);
-    o.u = dvc(t1, k.fric, k.r_fric, k.fast_div);
+    o.u = dvc(t1, k.q_fric, k.fast_div);
   }
   {
     const double adv = ((B(B_FXV, q) - B(B_FXV, q + 1)) + B(B_FYV, q)) - B(B_FYV, q + SX);
@@ -509,10 +509,9 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
     const double hpg = mlc<IC>(k.neg_g * Hv, k.dx_v, k.i_dx_v) * (A(A_SN, q + SX) - snc);
     const double num =
         A(A_VN, q) * Hv +
-        dvc(mlc<IC>(((adv + vis) + cor) + hpg, k.rdt, k.i_rdt), k.area_v, k.r_area_v,
-            k.fast_div);
+        dvc(mlc<IC>(((adv + vis) + cor) + hpg, k.rdt, k.i_rdt), k.q_area_v, k.fast_div);
     const double t1 = dvf(num, dhv, rhv);
-    o.v = dvc(t1, k.fric, k.r_fric, k.fast_div);
+    o.v = dvc(t1, k.q_fric, k.fast_div);
   }
   return o;
 }
@@ -538,7 +537,7 @@ __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q
   if (X) {
     const double u_w = A(A_UN, qw), v_w = A(A_VN, qw);
     // dudx at T(i,j): dudx_w of u face i, dudx_e of face i-1
-    B(B_GX, q) = dvc(u_c - u_w, k.dx_t, k.r_dx_t, k.fast_div) * D;
+    B(B_GX, q) = dvc(u_c - u_w, k.q_dx_t, k.fast_div) * D;
     // x-advective flux of u through T(i,j): uu_w * u_w * depw of face i
     const double U = mlc<IC>(half(u_c + u_w), k.dy_t, k.i_dy_t);
     B(B_FXU, q) = (upwind(U, u_c, u_w) * U) * D;
@@ -548,12 +547,12 @@ __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q
     const double Uw = mlc<IC>(half(uwc), k.dyu2, k.i_dyu2);
     const double depw = half((A(A_HUS, qw) + A(A_HU, qwn)) + A(A_SU, qwn));
     B(B_FXV, q) = (upwind(Uw, v_c, v_w) * Uw) * depw;
-    B(B_QX, q) = dvc(v_c - v_w, k.dxv2, k.r_dxv2, k.fast_div);
+    B(B_QX, q) = dvc(v_c - v_w, k.q_dxv2, k.fast_div);
   }
   if (Y) {
     const double u_s = A(A_UN, qs), v_s = A(A_VN, qs);
     // dvdy at T(i,j): dvdy_s of v face j, dvdy_n of face j-1
-    B(B_GY, q) = dvc(v_c - v_s, k.dy_t, k.r_dy_t, k.fast_div) * D;
+    B(B_GY, q) = dvc(v_c - v_s, k.q_dy_t, k.fast_div) * D;
     // y-advective flux of v through T(i,j): vv_s * v_s * deps of face j
     const double V = mlc<IC>(half(v_c + v_s), k.dx_t, k.i_dx_t);
     B(B_FYV, q) = (upwind(V, v_c, v_s) * V) * D;
@@ -563,7 +562,7 @@ __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q
     const double Vs = mlc<IC>(half(vsc), k.dxv2, k.i_dxv2);
     const double deps = half((A(A_HVS, qs) + A(A_HV, qse)) + A(A_SV, qse));
     B(B_FYU, q) = (upwind(Vs, u_c, u_s) * Vs) * deps;
-    B(B_QY, q) = dvc(u_c - u_s, k.dyu2, k.r_dyu2, k.fast_div);
+    B(B_QY, q) = dvc(u_c - u_s, k.q_dyu2, k.fast_div);
   }
 }
 
@@ -621,8 +620,7 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
     const int mm = mk[q], mn = mk[q + 1];
     if (fj <= d.ye && fi <= d.xe - 1 && mm + mn > 0) {
       if (mm * mn > 0)
-        su = dvc(half(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + 1)), k.area_u, k.r_area_u,
-                 k.fast_div);
+        su = dvc(half(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + 1)), k.q_area_u, k.fast_div);
       else
         su = mm <= 0 ? A(A_SN, q + 1) : A(A_SN, q);
     } else {
@@ -637,8 +635,7 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
     const int mm = mk[q], mn = mk[q + SX];
     if (fj <= d.ye - 1 && fi <= d.xe && mm + mn > 0) {
       if (mm * mn > 0)
-        sv = dvc(half(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + SX)), k.area_v, k.r_area_v,
-                 k.fast_div);
+        sv = dvc(half(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + SX)), k.q_area_v, k.fast_div);
       else
         sv = mm <= 0 ? A(A_SN, q + SX) : A(A_SN, q);
     } else {
@@ -730,7 +727,8 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
       reg[e] = regular;
       if (live && !regular) glist[atomicAdd(gcount, 1)] = row * TX + threadIdx.x;
     }
-    double dhu[NP], rhu[NP], dhv[NP], rhv[NP];
+    double dhu[NP], dhv[NP];
+    unsigned long long rhu[NP], rhv[NP];
 #pragma unroll
     for (int e = 0; e < NP; e++)
       if (reg[e]) {
@@ -786,6 +784,14 @@ inline IntFactor int_factor(double c) {
   return IntFactor{(unsigned)(m >> 21), ((unsigned)((int)(b >> 52) - 1023) - 1u) << 20};
 }
 
+// d as div_const's divisor (host side).
+inline IntDivisor int_divisor(double d) {
+  unsigned long long b;
+  memcpy(&b, &d, sizeof b);
+  const unsigned long long md = (b & 0xfffffffffffffULL) | (1ULL << 52);
+  return IntDivisor{d, md, recip64(md), (unsigned)(1021 - (int)(b >> 52 & 0x7ff)) << 20};
+}
+
 // The fast path's constants for one domain (host side).
 inline FastConst make_fast_const(const Scalars& s, const UniformMetrics& um) {
   FastConst k;
@@ -794,22 +800,22 @@ inline FastConst make_fast_const(const Scalars& s, const UniformMetrics& um) {
   k.dy_u = um.dy_u, k.dy_v = um.dy_v, k.dy_t = um.dy_t;
   k.dxv2 = um.dx_v + um.dx_v;
   k.dyu2 = um.dy_u + um.dy_u;
-  k.fric = 1.0 + s.cbfr * s.rdt;
   k.cor_u = 2. * s.omega * um.sin_u;
   k.cor_v = 2. * s.omega * um.sin_v;
   k.neg_g = -s.g;
   k.g = s.g;
   k.rdt = s.rdt;
   k.visc = s.visc;
+  const double fric = 1.0 + s.cbfr * s.rdt;
   const double divisors[8] = {k.area_t, k.area_u, k.area_v, k.dx_t, k.dy_t,
-                              k.dxv2,   k.dyu2,   k.fric};
+                              k.dxv2,   k.dyu2,   fric};
   bool fast = true;
   for (double v : divisors) fast = fast && in_fast_range(v);
   k.fast_div = fast ? 1 : 0;
-  k.r_area_t = 1.0 / k.area_t, k.r_area_u = 1.0 / k.area_u, k.r_area_v = 1.0 / k.area_v;
-  k.r_dx_t = 1.0 / k.dx_t, k.r_dy_t = 1.0 / k.dy_t;
-  k.r_dxv2 = 1.0 / k.dxv2, k.r_dyu2 = 1.0 / k.dyu2;
-  k.r_fric = 1.0 / k.fric;
+  k.q_area_t = int_divisor(k.area_t), k.q_area_u = int_divisor(k.area_u);
+  k.q_area_v = int_divisor(k.area_v), k.q_dx_t = int_divisor(k.dx_t);
+  k.q_dy_t = int_divisor(k.dy_t), k.q_dxv2 = int_divisor(k.dxv2);
+  k.q_dyu2 = int_divisor(k.dyu2), k.q_fric = int_divisor(fric);
   k.i_area_t = int_factor(k.area_t), k.i_area_u = int_factor(k.area_u);
   k.i_area_v = int_factor(k.area_v), k.i_dx_u = int_factor(k.dx_u);
   k.i_dx_v = int_factor(k.dx_v), k.i_dx_t = int_factor(k.dx_t);

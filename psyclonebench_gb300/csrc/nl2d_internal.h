@@ -33,10 +33,11 @@ struct Fields {
   double *area_t, *area_u, *area_v, *dx_u, *dx_v, *dx_t, *dy_u, *dy_v, *dy_t,
       *gphiu, *gphiv;
   double *sin_u, *sin_v;
-  // hu + ssha_u and hv + ssha_v (no step writes either operand) and RN(1 /
-  // them) (0 where out of the range the exact reciprocal division needs), for
-  // the fused step's regular cells.
-  double *d_hu, *d_hv, *r_hu, *r_hv;
+  // hu + ssha_u and hv + ssha_v (no step writes either operand) and their
+  // 64-bit reciprocals (recip64 of the significand; 0 where the value lies
+  // outside [2^-100, 2^100]), for the fused step.
+  double *d_hu, *d_hv;
+  unsigned long long *r_hu, *r_hv;
 };
 
 struct Dims {
@@ -131,9 +132,11 @@ void launch_df_ring(const Dims& d, const DfFields& ff, cudaStream_t st);
 void launch_df_step(const Fields& f, const FusedState& fs, const Dims& d, const Scalars& s,
                     const UniformMetrics& um, const DfFields& ff, double tide,
                     const double* tide_table, int tide_index, cudaStream_t st);
-// Split of one packed FP64 array into (hi, lo) pairs; the march flags of one
-// domain (tmask and reg point at the domain's first element).
-void launch_df_split(const double* a, float2* out, long long n, cudaStream_t st);
+// Split of one packed FP64 array into (hi, lo) pairs, or of its elements'
+// reciprocals (0 outside [2^-100, 2^100]); the march flags of one domain
+// (tmask and reg point at the domain's first element).
+void launch_df_split(const double* a, float2* out, long long n, bool reciprocal,
+                     cudaStream_t st);
 void launch_df_flags(const int* tmask, const Dims& d, unsigned char* reg, cudaStream_t st);
 
 // Recomputes Fields::d_hu / r_hu / d_hv / r_hv from hu, ssha_u, hv, ssha_v (array rows
