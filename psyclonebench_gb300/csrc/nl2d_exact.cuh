@@ -17,8 +17,8 @@
 //    x = +-0 returns x.  Dividends whose magnitude is tiny (below 2^-899,
 //    other than zero), huge (2^900 and above) or not finite use the IEEE
 //    divide, so no result leaves the normal range.
-//  * mul_const(x, f, c): x * c for a step constant c of at most 32
-//    significant bits, in integers.
+//  * mul_core: x * c for a step constant c of at most 32 significant bits,
+//    in integers.
 //  * half(x): 0.5 * x.  For normal x with a biased exponent >= 2 this is
 //    exact, i.e. the exponent minus one, done in integer arithmetic; zero
 //    keeps its bits; subnormal, smallest-normal and non-finite x use DMUL.
@@ -124,25 +124,19 @@ __device__ __forceinline__ double div_depth(double x, double d, unsigned long lo
 
 // A constant factor c > 0 in [2^-100, 2^100] of at most 32 significant bits
 // (grid spacings and time steps in whole or simply fractional units), as
-// mul_const takes it: co 2^e with co in [2^31, 2^32), and what the product's
+// mul_core takes it: co 2^e with co in [2^31, 2^32), and what the product's
 // exponent field gains.  co = 0: c is not of that kind.
 struct IntFactor {
   unsigned co, add;
 };
 
 // RN(x * c) in integers: the product of the significands (85 bits) is exact
-// in three words, normalised by its leading bit and rounded to nearest even.
-// Magnitudes of x below 2^-899 or from 2^900 take the IEEE product, +-0
-// itself.  About 20 instructions on the integer pipes, where the DMUL holds
-// a scheduler's share of the FP64 pipe for 64 issue slots.
-static __device__ __noinline__ double mul_ieee(double x, double c) { return x * c; }
-__device__ __forceinline__ double mul_const(double x, IntFactor f, double c) {
-  const unsigned long long b = (unsigned long long)bits(x);
-  const unsigned xl = (unsigned)b, xh = (unsigned)(b >> 32);
-  if (((xh >> 20) & 0x7ffu) - 124u > 1798u) {
-    if ((b & 0x7fffffffffffffffULL) == 0) return x;
-    return mul_ieee(x, c);
-  }
+// in three words, normalised by its leading bit and rounded to nearest even;
+// about 20 instructions on the integer pipes, where the DMUL holds a
+// scheduler's share of the FP64 pipe for 64 issue slots.  x normal, the
+// product too.
+__device__ __forceinline__ double mul_core(unsigned long long xb, IntFactor f) {
+  const unsigned xl = (unsigned)xb, xh = (unsigned)(xb >> 32);
   const unsigned long long p = (unsigned long long)xl * f.co;
   const unsigned long long t =
       (unsigned long long)((xh & 0xfffffu) | 0x100000u) * f.co + (p >> 32);
@@ -154,6 +148,68 @@ __device__ __forceinline__ double mul_const(double x, IntFactor f, double c) {
   if (frac > 0x80000000u - (ql & 1u)) q++;  // above half, or half and odd
   const unsigned eh = (xh & 0xfff00000u) + f.add + (top << 20);
   return from_bits((long long)(q + ((unsigned long long)eh << 32)));
+}
+
+// The bounded forms, for straight-line code on operands known to be +-0 or
+// normal with a normal result: no range test, +-0 selected (a branch per
+// operation would keep the compiler from interleaving independent chains).
+__device__ __forceinline__ double zero_or(double x, double y) {  // x if x is +-0, else y
+  return ((unsigned)((unsigned long long)bits(x) >> 32) & 0x7ff00000u) == 0 ? x : y;
+}
+__device__ __forceinline__ double mul_bounded(double x, IntFactor f) {
+  return zero_or(x, mul_core((unsigned long long)bits(x), f));
+}
+__device__ __forceinline__ double div_bounded(double x, const IntDivisor& v) {
+  return zero_or(x, div_core((unsigned long long)bits(x), v.md, v.rc, v.add));
+}
+__device__ __forceinline__ double div_bounded(double x, double d, unsigned long long rc) {
+  const unsigned long long db = (unsigned long long)bits(d);
+  return zero_or(x, div_core((unsigned long long)bits(x), (db & 0xfffffffffffffULL) | (1ULL << 52),
+                             rc, (1021u << 20) - ((unsigned)(db >> 32) & 0x7ff00000u)));
+}
+// RN(x * y): the 106-bit product of the significands in four words (x's
+// aligned so that the leading bit is bit 116 or 115), rounded to nearest
+// even; about 30 instructions.
+__device__ __forceinline__ double mul_bounded(double x, double y) {
+  const unsigned long long xb = (unsigned long long)bits(x), yb = (unsigned long long)bits(y);
+  const unsigned xl = (unsigned)xb, xh = (unsigned)(xb >> 32);
+  const unsigned yl = (unsigned)yb, yh = (unsigned)(yb >> 32);
+  const unsigned ah = __funnelshift_l(xl, xh, 11) | 0x80000000u, al = xl << 11;
+  const unsigned bh = (yh & 0xfffffu) | 0x100000u, bl = yl;
+  const unsigned long long p0 = (unsigned long long)al * bl;
+  const unsigned long long p1 = (unsigned long long)ah * bl + (p0 >> 32);
+  const unsigned long long p2 = (unsigned long long)al * bh + (unsigned)p1;
+  const unsigned long long hi = (unsigned long long)ah * bh + (p1 >> 32) + (p2 >> 32);
+  const unsigned w3 = (unsigned)(hi >> 32), w2 = (unsigned)hi, w1 = (unsigned)p2,
+                 w0 = (unsigned)p0;
+  const unsigned top = w3 >> 20, s = top ^ 1u;
+  const unsigned qh = __funnelshift_l(w2, w3, s), ql = __funnelshift_l(w1, w2, s);
+  const unsigned f1 = __funnelshift_l(w0, w1, s), f0 = w0 << s;
+  unsigned long long q = ((unsigned long long)qh << 32) | ql;
+  const unsigned most = (f0 | (ql & 1u)) ? 0x7fffffffu : 0x80000000u;
+  if (f1 > most) q++;  // above half, or half and odd
+  const unsigned sign = (xh ^ yh) & 0x80000000u;
+  const unsigned eh =
+      sign + (xh & 0x7ff00000u) + (yh & 0x7ff00000u) + (top << 20) - (1024u << 20);
+  const bool zero = (xh & 0x7ff00000u) == 0 || (yh & 0x7ff00000u) == 0;
+  const unsigned long long r = q + ((unsigned long long)eh << 32);
+  return from_bits((long long)(zero ? (unsigned long long)sign << 32 : r));
+}
+// upwind() for finite operands: the picked one, or, where that is a zero, a
+// zero with the AND of both signs.
+__device__ __forceinline__ double upwind_bounded(double w, double p, double q) {
+  const bool neg = bits(w) < 0;
+  const unsigned long long a = (unsigned long long)bits(neg ? p : q),
+                           z = (unsigned long long)bits(neg ? q : p);
+  const unsigned ah = (unsigned)(a >> 32), zh = (unsigned)(z >> 32);
+  const unsigned h = (ah & 0x7ff00000u) == 0 ? ah & zh : ah;
+  return from_bits((long long)(((unsigned long long)h << 32) | (unsigned)a));
+}
+// Whether x is neither +-0 nor of magnitude in [2^-n, 2^n).
+__device__ __forceinline__ bool beyond(double x, unsigned n) {
+  const unsigned h = (unsigned)((unsigned long long)bits(x) >> 32);
+  const bool zero = ((unsigned)bits(x) | (h << 1)) == 0;
+  return !zero && ((h >> 20) & 0x7ffu) - (1023u - n) >= 2u * n;
 }
 
 __device__ __forceinline__ double half(double x) {

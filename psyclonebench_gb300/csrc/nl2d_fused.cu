@@ -208,11 +208,12 @@ __global__ void k_selftest_exact(long long n, unsigned long long seed, IntDiviso
     const double q_ref = x / d;
     for (const double q : {div_const(x, v), div_depth(x, d, v.rc)})
       if (bits(q_ref) != bits(q) && !(q_ref != q_ref && q != q)) nd++;
+    const bool in = !beyond(x, 899);  // the bounded forms' operands, for any d
+    if (in && (bits(div_bounded(x, v)) != bits(q_ref) ||
+               bits(div_bounded(x, d, v.rc)) != bits(q_ref)))
+      nd++;
     // the product with d (counted with the quotients), where d has that form
-    if (fac.co != 0) {
-      const double p_ref = x * d, p = mul_const(x, fac, d);
-      if (bits(p_ref) != bits(p) && !(p_ref != p_ref && p != p)) nd++;
-    }
+    if (in && fac.co != 0 && bits(mul_bounded(x, fac)) != bits(x * d)) nd++;
     // Quotients within ~2^-53 ulp of a midpoint: RN((Q + ulp(Q)/2) * d) and
     // its neighbours; quotients at and next to a power of two.
     {
@@ -235,8 +236,18 @@ __global__ void k_selftest_exact(long long n, unsigned long long seed, IntDiviso
     if (bits(h_ref) != bits(h) && !(h_ref != h_ref && h != h)) nh++;
     const double p = sample(mix64(z + 1)), w = sample(mix64(z + 2));
     const double u_ref = (0.5 - copysign(0.5, w)) * x + (0.5 + copysign(0.5, w)) * p;
+    // products of operands whose product is normal (counted with the picks)
+    if (!beyond(x, 500) && !beyond(p, 500) && bits(mul_bounded(x, p)) != bits(x * p)) nu++;
+    {
+      const unsigned long long y = mix64(z + 5);
+      const double f = from_bits((long long)((y & 0x800fffffffffffffULL) | (1000ULL + (y >> 53) % 40) << 52));
+      const double s1 = from_bits((bits(f) >> (y % 53)) << (y % 53));  // a short significand
+      const double g = from_bits((bits(x) & 0x800fffffffffffffLL) | (1020LL << 52));
+      if (bits(mul_bounded(f, g)) != bits(f * g) || bits(mul_bounded(g, s1)) != bits(g * s1)) nu++;
+    }
     const double u = upwind(w, x, p);
     if (bits(u_ref) != bits(u) && !(u_ref != u_ref && u != u)) nu++;
+    if (!beyond(x, 899) && !beyond(p, 899) && bits(upwind_bounded(w, x, p)) != bits(u_ref)) nu++;
   }
   if (nd) atomicAdd(&bad[0], nd);
   if (nh) atomicAdd(&bad[1], nh);

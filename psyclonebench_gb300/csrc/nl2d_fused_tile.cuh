@@ -23,23 +23,46 @@ namespace {
 // the split.
 constexpr int NTHREADS = 256;
 
+// A constant factor of the tiles: c and its integer form.
+//
+// The tiles' regular update is straight-line code without range tests, on
+// fields (ssh, u, v and the depths) that are +-0 or of magnitude in [2^-200,
+// 2^200), and constants in [2^-40, 2^40].  Then every nonzero sum of fields is
+// at least 2^-252, a face height 2^-333, a total depth or a sum of them
+// 2^-385, and the smallest product formed (an advective flux: velocity, face
+// speed, depth) 2^-880: normal, so a power of two may move from an operand to
+// a constant without changing a bit.  Tendencies and momenta can cancel below
+// that, and are tested (2^-699) before they are scaled.  A tile with another
+// field, and a cell with another tendency, takes the general code.
+struct Factor {
+  double c;
+  IntFactor i;
+};
+constexpr unsigned kFieldRange = 200, kTendRange = 699;
+
 // Step-invariant constants of the fast path, evaluated on the host with the
 // operations the reference performs per point (e.g. dx_v[c] + dx_v[e] on a
 // uniform grid is one add of two equal values), so they are bit-identical.
 struct FastConst {
   double area_t, area_u, area_v, dx_u, dx_v, dx_t, dy_u, dy_v, dy_t;
   double dxv2, dyu2;                       // dx_v + dx_v, dy_u + dy_u
-  double cor_u, cor_v;                     // 2. * omega * sin(gphi * d2r)
+  double cor_u, cor_v, neg_cor_v;          // 2. * omega * sin(gphi * d2r)
   double neg_g, rdt, visc, g;
   // the constant divisors (fric: 1.0 + cbfr * rdt), and whether every one
   // lies in [2^-100, 2^100]
   IntDivisor q_area_t, q_area_u, q_area_v, q_dx_t, q_dy_t, q_dxv2, q_dyu2, q_fric;
   int fast_div;
-  // the grid's and the time step's constants as integer factors (mul_const),
-  // and whether all of them have that form
-  IntFactor i_area_t, i_area_u, i_area_v, i_dx_u, i_dx_v, i_dx_t, i_dy_u, i_dy_v, i_dy_t;
-  IntFactor i_dxv2, i_dyu2, i_rdt;
-  int int_mul;
+  // The tiles' factors, with the powers of two of the face averages folded in
+  // (the same bits: nothing they scale leaves the normal range, see Factor),
+  // and the face heights' divisors 2 area_u, 2 area_v.
+  Factor f_area_t, f_rdt, f_dy_u, f_dx_v, f_hdx_u, f_hdy_v;  // h: half
+  Factor f_U, f_V, f_Uw, f_Vs;                   // dy_t/2, dx_t/2, dyu2/8, dxv2/8
+  Factor f_cor_area_u, f_cor_area_v;             // area_u/4, area_v/4
+  IntDivisor q_2area_u, q_2area_v;
+  // whether the tiles' straight-line code applies: every constant divisor and
+  // factor lies in [2^-40, 2^40] (visc, cor and g may be zero); and whether
+  // all factors have the integer form
+  int bounded, int_mul;
 };
 
 // One domain of an ensemble (device-resident descriptor).
@@ -52,11 +75,11 @@ struct EnsDomain {
   FastConst k;
 };
 
-// Multiplication by a step constant, `kc` and its integer form `ic` (IC), the
-// same bits either way.
+// Multiplication by a constant: 20 instructions when every constant has the
+// integer form (IC), 30 otherwise.
 template <bool IC>
-__device__ __forceinline__ double mlc(double x, double kc, IntFactor ic) {
-  return IC ? mul_const(x, ic, kc) : x * kc;
+__device__ __forceinline__ double mlc(double x, const Factor& f) {
+  return IC ? mul_bounded(x, f.i) : mul_bounded(x, f.c);
 }
 
 // Division by a step constant: in integers when the constants allow it,
@@ -432,7 +455,7 @@ __host__ __device__ __forceinline__ void ring_pos(const Dims& d, int ja, int jb,
 // side: the loaded fields and the sshn_u / sshn_v this step sees, then the
 // terms that two neighbouring updates share.
 enum { A_SN, A_UN, A_VN, A_HU, A_HV, A_SU, A_SV, A_HUS, A_HVS, N_A0 };
-enum { B_FLXU, B_FLXV, B_GX, B_GY, B_FXU, B_FYV, B_VSC, B_FYU, B_QY, B_UWC, B_FXV, B_QX, N_B1 };
+enum { B_FLXU, B_FLXV, B_GX, B_GY, B_FXU, B_FYV, B_VS2, B_FYU, B_QY, B_UW2, B_FXV, B_QX, N_B1 };
 // area_t * sshn_t, needed until the face values are formed, shares the slot
 // of a term that is formed after them
 constexpr int B_AREA_SSH = B_QX;
@@ -448,7 +471,7 @@ struct Tile {
   static constexpr int S0 = SX * SY;  // staged positions (34 x 18 for 32 x 16)
   // + the mask, and the list of the tile's general (non-regular) cells
   static constexpr size_t kSmemBytes =
-      sizeof(double) * (N_A0 + N_B1) * S0 + sizeof(int) * (S0 + TX * TY + 1);
+      sizeof(double) * (N_A0 + N_B1) * S0 + sizeof(int) * (S0 + TX * TY + 2);
   // two CTAs of 256 threads per SM when their shared memory (with the 1 KB
   // the driver reserves per CTA) fits the SM's 228 KB
   static constexpr int kMinBlocks = 2 * (kSmemBytes + 1024) <= 228 * 1024 ? 2 : 1;
@@ -462,10 +485,13 @@ using DefaultTile = Tile<32, 16>;
 // A regular cell's new (sshn_t, un, vn) from the tile's staged fields (a0)
 // and shared terms (b1) at its slot q: continuity (continuity_kern.c:90-117)
 // and unmasked momentum (momentum_u_kern.c:184-261,
-// momentum_v_kern.c:159-239) in the reference's operation order.  dhu, rhu,
-// dhv, rhv: hu + ssha_u and hv + ssha_v at the cell and their reciprocals (dvf).
+// momentum_v_kern.c:159-239) in the reference's operation order, without a
+// branch.  dhu, rhu, dhv, rhv: hu + ssha_u and hv + ssha_v at the cell and
+// their reciprocals.  bad: a tendency or momentum is outside the bounded
+// forms' range (or a depth has no reciprocal), the results are not valid.
 struct RegOut {
   double ssh, u, v;
+  bool bad;
 };
 template <class T, bool IC>
 __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b1, int q,
@@ -475,43 +501,46 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
 #define A(qq, t) a0[(qq) * S0 + (t)]
 #define B(qq, t) b1[(qq) * S0 + (t)]
   RegOut o;
+  o.bad = rhu == 0 || rhv == 0;
   const double snc = A(A_SN, q), Hu = A(A_HUS, q), Hv = A(A_HVS, q);
-  const double ssh = mlc<IC>(
-      ((B(B_FLXU, q - 1) - B(B_FLXU, q)) + B(B_FLXV, q - SX)) - B(B_FLXV, q), k.rdt, k.i_rdt);
-  o.ssh = snc + dvc(ssh, k.q_area_t, k.fast_div);
+  const double ssh =
+      mlc<IC>(((B(B_FLXU, q - 1) - B(B_FLXU, q)) + B(B_FLXV, q - SX)) - B(B_FLXV, q), k.f_rdt);
+  o.ssh = snc + div_bounded(ssh, k.q_area_t);
   {
     const double adv = ((B(B_FXU, q) - B(B_FXU, q + 1)) + B(B_FYU, q)) - B(B_FYU, q + SX);
-    const double dudy_s = B(B_QY, q) * ((Hu + A(A_HU, q - SX)) + A(A_SU, q - SX));
-    const double dudy_n = B(B_QY, q + SX) * ((Hu + A(A_HU, q + SX)) + A(A_SU, q + SX));
-    double vis = mlc<IC>(B(B_GX, q + 1) - B(B_GX, q), k.dy_u, k.i_dy_u) +
-                 half(mlc<IC>(dudy_n - dudy_s, k.dx_u, k.i_dx_u));
-    vis = k.visc * vis;
-    const double cor = mlc<IC>(half(k.cor_u * (B(B_VSC, q) + B(B_VSC, q + SX))), k.area_u,
-                               k.i_area_u) *
-                       Hu;
-    const double hpg = mlc<IC>(k.neg_g * Hu, k.dy_u, k.i_dy_u) * (A(A_SN, q + 1) - snc);
+    const double dudy_s = mul_bounded(B(B_QY, q), (Hu + A(A_HU, q - SX)) + A(A_SU, q - SX));
+    const double dudy_n =
+        mul_bounded(B(B_QY, q + SX), (Hu + A(A_HU, q + SX)) + A(A_SU, q + SX));
+    double vis = mlc<IC>(B(B_GX, q + 1) - B(B_GX, q), k.f_dy_u) +
+                 mlc<IC>(dudy_n - dudy_s, k.f_hdx_u);
+    vis = mul_bounded(vis, k.visc);
+    const double cor = mul_bounded(
+        mlc<IC>(mul_bounded(B(B_VS2, q) + B(B_VS2, q + SX), k.cor_u), k.f_cor_area_u), Hu);
+    const double hpg =
+        mul_bounded(mlc<IC>(mul_bounded(Hu, k.neg_g), k.f_dy_u), A(A_SN, q + 1) - snc);
+    const double tend = ((adv + vis) + cor) + hpg;
     const double num =
-        A(A_UN, q) * Hu +
-        dvc(mlc<IC>(((adv + vis) + cor) + hpg, k.rdt, k.i_rdt), k.q_area_u, k.fast_div);
-    const double t1 = dvf(num, dhu, rhu);
-    o.u = dvc(t1, k.q_fric, k.fast_div);
+        mul_bounded(A(A_UN, q), Hu) + div_bounded(mlc<IC>(tend, k.f_rdt), k.q_area_u);
+    o.bad |= beyond(tend, kTendRange) || beyond(num, kTendRange);
+    o.u = div_bounded(div_bounded(num, dhu, rhu), k.q_fric);
   }
   {
     const double adv = ((B(B_FXV, q) - B(B_FXV, q + 1)) + B(B_FYV, q)) - B(B_FYV, q + SX);
-    const double dvdx_w = B(B_QX, q) * ((Hv + A(A_HV, q - 1)) + A(A_SV, q - 1));
-    const double dvdx_e = B(B_QX, q + 1) * ((Hv + A(A_HV, q + 1)) + A(A_SV, q + 1));
-    double vis = mlc<IC>(B(B_GY, q + SX) - B(B_GY, q), k.dx_v, k.i_dx_v) +
-                 half(mlc<IC>(dvdx_e - dvdx_w, k.dy_v, k.i_dy_v));
-    vis = k.visc * vis;
-    const double cor = mlc<IC>(-half(k.cor_v * (B(B_UWC, q + 1) + B(B_UWC, q))), k.area_v,
-                               k.i_area_v) *
-                       Hv;
-    const double hpg = mlc<IC>(k.neg_g * Hv, k.dx_v, k.i_dx_v) * (A(A_SN, q + SX) - snc);
+    const double dvdx_w = mul_bounded(B(B_QX, q), (Hv + A(A_HV, q - 1)) + A(A_SV, q - 1));
+    const double dvdx_e =
+        mul_bounded(B(B_QX, q + 1), (Hv + A(A_HV, q + 1)) + A(A_SV, q + 1));
+    double vis = mlc<IC>(B(B_GY, q + SX) - B(B_GY, q), k.f_dx_v) +
+                 mlc<IC>(dvdx_e - dvdx_w, k.f_hdy_v);
+    vis = mul_bounded(vis, k.visc);
+    const double cor = mul_bounded(
+        mlc<IC>(mul_bounded(B(B_UW2, q + 1) + B(B_UW2, q), k.neg_cor_v), k.f_cor_area_v), Hv);
+    const double hpg =
+        mul_bounded(mlc<IC>(mul_bounded(Hv, k.neg_g), k.f_dx_v), A(A_SN, q + SX) - snc);
+    const double tend = ((adv + vis) + cor) + hpg;
     const double num =
-        A(A_VN, q) * Hv +
-        dvc(mlc<IC>(((adv + vis) + cor) + hpg, k.rdt, k.i_rdt), k.q_area_v, k.fast_div);
-    const double t1 = dvf(num, dhv, rhv);
-    o.v = dvc(t1, k.q_fric, k.fast_div);
+        mul_bounded(A(A_VN, q), Hv) + div_bounded(mlc<IC>(tend, k.f_rdt), k.q_area_v);
+    o.bad |= beyond(tend, kTendRange) || beyond(num, kTendRange);
+    o.v = div_bounded(div_bounded(num, dhv, rhv), k.q_fric);
   }
   return o;
 }
@@ -520,9 +549,11 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
 // terms of the cell's west side, Y: of its south side (a tile's east and
 // north neighbours need one of the two only).  Every term is the exact
 // operation sequence of momentum_{u,v}_kern.c / continuity_kern.c for one of
-// the two updates that use it; for the other update the reference evaluates
-// the same operations on the same operands (addition commuted), so the bits
-// agree.  ht: the T depth at the cell.
+// the two updates that use it, up to powers of two moved into the constants
+// (the face speeds of B_FXV and B_FYU carry the half of their depth's
+// average, B_VS2 and B_UW2 are twice the averaged velocities); for the other
+// update the reference evaluates the same operations on the same operands
+// (addition commuted), so the bits agree.  ht: the T depth at the cell.
 template <class T, bool IC, bool X, bool Y>
 __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q, double ht,
                                              const FastConst& k) {
@@ -531,38 +562,38 @@ __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q
   const double D = ht + A(A_SN, q);  // ht + sshn at T(i,j)
   const double u_c = A(A_UN, q), v_c = A(A_VN, q);
   if (X && Y) {  // continuity fluxes (sshn_u + hu) * un and (sshn_v + hv) * vn
-    B(B_FLXU, q) = A(A_HUS, q) * u_c;
-    B(B_FLXV, q) = A(A_HVS, q) * v_c;
+    B(B_FLXU, q) = mul_bounded(A(A_HUS, q), u_c);
+    B(B_FLXV, q) = mul_bounded(A(A_HVS, q), v_c);
   }
   if (X) {
     const double u_w = A(A_UN, qw), v_w = A(A_VN, qw);
     // dudx at T(i,j): dudx_w of u face i, dudx_e of face i-1
-    B(B_GX, q) = dvc(u_c - u_w, k.q_dx_t, k.fast_div) * D;
+    B(B_GX, q) = mul_bounded(div_bounded(u_c - u_w, k.q_dx_t), D);
     // x-advective flux of u through T(i,j): uu_w * u_w * depw of face i
-    const double U = mlc<IC>(half(u_c + u_w), k.dy_t, k.i_dy_t);
-    B(B_FXU, q) = (upwind(U, u_c, u_w) * U) * D;
+    const double U = mlc<IC>(u_c + u_w, k.f_U);
+    B(B_FXU, q) = mul_bounded(mul_bounded(upwind_bounded(U, u_c, u_w), U), D);
     // west edge of v face (i,j): u_wc, u_w, depw, vv_w (unmasked form)
-    const double uwc = half(u_w + A(A_UN, qwn));
-    B(B_UWC, q) = uwc;
-    const double Uw = mlc<IC>(half(uwc), k.dyu2, k.i_dyu2);
-    const double depw = half((A(A_HUS, qw) + A(A_HU, qwn)) + A(A_SU, qwn));
-    B(B_FXV, q) = (upwind(Uw, v_c, v_w) * Uw) * depw;
-    B(B_QX, q) = dvc(v_c - v_w, k.q_dxv2, k.fast_div);
+    const double uw2 = u_w + A(A_UN, qwn);
+    B(B_UW2, q) = uw2;
+    const double Uw = mlc<IC>(uw2, k.f_Uw);
+    const double depw = (A(A_HUS, qw) + A(A_HU, qwn)) + A(A_SU, qwn);
+    B(B_FXV, q) = mul_bounded(mul_bounded(upwind_bounded(Uw, v_c, v_w), Uw), depw);
+    B(B_QX, q) = div_bounded(v_c - v_w, k.q_dxv2);
   }
   if (Y) {
     const double u_s = A(A_UN, qs), v_s = A(A_VN, qs);
     // dvdy at T(i,j): dvdy_s of v face j, dvdy_n of face j-1
-    B(B_GY, q) = dvc(v_c - v_s, k.q_dy_t, k.fast_div) * D;
+    B(B_GY, q) = mul_bounded(div_bounded(v_c - v_s, k.q_dy_t), D);
     // y-advective flux of v through T(i,j): vv_s * v_s * deps of face j
-    const double V = mlc<IC>(half(v_c + v_s), k.dx_t, k.i_dx_t);
-    B(B_FYV, q) = (upwind(V, v_c, v_s) * V) * D;
+    const double V = mlc<IC>(v_c + v_s, k.f_V);
+    B(B_FYV, q) = mul_bounded(mul_bounded(upwind_bounded(V, v_c, v_s), V), D);
     // south edge of u face (i,j): v_sc, v_s, deps, uu_s (unmasked form)
-    const double vsc = half(v_s + A(A_VN, qse));
-    B(B_VSC, q) = vsc;
-    const double Vs = mlc<IC>(half(vsc), k.dxv2, k.i_dxv2);
-    const double deps = half((A(A_HVS, qs) + A(A_HV, qse)) + A(A_SV, qse));
-    B(B_FYU, q) = (upwind(Vs, u_c, u_s) * Vs) * deps;
-    B(B_QY, q) = dvc(u_c - u_s, k.q_dyu2, k.fast_div);
+    const double vs2 = v_s + A(A_VN, qse);
+    B(B_VS2, q) = vs2;
+    const double Vs = mlc<IC>(vs2, k.f_Vs);
+    const double deps = (A(A_HVS, qs) + A(A_HV, qse)) + A(A_SV, qse);
+    B(B_FYU, q) = mul_bounded(mul_bounded(upwind_bounded(Vs, u_c, u_s), Vs), deps);
+    B(B_QY, q) = div_bounded(u_c - u_s, k.q_dyu2);
   }
 }
 
@@ -571,10 +602,13 @@ __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q
 //
 // The FP64 pipe bounds the step (about 1.7 instructions per clock per SM;
 // each holds a scheduler's share of it for 64 issue slots), so every phase
-// forms a value on exactly the positions that are read: a full warp per row
-// of the tile, and the edges' extra values (next column, next row) packed
-// into warps of their own.  140 -> 123 FP64 instructions per cell against the
-// form that formed everything on a 2- and a 1-cell halo.
+// forms a value on exactly the positions that are read (a full warp per row
+// of the tile, and the edges' extra values, next column and next row, packed
+// into warps of their own), and products and quotients are formed in
+// integers: the pipe has the step's adds only, 57 of the 140 instructions per
+// cell of the form that used it for everything on 2- and 1-cell halos.  The
+// integer forms pay only as straight-line code: with a range branch each,
+// the same products made the step slower.
 template <class T, bool IC>
 __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs, const Dims& d,
                                            const Scalars& p, const FastConst& k, double tide,
@@ -585,30 +619,41 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
   double* b1 = smem + N_A0 * S0;     // [N_B1][S0]
   int* mk = (int*)(b1 + N_B1 * S0);  // [S0]
   int* glist = mk + S0;              // [TX * TY] general cells of this tile
-  int* gcount = glist + TX * TY;
+  int* gcount = glist + TX * TY;     // their number
+  int* slow = gcount + 1;            // a field is outside the bounded forms' range
 
-  const int W = d.width, H = d.height;
+  const int W = d.width;
   const int tid = threadIdx.y * TX + threadIdx.x;
   const int i = i0 + threadIdx.x;
 
-  if (tid == 0) *gcount = 0;
-  // ---- the fields (positions past the array's end hold what the last
-  // column or row does; no cell that is written reads them) ----
+  if (tid == 0) {
+    *gcount = 0;
+    *slow = k.bounded ? 0 : 1;
+  }
+  // ---- the fields (positions past the copy region hold what its last column
+  // or row does; no cell that is written reads them) ----
+  const int imax = d.xe + 1, jmax = d.ye + 1;
+  bool out = false;  // a field of this thread's is out of range
   for (int t = tid; t < S0; t += NTHREADS) {
-    const int c = min(j0 - 1 + t / SX, H - 1) * W + min(i0 - 1 + t % SX, W - 1);
-    const double sn = fs.sshn_in[c];
+    const int c = min(j0 - 1 + t / SX, jmax) * W + min(i0 - 1 + t % SX, imax);
+    const double sn = fs.sshn_in[c], un = fs.un_in[c], vn = fs.vn_in[c], hu = f.hu[c],
+                 hv = f.hv[c];
+    out |= beyond(sn, kFieldRange) | beyond(un, kFieldRange) | beyond(vn, kFieldRange) |
+           beyond(hu, kFieldRange) | beyond(hv, kFieldRange);
     A(A_SN, t) = sn;
-    A(A_UN, t) = fs.un_in[c];
-    A(A_VN, t) = fs.vn_in[c];
-    A(A_HU, t) = f.hu[c];
-    A(A_HV, t) = f.hv[c];
+    A(A_UN, t) = un;
+    A(A_VN, t) = vn;
+    A(A_HU, t) = hu;
+    A(A_HV, t) = hv;
     mk[t] = f.tmask[c];
-    B(B_AREA_SSH, t) = mlc<IC>(sn, k.area_t, k.i_area_t);
+    B(B_AREA_SSH, t) = mlc<IC>(sn, k.f_area_t);
   }
   double ht[T::RPT];  // of this thread's own cells, for the shared terms
 #pragma unroll
-  for (int e = 0; e < T::RPT; e++)
-    ht[e] = f.ht[min(j0 + (int)threadIdx.y + e * T::RPP, H - 1) * W + min(i, W - 1)];
+  for (int e = 0; e < T::RPT; e++) {
+    ht[e] = f.ht[min(j0 + (int)threadIdx.y + e * T::RPP, jmax) * W + min(i, imax)];
+    out |= beyond(ht[e], kFieldRange);
+  }
   __syncthreads();
 
   // ---- the sshn_u / sshn_v this step reads: next_sshu_code /
@@ -619,12 +664,11 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
     double su;
     const int mm = mk[q], mn = mk[q + 1];
     if (fj <= d.ye && fi <= d.xe - 1 && mm + mn > 0) {
-      if (mm * mn > 0)
-        su = dvc(half(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + 1)), k.q_area_u, k.fast_div);
-      else
-        su = mm <= 0 ? A(A_SN, q + 1) : A(A_SN, q);
+      su = mm * mn > 0 ? div_bounded(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + 1), k.q_2area_u)
+                       : (mm <= 0 ? A(A_SN, q + 1) : A(A_SN, q));
     } else {
-      su = f.sshn_u[min(fj, H - 1) * W + min(fi, W - 1)];
+      su = f.sshn_u[min(fj, jmax) * W + min(fi, imax)];
+      out |= beyond(su, kFieldRange);
     }
     A(A_SU, q) = su;
     if (sum) A(A_HUS, q) = A(A_HU, q) + su;
@@ -634,12 +678,11 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
     double sv;
     const int mm = mk[q], mn = mk[q + SX];
     if (fj <= d.ye - 1 && fi <= d.xe && mm + mn > 0) {
-      if (mm * mn > 0)
-        sv = dvc(half(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + SX)), k.q_area_v, k.fast_div);
-      else
-        sv = mm <= 0 ? A(A_SN, q + SX) : A(A_SN, q);
+      sv = mm * mn > 0 ? div_bounded(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + SX), k.q_2area_v)
+                       : (mm <= 0 ? A(A_SN, q + SX) : A(A_SN, q));
     } else {
-      sv = f.sshn_v[min(fj, H - 1) * W + min(fi, W - 1)];
+      sv = f.sshn_v[min(fj, jmax) * W + min(fi, imax)];
+      out |= beyond(sv, kFieldRange);
     }
     A(A_SV, q) = sv;
     if (sum) A(A_HVS, q) = A(A_HV, q) + sv;
@@ -680,80 +723,89 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
   for (int t = tid; t < 2 * RX + 2 * RY; t += NTHREADS) {
     int e = t;
     if (e < RX) {
-      if (e < TX)
-        shared_terms<T, IC, false, true>(a0, b1, (TY + 1) * SX + e + 1,
-                                     f.ht[min(j0 + TY, H - 1) * W + min(i0 + e, W - 1)], k);
+      if (e < TX) {
+        const double h = f.ht[min(j0 + TY, jmax) * W + min(i0 + e, imax)];
+        out |= beyond(h, kFieldRange);
+        shared_terms<T, IC, false, true>(a0, b1, (TY + 1) * SX + e + 1, h, k);
+      }
     } else if ((e -= RX) < RY) {
-      if (e < TY)
-        shared_terms<T, IC, true, false>(a0, b1, (e + 1) * SX + TX + 1,
-                                     f.ht[min(j0 + e, H - 1) * W + min(i0 + TX, W - 1)], k);
+      if (e < TY) {
+        const double h = f.ht[min(j0 + e, jmax) * W + min(i0 + TX, imax)];
+        out |= beyond(h, kFieldRange);
+        shared_terms<T, IC, true, false>(a0, b1, (e + 1) * SX + TX + 1, h, k);
+      }
     } else if ((e -= RY) < RY) {
       const int q = (e + 1) * SX;
-      if (e < TY) B(B_FLXU, q) = A(A_HUS, q) * A(A_UN, q);
+      if (e < TY) B(B_FLXU, q) = mul_bounded(A(A_HUS, q), A(A_UN, q));
     } else {
       e -= RY;
       const int q = e + 1;
-      if (e < TX) B(B_FLXV, q) = A(A_HVS, q) * A(A_VN, q);
+      if (e < TX) B(B_FLXV, q) = mul_bounded(A(A_HVS, q), A(A_VN, q));
     }
   }
+  if (out) *slow = 1;
   __syncthreads();
 
   // ---- the update ----
   // Each thread owns the cells (i, j0 + row) of its rows.  Regular cells
   // (wet 3x3 neighbourhood: continuity without bc_ssh, unmasked momentum, no
-  // solid-wall or Flather change) are computed here; the others are queued
-  // for the packed general pass below, so that a warp holding a few land-side
-  // cells does not run both paths.  When both of a thread's cells are
-  // regular they are computed in one straight-line block, so the compiler
-  // can interleave two independent FP64 chains; the per-face global inputs
-  // are loaded first and the results stored last, so no store can alias a
-  // later load.
+  // solid-wall or Flather change; values in the bounded forms' range) are
+  // computed here, two of a thread's cells in one straight-line block, so
+  // that the compiler interleaves independent FP64 chains; the others are
+  // queued for the packed general pass below, so that a warp holding a few
+  // land-side cells does not run both paths.  The per-face global inputs are
+  // loaded first and the results stored last, so no store can alias a later
+  // load.
+  const bool tile_slow = *slow != 0;
 #pragma unroll
   for (int pb = 0; pb < T::RPT; pb += 2) {
     constexpr int NP = T::RPT >= 2 ? 2 : 1;  // rows taken together
     int c[NP], q[NP];
-    bool reg[NP];
+    bool live[NP], reg[NP];
+    bool any = false;
 #pragma unroll
     for (int e = 0; e < NP; e++) {
       const int row = threadIdx.y + (pb + e) * T::RPP, j = j0 + row;
       c[e] = j * W + i;
       q[e] = (row + 1) * SX + (threadIdx.x + 1);
-      const bool live = i <= d.xe - 1 && j <= d.ye - 1;
-      bool regular = live;
+      live[e] = i <= d.xe - 1 && j <= d.ye - 1;
+      bool regular = live[e] && !tile_slow;
 #pragma unroll
       for (int dj = -1; dj <= 1; dj++)
 #pragma unroll
         for (int di = -1; di <= 1; di++) regular &= mk[q[e] + dj * SX + di] > 0;
       reg[e] = regular;
-      if (live && !regular) glist[atomicAdd(gcount, 1)] = row * TX + threadIdx.x;
+      any |= regular;
     }
-    double dhu[NP], dhv[NP];
-    unsigned long long rhu[NP], rhv[NP];
+    if (any) {
+      double dhu[NP], dhv[NP];
+      unsigned long long rhu[NP], rhv[NP];
 #pragma unroll
-    for (int e = 0; e < NP; e++)
-      if (reg[e]) {
-        dhu[e] = f.d_hu[c[e]];
-        rhu[e] = f.r_hu[c[e]];
-        dhv[e] = f.d_hv[c[e]];
-        rhv[e] = f.r_hv[c[e]];
+      for (int e = 0; e < NP; e++) {  // (a cell that is not regular: the other's values)
+        const int cc = reg[e] ? c[e] : c[NP - 1 - e];
+        dhu[e] = f.d_hu[cc];
+        rhu[e] = f.r_hu[cc];
+        dhv[e] = f.d_hv[cc];
+        rhv[e] = f.r_hv[cc];
       }
-    RegOut o[NP];
-    if (NP == 2 && reg[0] && reg[NP - 1]) {
-      o[0] = regular_cell<T, IC>(a0, b1, q[0], dhu[0], rhu[0], dhv[0], rhv[0], k);
-      o[NP - 1] = regular_cell<T, IC>(a0, b1, q[NP - 1], dhu[NP - 1], rhu[NP - 1], dhv[NP - 1],
-                                  rhv[NP - 1], k);
-    } else {
+      RegOut o[NP];
 #pragma unroll
       for (int e = 0; e < NP; e++)
-        if (reg[e]) o[e] = regular_cell<T, IC>(a0, b1, q[e], dhu[e], rhu[e], dhv[e], rhv[e], k);
+        o[e] = regular_cell<T, IC>(a0, b1, q[e], dhu[e], rhu[e], dhv[e], rhv[e], k);
+#pragma unroll
+      for (int e = 0; e < NP; e++) {
+        reg[e] = reg[e] && !o[e].bad;
+        if (reg[e]) {
+          fs.sshn_out[c[e]] = o[e].ssh;
+          fs.un_out[c[e]] = o[e].u;
+          fs.vn_out[c[e]] = o[e].v;
+        }
+      }
     }
 #pragma unroll
     for (int e = 0; e < NP; e++)
-      if (reg[e]) {
-        fs.sshn_out[c[e]] = o[e].ssh;
-        fs.un_out[c[e]] = o[e].u;
-        fs.vn_out[c[e]] = o[e].v;
-      }
+      if (live[e] && !reg[e])
+        glist[atomicAdd(gcount, 1)] = (threadIdx.y + (pb + e) * T::RPP) * TX + threadIdx.x;
   }
   __syncthreads();
 
@@ -772,7 +824,7 @@ bool in_fast_range(double d) {
   return d > 0.0 && d >= 0x1p-100 && d <= 0x1p100;
 }
 
-// c as mul_const's factor (host side).
+// c as mul_core's factor (host side).
 inline IntFactor int_factor(double c) {
   if (!in_fast_range(c)) return IntFactor{0, 0};
   unsigned long long b;
@@ -783,6 +835,8 @@ inline IntFactor int_factor(double c) {
   // leading bit, added there); minus one for q's own leading bit
   return IntFactor{(unsigned)(m >> 21), ((unsigned)((int)(b >> 52) - 1023) - 1u) << 20};
 }
+
+inline Factor factor(double c) { return Factor{c, int_factor(c)}; }
 
 // d as div_const's divisor (host side).
 inline IntDivisor int_divisor(double d) {
@@ -816,16 +870,27 @@ inline FastConst make_fast_const(const Scalars& s, const UniformMetrics& um) {
   k.q_area_v = int_divisor(k.area_v), k.q_dx_t = int_divisor(k.dx_t);
   k.q_dy_t = int_divisor(k.dy_t), k.q_dxv2 = int_divisor(k.dxv2);
   k.q_dyu2 = int_divisor(k.dyu2), k.q_fric = int_divisor(fric);
-  k.i_area_t = int_factor(k.area_t), k.i_area_u = int_factor(k.area_u);
-  k.i_area_v = int_factor(k.area_v), k.i_dx_u = int_factor(k.dx_u);
-  k.i_dx_v = int_factor(k.dx_v), k.i_dx_t = int_factor(k.dx_t);
-  k.i_dy_u = int_factor(k.dy_u), k.i_dy_v = int_factor(k.dy_v);
-  k.i_dy_t = int_factor(k.dy_t), k.i_dxv2 = int_factor(k.dxv2);
-  k.i_dyu2 = int_factor(k.dyu2), k.i_rdt = int_factor(k.rdt);
-  const IntFactor all[12] = {k.i_area_t, k.i_area_u, k.i_area_v, k.i_dx_u, k.i_dx_v, k.i_dx_t,
-                             k.i_dy_u,   k.i_dy_v,   k.i_dy_t,   k.i_dxv2, k.i_dyu2, k.i_rdt};
+  k.neg_cor_v = -k.cor_v;
+  k.f_area_t = factor(k.area_t), k.f_rdt = factor(k.rdt);
+  k.f_dy_u = factor(k.dy_u), k.f_dx_v = factor(k.dx_v);
+  k.f_hdx_u = factor(0.5 * k.dx_u), k.f_hdy_v = factor(0.5 * k.dy_v);
+  k.f_U = factor(0.5 * k.dy_t), k.f_V = factor(0.5 * k.dx_t);
+  k.f_Uw = factor(0.125 * k.dyu2), k.f_Vs = factor(0.125 * k.dxv2);
+  k.f_cor_area_u = factor(0.25 * k.area_u), k.f_cor_area_v = factor(0.25 * k.area_v);
+  k.q_2area_u = int_divisor(2.0 * k.area_u), k.q_2area_v = int_divisor(2.0 * k.area_v);
+  const Factor* all[12] = {&k.f_area_t, &k.f_rdt, &k.f_dy_u, &k.f_dx_v, &k.f_hdx_u, &k.f_hdy_v,
+                           &k.f_U, &k.f_V, &k.f_Uw, &k.f_Vs, &k.f_cor_area_u, &k.f_cor_area_v};
   k.int_mul = 1;
-  for (const IntFactor& q : all) k.int_mul &= q.co != 0;
+  for (const Factor* q : all) k.int_mul &= q->i.co != 0;
+  bool bounded = fast;
+  for (double v : {k.area_t, k.area_u, k.area_v, k.dx_u, k.dx_v, k.dx_t, k.dy_u, k.dy_v, k.dy_t,
+                   k.dxv2, k.dyu2, k.rdt, fric})
+    bounded = bounded && v >= 0x1p-40 && v <= 0x1p40;
+  for (double v : {k.visc, k.cor_u, k.cor_v, k.neg_g}) {
+    const double a = v < 0 ? -v : v;
+    bounded = bounded && (a == 0.0 || (a >= 0x1p-40 && a <= 0x1p40));
+  }
+  k.bounded = bounded ? 1 : 0;
   return k;
 }
 
