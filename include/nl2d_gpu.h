@@ -229,17 +229,16 @@ int nl2d_ens_set_domain(int dom, const int *tmask, const double *ht,
 /* Schedule knobs the autotuner searches: persistent CTAs per SM (1, 2),
  * tile assignment (0 contiguous cost-balanced chunks, 1 longest processing
  * time first, 2 one tile per CTA with as many CTAs as tiles, balanced by the
- * hardware block scheduler; the CTA count then does not apply) and the
- * cost weight of a ring cell (a cell of the domain's boundary rows and
+ * hardware block scheduler, the default; the CTA count then does not apply)
+ * and the cost weight of a ring cell (a cell of the domain's boundary rows and
  * columns, which takes the general per-cell code) against a regular one. */
 int nl2d_ens_schedule(int ctas_per_sm, int policy, double boundary_weight);
 /* Tile knobs the autotuner searches (the reference's tiled OpenMP layer,
  * psykal_omp/time_step_mod.f90:587-1182, fixes its tile size per run): the
- * FP64 kernel's tile shape tx x ty, one of 32 x 16 (the default), 32 x 8,
+ * FP64 kernel's tile shape tx x ty, one of 32 x 16, 32 x 8 (the default),
  * 16 x 16, 64 x 8 and 32 x 32, and the column marches' strip height (the
  * mixed and FP64-equivalent forms), 8, 16, 32 (the default) or 64 rows.
- * Results do not depend on
- * either.  A new ensemble starts with the defaults.  Returns NL2D_ERR_ARGS
+ * Results do not depend on either.  A new ensemble starts with the defaults.  Returns NL2D_ERR_ARGS
  * for other values. */
 int nl2d_ens_tile(int tx, int ty, int march_rows);
 /* Advances every domain nsteps steps (istep = istep0 ...); per-domain

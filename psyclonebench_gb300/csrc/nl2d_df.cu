@@ -54,11 +54,7 @@ __global__ void __launch_bounds__(32 * WARPS, 3)
     if (part < kParts) {
       const int c = ff.ring[g - part * ff.n_ring];
       const int j = c / d.width, i = c - j * d.width;
-      const GlobalCtx x{fs.sshn_in, fs.un_in,    fs.vn_in, f.hu,      f.hv,
-                        f.ht,       f.ssha_u,    f.ssha_v, f.r_hu,    f.r_hv,
-                        f.tmask,    f.sshn_u,    f.sshn_v, d.width,   d,
-                        fk};
-      general_part(x, f, fs, p, tide_table ? tide_table[tide_index] : tide, part, i, j);
+      general_part(f, fs, d, p, fk, tide_table ? tide_table[tide_index] : tide, part, i, j);
     }
     return;
   }

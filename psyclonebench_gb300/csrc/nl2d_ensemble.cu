@@ -80,10 +80,11 @@ __global__ void k_mixed_statics(const double* __restrict__ ht, const double* __r
 
 // Ensemble: a persistent grid walks a list spanning many independent
 // domains; CTA b takes entries [first[b], first[b+1]).  An entry (domain, i0,
-// j0, -1) is a tile, (domain, -, -, g) parts g .. g + NTHREADS - 1 of the
+// j0, -1) is a tile, (domain, -, -, g) parts g .. g + kRingUnit - 1 of the
 // domain's ring cells.  `tides` holds this step's bc_ssh value per domain.
+constexpr int kRingUnit = 256;
 template <class T, bool IC>
-__global__ void __launch_bounds__(NTHREADS, T::kMinBlocks)
+__global__ void __launch_bounds__(T::NTHREADS, T::kMinBlocks)
     k_ensemble_step(const EnsDomain* __restrict__ doms, const int4* __restrict__ tiles,
                     const int* __restrict__ first, int parity,
                     const double* __restrict__ tides) {
@@ -116,12 +117,8 @@ __global__ void __launch_bounds__(NTHREADS, T::kMinBlocks)
 __device__ __forceinline__ void ring_cell(const EnsDomain* __restrict__ doms, int2 e, int part,
                                           int parity, const double* __restrict__ tides) {
   const EnsDomain& D = doms[e.x];
-  const FusedState& st = D.fs[parity];
-  const GlobalCtx x{st.sshn_in, st.un_in,   st.vn_in, D.f.hu,    D.f.hv,    D.f.ht,
-                    D.f.ssha_u, D.f.ssha_v, D.f.r_hu, D.f.r_hv,  D.f.tmask, D.f.sshn_u,
-                    D.f.sshn_v, D.d.width,  D.d,      D.k};
   const int j = e.y / D.d.width, i = e.y - j * D.d.width;
-  general_part(x, D.f, st, D.p, tides[e.x], part, i, j);
+  general_part(D.f, D.fs[parity], D.d, D.p, D.k, tides[e.x], part, i, j);
 }
 
 // One launch per step of the FP64-equivalent form.  A block takes one of two
@@ -176,9 +173,13 @@ __global__ void __launch_bounds__(32 * dfm::WARPS, 3)
 constexpr int kDefaultMarchRows = 32;
 
 // The tile shapes the ensemble's FP64 kernel is built for (the autotuner's
-// search space); shape 0 is the single-domain kernel's.
+// search space).  Until it or the caller chooses, 32 x 8 with one tile per CTA
+// (the fastest or within 5 % of it from rest and in motion: 8 domains of 256^2
+// in motion 85.6 us per step, 32 x 16 in contiguous chunks 103.8; from rest
+// 159 and 265).
 constexpr int kNumShapes = 5;
 constexpr int kShapes[kNumShapes][2] = {{32, 16}, {32, 8}, {16, 16}, {64, 8}, {32, 32}};
+constexpr int kDefaultShape = 1;
 
 template <class T>
 bool set_ens_attr() {
@@ -197,8 +198,8 @@ bool set_ens_attr() {
 // stream capture).
 bool prepare_ens_step(int shape) {
   switch (shape) {
-    case 1: return set_ens_attr<Tile<32, 8>>();
-    case 2: return set_ens_attr<Tile<16, 16>>();
+    case 1: return set_ens_attr<Tile<32, 8, 256, 3>>();
+    case 2: return set_ens_attr<Tile<16, 16, 256, 3>>();
     case 3: return set_ens_attr<Tile<64, 8>>();
     case 4: return set_ens_attr<Tile<32, 32>>();
     default: return set_ens_attr<DefaultTile>();
@@ -218,8 +219,8 @@ void launch_ens_step(int shape, bool int_mul, int nctas, const EnsDomain* doms,
                      cudaStream_t st) {
   auto launch = launch_ens_step_shape<DefaultTile>;
   switch (shape) {
-    case 1: launch = launch_ens_step_shape<Tile<32, 8>>; break;
-    case 2: launch = launch_ens_step_shape<Tile<16, 16>>; break;
+    case 1: launch = launch_ens_step_shape<Tile<32, 8, 256, 3>>; break;
+    case 2: launch = launch_ens_step_shape<Tile<16, 16, 256, 3>>; break;
     case 3: launch = launch_ens_step_shape<Tile<64, 8>>; break;
     case 4: launch = launch_ens_step_shape<Tile<32, 32>>; break;
     default: break;
@@ -306,7 +307,7 @@ struct Ens {
   EnsDomain* d_desc = nullptr;
   int4* d_tiles = nullptr;
   int* d_first = nullptr;
-  int ntiles = 0, nctas = 0, ctas_per_sm = 2, policy = 0;
+  int ntiles = 0, nctas = 0, ctas_per_sm = 2, policy = 2;
   double boundary_weight = 4.0;
   double* d_tides = nullptr;
   size_t tides_cap = 0;
@@ -322,7 +323,7 @@ struct Ens {
   int graph_key[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
   bool built = false;
   bool int_mul = false;  // every domain's constants have the integer form
-  int shape = 0;        // index into kShapes: the FP64 kernel's tile
+  int shape = kDefaultShape;  // index into kShapes: the FP64 kernel's tile
   int march_rows = kDefaultMarchRows;  // strip height of the column marches
   // mixed-precision form
   int precision = 0;
@@ -434,7 +435,7 @@ void ens_free() {
   e.built = false;
   e.ndom = 0;
   e.dom.clear();
-  e.shape = 0;
+  e.shape = kDefaultShape;
   e.march_rows = kDefaultMarchRows;
 }
 
@@ -485,8 +486,8 @@ bool build_schedule(int TXv, int TYv) {
     const DomainHost& D = e.dom[k];
     const Dims d{D.xs, D.xe, D.ys, D.ye, D.W, D.H};
     const int nr = kParts * ring_count(d, D.ys - 1, D.ye + 1);
-    for (int g = 0; g < nr; g += NTHREADS)
-      tiles.push_back({k, 0, 0, g, e.boundary_weight * std::min(NTHREADS, nr - g) / kParts});
+    for (int g = 0; g < nr; g += kRingUnit)
+      tiles.push_back({k, 0, 0, g, e.boundary_weight * std::min(kRingUnit, nr - g) / kParts});
     const int nx = D.xe - D.xs - 1, ny = D.ye - D.ys - 1;
     if (nx < 1 || ny < 1) continue;
     const int ntx = (nx + TXv - 1) / TXv, nty = (ny + TYv - 1) / TYv;

@@ -17,8 +17,8 @@
 //    x = +-0 returns x.  Dividends whose magnitude is tiny (below 2^-899,
 //    other than zero), huge (2^900 and above) or not finite use the IEEE
 //    divide, so no result leaves the normal range.
-//  * mul_core: x * c for a step constant c of at most 32 significant bits,
-//    in integers.
+//  * mul_bounded, div_bounded, upwind_bounded: the operations of the tiles'
+//    straight-line code, on operands whose range has been tested.
 //  * half(x): 0.5 * x.  For normal x with a biased exponent >= 2 this is
 //    exact, i.e. the exponent minus one, done in integer arithmetic; zero
 //    keeps its bits; subnormal, smallest-normal and non-finite x use DMUL.
@@ -73,27 +73,36 @@ __host__ __device__ __forceinline__ unsigned long long recip64_of(double d) {
   return recip64((b & 0xfffffffffffffULL) | (1ULL << 52));
 }
 
-// The quotient's bits for a dividend of biased exponent 124 .. 1922 (bits
-// xb), the divisor's significand md, its reciprocal rc and what the
-// quotient's exponent field gains, `add` = (1023 - the divisor's biased
-// exponent - 2) << 20.  With mx the dividend's significand, t = hi64(2^11 mx
-// rc) is mx / md 2^63 to within 4 units below (the low partial product is
-// left out): its leading bit says whether mx >= md, and q, its top 53 bits,
-// is less than 1.01 below the quotient mx 2^s / md (s = 52 or 53).  The
-// remainder mx 2^s - q md is below 2^54, so its low 64 bits are all of it,
-// and q rounds up exactly when it is above md / 2 (a quotient of two
-// significands is never a midpoint).
-__device__ __forceinline__ double div_core(unsigned long long xb, unsigned long long md,
-                                           unsigned long long rc, unsigned add) {
+// The significand q in [2^52, 2^53] of x / d rounded to nearest, for a
+// normal x (bits xb), the divisor's significand md and its reciprocal rc; top
+// = 1 where x's significand is at least d's.  With mx the dividend's
+// significand, t = hi64(2^11 mx rc) is mx / md 2^63 to within 4 units below
+// (the low partial product is left out): its leading bit says whether mx >=
+// md, and its top 53 bits are less than 1.01 below the quotient mx 2^s / md
+// (s = 52 or 53).  The remainder mx 2^s - q md is below 2^54, so its low 64
+// bits are all of it, and q rounds up exactly when it is above md / 2 (a
+// quotient of two significands is never a midpoint).
+__device__ __forceinline__ unsigned long long div_significand(unsigned long long xb,
+                                                              unsigned long long md,
+                                                              unsigned long long rc,
+                                                              unsigned& top) {
   const unsigned xl = (unsigned)xb, xh = (unsigned)(xb >> 32);
   const unsigned rl = (unsigned)rc, rh = (unsigned)(rc >> 32);
   const unsigned ah = __funnelshift_l(xl, xh, 11) | 0x80000000u, al = xl << 11;
   const unsigned long long t = (unsigned long long)ah * rh + __umulhi(ah, rl) + __umulhi(al, rh);
-  const unsigned top = (unsigned)(t >> 32) >> 31;
+  top = (unsigned)(t >> 32) >> 31;
   unsigned long long q = t >> (10 + top);
   const unsigned long long rem = ((unsigned long long)(xl << (21 - top)) << 32) - q * md;
   if ((long long)rem > (long long)(md >> 1)) q++;
-  const unsigned eh = (xh & 0xfff00000u) + add + (top << 20);
+  return q;
+}
+// The quotient for a dividend of biased exponent 124 .. 1922; add = (1023 -
+// the divisor's biased exponent - 2) << 20 is what its exponent field gains.
+__device__ __forceinline__ double div_core(unsigned long long xb, unsigned long long md,
+                                           unsigned long long rc, unsigned add) {
+  unsigned top;
+  const unsigned long long q = div_significand(xb, md, rc, top);
+  const unsigned eh = ((unsigned)(xb >> 32) & 0xfff00000u) + add + (top << 20);
   return from_bits((long long)(q + ((unsigned long long)eh << 32)));
 }
 
@@ -124,18 +133,30 @@ __device__ __forceinline__ double div_depth(double x, double d, unsigned long lo
 
 // A constant factor c > 0 in [2^-100, 2^100] of at most 32 significant bits
 // (grid spacings and time steps in whole or simply fractional units), as
-// mul_core takes it: co 2^e with co in [2^31, 2^32), and what the product's
+// mul_bounded takes it: co 2^e with co in [2^31, 2^32), and what the product's
 // exponent field gains.  co = 0: c is not of that kind.
 struct IntFactor {
   unsigned co, add;
 };
 
-// RN(x * c) in integers: the product of the significands (85 bits) is exact
-// in three words, normalised by its leading bit and rounded to nearest even;
-// about 20 instructions on the integer pipes, where the DMUL holds a
-// scheduler's share of the FP64 pipe for 64 issue slots.  x normal, the
-// product too.
-__device__ __forceinline__ double mul_core(unsigned long long xb, IntFactor f) {
+// The bounded forms, for straight-line code (a range branch per operation
+// would keep the compiler from interleaving independent chains): operands are
+// +-0 or normal, results too.
+//
+// The result with exponent field e (less q's leading bit), sign bit sign,
+// significand q in [2^52, 2^53].
+__device__ __forceinline__ double bounded_result(bool zero, unsigned sign, unsigned e,
+                                                 unsigned long long q) {
+  const unsigned long long r = q + ((unsigned long long)(e + sign) << 32);
+  return from_bits((long long)(zero ? (unsigned long long)sign << 32 : r));
+}
+
+// RN(x * c): the product of the significands (85 bits) is exact in three
+// words, normalised by its leading bit and rounded to nearest even.  About 25
+// instructions on the integer pipes, where a DMUL holds its scheduler's FP64
+// unit for 64 clocks.
+__device__ __forceinline__ double mul_bounded(double x, IntFactor f) {
+  const unsigned long long xb = (unsigned long long)bits(x);
   const unsigned xl = (unsigned)xb, xh = (unsigned)(xb >> 32);
   const unsigned long long p = (unsigned long long)xl * f.co;
   const unsigned long long t =
@@ -146,30 +167,13 @@ __device__ __forceinline__ double mul_core(unsigned long long xb, IntFactor f) {
   const unsigned frac = w0 << s;
   unsigned long long q = ((unsigned long long)qh << 32) | ql;
   if (frac > 0x80000000u - (ql & 1u)) q++;  // above half, or half and odd
-  const unsigned eh = (xh & 0xfff00000u) + f.add + (top << 20);
-  return from_bits((long long)(q + ((unsigned long long)eh << 32)));
+  const unsigned ex = xh & 0x7ff00000u;
+  return bounded_result(ex == 0, xh & 0x80000000u, ex + f.add + (top << 20), q);
 }
 
-// The bounded forms, for straight-line code on operands known to be +-0 or
-// normal with a normal result: no range test, +-0 selected (a branch per
-// operation would keep the compiler from interleaving independent chains).
-__device__ __forceinline__ double zero_or(double x, double y) {  // x if x is +-0, else y
-  return ((unsigned)((unsigned long long)bits(x) >> 32) & 0x7ff00000u) == 0 ? x : y;
-}
-__device__ __forceinline__ double mul_bounded(double x, IntFactor f) {
-  return zero_or(x, mul_core((unsigned long long)bits(x), f));
-}
-__device__ __forceinline__ double div_bounded(double x, const IntDivisor& v) {
-  return zero_or(x, div_core((unsigned long long)bits(x), v.md, v.rc, v.add));
-}
-__device__ __forceinline__ double div_bounded(double x, double d, unsigned long long rc) {
-  const unsigned long long db = (unsigned long long)bits(d);
-  return zero_or(x, div_core((unsigned long long)bits(x), (db & 0xfffffffffffffULL) | (1ULL << 52),
-                             rc, (1021u << 20) - ((unsigned)(db >> 32) & 0x7ff00000u)));
-}
 // RN(x * y): the 106-bit product of the significands in four words (x's
 // aligned so that the leading bit is bit 116 or 115), rounded to nearest
-// even; about 30 instructions.
+// even; about 35 instructions.
 __device__ __forceinline__ double mul_bounded(double x, double y) {
   const unsigned long long xb = (unsigned long long)bits(x), yb = (unsigned long long)bits(y);
   const unsigned xl = (unsigned)xb, xh = (unsigned)(xb >> 32);
@@ -188,15 +192,31 @@ __device__ __forceinline__ double mul_bounded(double x, double y) {
   unsigned long long q = ((unsigned long long)qh << 32) | ql;
   const unsigned most = (f0 | (ql & 1u)) ? 0x7fffffffu : 0x80000000u;
   if (f1 > most) q++;  // above half, or half and odd
-  const unsigned sign = (xh ^ yh) & 0x80000000u;
-  const unsigned eh =
-      sign + (xh & 0x7ff00000u) + (yh & 0x7ff00000u) + (top << 20) - (1024u << 20);
-  const bool zero = (xh & 0x7ff00000u) == 0 || (yh & 0x7ff00000u) == 0;
-  const unsigned long long r = q + ((unsigned long long)eh << 32);
-  return from_bits((long long)(zero ? (unsigned long long)sign << 32 : r));
+  const unsigned ex = xh & 0x7ff00000u, ey = yh & 0x7ff00000u;
+  return bounded_result(ex == 0 || ey == 0, (xh ^ yh) & 0x80000000u,
+                        ex + ey + (top << 20) - (1024u << 20), q);
 }
-// upwind() for finite operands: the picked one, or, where that is a zero, a
-// zero with the AND of both signs.
+
+// RN(x / d), see div_core.
+__device__ __forceinline__ double div_bounded(double x, unsigned long long md,
+                                              unsigned long long rc, unsigned add) {
+  const unsigned long long xb = (unsigned long long)bits(x);
+  const unsigned xh = (unsigned)(xb >> 32);
+  const unsigned ex = xh & 0x7ff00000u;
+  unsigned top;
+  const unsigned long long q = div_significand(xb, md, rc, top);
+  return bounded_result(ex == 0, xh & 0x80000000u, ex + add + (top << 20), q);
+}
+__device__ __forceinline__ double div_bounded(double x, const IntDivisor& v) {
+  return div_bounded(x, v.md, v.rc, v.add);
+}
+__device__ __forceinline__ double div_bounded(double x, double d, unsigned long long rc) {
+  const unsigned long long db = (unsigned long long)bits(d);
+  return div_bounded(x, (db & 0xfffffffffffffULL) | (1ULL << 52), rc,
+                     (1021u << 20) - ((unsigned)(db >> 32) & 0x7ff00000u));
+}
+// upwind() for operands that are +-0 or normal: the picked one, or, where
+// that is a zero, a zero with the AND of both signs.
 __device__ __forceinline__ double upwind_bounded(double w, double p, double q) {
   const bool neg = bits(w) < 0;
   const unsigned long long a = (unsigned long long)bits(neg ? p : q),
@@ -205,11 +225,11 @@ __device__ __forceinline__ double upwind_bounded(double w, double p, double q) {
   const unsigned h = (ah & 0x7ff00000u) == 0 ? ah & zh : ah;
   return from_bits((long long)(((unsigned long long)h << 32) | (unsigned)a));
 }
-// Whether x is neither +-0 nor of magnitude in [2^-n, 2^n).
-__device__ __forceinline__ bool beyond(double x, unsigned n) {
+// Whether x is neither +-0 nor of magnitude in [2^-lo, 2^hi).
+__device__ __forceinline__ bool beyond(double x, unsigned lo, unsigned hi) {
   const unsigned h = (unsigned)((unsigned long long)bits(x) >> 32);
   const bool zero = ((unsigned)bits(x) | (h << 1)) == 0;
-  return !zero && ((h >> 20) & 0x7ffu) - (1023u - n) >= 2u * n;
+  return !zero && ((h >> 20) & 0x7ffu) - (1023u - lo) >= lo + hi;
 }
 
 __device__ __forceinline__ double half(double x) {

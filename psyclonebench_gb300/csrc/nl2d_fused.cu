@@ -32,18 +32,22 @@
 namespace nl2d {
 namespace {
 
-using T = DefaultTile;
-// Domains too small to give every SM a few 32 x 16 tiles take 16 x 16 ones:
-// one cell per thread instead of two, twice the tiles, the same bits (the
-// arithmetic does not depend on the shape).
-using SmallTile = Tile<16, 16>;
+// 32 x 8 cells, one per thread, three CTAs per SM (80 registers): the integer
+// forms' long dependency chains need warps more than they need a second cell
+// per thread (2048^2: 32 x 16 and two CTAs 597 us, 16 x 16 and three 540,
+// 32 x 12 and two CTAs of 384 threads 565, 32 x 8 and two 620, three 537).
+using T = Tile<32, 8, 256, 3>;
+// Domains too small to give every SM a few of those take 16 x 8 cells and 128
+// threads: twice the tiles, the same bits (the arithmetic does not depend on
+// the shape; 256^2: 19.4 us with 16 x 16, 16.3 with 16 x 8).
+using SmallTile = Tile<16, 8, 128, 4>;
 
 // One step of copy-region rows [ja, jb).  The first nring blocks take the
 // ring's cells in those rows, rc parts of them each (one per thread: their
 // long FP64 chains start first and run beside the tiles); the others one tile
 // each of the ntx per row of tiles, from tile row row0.
 template <class TT, bool IC>
-__global__ void __launch_bounds__(NTHREADS, TT::kMinBlocks)
+__global__ void __launch_bounds__(TT::NTHREADS, TT::kMinBlocks)
     k_fused_step(const __grid_constant__ Fields f, const __grid_constant__ FusedState fs,
                  const __grid_constant__ Dims d, const __grid_constant__ Scalars p,
                  const __grid_constant__ FastConst k, const double* __restrict__ tide_table,
@@ -71,7 +75,6 @@ int tiles_over(int n, int t) { return n > 0 ? (n + t - 1) / t : 0; }
 int interior_x(const Dims& d) { return d.xe - d.xs - 1; }
 int interior_y(const Dims& d) { return d.ye - d.ys - 1; }
 
-// Domains too small for four 32 x 16 tiles per SM take 16 x 16 tiles.
 bool small_tiles(const Dims& d) {
   return (long long)tiles_over(interior_x(d), T::TX) * tiles_over(interior_y(d), T::TY) <
          4LL * 152;
@@ -90,7 +93,7 @@ void launch_rows(const Fields& f, const FusedState& fs, const Dims& d, const Sca
   // block per SM: each is ~100 dependent FP64 operations.
   const int nr = kParts * ring_count(d, ja, jb);
   int rc = 32;
-  while (rc < NTHREADS && nr > rc * 152) rc *= 2;
+  while (rc < TT::NTHREADS && nr > rc * 152) rc *= 2;
   const int nring = (nr + rc - 1) / rc;
   const FastConst k = make_fast_const(s, um);
   auto step = k.int_mul ? k_fused_step<TT, true> : k_fused_step<TT, false>;
@@ -208,12 +211,13 @@ __global__ void k_selftest_exact(long long n, unsigned long long seed, IntDiviso
     const double q_ref = x / d;
     for (const double q : {div_const(x, v), div_depth(x, d, v.rc)})
       if (bits(q_ref) != bits(q) && !(q_ref != q_ref && q != q)) nd++;
-    const bool in = !beyond(x, 899);  // the bounded forms' operands, for any d
-    if (in && (bits(div_bounded(x, v)) != bits(q_ref) ||
-               bits(div_bounded(x, d, v.rc)) != bits(q_ref)))
-      nd++;
-    // the product with d (counted with the quotients), where d has that form
-    if (in && fac.co != 0 && bits(mul_bounded(x, fac)) != bits(x * d)) nd++;
+    // the bounded forms on zeros and normal operands with normal results
+    if (!beyond(x, 900, 900)) {
+      if (bits(div_bounded(x, v)) != bits(q_ref) || bits(div_bounded(x, d, v.rc)) != bits(q_ref))
+        nd++;
+      // the product with d (counted with the quotients), where d has that form
+      if (fac.co != 0 && bits(mul_bounded(x, fac)) != bits(x * d)) nd++;
+    }
     // Quotients within ~2^-53 ulp of a midpoint: RN((Q + ulp(Q)/2) * d) and
     // its neighbours; quotients at and next to a power of two.
     {
@@ -236,18 +240,23 @@ __global__ void k_selftest_exact(long long n, unsigned long long seed, IntDiviso
     if (bits(h_ref) != bits(h) && !(h_ref != h_ref && h != h)) nh++;
     const double p = sample(mix64(z + 1)), w = sample(mix64(z + 2));
     const double u_ref = (0.5 - copysign(0.5, w)) * x + (0.5 + copysign(0.5, w)) * p;
-    // products of operands whose product is normal (counted with the picks)
-    if (!beyond(x, 500) && !beyond(p, 500) && bits(mul_bounded(x, p)) != bits(x * p)) nu++;
+    // products (counted with the picks): of x and p, and of moderate operands
+    // with full, short and trailing significands
     {
+      auto wrong = [](double a, double c) {
+        return !beyond(a, 1022, 1024) && !beyond(c, 1022, 1024) && !beyond(a * c, 1022, 1024) &&
+               ((a * c != 0.0) || a == 0.0 || c == 0.0) && bits(mul_bounded(a, c)) != bits(a * c);
+      };
       const unsigned long long y = mix64(z + 5);
-      const double f = from_bits((long long)((y & 0x800fffffffffffffULL) | (1000ULL + (y >> 53) % 40) << 52));
+      const double f = from_bits((long long)((y & 0x800fffffffffffffULL) |
+                                             (1000ULL + (y >> 53) % 40) << 52));
       const double s1 = from_bits((bits(f) >> (y % 53)) << (y % 53));  // a short significand
       const double g = from_bits((bits(x) & 0x800fffffffffffffLL) | (1020LL << 52));
-      if (bits(mul_bounded(f, g)) != bits(f * g) || bits(mul_bounded(g, s1)) != bits(g * s1)) nu++;
+      if (wrong(x, p) || wrong(f, g) || wrong(g, s1) || wrong(s1, s1)) nu++;
     }
     const double u = upwind(w, x, p);
     if (bits(u_ref) != bits(u) && !(u_ref != u_ref && u != u)) nu++;
-    if (!beyond(x, 899) && !beyond(p, 899) && bits(upwind_bounded(w, x, p)) != bits(u_ref)) nu++;
+    if (!beyond(x, 1022, 1024) && !beyond(p, 1022, 1024) && bits(upwind_bounded(w, x, p)) != bits(u_ref)) nu++;
   }
   if (nd) atomicAdd(&bad[0], nd);
   if (nh) atomicAdd(&bad[1], nh);

@@ -4,6 +4,7 @@
 // is bit-identical to the reference.
 #pragma once
 #include <cstring>
+#include <type_traits>
 
 #include "nl2d_exact.cuh"
 #include "nl2d_internal.h"
@@ -21,24 +22,30 @@ namespace {
 // per-cell code, a long FP64 chain, and are taken one per thread by blocks of
 // their own that run beside the tiles.  The arithmetic does not depend on
 // the split.
-constexpr int NTHREADS = 256;
 
 // A constant factor of the tiles: c and its integer form.
 //
-// The tiles' regular update is straight-line code without range tests, on
-// fields (ssh, u, v and the depths) that are +-0 or of magnitude in [2^-200,
-// 2^200), and constants in [2^-40, 2^40].  Then every nonzero sum of fields is
-// at least 2^-252, a face height 2^-333, a total depth or a sum of them
-// 2^-385, and the smallest product formed (an advective flux: velocity, face
-// speed, depth) 2^-880: normal, so a power of two may move from an operand to
-// a constant without changing a bit.  Tendencies and momenta can cancel below
-// that, and are tested (2^-699) before they are scaled.  A tile with another
-// field, and a cell with another tendency, takes the general code.
+// Where every field a tile reads (ssh, u, v, the depths, stored face heights)
+// is +-0 or of magnitude in [2^-200, 2^200) and the constants lie in [2^-40,
+// 2^40], its update is straight-line code in the bounded forms
+// (nl2d_exact.cuh): no product overflows (the largest, an advective flux, is
+// below 2^730), every nonzero sum of fields is at least 2^-252, a face height
+// 2^-333, a sum of depths 2^-385, and the smallest product (an advective
+// flux: velocity, face speed, depth) 2^-880, normal, so a power of two may
+// move between an operand and a constant without changing a bit.  Tendencies
+// and momenta can cancel below that and are tested before they are scaled.
+//
+// Other tiles ("wide") run the same update with the plain operations and the
+// exact helpers that branch to the IEEE ones.  From rest the tide sends ahead
+// of it values that fall by five decades per cell down to the smallest
+// subnormal, for thousands of steps: half of a 128^2 domain holds values
+// below 2^-200 after 1000 steps, so this form matters too (per-cell fallback
+// to the general code made steps from rest up to 4 times slower).
 struct Factor {
   double c;
   IntFactor i;
 };
-constexpr unsigned kFieldRange = 200, kTendRange = 699;
+__device__ __forceinline__ bool out_of_range(double field) { return beyond(field, 200, 200); }
 
 // Step-invariant constants of the fast path, evaluated on the host with the
 // operations the reference performs per point (e.g. dx_v[c] + dx_v[e] on a
@@ -115,6 +122,11 @@ struct GlobalCtx {
   const Dims& d;
   const FastConst& k;
 
+  __device__ __forceinline__ GlobalCtx(const Fields& f, const FusedState& fs, const Dims& dd,
+                                       const FastConst& kk)
+      : sn(fs.sshn_in), un(fs.un_in), vn(fs.vn_in), hu(f.hu), hv(f.hv), ht(f.ht),
+        ssha_u(f.ssha_u), ssha_v(f.ssha_v), r_hu(f.r_hu), r_hv(f.r_hv), m(f.tmask), sshn_u(f.sshn_u), sshn_v(f.sshn_v), W(dd.width), d(dd), k(kk) {}
+
   __device__ __forceinline__ bool in_copy(int i, int j) const {
     return i >= d.xs - 1 && i <= d.xe + 1 && j >= d.ys - 1 && j <= d.ye;
   }
@@ -170,8 +182,7 @@ __device__ __forceinline__ double hi_only(double w, double p) {
 // range, with the masked (slip-wall) branches; returns false where the
 // kernel returns early (ua keeps its value).  Same operations as the
 // reference, with the exact helpers for halving, upwind picks and division.
-template <class X>
-__device__ __forceinline__ bool mom_u(const X& x, int i, int j, double& out) {
+__device__ __forceinline__ bool mom_u(const GlobalCtx& x, int i, int j, double& out) {
   const int W = x.W, c = j * W + i, e = c + 1, wst = c - 1, s = c - W, n = c + W,
             se = s + 1, ne = n + 1;
   const FastConst& k = x.k;
@@ -240,8 +251,7 @@ __device__ __forceinline__ bool mom_u(const X& x, int i, int j, double& out) {
 }
 
 // momentum_v_code (momentum_v_kern.c:125-241) at v face (i,j).
-template <class X>
-__device__ __forceinline__ bool mom_v(const X& x, int i, int j, double& out) {
+__device__ __forceinline__ bool mom_v(const GlobalCtx& x, int i, int j, double& out) {
   const int W = x.W, c = j * W + i, e = c + 1, wst = c - 1, s = c - W, n = c + W,
             nw = n - 1, ne = n + 1;
   const FastConst& k = x.k;
@@ -311,9 +321,8 @@ __device__ __forceinline__ bool mom_v(const X& x, int i, int j, double& out) {
 // ua at u face (i,j) after momentum_u and bc_solid_u, before Flather: the
 // value bc_flather_u reads.  On the copy region the previous step's ua is
 // the current un; elsewhere it is the ua array, which no fused step changes.
-template <class X>
-__device__ __forceinline__ double ua_pre_flather(const X& x, const double* ua_arr,
-                                                 int i, int j) {
+__device__ __forceinline__ double ua_pre_flather(const GlobalCtx& x, const double* ua_arr, int i,
+                                                 int j) {
   const int c = j * x.W + i;
   double ua = x.in_copy(i, j) ? x.un[c] : ua_arr[c];
   if (i >= x.d.xs && i <= x.d.xe - 1 && j >= x.d.ys && j <= x.d.ye) {
@@ -326,9 +335,8 @@ __device__ __forceinline__ double ua_pre_flather(const X& x, const double* ua_ar
   return ua;
 }
 
-template <class X>
-__device__ __forceinline__ double va_pre_flather(const X& x, const double* va_arr,
-                                                 int i, int j) {
+__device__ __forceinline__ double va_pre_flather(const GlobalCtx& x, const double* va_arr, int i,
+                                                 int j) {
   const int c = j * x.W + i;
   double va = x.in_copy(i, j) ? x.vn[c] : va_arr[c];
   if (i >= x.d.xs && i <= x.d.xe && j >= x.d.ys && j <= x.d.ye - 1) {
@@ -348,14 +356,15 @@ __device__ __forceinline__ double va_pre_flather(const X& x, const double* va_ar
 // bc_flather_u), sea-surface height (continuity_kern.c:90-117, then bc_ssh).
 // A Flather face takes the momentum of the face next to it instead of its
 // own (bc_flather replaces it), so each part evaluates one momentum update.
+// (The IEEE operations and branching helpers here, not the tiles' bounded
+// forms: with those a small domain's step was no shorter, and the
+// FP64-equivalent form's, whose march fills the integer pipes, 4 % longer.)
 enum { kPartV, kPartU, kPartSsh, kParts };
-template <class X>
-__device__ __forceinline__ void general_part(const X& x, const Fields& f, const FusedState& fs,
-                                             const Scalars& p, double tide, int part, int i,
-                                             int j) {
-  const int W = x.W;
-  const Dims& d = x.d;
-  const FastConst& k = x.k;
+__device__ __forceinline__ void general_part(const Fields& f, const FusedState& fs,
+                                             const Dims& d, const Scalars& p, const FastConst& k,
+                                             double tide, int part, int i, int j) {
+  const GlobalCtx x(f, fs, d, k);
+  const int W = d.width;
   const int* __restrict__ m = x.m;
   const int c = j * W + i;
 
@@ -405,17 +414,14 @@ __device__ __forceinline__ void general_part(const X& x, const Fields& f, const 
   }
 }
 
-// general_part on the domain's arrays, out of line: the tiles' registers are
-// sized by the regular update, and the few land-side cells of a tile and the
-// ring's cells share one copy of the code.
+// general_part out of line: the tiles' registers are sized by the regular
+// update, and the few land-side cells of a tile and the ring's cells share
+// one copy of the code.
 static __device__ __noinline__ void general_at(const Fields& f, const FusedState& fs,
                                                const Dims& d, const Scalars& p,
                                                const FastConst& k, double tide, int part, int i,
                                                int j) {
-  const GlobalCtx x{fs.sshn_in, fs.un_in, fs.vn_in, f.hu,     f.hv,     f.ht,
-                    f.ssha_u,   f.ssha_v, f.r_hu,   f.r_hv,   f.tmask,  f.sshn_u,
-                    f.sshn_v,   d.width,  d,        k};
-  general_part(x, f, fs, p, tide, part, i, j);
+  general_part(f, fs, d, p, k, tide, part, i, j);
 }
 
 // The ring: the copy region's cells outside the interior, rows ys-1, ys, ye
@@ -454,33 +460,46 @@ __host__ __device__ __forceinline__ void ring_pos(const Dims& d, int ja, int jb,
 // Shared-memory layout of one tile, all on the tile plus one cell on each
 // side: the loaded fields and the sshn_u / sshn_v this step sees, then the
 // terms that two neighbouring updates share.
-enum { A_SN, A_UN, A_VN, A_HU, A_HV, A_SU, A_SV, A_HUS, A_HVS, N_A0 };
+enum { A_SN, A_UN, A_VN, A_HU, A_HV, A_HT, A_SU, A_SV, A_HUS, A_HVS, N_A0 };
 enum { B_FLXU, B_FLXV, B_GX, B_GY, B_FXU, B_FYV, B_VS2, B_FYU, B_QY, B_UW2, B_FXV, B_QX, N_B1 };
 // area_t * sshn_t, needed until the face values are formed, shares the slot
 // of a term that is formed after them
 constexpr int B_AREA_SSH = B_QX;
 
-template <int TX_, int TY_>
+// NT threads per CTA.  MB: CTAs per SM to hold the registers to, 0 for what
+// the shared memory allows, up to two.
+template <int TX_, int TY_, int NT = 256, int MB = 0>
 struct Tile {
-  static constexpr int TX = TX_, TY = TY_;
+  static constexpr int TX = TX_, TY = TY_, NTHREADS = NT;
   static constexpr int RPP = NTHREADS / TX;  // rows per pass of the thread block
   static constexpr int RPT = TY / RPP;       // cells per thread in the update phase
   static_assert(NTHREADS % TX == 0 && TY % RPP == 0 && (RPT == 1 || RPT == 2 || RPT == 4),
                 "tile shape");
   static constexpr int SX = TX + 2, SY = TY + 2;
   static constexpr int S0 = SX * SY;  // staged positions (34 x 18 for 32 x 16)
-  // + the mask, and the list of the tile's general (non-regular) cells
+  // + the mask, the list of the tile's general (non-regular) cells
   static constexpr size_t kSmemBytes =
-      sizeof(double) * (N_A0 + N_B1) * S0 + sizeof(int) * (S0 + TX * TY + 2);
-  // two CTAs of 256 threads per SM when their shared memory (with the 1 KB
-  // the driver reserves per CTA) fits the SM's 228 KB
-  static constexpr int kMinBlocks = 2 * (kSmemBytes + 1024) <= 228 * 1024 ? 2 : 1;
+      sizeof(double) * (N_A0 + N_B1) * S0 + sizeof(int) * (S0 + TX * TY + 1);
+  // shared memory per CTA (with the 1 KB the driver reserves) against the
+  // SM's 228 KB
+  static constexpr int kMinBlocks = MB > 0 ? MB : 2 * (kSmemBytes + 1024) <= 228 * 1024 ? 2 : 1;
+  static_assert(kMinBlocks * (kSmemBytes + 1024) <= 228 * 1024 || kMinBlocks == 1, "tile shape");
   // Items along the tile's edges are handled by whole warps: an edge's items
   // start at a multiple of 32 of the thread index.
   static constexpr int RX = (TX + 31) / 32 * 32, RY = (TY + 31) / 32 * 32,
                        RY1 = (TY + 32) / 32 * 32;
 };
 using DefaultTile = Tile<32, 16>;
+
+template <class T>
+struct TileSmem {
+  double *a0, *b1;       // [N_A0][S0], [N_B1][S0]
+  int* mk;               // [S0] the mask
+  int *glist, *gcount;   // [TX * TY] the tile's general cells, their number
+  __device__ __forceinline__ explicit TileSmem(double* smem)
+      : a0(smem), b1(smem + N_A0 * T::S0), mk((int*)(b1 + N_B1 * T::S0)), glist(mk + T::S0),
+        gcount(glist + T::TX * T::TY) {}
+};
 
 // A regular cell's new (sshn_t, un, vn) from the tile's staged fields (a0)
 // and shared terms (b1) at its slot q: continuity (continuity_kern.c:90-117)
@@ -521,7 +540,7 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
     const double tend = ((adv + vis) + cor) + hpg;
     const double num =
         mul_bounded(A(A_UN, q), Hu) + div_bounded(mlc<IC>(tend, k.f_rdt), k.q_area_u);
-    o.bad |= beyond(tend, kTendRange) || beyond(num, kTendRange);
+    o.bad |= beyond(tend, 699, 699) || beyond(num, 699, 699);
     o.u = div_bounded(div_bounded(num, dhu, rhu), k.q_fric);
   }
   {
@@ -539,8 +558,49 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
     const double tend = ((adv + vis) + cor) + hpg;
     const double num =
         mul_bounded(A(A_VN, q), Hv) + div_bounded(mlc<IC>(tend, k.f_rdt), k.q_area_v);
-    o.bad |= beyond(tend, kTendRange) || beyond(num, kTendRange);
+    o.bad |= beyond(tend, 699, 699) || beyond(num, 699, 699);
     o.v = div_bounded(div_bounded(num, dhv, rhv), k.q_fric);
+  }
+  return o;
+}
+
+// The same in the plain operations and the helpers that take any value.
+template <class T>
+__device__ __forceinline__ RegOut regular_cell_any(const double* a0, const double* b1, int q,
+                                                   double dhu, unsigned long long rhu, double dhv,
+                                                   unsigned long long rhv, const FastConst& k) {
+  constexpr int S0 = T::S0, SX = T::SX;
+  RegOut o;
+  o.bad = false;
+  const double snc = A(A_SN, q), Hu = A(A_HUS, q), Hv = A(A_HVS, q);
+  const double ssh = (((B(B_FLXU, q - 1) - B(B_FLXU, q)) + B(B_FLXV, q - SX)) - B(B_FLXV, q)) *
+                     k.rdt;
+  o.ssh = snc + dvc(ssh, k.q_area_t, k.fast_div);
+  {
+    const double adv = ((B(B_FXU, q) - B(B_FXU, q + 1)) + B(B_FYU, q)) - B(B_FYU, q + SX);
+    const double dudy_s = B(B_QY, q) * ((Hu + A(A_HU, q - SX)) + A(A_SU, q - SX));
+    const double dudy_n = B(B_QY, q + SX) * ((Hu + A(A_HU, q + SX)) + A(A_SU, q + SX));
+    double vis = (B(B_GX, q + 1) - B(B_GX, q)) * k.dy_u + half((dudy_n - dudy_s) * k.dx_u);
+    vis = k.visc * vis;
+    const double cor = (half(k.cor_u * (B(B_VS2, q) + B(B_VS2, q + SX))) * k.area_u) * Hu;
+    const double hpg = ((k.neg_g * Hu) * k.dy_u) * (A(A_SN, q + 1) - snc);
+    const double num =
+        A(A_UN, q) * Hu + dvc(k.rdt * (((adv + vis) + cor) + hpg), k.q_area_u, k.fast_div);
+    const double t1 = dvf(num, dhu, rhu);
+    o.u = dvc(t1, k.q_fric, k.fast_div);
+  }
+  {
+    const double adv = ((B(B_FXV, q) - B(B_FXV, q + 1)) + B(B_FYV, q)) - B(B_FYV, q + SX);
+    const double dvdx_w = B(B_QX, q) * ((Hv + A(A_HV, q - 1)) + A(A_SV, q - 1));
+    const double dvdx_e = B(B_QX, q + 1) * ((Hv + A(A_HV, q + 1)) + A(A_SV, q + 1));
+    double vis = (B(B_GY, q + SX) - B(B_GY, q)) * k.dx_v + half((dvdx_e - dvdx_w) * k.dy_v);
+    vis = k.visc * vis;
+    const double cor = (-half(k.cor_v * (B(B_UW2, q + 1) + B(B_UW2, q))) * k.area_v) * Hv;
+    const double hpg = ((k.neg_g * Hv) * k.dx_v) * (A(A_SN, q + SX) - snc);
+    const double num =
+        A(A_VN, q) * Hv + dvc(k.rdt * (((adv + vis) + cor) + hpg), k.q_area_v, k.fast_div);
+    const double t1 = dvf(num, dhv, rhv);
+    o.v = dvc(t1, k.q_fric, k.fast_div);
   }
   return o;
 }
@@ -553,13 +613,13 @@ __device__ __forceinline__ RegOut regular_cell(const double* a0, const double* b
 // (the face speeds of B_FXV and B_FYU carry the half of their depth's
 // average, B_VS2 and B_UW2 are twice the averaged velocities); for the other
 // update the reference evaluates the same operations on the same operands
-// (addition commuted), so the bits agree.  ht: the T depth at the cell.
+// (addition commuted), so the bits agree.
 template <class T, bool IC, bool X, bool Y>
-__device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q, double ht,
+__device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q,
                                              const FastConst& k) {
   constexpr int S0 = T::S0, SX = T::SX;
   const int qw = q - 1, qs = q - SX, qse = qs + 1, qwn = qw + SX;
-  const double D = ht + A(A_SN, q);  // ht + sshn at T(i,j)
+  const double D = A(A_HT, q) + A(A_SN, q);  // ht + sshn at T(i,j)
   const double u_c = A(A_UN, q), v_c = A(A_VN, q);
   if (X && Y) {  // continuity fluxes (sshn_u + hu) * un and (sshn_v + hv) * vn
     B(B_FLXU, q) = mul_bounded(A(A_HUS, q), u_c);
@@ -597,78 +657,78 @@ __device__ __forceinline__ void shared_terms(const double* a0, double* b1, int q
   }
 }
 
-// One tile of the fused step: interior cells [i0, i0+TX) x [j0, j0+TY) of one
-// domain.  `tide` is this step's bc_ssh value (general cells).
-//
-// The FP64 pipe bounds the step (about 1.7 instructions per clock per SM;
-// each holds a scheduler's share of it for 64 issue slots), so every phase
-// forms a value on exactly the positions that are read (a full warp per row
-// of the tile, and the edges' extra values, next column and next row, packed
-// into warps of their own), and products and quotients are formed in
-// integers: the pipe has the step's adds only, 57 of the 140 instructions per
-// cell of the form that used it for everything on 2- and 1-cell halos.  The
-// integer forms pay only as straight-line code: with a range branch each,
-// the same products made the step slower.
-template <class T, bool IC>
-__device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs, const Dims& d,
-                                           const Scalars& p, const FastConst& k, double tide,
+// The same in the plain operations and the helpers that take any value
+// (B_VS2 and B_UW2 hold the averaged velocities themselves).
+template <class T, bool X, bool Y>
+__device__ __forceinline__ void shared_terms_any(const double* a0, double* b1, int q,
+                                                 const FastConst& k) {
+  constexpr int S0 = T::S0, SX = T::SX;
+  const int qw = q - 1, qs = q - SX, qse = qs + 1, qwn = qw + SX;
+  const double D = A(A_HT, q) + A(A_SN, q);  // ht + sshn at T(i,j)
+  const double u_c = A(A_UN, q), v_c = A(A_VN, q);
+  if (X && Y) {  // continuity fluxes (sshn_u + hu) * un and (sshn_v + hv) * vn
+    B(B_FLXU, q) = A(A_HUS, q) * u_c;
+    B(B_FLXV, q) = A(A_HVS, q) * v_c;
+  }
+  if (X) {
+    const double u_w = A(A_UN, qw), v_w = A(A_VN, qw);
+    // dudx at T(i,j): dudx_w of u face i, dudx_e of face i-1
+    B(B_GX, q) = dvc(u_c - u_w, k.q_dx_t, k.fast_div) * D;
+    // x-advective flux of u through T(i,j): uu_w * u_w * depw of face i
+    const double U = half(u_c + u_w) * k.dy_t;
+    B(B_FXU, q) = (upwind(U, u_c, u_w) * U) * D;
+    // west edge of v face (i,j): u_wc, u_w, depw, vv_w (unmasked form)
+    const double uwc = half(u_w + A(A_UN, qwn));
+    B(B_UW2, q) = uwc;
+    const double Uw = half(uwc) * k.dyu2;
+    const double depw = half((A(A_HUS, qw) + A(A_HU, qwn)) + A(A_SU, qwn));
+    B(B_FXV, q) = (upwind(Uw, v_c, v_w) * Uw) * depw;
+    B(B_QX, q) = dvc(v_c - v_w, k.q_dxv2, k.fast_div);
+  }
+  if (Y) {
+    const double u_s = A(A_UN, qs), v_s = A(A_VN, qs);
+    // dvdy at T(i,j): dvdy_s of v face j, dvdy_n of face j-1
+    B(B_GY, q) = dvc(v_c - v_s, k.q_dy_t, k.fast_div) * D;
+    // y-advective flux of v through T(i,j): vv_s * v_s * deps of face j
+    const double V = half(v_c + v_s) * k.dx_t;
+    B(B_FYV, q) = (upwind(V, v_c, v_s) * V) * D;
+    // south edge of u face (i,j): v_sc, v_s, deps, uu_s (unmasked form)
+    const double vsc = half(v_s + A(A_VN, qse));
+    B(B_VS2, q) = vsc;
+    const double Vs = half(vsc) * k.dxv2;
+    const double deps = half((A(A_HVS, qs) + A(A_HV, qse)) + A(A_SV, qse));
+    B(B_FYU, q) = (upwind(Vs, u_c, u_s) * Vs) * deps;
+    B(B_QY, q) = dvc(u_c - u_s, k.q_dyu2, k.fast_div);
+  }
+}
+
+// The sshn_u / sshn_v this step reads: next_sshu_code / next_sshv_code
+// (time_update_kern.c:90-155) over their loop ranges; other faces keep the
+// stored value, which is read only for them.  Returns whether this thread met
+// a stored value out of range (the wide form takes any).
+template <class T, bool WIDE>
+__device__ __forceinline__ bool tile_faces(const Fields& f, const Dims& d, const FastConst& k,
                                            int i0, int j0, double* smem) {
-  constexpr int TX = T::TX, TY = T::TY, SX = T::SX, S0 = T::S0;
+  constexpr int TX = T::TX, TY = T::TY, SX = T::SX, S0 = T::S0, NTHREADS = T::NTHREADS;
   constexpr int RX = T::RX, RY = T::RY, RY1 = T::RY1;
-  double* a0 = smem;                 // [N_A0][S0]
-  double* b1 = smem + N_A0 * S0;     // [N_B1][S0]
-  int* mk = (int*)(b1 + N_B1 * S0);  // [S0]
-  int* glist = mk + S0;              // [TX * TY] general cells of this tile
-  int* gcount = glist + TX * TY;     // their number
-  int* slow = gcount + 1;            // a field is outside the bounded forms' range
-
-  const int W = d.width;
+  const TileSmem<T> sm(smem);
+  double *a0 = sm.a0, *b1 = sm.b1;
+  const int* mk = sm.mk;
+  const int W = d.width, imax = d.xe + 1, jmax = d.ye + 1;
   const int tid = threadIdx.y * TX + threadIdx.x;
-  const int i = i0 + threadIdx.x;
-
-  if (tid == 0) {
-    *gcount = 0;
-    *slow = k.bounded ? 0 : 1;
-  }
-  // ---- the fields (positions past the copy region hold what its last column
-  // or row does; no cell that is written reads them) ----
-  const int imax = d.xe + 1, jmax = d.ye + 1;
-  bool out = false;  // a field of this thread's is out of range
-  for (int t = tid; t < S0; t += NTHREADS) {
-    const int c = min(j0 - 1 + t / SX, jmax) * W + min(i0 - 1 + t % SX, imax);
-    const double sn = fs.sshn_in[c], un = fs.un_in[c], vn = fs.vn_in[c], hu = f.hu[c],
-                 hv = f.hv[c];
-    out |= beyond(sn, kFieldRange) | beyond(un, kFieldRange) | beyond(vn, kFieldRange) |
-           beyond(hu, kFieldRange) | beyond(hv, kFieldRange);
-    A(A_SN, t) = sn;
-    A(A_UN, t) = un;
-    A(A_VN, t) = vn;
-    A(A_HU, t) = hu;
-    A(A_HV, t) = hv;
-    mk[t] = f.tmask[c];
-    B(B_AREA_SSH, t) = mlc<IC>(sn, k.f_area_t);
-  }
-  double ht[T::RPT];  // of this thread's own cells, for the shared terms
-#pragma unroll
-  for (int e = 0; e < T::RPT; e++) {
-    ht[e] = f.ht[min(j0 + (int)threadIdx.y + e * T::RPP, jmax) * W + min(i, imax)];
-    out |= beyond(ht[e], kFieldRange);
-  }
-  __syncthreads();
-
-  // ---- the sshn_u / sshn_v this step reads: next_sshu_code /
-  // next_sshv_code (time_update_kern.c:90-155) over their loop ranges; other
-  // faces keep the stored value, which is read only for them ----
+  bool out = false;
   auto face_u = [&](int tx, int ty, bool sum) {
     const int q = (ty + 1) * SX + tx + 1, fi = i0 + tx, fj = j0 + ty;
     double su;
     const int mm = mk[q], mn = mk[q + 1];
     if (fj <= d.ye && fi <= d.xe - 1 && mm + mn > 0) {
-      su = mm * mn > 0 ? div_bounded(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + 1), k.q_2area_u)
-                       : (mm <= 0 ? A(A_SN, q + 1) : A(A_SN, q));
+      const double two = B(B_AREA_SSH, q) + B(B_AREA_SSH, q + 1);
+      const double both = WIDE ? dvc(half(two), k.q_area_u, k.fast_div)
+                               : div_bounded(two, k.q_2area_u);
+      su = mm * mn > 0 ? both : (mm <= 0 ? A(A_SN, q + 1) : A(A_SN, q));
     } else {
       su = f.sshn_u[min(fj, jmax) * W + min(fi, imax)];
-      out |= beyond(su, kFieldRange);
+      out |= out_of_range(su);
     }
     A(A_SU, q) = su;
     if (sum) A(A_HUS, q) = A(A_HU, q) + su;
@@ -678,11 +738,13 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
     double sv;
     const int mm = mk[q], mn = mk[q + SX];
     if (fj <= d.ye - 1 && fi <= d.xe && mm + mn > 0) {
-      sv = mm * mn > 0 ? div_bounded(B(B_AREA_SSH, q) + B(B_AREA_SSH, q + SX), k.q_2area_v)
-                       : (mm <= 0 ? A(A_SN, q + SX) : A(A_SN, q));
+      const double two = B(B_AREA_SSH, q) + B(B_AREA_SSH, q + SX);
+      const double both = WIDE ? dvc(half(two), k.q_area_v, k.fast_div)
+                               : div_bounded(two, k.q_2area_v);
+      sv = mm * mn > 0 ? both : (mm <= 0 ? A(A_SN, q + SX) : A(A_SN, q));
     } else {
       sv = f.sshn_v[min(fj, jmax) * W + min(fi, imax)];
-      out |= beyond(sv, kFieldRange);
+      out |= out_of_range(sv);
     }
     A(A_SV, q) = sv;
     if (sum) A(A_HVS, q) = A(A_HV, q) + sv;
@@ -711,39 +773,59 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
       if (e < TY) face_v(-1, e, false);
     }
   }
-  __syncthreads();
+  return out;
+}
+
+// The shared terms and the regular cells' update; the other cells go to
+// the tile's list.
+template <class T, bool IC, bool WIDE>
+__device__ __forceinline__ void tile_update(const Fields& f, const FusedState& fs, const Dims& d,
+                                            const FastConst& k, int i0, int j0, double* smem) {
+  constexpr int TX = T::TX, TY = T::TY, SX = T::SX, S0 = T::S0, NTHREADS = T::NTHREADS;
+  constexpr int RX = T::RX, RY = T::RY;
+  const TileSmem<T> sm(smem);
+  double *a0 = sm.a0, *b1 = sm.b1;
+  int *mk = sm.mk, *glist = sm.glist, *gcount = sm.gcount;
+  const int W = d.width;
+  const int tid = threadIdx.y * TX + threadIdx.x;
+  const int i = i0 + threadIdx.x;
 
   // ---- the terms shared by neighbouring updates ----
+  auto terms = [&](auto x, auto y, int q) {
+    if constexpr (WIDE)
+      shared_terms_any<T, decltype(x)::value, decltype(y)::value>(a0, b1, q, k);
+    else
+      shared_terms<T, IC, decltype(x)::value, decltype(y)::value>(a0, b1, q, k);
+  };
+  auto flux = [&](double h, double v) { return WIDE ? h * v : mul_bounded(h, v); };
 #pragma unroll
-  for (int e = 0; e < T::RPT; e++)
-    shared_terms<T, IC, true, true>(a0, b1, (threadIdx.y + e * T::RPP + 1) * SX + threadIdx.x + 1,
-                                ht[e], k);
+  for (int e = 0; e < T::RPT; e++) {
+    const int q = (threadIdx.y + e * T::RPP + 1) * SX + threadIdx.x + 1;
+    terms(std::true_type{}, std::true_type{}, q);
+  }
   // the south terms of row TY, the west terms of column TX, and the fluxes
   // through the tile's west and south edges
   for (int t = tid; t < 2 * RX + 2 * RY; t += NTHREADS) {
     int e = t;
     if (e < RX) {
       if (e < TX) {
-        const double h = f.ht[min(j0 + TY, jmax) * W + min(i0 + e, imax)];
-        out |= beyond(h, kFieldRange);
-        shared_terms<T, IC, false, true>(a0, b1, (TY + 1) * SX + e + 1, h, k);
+        const int q = (TY + 1) * SX + e + 1;
+        terms(std::false_type{}, std::true_type{}, q);
       }
     } else if ((e -= RX) < RY) {
       if (e < TY) {
-        const double h = f.ht[min(j0 + e, jmax) * W + min(i0 + TX, imax)];
-        out |= beyond(h, kFieldRange);
-        shared_terms<T, IC, true, false>(a0, b1, (e + 1) * SX + TX + 1, h, k);
+        const int q = (e + 1) * SX + TX + 1;
+        terms(std::true_type{}, std::false_type{}, q);
       }
     } else if ((e -= RY) < RY) {
       const int q = (e + 1) * SX;
-      if (e < TY) B(B_FLXU, q) = mul_bounded(A(A_HUS, q), A(A_UN, q));
+      if (e < TY) B(B_FLXU, q) = flux(A(A_HUS, q), A(A_UN, q));
     } else {
       e -= RY;
       const int q = e + 1;
-      if (e < TX) B(B_FLXV, q) = mul_bounded(A(A_HVS, q), A(A_VN, q));
+      if (e < TX) B(B_FLXV, q) = flux(A(A_HVS, q), A(A_VN, q));
     }
   }
-  if (out) *slow = 1;
   __syncthreads();
 
   // ---- the update ----
@@ -756,7 +838,6 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
   // land-side cells does not run both paths.  The per-face global inputs are
   // loaded first and the results stored last, so no store can alias a later
   // load.
-  const bool tile_slow = *slow != 0;
 #pragma unroll
   for (int pb = 0; pb < T::RPT; pb += 2) {
     constexpr int NP = T::RPT >= 2 ? 2 : 1;  // rows taken together
@@ -769,7 +850,7 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
       c[e] = j * W + i;
       q[e] = (row + 1) * SX + (threadIdx.x + 1);
       live[e] = i <= d.xe - 1 && j <= d.ye - 1;
-      bool regular = live[e] && !tile_slow;
+      bool regular = live[e];
 #pragma unroll
       for (int dj = -1; dj <= 1; dj++)
 #pragma unroll
@@ -791,7 +872,8 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
       RegOut o[NP];
 #pragma unroll
       for (int e = 0; e < NP; e++)
-        o[e] = regular_cell<T, IC>(a0, b1, q[e], dhu[e], rhu[e], dhv[e], rhv[e], k);
+        o[e] = WIDE ? regular_cell_any<T>(a0, b1, q[e], dhu[e], rhu[e], dhv[e], rhv[e], k)
+                    : regular_cell<T, IC>(a0, b1, q[e], dhu[e], rhu[e], dhv[e], rhv[e], k);
 #pragma unroll
       for (int e = 0; e < NP; e++) {
         reg[e] = reg[e] && !o[e].bad;
@@ -808,6 +890,76 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
         glist[atomicAdd(gcount, 1)] = (threadIdx.y + (pb + e) * T::RPP) * TX + threadIdx.x;
   }
   __syncthreads();
+}
+
+// One tile of the fused step: interior cells [i0, i0+TX) x [j0, j0+TY) of one
+// domain.  `tide` is this step's bc_ssh value (general cells).
+//
+// The FP64 pipe bounds the step (about 1.7 instructions per clock per SM;
+// each holds a scheduler's share of it for 64 issue slots), so every phase
+// forms a value on exactly the positions that are read (a full warp per row
+// of the tile, and the edges' extra values, next column and next row, packed
+// into warps of their own), and products and quotients are formed in
+// integers: the pipe has the step's adds only, 57 of the 140 instructions per
+// cell of the form that used it for everything on 2- and 1-cell halos.  The
+// integer forms pay only as straight-line code: with a range branch each,
+// the same products made the step slower.
+template <class T, bool IC>
+__device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs, const Dims& d,
+                                           const Scalars& p, const FastConst& k, double tide,
+                                           int i0, int j0, double* smem) {
+  constexpr int TX = T::TX, TY = T::TY, SX = T::SX, S0 = T::S0;
+  constexpr int NTHREADS = T::NTHREADS;
+  const TileSmem<T> sm(smem);
+  double *a0 = sm.a0, *b1 = sm.b1;
+  int *mk = sm.mk, *glist = sm.glist, *gcount = sm.gcount;
+
+  const int W = d.width;
+  const int tid = threadIdx.y * TX + threadIdx.x;
+
+  if (tid == 0) {
+    *gcount = 0;
+  }
+  // ---- the fields (positions past the copy region hold what its last column
+  // or row does; no cell that is written reads them) ----
+  const int imax = d.xe + 1, jmax = d.ye + 1;
+  bool wide = !k.bounded;
+  for (int t = tid; t < S0; t += NTHREADS) {
+    const int c = min(j0 - 1 + t / SX, jmax) * W + min(i0 - 1 + t % SX, imax);
+    const double sn = fs.sshn_in[c], un = fs.un_in[c], vn = fs.vn_in[c], hu = f.hu[c],
+                 hv = f.hv[c], ht = f.ht[c];
+    wide |= out_of_range(sn) | out_of_range(un) | out_of_range(vn) | out_of_range(hu) |
+            out_of_range(hv) | out_of_range(ht);
+    A(A_SN, t) = sn;
+    A(A_UN, t) = un;
+    A(A_VN, t) = vn;
+    A(A_HU, t) = hu;
+    A(A_HV, t) = hv;
+    A(A_HT, t) = ht;
+    mk[t] = f.tmask[c];
+    B(B_AREA_SSH, t) = mlc<IC>(sn, k.f_area_t);
+  }
+  // what the update will read from global memory, into L2 meanwhile: one line
+  // (16 doubles) per thread (2048^2: 615 -> 597 us)
+  for (int t = tid; t < 4 * TY * (TX / 16); t += NTHREADS) {
+    const int l = t % (TX / 16), r = t / (TX / 16) % TY, a = t / (TX / 16 * TY);
+    const double* base = a == 0   ? f.d_hu
+                         : a == 1 ? f.d_hv
+                                  : reinterpret_cast<const double*>(a == 2 ? f.r_hu : f.r_hv);
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(
+        base + min(j0 + r, jmax) * W + min(i0 + 16 * l, imax)));
+  }
+  bool any_wide = __syncthreads_or(wide);
+  if (!any_wide) any_wide = __syncthreads_or(tile_faces<T, false>(f, d, k, i0, j0, smem));
+  if (!any_wide) {
+    tile_update<T, IC, false>(f, fs, d, k, i0, j0, smem);
+  } else {
+    for (int t = tid; t < S0; t += NTHREADS) B(B_AREA_SSH, t) = k.area_t * A(A_SN, t);
+    __syncthreads();
+    tile_faces<T, true>(f, d, k, i0, j0, smem);
+    __syncthreads();
+    tile_update<T, IC, true>(f, fs, d, k, i0, j0, smem);
+  }
 
   // ---- general cells: the reference's per-point code, in its order ----
   const int ngen = *gcount;
