@@ -88,15 +88,10 @@ constexpr int kRowPix = 136;
 // every role's loop, and the MMA thread waits for its last commit before the
 // tensor memory is freed.
 constexpr int kStripRows = 8;
-constexpr int kSlots = 4;      // the weight gradient's X ring
 constexpr int kConvSlots = 5;  // the convolution's input ring: 3 rows read, 2 in flight
 constexpr int kPipeThreads = 256;
 constexpr int kEpiWarps = 4;
 constexpr int kStageThreads = 96;  // warps 5-7
-// 16-byte loads per staging thread per row: 8 channel groups x 136 pixels
-// (cin = 64, the widest) fit in 96 x 12
-constexpr int kStageBatch = 12;
-static_assert(8 * kRowPix <= kStageThreads * kStageBatch, "a staged row must fit one batch");
 constexpr int kPipeTmemCols = 128;  // two accumulators of up to 64 columns
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -112,6 +107,17 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
       "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
           smem_u32(bar))
       : "memory");
+}
+// 16 FP32 columns of 32 tensor-memory lanes; the values are there after
+// tcgen05.wait::ld (which the caller puts before their first use).
+__device__ __forceinline__ void tmem_ld16(uint32_t (&r)[16], uint32_t ta) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,"
+      "%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(ta));
 }
 // Waits for the phase with the given parity to complete; false if the wait
 // ran out after max_cycles (flag and error set) or another role aborted.
@@ -407,53 +413,106 @@ __global__ void k_flip_transpose(const __nv_bfloat16* __restrict__ w,
 
 // Weight gradient on the tensor cores.  For each tap it is a GEMM over
 // pixels, D[co][ci] = sum_p dY[p][co] X[p + off][ci], with both operands
-// "MN-major" (channels contiguous per pixel, as the data already is):
-// M = co (padded to 128 with zero rows), N = ci, K = pixels.  X is staged as
-// in the convolution, so the tap (dy, dx) operand is again a row block
-// started 16 * dx bytes later.  The nine accumulators (9 x ci FP32 columns)
-// stay in tensor memory for the CTA's lifetime; at the end each CTA writes
-// its partial sums to its own slot of `part`, and k_sum_parts adds the
-// slots in CTA order, so that the gradient has the same bits on every run
-// (atomic additions would sum in whatever order the CTAs finished).
+// "MN-major" (channels contiguous per pixel, as the data already is): M =
+// output channels, N = input channels, K = pixels.  X is staged as in the
+// convolution, so the tap (dy, dx) operand is again a row block started 16 *
+// dx bytes later.
+//
+// What bounds it is the tensor core's operand reads from shared memory: an M
+// = 128, N = 48 MMA reads 5.6 KB for 48 of its 128 rows' worth of products.
+// So two adjacent rows are stacked on each side (cout <= 64): A = dY rows (r,
+// r+1), B = X rows (r, r+1), and the four quadrants of one accumulator are
+// dY(r) X(r): dy = 1, dY(r) X(r+1): dy = 2, dY(r+1) X(r): dy = 0, and dY(r+1)
+// X(r+1), which is not used (every row meets itself in the first).  As r runs
+// over the rows, with zero rows of dY before and after, each quadrant sums
+// its tap over all of them: 24 MMAs of N = 96 per row of 48 channels instead
+// of 72 of N = 48.  Rows lie in a ring of slots, adjacent rows in adjacent
+// slots (slot 0 is staged a second time behind the last).  cout > 64: one row
+// of dY, and the nine taps as separate MMAs.
+//
+// The accumulators stay in tensor memory for the CTA's lifetime; at the end
+// each CTA writes its partial sums to its own slot of `part`, and k_sum_parts
+// adds the slots in a fixed order, so that the gradient has the same bits on
+// every run (atomic additions would sum in whatever order the CTAs finished).
+// A CTA (alone on its SM: it holds all 512 TMEM columns) takes an equal,
+// contiguous share of the rows of all 128-pixel columns.  Roles:
+//   warps 0-6  stage rows of X and dY by cp.async, kWgDepth rows in flight,
+//              and add up their dY values for the bias gradient; at the end
+//              warps 0-3 move the accumulators out of TMEM
+//   warp 7     one thread issues the MMAs
+// 48 -> 48 channels at 16 x 256^2: 193 us (9 x N = 48 per row, one row in
+// flight in registers) plus 24 us for a separate bias pass before.
 constexpr int kWgTmemCols = 512;
-constexpr int kWgGroups = 16;  // 128 M rows = 16 groups of 8 output channels
-constexpr size_t kWgSmem = 120 * 1024;
+#ifndef WGW
+#define WGW 8
+#endif
+constexpr int kWgThreads = 32 * WGW, kWgStagers = kWgThreads - 32;  // the last warp issues
+constexpr int kWgDepth = 3;      // rows in flight per CTA (fewer where slots are scarce)
+constexpr int kWgMaxSlots = 8;
+constexpr uint32_t kWgLboY = kTileM * 16 + 16;   // next 8 output channels (padded: banks)
+constexpr uint32_t kWgLboX = kRowPix * 16 + 16;  // next 8 input channels
+constexpr size_t kWgMaxSmem = 216 * 1024;
 
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
          ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
 }
+// One slot: a row of dY and a row of X.
+__host__ __device__ constexpr uint32_t wg_ybytes(int cout) { return (cout >> 3) * kWgLboY; }
+__host__ __device__ constexpr uint32_t wg_xbytes(int cin) { return (cin >> 3) * kWgLboX; }
+// dY slots, then X slots, each with the copy of slot 0 where rows are paired;
+// an operand of M = 128 reads 16 channel groups from its first row on.
+__host__ __device__ constexpr size_t wg_smem(int cin, int cout, int slots) {
+  const int n = slots + (cout <= 64 ? 1 : 0);
+  const size_t all = (size_t)n * (wg_ybytes(cout) + wg_xbytes(cin));
+  const size_t last = (size_t)(slots - 1) * wg_ybytes(cout) + 16 * kWgLboY;
+  return all > last ? all : last;
+}
+// Rows in flight: an MMA step frees a row once the next one (paired) or the
+// next two are marked full, which the stagers do depth - 1 rows later.
+__host__ __device__ constexpr int wg_depth(int cout, int slots) {
+  const int d = slots - (cout <= 64 ? 1 : 2);
+  return d < kWgDepth ? d : kWgDepth;
+}
 
-// Laid out like the convolution: a CTA (alone on its SM: it holds all 512
-// TMEM columns) walks strips of kStripRows rows of one 128-pixel segment:
-//   warps 5-7  stage input rows (X) into a ring of kSlots slots
-//   warps 0-3  stage gradient rows (dY) into a ring of 2 slots, then, at
-//              the end, move the nine accumulators out of TMEM into dw
-//   warp 4     one thread issues, per row, the 9 taps x 8 pixel chunks of
-//              MMAs into the accumulators, which stay in TMEM throughout
-// The bias gradient is a separate reduction (k_bias_grad).
-constexpr int kWgYSlots = 2;
-constexpr int kWgYThreads = 128;   // warps 0-3
-constexpr int kWgYBatch = 16;      // 16-byte loads per thread per dY row (cout <= 128)
+// A CTA's share of the rows: rows [g, end) of the list of all columns' rows,
+// cut into segments of one column each.
+struct RowSegments {
+  long long g, end;
+  int H, segs;
+  __device__ RowSegments(int batch, int H_, int segs_) : H(H_), segs(segs_) {
+    const long long total = (long long)batch * segs * H;
+    g = total * blockIdx.x / gridDim.x;
+    end = total * (blockIdx.x + 1) / gridDim.x;
+  }
+  __device__ bool next(int& img, int& x0, int& y0, int& rows) {
+    if (g >= end) return false;
+    const long long col = g / H;
+    img = (int)(col / segs);
+    x0 = (int)(col - (long long)img * segs) * kTileM;
+    y0 = (int)(g - col * H);
+    rows = (int)(end - g < H - y0 ? end - g : H - y0);
+    g += rows;
+    return true;
+  }
+};
 
-__global__ void __launch_bounds__(kPipeThreads)
+__global__ void __launch_bounds__(kWgThreads)
     k_conv_wgrad_pipe(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                       float* __restrict__ part, int batch, int H, int W, int cin, int cout,
-                      int* __restrict__ err) {
+                      int slots, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t xfull[kSlots], xempty[kSlots];
-  __shared__ __align__(8) uint64_t yfull[kWgYSlots], yempty[kWgYSlots], last_bar;
+  __shared__ __align__(8) uint64_t full_bar[kWgMaxSlots], empty_bar[kWgMaxSlots], last_bar;
   __shared__ uint32_t taddr_slot;
   __shared__ int abort_flag, s_issued;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int kc = cin >> 3, kco = cout >> 3;
-  const uint32_t lbo_y = kTileM * 16;  // next group of 8 output channels (M)
-  const uint32_t lbo_x = kRowPix * 16; // next group of 8 input channels (N)
-  const uint32_t row_bytes = (uint32_t)kc * lbo_x;
-  const uint32_t yslot_bytes = (uint32_t)kWgGroups * lbo_y;
-  unsigned char* yring = smem;                               // kWgYSlots x 32 KB
-  unsigned char* xring = smem + kWgYSlots * yslot_bytes;     // kSlots staged X rows
+  const bool pair = cout <= 64;
+  const uint32_t ybytes = wg_ybytes(cout), xbytes = wg_xbytes(cin);
+  unsigned char* yring = smem;
+  unsigned char* xring = smem + (size_t)(slots + (pair ? 1 : 0)) * ybytes;
+  const int depth = wg_depth(cout, slots);
   volatile int* abort_v = &abort_flag;
 
   if (warp == 0) {
@@ -463,120 +522,100 @@ __global__ void __launch_bounds__(kPipeThreads)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    for (int q = 0; q < kSlots; q++) {
-      mbar_init(&xfull[q], kStageThreads);
-      mbar_init(&xempty[q], 1);
-    }
-    for (int q = 0; q < kWgYSlots; q++) {
-      mbar_init(&yfull[q], kWgYThreads);
-      mbar_init(&yempty[q], 1);
+    for (int q = 0; q < slots; q++) {
+      mbar_init(&full_bar[q], kWgStagers / 32);
+      mbar_init(&empty_bar[q], 1);
     }
     mbar_init(&last_bar, 1);
     abort_flag = 0;
     s_issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
-  // rows co >= cout of the M = 128 operand stay zero in both dY slots
-  for (int t = tid; t < kWgYSlots * kWgGroups * kTileM; t += kPipeThreads)
-    *reinterpret_cast<uint4*>(yring + t * 16) = make_uint4(0, 0, 0, 0);
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t taddr = taddr_slot;
   const int segs = W / kTileM;
-  const long long units = (long long)batch * ((H + kStripRows - 1) / kStripRows) * segs;
+  const long long nel = 9LL * cout * cin;
+  float* mine = part + (size_t)blockIdx.x * (nel + cout);
 
-  if (warp >= 5) {
-    // ---- X stagers: input rows y0-1 .. y0+rows of every strip ----
-    const int st = tid - 5 * 32;
-    long long q = 0;
-    for (long long u = blockIdx.x; u < units && !*abort_v; u += gridDim.x) {
-      const StripWalk sw(u, H, segs);
-      for (int a = 0; a < sw.rows + 2 && !*abort_v; a++, q++) {
-        const int slot = (int)(q % kSlots);
-        const int yy = sw.y0 - 1 + a;
-        uint4 v[kStageBatch];
-#pragma unroll
-        for (int b = 0; b < kStageBatch; b++) {
-          const int t = st + b * kStageThreads;
-          v[b] = make_uint4(0, 0, 0, 0);
-          if (t < kc * kRowPix) {
-            const int p = t % kRowPix, ch = t / kRowPix;
-            const int xx = sw.x0 - 1 + p;
-            if (yy >= 0 && yy < H && xx >= 0 && xx < W)
-              v[b] = *reinterpret_cast<const uint4*>(
-                  x + (((size_t)sw.img * H + yy) * W + xx) * cin + ch * 8);
-          }
-        }
-        if (q >= kSlots &&
-            !mbar_wait(&xempty[slot], (uint32_t)((q / kSlots - 1) & 1), abort_v, err))
-          break;
-        unsigned char* dst = xring + slot * row_bytes;
-#pragma unroll
-        for (int b = 0; b < kStageBatch; b++) {
-          const int t = st + b * kStageThreads;
-          if (t < kc * kRowPix) {
-            const int p = t % kRowPix, ch = t / kRowPix;
-            *reinterpret_cast<uint4*>(dst + ch * lbo_x + p * 16) = v[b];
-          }
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive(&xfull[slot]);
-      }
-    }
-  } else if (warp == 4) {
+  if (tid >= kWgStagers) {
     // ---- MMA issuer ----
     if (lane == 0) {
-      const uint32_t idesc = idesc_bf16_mn(cin);
-      long long q = 0, p = 0;
+      const uint32_t idesc = idesc_bf16_mn(pair ? 2 * cin : cin);
+      RowSegments rs(batch, H, segs);
       bool issued = false, ok = true;
-      for (long long u = blockIdx.x; u < units && ok && !*abort_v; u += gridDim.x) {
-        const StripWalk sw(u, H, segs);
-        const long long qb = q;
-        ok = mbar_wait(&xfull[qb % kSlots], (uint32_t)((qb / kSlots) & 1), abort_v, err) &&
-             mbar_wait(&xfull[(qb + 1) % kSlots], (uint32_t)(((qb + 1) / kSlots) & 1),
-                       abort_v, err);
-        for (int o = 0; o < sw.rows && ok; o++, p++) {
-          const long long qn = qb + o + 2;
-          const int ys = (int)(p % kWgYSlots);
-          ok = mbar_wait(&xfull[qn % kSlots], (uint32_t)((qn / kSlots) & 1), abort_v, err) &&
-               mbar_wait(&yfull[ys], (uint32_t)((p / kWgYSlots) & 1), abort_v, err);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          // MN-major, no swizzle: LBO steps along K (8 pixels = 128 B), SBO
-          // along M / N (the next 8 channels).  Descriptors built once per
-          // row and advanced by adding byte offsets / 16 to their address
-          // field (shared addresses stay below 256 KB): + 256 / 16 per
-          // K-step, + dx for the tap's pixel shift.
-          const uint64_t yrow = smem_desc(smem_u32(yring + ys * yslot_bytes), 128, lbo_y);
-          uint64_t xrow[3];
+      int img, x0, y0, rows;
+      // Ring positions are counted in 32 bits, slot and parity apart, and the
+      // slots' descriptors formed by one multiply-add: this thread's work per
+      // row is what the tensor core waits for between rows.
+      struct Pos {
+        int slot;
+        uint32_t par;
+      };
+      auto next = [&](Pos p) {
+        const bool wrap = p.slot + 1 == slots;
+        return Pos{wrap ? 0 : p.slot + 1, p.par ^ (wrap ? 1u : 0u)};
+      };
+      auto full = [&](Pos p) { return mbar_wait(&full_bar[p.slot], p.par, abort_v, err); };
+      const uint64_t yd0 = smem_desc(smem_u32(yring), 128, kWgLboY);
+      const uint64_t xd0 = smem_desc(smem_u32(xring), 128, kWgLboX);
+      auto mma = [&](uint32_t dcol, uint64_t ad, uint64_t bd) {
+        // MN-major, no swizzle: LBO steps along K (8 pixels = 128 B), SBO
+        // along M / N (the next 8 channels); + 256 / 16 per K-step of 16
+        // pixels (the address field never carries: shared addresses stay
+        // below 256 KB)
 #pragma unroll
-          for (int dyr = 0; dyr < 3; dyr++)
-            xrow[dyr] = smem_desc(smem_u32(xring + (int)((qb + o + dyr) % kSlots) * row_bytes),
-                                  128, lbo_x);
+        for (int kq = 0; kq < kTileM / 16; kq++, ad += 256 >> 4, bd += 256 >> 4) {
+          const uint32_t acc = (issued || kq > 0) ? 1u : 0u;
+          asm volatile(
+              "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dcol),
+              "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+        }
+      };
+      Pos cur{0, 0};  // the ring row of the segment's row y0 - 1, then of each row
+      while (ok && rs.next(img, x0, y0, rows) && !*abort_v) {
+        ok = full(cur);
+        if (pair) {
+          for (int o = 0; o <= rows && ok; o++) {  // rows (cur, nxt)
+            const Pos nxt = next(cur);
+            ok = full(nxt);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t yd = yd0 + (uint64_t)((uint32_t)cur.slot * (ybytes >> 4));
+            const uint64_t xd = xd0 + (uint64_t)((uint32_t)cur.slot * (xbytes >> 4));
 #pragma unroll
-          for (int tap = 0; tap < 9; tap++) {
-            uint64_t ad = yrow, bd = xrow[tap / 3] + (uint64_t)(tap % 3);
-#pragma unroll
-            for (int kq = 0; kq < kTileM / 16; kq++, ad += 256 >> 4, bd += 256 >> 4) {
-              const uint32_t acc = (issued || kq > 0) ? 1u : 0u;
-              asm volatile(
-                  "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(
-                      taddr + (uint32_t)(tap * cin)),
-                  "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-            }
+            for (int dx = 0; dx < 3; dx++)
+              mma(taddr + (uint32_t)(dx * 2 * cin), yd, xd + (uint64_t)dx);
+            issued = true;
+            tc_commit(&empty_bar[cur.slot]);  // no later step of this segment reads cur
+            cur = nxt;
           }
-          issued = true;
-          tc_commit(&yempty[ys]);
-          tc_commit(&xempty[(qb + o) % kSlots]);
+        } else {
+          Pos mid = next(cur);
+          ok = ok && full(mid);
+          for (int o = 1; o <= rows && ok; o++) {  // dY row mid, X rows cur, mid, nxt
+            const Pos nxt = next(mid);
+            ok = full(nxt);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t yd = yd0 + (uint64_t)((uint32_t)mid.slot * (ybytes >> 4));
+            const int xs[3] = {cur.slot, mid.slot, nxt.slot};
+#pragma unroll
+            for (int tap = 0; tap < 9; tap++)
+              mma(taddr + (uint32_t)(tap * cin), yd,
+                  xd0 + (uint64_t)((uint32_t)xs[tap / 3] * (xbytes >> 4)) + (uint64_t)(tap % 3));
+            issued = true;
+            tc_commit(&empty_bar[cur.slot]);
+            cur = mid;
+            mid = nxt;
+          }
+          if (ok) tc_commit(&empty_bar[cur.slot]);
+          cur = mid;
         }
-        q = qb + sw.rows + 2;
-        if (ok) {
-          tc_commit(&xempty[(q - 2) % kSlots]);
-          tc_commit(&xempty[(q - 1) % kSlots]);
-        }
+        if (ok) tc_commit(&empty_bar[cur.slot]);
+        cur = next(cur);
       }
       s_issued = (issued && ok) ? 1 : 0;
       __threadfence_block();
@@ -586,60 +625,152 @@ __global__ void __launch_bounds__(kPipeThreads)
         mbar_arrive(&last_bar);
     }
   } else {
-    // ---- dY stagers, then the epilogue ----
-    long long p = 0;
-    for (long long u = blockIdx.x; u < units && !*abort_v; u += gridDim.x) {
-      const StripWalk sw(u, H, segs);
-      for (int o = 0; o < sw.rows && !*abort_v; o++, p++) {
-        const int ys = (int)(p % kWgYSlots);
-        const size_t pix0 = ((size_t)sw.img * H + sw.y0 + o) * W + sw.x0;
-        uint4 v[kWgYBatch];
+    // ---- stagers.  Consecutive threads take consecutive 16-byte channel
+    // groups of a pixel, so a warp's copies cover whole lines; every thread
+    // keeps one channel group of dY and so its eight bias sums.  A thread's
+    // chunks of a row have the same offsets in every row (formed once: index
+    // arithmetic per chunk had the stagers at 700 instructions per warp and
+    // row, longer than the row's MMAs).
+    const int yg = tid % kco, yl = tid / kco, yL = kWgStagers / kco;  // group, first pixel, step
+    const int yn = yl < yL ? (kTileM - yl + yL - 1) / yL : 0;         // its pixels
+    const uint32_t ydst = (uint32_t)(yg * kWgLboY + yl * 16);
+    const int ysrc = yl * cout + yg * 8;
+    constexpr int kX = (6 * kRowPix + kWgStagers - 1) / kWgStagers;  // cin <= 48
+    uint32_t xdst[kX];
+    int xpix[kX], xsrc[kX];
 #pragma unroll
-        for (int b = 0; b < kWgYBatch; b++) {
-          const int t = tid + b * kWgYThreads;  // pixel t % 128, group t / 128
-          if (t < kco * kTileM)
-            v[b] = *reinterpret_cast<const uint4*>(dy + (pix0 + (t % kTileM)) * cout +
-                                                   (t / kTileM) * 8);
-        }
-        if (p >= kWgYSlots &&
-            !mbar_wait(&yempty[ys], (uint32_t)((p / kWgYSlots - 1) & 1), abort_v, err))
-          break;
-        unsigned char* dst = yring + ys * yslot_bytes;
+    for (int k = 0; k < kX; k++) {
+      const int t = tid + k * kWgStagers, p = t / kc, ch = t - p * kc;
+      xpix[k] = p < kRowPix ? p - 1 : -2;  // -2: no chunk
+      xdst[k] = (uint32_t)(ch * kWgLboX + p * 16);
+      xsrc[k] = (p - 1) * cin + ch * 8;
+    }
+    float bs[8] = {};
+    long long q = 0, done = 0;      // rows started, rows marked full
+    int qslot = 0, dslot = 0;       // their slots
+    uint32_t qphase = 1;            // parity of empty_bar the next row waits for
+    unsigned real = 0;              // bit k: ring row q-1-k carries dY values
+    auto finish = [&]() {           // row `done` has landed
+      if (real >> (int)(q - 1 - done) & 1u) {
+        const unsigned char* src = yring + dslot * ybytes + ydst;
+        for (int k = 0; k < yn; k++, src += yL * 16) {
+          const uint4 v = *reinterpret_cast<const uint4*>(src);
+          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int b = 0; b < kWgYBatch; b++) {
-          const int t = tid + b * kWgYThreads;
-          if (t < kco * kTileM)
-            *reinterpret_cast<uint4*>(dst + (t / kTileM) * lbo_y + (t % kTileM) * 16) = v[b];
+          for (int e = 0; e < 4; e++) {
+            bs[2 * e] += __uint_as_float(w[e] << 16);
+            bs[2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u);
+          }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive(&yfull[ys]);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();  // one arrival per warp: 224 serialised ones took longer than the copies
+      if (lane == 0) mbar_arrive(&full_bar[dslot]);
+      done++;
+      if (++dslot == slots) dslot = 0;
+    };
+    RowSegments rs(batch, H, segs);
+    int img, x0, y0, rows;
+    bool ok = true;
+    while (ok && rs.next(img, x0, y0, rows) && !*abort_v) {
+      unsigned xin = 0;  // bit k: chunk k lies inside the image's columns
+#pragma unroll
+      for (int k = 0; k < kX; k++)
+        if (xpix[k] >= -1 && x0 + xpix[k] >= 0 && x0 + xpix[k] < W) xin |= 1u << k;
+      const size_t row0 = ((size_t)img * H + y0) * W + x0;  // the segment's first pixel
+      const __nv_bfloat16* yrow_p = dy + row0 * cout + ysrc;
+      const __nv_bfloat16* xrow_p = x + row0 * cin;
+      for (int a = 0; a < rows + 2; a++) {
+        const long long dr = a - 1;
+        if (q >= slots) ok = mbar_wait(&empty_bar[qslot], qphase, abort_v, err);
+        if (!ok) break;
+        const bool yrow = a >= 1 && a <= rows, xrow = y0 + dr >= 0 && y0 + dr < H;
+        const __nv_bfloat16* ys = yrow ? yrow_p + dr * W * cout : dy;
+        const __nv_bfloat16* xs = xrow_p + dr * W * cin;
+        const int ystep = yrow ? yL * cout : 0;
+        for (int copy = qslot; copy <= slots; copy += slots) {  // slot 0: twice, paired
+          uint32_t yd = smem_u32(yring + copy * ybytes) + ydst;
+          const __nv_bfloat16* yp = ys;
+          for (int k = 0; k < yn; k++, yd += yL * 16, yp += ystep)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(yd), "l"(yp),
+                         "r"(yrow ? 16 : 0)
+                         : "memory");
+          const uint32_t xd = smem_u32(xring + copy * xbytes);
+#pragma unroll
+          for (int k = 0; k < kX; k++)
+            if (xpix[k] >= -1) {
+              const bool in = xrow && (xin >> k & 1u);
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(xd + xdst[k]),
+                           "l"(in ? xs + xsrc[k] : x), "r"(in ? 16 : 0)
+                           : "memory");
+            }
+          if (qslot != 0 || !pair) break;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        real = real << 1 | (yrow ? 1u : 0u);
+        q++;
+        if (++qslot == slots) {
+          qslot = 0;
+          qphase ^= 1u;
+        }
+        if (q - done >= depth) {  // all but the newest depth - 1 rows must have landed
+          switch (depth) {
+            case 1: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+            case 2: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+            case 3: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+            default: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+          }
+          finish();
+        }
       }
     }
-    // the accumulators: row co (lanes 32w .. 32w+31), 9 x cin columns
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    while (done < q && !*abort_v) finish();
+    // the accumulators: rows 32w .. 32w+31 of M
     volatile int never = 0;
-    const bool done = mbar_wait(&last_bar, 0, &never, err);
-    if (__all_sync(0xffffffffu, done) && s_issued && !*abort_v) {
+    const bool mmas = mbar_wait(&last_bar, 0, &never, err);
+    if (warp < 4 && __all_sync(0xffffffffu, mmas) && s_issued && !*abort_v) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int co = warp * 32 + lane;
-      for (int c0 = 0; c0 < 9 * cin; c0 += 16) {
-        uint32_t r[16];
-        const uint32_t ta = taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
-            "%13,%14,%15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-              "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-              "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(ta));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (co < cout) {
-          const int tap = c0 / cin, ci0 = c0 - tap * cin;
-          float* mine = part + (size_t)blockIdx.x * 9 * cout * cin;
+      const int m = warp * 32 + lane;
+      const bool second = pair && m >= cout;  // dY row r+1: the tap dy = 0
+      const int co = second ? m - cout : m;
+      const int ncols = pair ? 6 * cin : 9 * cin;
+      // (ncols is a multiple of 48: three loads in flight)
+      for (int c0 = 0; c0 < ncols; c0 += 48) {
+        uint32_t r[3][16];
 #pragma unroll
-          for (int k = 0; k < 16; k++)
-            mine[((size_t)tap * cout + co) * cin + ci0 + k] = __uint_as_float(r[k]);
+        for (int l = 0; l < 3; l++)
+          tmem_ld16(r[l], taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c0 + 16 * l));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int l = 0; l < 3; l++) {
+          const int c = c0 + 16 * l;
+          const int blk = c / cin, ci0 = c - blk * cin;  // (dx, X row) or the tap
+          int tap = blk;
+          if (pair) {
+            const int dx = blk >> 1, xr = blk & 1;
+            tap = second ? (xr ? -1 : dx) : (xr ? 6 + dx : 3 + dx);
+          }
+          if (co < cout && tap >= 0)
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+              *reinterpret_cast<float4*>(mine + ((size_t)tap * cout + co) * cin + ci0 + 4 * k) =
+                  make_float4(__uint_as_float(r[l][4 * k]), __uint_as_float(r[l][4 * k + 1]),
+                              __uint_as_float(r[l][4 * k + 2]), __uint_as_float(r[l][4 * k + 3]));
         }
       }
+    }
+    // the bias sums, added over the threads of a channel group in thread order
+    float* sb = reinterpret_cast<float*>(smem);  // [yL][cout]: the rings are done with
+    asm volatile("bar.sync 1, %0;" ::"n"(kWgStagers) : "memory");
+    if (yl < yL)
+#pragma unroll
+      for (int k = 0; k < 8; k++) sb[yl * cout + yg * 8 + k] = bs[k];
+    asm volatile("bar.sync 1, %0;" ::"n"(kWgStagers) : "memory");
+    for (int c = tid; c < cout; c += kWgStagers) {
+      float acc = 0.f;
+      for (int r = 0; r < yL; r++) acc += sb[r * cout + c];
+      mine[nel + c] = acc;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -650,45 +781,33 @@ __global__ void __launch_bounds__(kPipeThreads)
                  "r"(kWgTmemCols));
 }
 
-// Block b's partial bias gradient, part[b][co] = sum over its pixels of
-// dy[p][co], in a fixed order (each thread a channel pair over a fixed set
-// of rows, then the block's rows in order); k_sum_parts adds the blocks.
-__global__ void __launch_bounds__(256)
-    k_bias_grad(const __nv_bfloat16* __restrict__ dy, float* __restrict__ part, long long P,
-                int cout) {
-  __shared__ float sp[256 * 2];
-  // thread -> one channel pair, rows strided over the grid
-  const int pairs = cout >> 1;
-  const int lanes_per_row = pairs;  // <= 64
-  const int rows_per_block = blockDim.x / lanes_per_row;
-  const int c2 = threadIdx.x % lanes_per_row, r0 = threadIdx.x / lanes_per_row;
-  if (r0 < rows_per_block) {
-    float s0 = 0.f, s1 = 0.f;
-    for (long long pix = (long long)blockIdx.x * rows_per_block + r0; pix < P;
-         pix += (long long)gridDim.x * rows_per_block) {
-      const __nv_bfloat162 v = reinterpret_cast<const __nv_bfloat162*>(dy + pix * cout)[c2];
-      s0 += __low2float(v);
-      s1 += __high2float(v);
-    }
-    sp[r0 * cout + 2 * c2] = s0;
-    sp[r0 * cout + 2 * c2 + 1] = s1;
+// out[e] += the sum over the parts' slots of nel + cout values (dw, then db):
+// kSumWays threads add a contiguous share of the slots each, in order, and
+// their sums are added in order.  (One thread per element made the 1216 bias
+// parts of a separate pass 100 us of dependent loads, the 152 weight parts 17.)
+constexpr int kSumWays = 8, kSumElems = 32;
+__global__ void __launch_bounds__(kSumWays * kSumElems)
+    k_sum_parts(const float* __restrict__ part, int nparts, long long nel, int cout,
+                float* __restrict__ dw, float* __restrict__ db) {
+  __shared__ float sums[kSumWays][kSumElems];
+  const int lane = threadIdx.x % kSumElems, way = threadIdx.x / kSumElems;
+  const long long n = nel + cout, e = (long long)blockIdx.x * kSumElems + lane;
+  const int b0 = (int)((long long)nparts * way / kSumWays),
+            b1 = (int)((long long)nparts * (way + 1) / kSumWays);
+  float acc = 0.f;
+  if (e < n) {
+#pragma unroll 8
+    for (int b = b0; b < b1; b++) acc += part[(size_t)b * n + e];
   }
+  sums[way][lane] = acc;
   __syncthreads();
-  for (int c = threadIdx.x; c < cout; c += blockDim.x) {
-    float acc = 0.f;
-    for (int r = 0; r < rows_per_block; r++) acc += sp[r * cout + c];
-    part[(size_t)blockIdx.x * cout + c] = acc;
-  }
-}
-
-// out[e] += part[0][e] + part[1][e] + ... in that order.
-__global__ void k_sum_parts(const float* __restrict__ part, int nparts, long long nel,
-                            float* __restrict__ out) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nel;
-       e += (long long)gridDim.x * blockDim.x) {
-    float acc = 0.f;
-    for (int b = 0; b < nparts; b++) acc += part[(size_t)b * nel + e];
-    out[e] += acc;
+  if (way == 0 && e < n) {
+#pragma unroll
+    for (int w = 1; w < kSumWays; w++) acc += sums[w][lane];
+    if (e < nel)
+      dw[e] += acc;
+    else
+      db[e - nel] += acc;
   }
 }
 
@@ -989,38 +1108,35 @@ int nl2d_emu_conv_wgrad(const void* x, const void* dy, float* dw, float* db, int
   if (!x || !dy || !dw || !db || !err || cin % 16 || cin < 16 || 9 * cin > kWgTmemCols ||
       cout % 8 || cout < 8 || cout > 128 || W % kTileM || H < 1 || batch < 1)
     return NL2D_ERR_ARGS;
+  // As many ring slots as fit (at least one row in flight: wg_depth).
   // The kernel holds all 512 TMEM columns, so it must be alone on its SM:
   // asking for more than half an SM's shared memory guarantees that.
-  const size_t need = (size_t)kWgYSlots * kWgGroups * kTileM * 16 +
-                      (size_t)kSlots * (cin / 8) * kRowPix * 16;
-  const size_t smem = need > kWgSmem ? need : kWgSmem;
-  constexpr size_t kMaxSmem = 200 * 1024;
+  int slots = kWgMaxSlots;
+  while (slots > 3 && wg_smem(cin, cout, slots) > kWgMaxSmem) slots--;
+  const size_t need = wg_smem(cin, cout, slots);
+  const size_t smem = need > 120 * 1024 ? need : 120 * 1024;
   static bool attr = false;
   if (!attr) {
     if (cudaFuncSetAttribute(k_conv_wgrad_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kMaxSmem) != cudaSuccess)
+                             (int)kWgMaxSmem) != cudaSuccess)
       return NL2D_ERR_CUDA;
     attr = true;
   }
-  if (smem > kMaxSmem) return NL2D_ERR_ARGS;
+  if (smem > kWgMaxSmem) return NL2D_ERR_ARGS;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long units =
-      (long long)batch * ((H + kStripRows - 1) / kStripRows) * (W / kTileM);
-  const int grid = (int)(units < sms ? units : sms);  // 512 TMEM columns: one CTA per SM
-  constexpr int kBiasBlocks = 152 * 8;
+  // one CTA per SM (512 TMEM columns), with four rows or more each
+  const long long rows = (long long)batch * H * (W / kTileM);
+  const int grid = (int)std::max<long long>(1, std::min<long long>(rows / 4, sms));
   const long long nel = 9LL * cout * cin;
-  if (!ensure_parts((size_t)std::max<long long>(grid * nel, (long long)kBiasBlocks * cout)))
-    return NL2D_ERR_CUDA;
+  if (!ensure_parts((size_t)(grid * (nel + cout)))) return NL2D_ERR_CUDA;
   const cudaStream_t st = (cudaStream_t)stream;
-  k_conv_wgrad_pipe<<<grid, kPipeThreads, smem, st>>>(
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, g_parts, batch, H, W, cin, cout, err);
-  k_sum_parts<<<(int)((nel + 255) / 256), 256, 0, st>>>(g_parts, grid, nel, dw);
-  if (cudaGetLastError() != cudaSuccess) return NL2D_ERR_CUDA;
-  k_bias_grad<<<kBiasBlocks, 256, 0, st>>>((const __nv_bfloat16*)dy, g_parts,
-                                            (long long)batch * H * W, cout);
-  k_sum_parts<<<1, 128, 0, st>>>(g_parts, kBiasBlocks, cout, db);
+  k_conv_wgrad_pipe<<<grid, kWgThreads, smem, st>>>((const __nv_bfloat16*)x,
+                                                      (const __nv_bfloat16*)dy, g_parts, batch,
+                                                      H, W, cin, cout, slots, err);
+  k_sum_parts<<<(int)((nel + cout + kSumElems - 1) / kSumElems), kSumWays * kSumElems, 0, st>>>(
+      g_parts, grid, nel, cout, dw, db);
   return cudaGetLastError() == cudaSuccess ? NL2D_OK : NL2D_ERR_CUDA;
 }
 
