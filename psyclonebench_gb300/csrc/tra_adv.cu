@@ -7,14 +7,15 @@
 // Layout: Fortran a(ji, jj, jk) is a[(k * J + j) * I + i], 0-based.
 //
 // One iteration is two kernels:
-//  * k_tra_horizontal_tiled: for every interior point (1 <= i <= I-2,
-//    1 <= j <= J-2, k <= K-2) the x / y differences, MUSCL slopes with their
-//    limiter, the upstream fluxes and the flux-divergence update, from the
-//    previous iteration's field (ping-pong buffers: the update of one point
-//    never sees another point's new value, as in the reference's separate
-//    loops).
-//  * k_tra_vertical: one thread per interior column marches up in k through
-//    the vertical differences, slopes, fluxes and the final assignment.
+//  * k_tra_horizontal: for every interior point (1 <= i <= I-2, 1 <= j <=
+//    J-2, k <= K-2) the x / y differences, MUSCL slopes with their limiter,
+//    the upstream fluxes and the flux-divergence update, from the field into
+//    a second buffer (the update of one point never sees another point's new
+//    value, as in the reference's separate loops).
+//  * k_tra_vertical: back from the second buffer into the field; a thread
+//    marches up in k through the vertical differences, slopes, fluxes and the
+//    final assignment of an interior column, or of a run of its levels where
+//    there are too few columns to fill the GPU.
 // Work arrays are never stored: each value is recomputed where it is used.
 // Two of the reference's work-array entries are read before the iteration
 // writes them, so they come from earlier calls:
@@ -126,159 +127,298 @@ __device__ __forceinline__ double upstream(double vel, double f1, double f0, dou
   return vel * ((bits(vel) < 0) ? pick(zzwx, zzwy) : pick(zzwy, zzwx));
 }
 
+// The same on operands of known range, without a branch and with the products
+// in integers (nl2d_exact.cuh's bounded forms): the FP64 pipe, which bounds
+// the iteration, is left 15 adds of 38 instructions per point.  Velocities
+// are +-0 or of magnitude in [2^-100, 2^100), masks and zind in [2^-60,
+// 2^10), the field in [2^-400, 2^700): a difference is at least 2^-512, a
+// slope 2^-565, the Courant factor (1 - |v|) / 2 and zind = 1 - z 2^-54, a
+// weighted slope 2^-673 and the sum it enters 2^-725, a flux 2^-825; nothing
+// reaches 2^1023.
+using nl2d::beyond;
+using nl2d::mul_bounded;
+__device__ __forceinline__ bool field_out(double m) { return beyond(m, 400, 700); }
+__device__ __forceinline__ bool vel_out(double v) { return beyond(v, 100, 100); }
+__device__ __forceinline__ bool mask_out(double v) { return beyond(v, 60, 10); }
+__device__ __forceinline__ bool is_zero(double x) {  // of operands that are +-0 or normal
+  return ((unsigned)((unsigned long long)bits(x) >> 32) & 0x7ff00000u) == 0;
+}
+__device__ __forceinline__ double half_b(double x) {
+  return is_zero(x) ? x : from_bits(bits(x) - (1LL << 52));
+}
+__device__ __forceinline__ long long twice_b(double x) {
+  return is_zero(x) ? 0 : (bits(x) & kMag) + (1LL << 52);
+}
+__device__ __forceinline__ double limited_slope_b(double a, double b) {
+  const double s = a + b;
+  const double h = (bits(a) ^ bits(b)) < 0 ? from_bits(bits(s) & kSign) : half_b(s);
+  const long long hm = bits(h) & kMag, p = twice_b(b), q = twice_b(a);
+  const long long m = hm < p ? hm : p;
+  return from_bits((m < q ? m : q) | (bits(h) & kSign));
+}
+// The flux takes one operand, f + zind (zu s), plus a zero with the other
+// one's sign (pick), which matters only where the first is a zero.  The other
+// one's sign follows without computing it where its slope term is a zero (on
+// land, say); else it is computed.
+// zu: the Courant factor, made at registration.
+__device__ __forceinline__ double upstream_b(double vel, double zu, double f1, double f0,
+                                             double zind, double s1, double s0, bool far) {
+  const double f = far ? f1 : f0, s = far ? s1 : s0;
+  const double fo = far ? f0 : f1, so = far ? s0 : s1;
+  double w = f + mul_bounded(zind, mul_bounded(zu, s));
+  const bool wz = is_zero(w), tz = is_zero(zind) || is_zero(zu) || is_zero(so);
+  const long long st = bits(zind) ^ bits(zu) ^ bits(so);
+  const long long other = is_zero(fo) ? bits(fo) & st : bits(fo);
+  if (wz) w = from_bits(bits(w) & other & kSign);
+  if (wz && !tz) w = pick(f + zind * (zu * s), fo + zind * (zu * so));
+  return mul_bounded(vel, w);
+}
+
 struct TraDev {
   const double *pun, *pvn, *pwn, *umask, *vmask, *tmask, *zind;
+  const double *cun, *cvn, *cwn;  // the velocities' Courant factors zu
   int I, J, K;
 };
 
+// zind, the Courant factors, and whether an input is outside the bounded
+// forms' range (*wide).
 __global__ void k_tra_zind(const double* __restrict__ tsn, const double* __restrict__ ztfreez,
                            const double* __restrict__ rnfmsk, const double* __restrict__ upsmsk,
-                           const double* __restrict__ rnfmsk_z,
-                           const double* __restrict__ tmask, double* __restrict__ zind, int I,
-                           int J, int K) {
-  const long long n = (long long)I * J * K;
+                           const double* __restrict__ rnfmsk_z, TraDev d,
+                           double* __restrict__ zind, double* __restrict__ cun,
+                           double* __restrict__ cvn, double* __restrict__ cwn,
+                           int* __restrict__ wide) {
+  const long long n = (long long)d.I * d.J * d.K;
+  bool out = false;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(t / ((long long)I * J));
-    const long long p2 = t - (long long)k * I * J;
+    const int k = (int)(t / ((long long)d.I * d.J));
+    const long long p2 = t - (long long)k * d.I * d.J;
+    const double tm = d.tmask[t];
     const double zice = tsn[t] <= ztfreez[p2] + 0.1 ? 1.0 : 0.0;
-    double z = max2(max2(rnfmsk[p2] * rnfmsk_z[k], upsmsk[p2]), zice) * tmask[t];
+    double z = max2(max2(rnfmsk[p2] * rnfmsk_z[k], upsmsk[p2]), zice) * tm;
     zind[t] = 1 - z;
+    const double u = d.pun[t], v = d.pvn[t], w = d.pwn[t];
+    cun[t] = courant(half_sign(u), u);
+    cvn[t] = courant(half_sign(v), v);
+    cwn[t] = courant(half_sign(w), w);
+    out |= vel_out(u) | vel_out(v) | vel_out(w) | mask_out(d.umask[t]) | mask_out(d.vmask[t]) |
+           mask_out(tm) | mask_out(1 - z);
   }
+  if (out) *wide = 1;
 }
 
 // tra_adv.F90:122-194 for the interior points, from `mo` (the field before
 // the iteration) into `mn` (whose other points already hold their
-// unchanging values).  A CTA of kTx x kTy threads owns kTx x kTy interior
-// points of one level and stages, in shared memory, the field with a
-// 2-point halo, then the x / y differences, the limited slopes and the
-// fluxes its points need, each once, shared by the neighbours.  The
-// x difference east of the last interior column (i = I-1) is the entry the
-// previous iteration's vertical part left in the reference's zwx (zero on
-// the first iteration); y differences on the row j = J-1 are zero (never
-// written there).
-constexpr int kTx = 32, kTy = 16;
+// unchanging values).  A CTA owns kTx x kTy interior points of one level, one
+// per thread, and stages, in shared memory, the field with a 2-point halo,
+// then the x / y differences, the limited slopes and the fluxes its points
+// need, each once, shared by the neighbours: a thread forms those of its own
+// point, and the edges' extra ones are packed into whole warps (FP64
+// instructions cost a scheduler 64 issue slots each whether a warp is full or
+// not).  WIDE: the forms that take any value.  The x difference east of the
+// last interior column (i = I-1) is the entry the previous iteration's
+// vertical part left in the reference's zwx (zero on the first iteration); y
+// differences on the row j = J-1 are zero (never written there).
+constexpr int kTx = 32, kTy = 8;
 
-__global__ void __launch_bounds__(kTx * kTy)
-    k_tra_horizontal_tiled(const double* __restrict__ mo, double* __restrict__ mn, TraDev d,
-                           int first) {
-  __shared__ double sm[kTy + 4][kTx + 4];   // m at (j0-2+r, i0-2+c)
-  __shared__ double dx_[kTy][kTx + 3];      // x difference at i0-2+c
-  __shared__ double dy_[kTy + 3][kTx];      // y difference at j0-2+r
-  __shared__ double sx_[kTy][kTx + 2];      // x slope at i0-1+c
-  __shared__ double sy_[kTy + 2][kTx];      // y slope at j0-1+r
-  __shared__ double fx_[kTy][kTx + 1];      // x flux at i0-1+c
-  __shared__ double fy_[kTy + 1][kTx];      // y flux at j0-1+r
-  const int tid = threadIdx.y * kTx + threadIdx.x, nt = kTx * kTy;
-  const int i0 = 1 + blockIdx.x * kTx, j0 = 1 + blockIdx.y * kTy, k = blockIdx.z;
+struct TraTile {
+  double m[kTy + 4][kTx + 4];   // m at (j0-2+r, i0-2+c)
+  double dx[kTy][kTx + 3];      // x difference at i0-2+c
+  double dy[kTy + 3][kTx];      // y difference at j0-2+r
+  double sx[kTy][kTx + 2];      // x slope at i0-1+c
+  double sy[kTy + 2][kTx];      // y slope at j0-1+r
+  double fx[kTy][kTx + 1];      // x flux at i0-1+c
+  double fy[kTy + 1][kTx];      // y flux at j0-1+r
+};
+
+template <bool WIDE>
+__device__ __forceinline__ double tra_mul(double a, double b) {
+  return WIDE ? a * b : mul_bounded(a, b);
+}
+template <bool WIDE>
+__device__ __forceinline__ double tra_slope(double a, double b) {
+  return WIDE ? limit(slope_raw(a, b), b, a) : limited_slope_b(a, b);
+}
+template <bool WIDE>
+__device__ __forceinline__ double tra_upstream(double vel, double zu, double f1, double f0,
+                                               double zind, double s1, double s0) {
+  return WIDE ? upstream(vel, f1, f0, zind, s1, s0)
+              : upstream_b(vel, zu, f1, f0, zind, s1, s0, bits(vel) < 0);
+}
+
+template <bool WIDE>
+__device__ __forceinline__ void tra_tile(TraTile& s, const double* __restrict__ mo,
+                                         double* __restrict__ mn, const TraDev& d, bool first,
+                                         int i0, int j0, int k) {
+  const int tx = threadIdx.x, ty = threadIdx.y;  // a warp per row of the tile
   const int I = d.I, J = d.J;
   const size_t lev = (size_t)k * J * I;
-  const bool f = first != 0;
-
-  for (int t = tid; t < (kTy + 4) * (kTx + 4); t += nt) {
-    const int r = t / (kTx + 4), c = t - r * (kTx + 4);
-    const int i = i0 - 2 + c, j = j0 - 2 + r;
-    sm[r][c] = (i >= 0 && i < I && j >= 0 && j < J) ? mo[lev + (size_t)j * I + i] : 0.0;
-  }
-  __syncthreads();
-  for (int t = tid; t < kTy * (kTx + 3); t += nt) {  // x differences
-    const int r = t / (kTx + 3), c = t - r * (kTx + 3);
+  auto diff_x = [&](int c, int r) {  // at (i0-2+c, j0+r)
     const int i = i0 - 2 + c, j = j0 + r;
     double v = 0.0;
     if (i >= 0 && j < J) {
       const size_t g = lev + (size_t)j * I + i;
-      if (i <= I - 2) v = d.umask[g] * (sm[r + 2][c + 1] - sm[r + 2][c]);
-      else if (i == I - 1 && !f)
-        v = (k == 0) ? d.pwn[g] * sm[r + 2][c] : d.tmask[g] * (mo[g - (size_t)I * J] - sm[r + 2][c]);
+      if (i <= I - 2)
+        v = tra_mul<WIDE>(d.umask[g], s.m[r + 2][c + 1] - s.m[r + 2][c]);
+      else if (i == I - 1 && !first)
+        v = (k == 0) ? d.pwn[g] * s.m[r + 2][c]
+                     : d.tmask[g] * (mo[g - (size_t)I * J] - s.m[r + 2][c]);
     }
-    dx_[r][c] = v;
-  }
-  for (int t = tid; t < (kTy + 3) * kTx; t += nt) {  // y differences
-    const int r = t / kTx, c = t - r * kTx;
+    s.dx[r][c] = v;
+  };
+  auto diff_y = [&](int c, int r) {  // at (i0+c, j0-2+r)
     const int i = i0 + c, j = j0 - 2 + r;
     double v = 0.0;
-    if (j >= 0 && j <= J - 2 && i < I) {
-      const size_t g = lev + (size_t)j * I + i;
-      v = d.vmask[g] * (sm[r + 1][c + 2] - sm[r][c + 2]);
-    }
-    dy_[r][c] = v;
+    if (j >= 0 && j <= J - 2 && i < I)
+      v = tra_mul<WIDE>(d.vmask[lev + (size_t)j * I + i], s.m[r + 1][c + 2] - s.m[r][c + 2]);
+    s.dy[r][c] = v;
+  };
+  // the velocities and zind of the fluxes, loaded while the differences form
+  const int i = i0 + tx, j = j0 + ty;
+  const bool live = i <= I - 2 && j <= J - 2;
+  const size_t g = lev + (size_t)min(j, J - 1) * I + min(i, I - 1);
+  const double pun = d.pun[g], pvn = d.pvn[g], zind = d.zind[g], cun = d.cun[g], cvn = d.cvn[g];
+  diff_x(tx + 2, ty);
+  diff_y(tx, ty + 2);
+  if (ty == 0) {  // columns i0-2, i0-1, i0+32: 24 differences
+    if (tx < 3 * kTy) diff_x(tx / kTy == 2 ? kTx + 2 : tx / kTy, tx % kTy);
+  } else if (ty <= 3) {  // rows j0-2, j0-1, j0+8
+    diff_y(tx, ty == 3 ? kTy + 2 : ty - 1);
   }
   __syncthreads();
-  for (int t = tid; t < kTy * (kTx + 2); t += nt) {  // x slopes at i0-1+c
-    const int r = t / (kTx + 2), c = t - r * (kTx + 2);
-    const double a = dx_[r][c + 1], b = dx_[r][c];
-    sx_[r][c] = limit(slope_raw(a, b), b, a);
-  }
-  for (int t = tid; t < (kTy + 2) * kTx; t += nt) {  // y slopes at j0-1+r
-    const int r = t / kTx, c = t - r * kTx;
-    const double a = dy_[r + 1][c], b = dy_[r][c];
-    sy_[r][c] = limit(slope_raw(a, b), b, a);
-  }
-  __syncthreads();
-  for (int t = tid; t < kTy * (kTx + 1); t += nt) {  // x fluxes at i0-1+c
-    const int r = t / (kTx + 1), c = t - r * (kTx + 1);
-    const int i = i0 - 1 + c, j = j0 + r;
-    double v = 0.0;
-    if (i == 0) {
-      v = dx_[r][c + 1];  // the flux loop starts at ji = 2: zwx(1) is still the difference
-    } else if (i <= I - 2 && j < J) {
-      const size_t g = lev + (size_t)j * I + i;
-      v = upstream(d.pun[g], sm[r + 2][c + 2], sm[r + 2][c + 1], d.zind[g], sx_[r][c + 1],
-                   sx_[r][c]);
-    }
-    fx_[r][c] = v;
-  }
-  for (int t = tid; t < (kTy + 1) * kTx; t += nt) {  // y fluxes at j0-1+r
-    const int r = t / kTx, c = t - r * kTx;
-    const int i = i0 + c, j = j0 - 1 + r;
-    double v = 0.0;
-    if (j == 0) {
-      v = dy_[r + 1][c];
-    } else if (j <= J - 2 && i < I) {
-      const size_t g = lev + (size_t)j * I + i;
-      v = upstream(d.pvn[g], sm[r + 2][c + 2], sm[r + 1][c + 2], d.zind[g], sy_[r + 1][c],
-                   sy_[r][c]);
-    }
-    fy_[r][c] = v;
+  auto slope_x = [&](int c, int r) {  // at i0-1+c
+    s.sx[r][c] = tra_slope<WIDE>(s.dx[r][c + 1], s.dx[r][c]);
+  };
+  auto slope_y = [&](int c, int r) {  // at j0-1+r
+    s.sy[r][c] = tra_slope<WIDE>(s.dy[r + 1][c], s.dy[r][c]);
+  };
+  slope_x(tx + 1, ty);
+  slope_y(tx, ty + 1);
+  if (ty == 4) {  // columns i0-1, i0+32
+    if (tx < 2 * kTy) slope_x(tx / kTy == 1 ? kTx + 1 : 0, tx % kTy);
+  } else if (ty == 5 || ty == 6) {  // rows j0-1, j0+8
+    slope_y(tx, ty == 6 ? kTy + 1 : 0);
   }
   __syncthreads();
-  const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
-  if (i <= I - 2 && j <= J - 2) {
-    const int r = threadIdx.y, c = threadIdx.x;
-    const double ztra = -(1.0 * (fx_[r][c + 1] - fx_[r][c] + fy_[r + 1][c] - fy_[r][c]));
-    mn[lev + (size_t)j * I + i] = sm[r + 2][c + 2] + ztra;
+  auto flux_x = [&](int c, int r, double vel, double zu, double zi) {  // at i0-1+c >= 1
+    s.fx[r][c] = tra_upstream<WIDE>(vel, zu, s.m[r + 2][c + 2], s.m[r + 2][c + 1], zi,
+                                    s.sx[r][c + 1], s.sx[r][c]);
+  };
+  auto flux_y = [&](int c, int r, double vel, double zu, double zi) {  // at j0-1+r >= 1
+    s.fy[r][c] = tra_upstream<WIDE>(vel, zu, s.m[r + 2][c + 2], s.m[r + 1][c + 2], zi,
+                                    s.sy[r + 1][c], s.sy[r][c]);
+  };
+  if (live) {
+    flux_x(tx + 1, ty, pun, cun, zind);
+    flux_y(tx, ty + 1, pvn, cvn, zind);
+  }
+  if (ty == 7) {  // row j0-1
+    if (i <= I - 2) {
+      const size_t gs = lev + (size_t)(j0 - 1) * I + i;
+      if (j0 == 1)
+        s.fy[0][tx] = s.dy[1][tx];  // the flux loop starts at jj = 2: still the difference
+      else
+        flux_y(tx, 0, d.pvn[gs], d.cvn[gs], d.zind[gs]);
+    }
+  } else if (ty == 0 && tx < kTy && j0 + tx <= J - 2) {  // column i0-1
+    const size_t gw = lev + (size_t)(j0 + tx) * I + i0 - 1;
+    if (i0 == 1)
+      s.fx[tx][0] = s.dx[tx][1];
+    else
+      flux_x(0, tx, d.pun[gw], d.cun[gw], d.zind[gw]);
+  }
+  __syncthreads();
+  if (live) {
+    const double ztra = -(1.0 * (s.fx[ty][tx + 1] - s.fx[ty][tx] + s.fy[ty + 1][tx] - s.fy[ty][tx]));
+    mn[g] = s.m[ty + 2][tx + 2] + ztra;
   }
 }
 
-// tra_adv.F90:196-251 for one interior column, in place on m (the field
-// after the horizontal update).
-__global__ void __launch_bounds__(256) k_tra_vertical(double* __restrict__ m, TraDev d) {
+// (512 x 512 x 75, both kernels: four CTAs per SM 1121 us, five 1035, six 991;
+// with the Courant factors made at registration six 926, seven 895.)
+__global__ void __launch_bounds__(kTx * kTy, 7)
+    k_tra_horizontal(const double* __restrict__ mo, double* __restrict__ mn, TraDev d, int first,
+                     int wide) {
+  __shared__ TraTile s;
+  const int tid = threadIdx.y * kTx + threadIdx.x;
+  const int i0 = 1 + blockIdx.x * kTx, j0 = 1 + blockIdx.y * kTy, k = blockIdx.z;
+  const size_t lev = (size_t)k * d.J * d.I;
+  bool out = wide != 0;
+  for (int t = tid; t < (kTy + 4) * (kTx + 4); t += kTx * kTy) {
+    const int r = t / (kTx + 4), c = t - r * (kTx + 4);
+    const int i = i0 - 2 + c, j = j0 - 2 + r;
+    const double v = (i >= 0 && i < d.I && j >= 0 && j < d.J) ? mo[lev + (size_t)j * d.I + i] : 0.0;
+    out |= field_out(v);
+    s.m[r][c] = v;
+  }
+  // the level below enters the difference east of the last interior column
+  if (i0 + kTx >= d.I - 1 && k > 0 && tid < kTy + 4 && j0 + tid < d.J)
+    out |= field_out(mo[lev - (size_t)d.J * d.I + (size_t)(j0 + tid) * d.I + d.I - 1]);
+  if (__syncthreads_or(out))
+    tra_tile<true>(s, mo, mn, d, first != 0, i0, j0, k);
+  else
+    tra_tile<false>(s, mo, mn, d, first != 0, i0, j0, k);
+}
+
+// tra_adv.F90:196-251 for levels [ks, ke) of one interior column, from mi
+// (the field after the horizontal update) into mo.  Level ks's lower flux is
+// formed by a pass over level ks-1 that stores nothing.  A thread that meets
+// a value out of the bounded forms' range takes the other forms from there on.
+template <bool WIDE>
+__device__ __forceinline__ void tra_level(int K, int k, double mk, double mk1, double mk2,
+                                          double zd1, double slk, double tm2, double p1, double zw1, double zind,
+                                          double& zd2, double& slk1, double& fwk1) {
+  zd2 = k + 2 <= K - 2 ? tra_mul<WIDE>(tm2, mk1 - mk2) : 0.0;
+  slk1 = k + 1 <= K - 2 ? tra_slope<WIDE>(zd1, zd2) : 0.0;
+  // zalpha = 0.5 + SIGN(0.5, pwn): 1 for pwn >= +0, else +0
+  if (WIDE) {
+    const double z0w = half_sign(p1);
+    const double zw = courant(z0w, p1);
+    const double zzwx = mk1 + zind * (zw * slk1);
+    const double zzwy = mk + zind * (zw * slk);
+    fwk1 = p1 * ((bits(p1) < 0) ? pick(zzwy, zzwx) : pick(zzwx, zzwy));
+  } else {
+    fwk1 = upstream_b(p1, zw1, mk1, mk, zind, slk1, slk, bits(p1) >= 0);
+  }
+}
+
+__global__ void __launch_bounds__(256, 6)
+    k_tra_vertical(const double* __restrict__ mi, double* __restrict__ mo, TraDev d, int nseg,
+                   int wide) {
   const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
   if (i > d.I - 2 || j > d.J - 2) return;
   const size_t s = (size_t)d.I * d.J;
   const size_t c0 = (size_t)j * d.I + i;
   const int K = d.K;
-  double mk = m[c0];
-  double mk1 = m[c0 + s];  // K >= 2
-  double zd1 = (1 <= K - 2) ? d.tmask[c0 + s] * (mk - mk1) : 0.0;
-  double slk = 0.0;               // zslpx(:,:,1) = 0
-  double fwk = d.pwn[c0] * mk;    // zwx(:,:,1) = pwn m
-  for (int k = 0; k <= K - 2; k++) {
+  const int ks = (int)((long long)(K - 1) * blockIdx.z / nseg),
+            ke = (int)((long long)(K - 1) * (blockIdx.z + 1) / nseg);
+  const int k0 = ks > 0 ? ks - 1 : 0;  // the first level passed over
+  bool out = wide != 0;
+  double mk = mi[c0 + k0 * s], mk1 = mi[c0 + (k0 + 1) * s];  // K >= 2
+  double zd1 = (k0 + 1 <= K - 2) ? d.tmask[c0 + (k0 + 1) * s] * (mk - mk1) : 0.0;
+  double slk = 0.0;            // zslpx(:,:,1) = 0
+  double fwk = d.pwn[c0] * mk;  // zwx(:,:,1) = pwn m (overwritten where ks > 0)
+  out |= field_out(mk) | field_out(mk1);
+  if (k0 > 0) {  // the slope at k0, from the differences at k0 and k0 + 1
+    const double mb = mi[c0 + (k0 - 1) * s];
+    out |= field_out(mb);
+    const double zd0 = d.tmask[c0 + k0 * s] * (mb - mk);
+    slk = k0 <= K - 2 ? limit(slope_raw(zd0, zd1), zd1, zd0) : 0.0;
+  }
+  for (int k = k0; k < ke; k++) {
     const size_t c = c0 + (size_t)k * s;
-    double mk2 = 0.0, zd2 = 0.0;
-    if (k + 2 <= K - 1) mk2 = m[c + 2 * s];
-    if (k + 2 <= K - 2) zd2 = d.tmask[c + 2 * s] * (mk1 - mk2);
-    const double slk1 = (k + 1 <= K - 2) ? limit(slope_raw(zd1, zd2), zd2, zd1) : 0.0;
-    const double p1 = d.pwn[c + s];
-    const double z0w = half_sign(p1);
-    const double zw = courant(z0w, p1);
-    const double zind = d.zind[c];
-    const double zzwx = mk1 + zind * (zw * slk1);
-    const double zzwy = mk + zind * (zw * slk);
-    // zalpha = 0.5 + SIGN(0.5, pwn): 1 for pwn >= +0, else +0
-    const double fwk1 = p1 * ((bits(p1) < 0) ? pick(zzwy, zzwx) : pick(zzwx, zzwy));
-    m[c] = -(1.0 * (fwk - fwk1));
+    const double mk2 = k + 2 <= K - 1 ? mi[c + 2 * s] : 0.0;
+    const double tm2 = k + 2 <= K - 2 ? d.tmask[c + 2 * s] : 0.0;
+    const double p1 = d.pwn[c + s], zw1 = d.cwn[c + s], zind = d.zind[c];
+    double zd2, slk1, fwk1;
+    out |= field_out(mk2);
+    if (out)
+      tra_level<true>(K, k, mk, mk1, mk2, zd1, slk, tm2, p1, zw1, zind, zd2, slk1, fwk1);
+    else
+      tra_level<false>(K, k, mk, mk1, mk2, zd1, slk, tm2, p1, zw1, zind, zd2, slk1, fwk1);
+    if (k >= ks) mo[c] = -(1.0 * (fwk - fwk1));
     mk = mk1;
     mk1 = mk2;
     zd1 = zd2;
@@ -298,10 +438,10 @@ struct TraState {
   const void* key[12] = {};
   int I = 0, J = 0, K = 0;
   bool registered = false;
-  double* m[2] = {nullptr, nullptr};  // ping-pong copies of mydomain
+  double* m[2] = {nullptr, nullptr};  // mydomain, and the field between the two kernels
   double *pun = nullptr, *pvn = nullptr, *pwn = nullptr, *umask = nullptr, *vmask = nullptr,
-         *tmask = nullptr, *zind = nullptr;
-  int cur = 0;                 // buffer holding the current field
+         *tmask = nullptr, *zind = nullptr, *cun = nullptr, *cvn = nullptr, *cwn = nullptr;
+  int wide = 0;                // an input is outside the bounded forms' range
   long long iters = 0;         // iterations since registration
   cudaStream_t stream = nullptr;
   int status = NL2D_OK;
@@ -327,7 +467,7 @@ bool tra_ck(cudaError_t e, const char* what) {
 void tra_release() {
   TraState& s = g_tra;
   for (double** p : {&s.m[0], &s.m[1], &s.pun, &s.pvn, &s.pwn, &s.umask, &s.vmask, &s.tmask,
-                     &s.zind}) {
+                     &s.zind, &s.cun, &s.cvn, &s.cwn}) {
     if (*p) cudaFree(*p);
     *p = nullptr;
   }
@@ -336,19 +476,25 @@ void tra_release() {
 
 TraDev tra_dev() {
   const TraState& s = g_tra;
-  return TraDev{s.pun, s.pvn, s.pwn, s.umask, s.vmask, s.tmask, s.zind, s.I, s.J, s.K};
+  return TraDev{s.pun,  s.pvn, s.pwn, s.umask, s.vmask, s.tmask, s.zind,
+                s.cun,  s.cvn, s.cwn, s.I,     s.J,     s.K};
 }
 
 // One iteration's two launches on the library's stream.
-void tra_launch_iteration(int cur, bool first) {
+void tra_launch_iteration(bool first) {
   TraState& s = g_tra;
   const dim3 blk(kTx, kTy);
   const dim3 grd((s.I - 2 + kTx - 1) / kTx, (s.J - 2 + kTy - 1) / kTy, s.K - 1);
-  k_tra_horizontal_tiled<<<grd, blk, 0, s.stream>>>(s.m[cur], s.m[cur ^ 1], tra_dev(),
-                                                     first ? 1 : 0);
-  const dim3 vblk(32, 8);
-  const dim3 vgrd((s.I - 2 + 31) / 32, (s.J - 2 + 7) / 8, 1);
-  k_tra_vertical<<<vgrd, vblk, 0, s.stream>>>(s.m[cur ^ 1], tra_dev());
+  k_tra_horizontal<<<grd, blk, 0, s.stream>>>(s.m[0], s.m[1], tra_dev(), first ? 1 : 0, s.wide);
+  // Columns cut into runs of levels until the grid holds eight blocks of 256
+  // threads per SM, a run at least three levels (it passes over one more than
+  // it stores): 512 x 512 columns of 75 levels in two runs each 926 us per
+  // iteration, whole 936; 93 x 67 of 31 in eight.
+  const int bx = (s.I - 2 + 31) / 32, by = (s.J - 2 + 7) / 8;
+  int nseg = 1;
+  while (bx * by * nseg < 8 * 152 && (s.K - 1) / (2 * nseg) >= 3) nseg *= 2;
+  k_tra_vertical<<<dim3(bx, by, nseg), dim3(32, 8), 0, s.stream>>>(s.m[1], s.m[0], tra_dev(),
+                                                                   nseg, s.wide);
 }
 
 bool tra_register(const double* ztfreez, const double* pun, const double* pvn, const double* pwn,
@@ -367,10 +513,12 @@ bool tra_register(const double* ztfreez, const double* pun, const double* pvn, c
   const size_t n3 = (size_t)I * J * K, b3 = n3 * sizeof(double);
   const size_t b2 = (size_t)I * J * sizeof(double);
   for (double** p : {&s.m[0], &s.m[1], &s.pun, &s.pvn, &s.pwn, &s.umask, &s.vmask, &s.tmask,
-                     &s.zind})
+                     &s.zind, &s.cun, &s.cvn, &s.cwn})
     if (!tra_ck(cudaMalloc(p, b3), "cudaMalloc")) return false;
   double *d_tsn = nullptr, *d2[3] = {nullptr, nullptr, nullptr}, *d_rz = nullptr;
+  int* d_wide = nullptr;
   bool ok = tra_ck(cudaMalloc(&d_tsn, b3), "cudaMalloc") &&
+            tra_ck(cudaMalloc(&d_wide, sizeof(int)), "cudaMalloc") &&
             tra_ck(cudaMalloc(&d_rz, K * sizeof(double)), "cudaMalloc");
   for (int q = 0; q < 3 && ok; q++) ok = tra_ck(cudaMalloc(&d2[q], b2), "cudaMalloc");
   const struct {
@@ -387,13 +535,20 @@ bool tra_register(const double* ztfreez, const double* pun, const double* pvn, c
   if (ok) {
     ok = tra_ck(cudaMemcpyAsync(s.m[1], s.m[0], b3, cudaMemcpyDeviceToDevice, s.stream),
                 "copy");
-    k_tra_zind<<<152 * 8, 256, 0, s.stream>>>(d_tsn, d2[0], d2[1], d2[2], d_rz, s.tmask, s.zind,
-                                              I, J, K);
+    TraDev d = tra_dev();
+    d.I = I, d.J = J, d.K = K;
+    ok = ok && tra_ck(cudaMemsetAsync(d_wide, 0, sizeof(int), s.stream), "memset");
+    if (ok)
+      k_tra_zind<<<152 * 8, 256, 0, s.stream>>>(d_tsn, d2[0], d2[1], d2[2], d_rz, d, s.zind,
+                                                s.cun, s.cvn, s.cwn, d_wide);
     ok = ok && tra_ck(cudaGetLastError(), "k_tra_zind") &&
+         tra_ck(cudaMemcpyAsync(&s.wide, d_wide, sizeof(int), cudaMemcpyDeviceToHost, s.stream),
+                "registration") &&
          tra_ck(cudaStreamSynchronize(s.stream), "registration");
   }
   cudaFree(d_tsn);
   cudaFree(d_rz);
+  cudaFree(d_wide);
   for (double* p : d2) cudaFree(p);
   if (!ok) {
     tra_release();
@@ -403,7 +558,6 @@ bool tra_register(const double* ztfreez, const double* pun, const double* pvn, c
   s.I = I;
   s.J = J;
   s.K = K;
-  s.cur = 0;
   s.iters = 0;
   s.registered = true;
   return true;
@@ -430,9 +584,8 @@ void tra_adv_compute(const double* ztfreez, const double* pun, const double* pvn
                     mydomain, tsn, jpi, jpj, jpk))
     return;
   TraState& s = g_tra;
-  tra_launch_iteration(s.cur, s.iters == 0);
+  tra_launch_iteration(s.iters == 0);
   if (!tra_ck(cudaGetLastError(), "tra_adv iteration")) return;
-  s.cur ^= 1;
   s.iters++;
 }
 
@@ -447,8 +600,7 @@ int tra_adv_run(int niter, double* ms) {
     return NL2D_ERR_CUDA;
   cudaEventRecord(e0, s.stream);
   for (int t = 0; t < niter; t++) {
-    tra_launch_iteration(s.cur, s.iters == 0);
-    s.cur ^= 1;
+    tra_launch_iteration(s.iters == 0);
     s.iters++;
   }
   cudaEventRecord(e1, s.stream);
@@ -467,7 +619,7 @@ int tra_adv_read(double* mydomain) {
   if (!s.registered) return NL2D_ERR_STATE;
   if (!mydomain) return NL2D_ERR_ARGS;
   const size_t b3 = (size_t)s.I * s.J * s.K * sizeof(double);
-  if (!tra_ck(cudaMemcpyAsync(mydomain, s.m[s.cur], b3, cudaMemcpyDeviceToHost, s.stream),
+  if (!tra_ck(cudaMemcpyAsync(mydomain, s.m[0], b3, cudaMemcpyDeviceToHost, s.stream),
               "tra_adv_read") ||
       !tra_ck(cudaStreamSynchronize(s.stream), "tra_adv_read"))
     return NL2D_ERR_CUDA;
