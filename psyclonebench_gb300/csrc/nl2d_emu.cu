@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "../../include/nl2d_gpu.h"
 
@@ -67,32 +68,48 @@ constexpr int kRowPix = 136;
 
 // ---- 3x3 convolution ------------------------------------------------------
 //
-// Implicit GEMM on the tensor cores: M = 128 pixels of one image row,
-// N = cout, K = 9 taps x cin.  The 9 weight taps stay in shared memory for
-// the CTA's lifetime.  A staged input row keeps each 8-channel group of its
-// pixels 16 bytes apart, so the operand of tap (dy, dx) is the dy-th row of
-// the window started dx pixels (16 * dx bytes) later: a descriptor offset,
-// no per-tap copies.  Warp-specialised and persistent: a CTA walks strips
-// of kStripRows output rows of one 128-pixel column segment.  Input rows pass
-// through a ring of kSlots shared-memory slots (each input row is staged
-// once per strip instead of three times), the accumulator alternates
-// between two TMEM buffers, and the three roles overlap:
+// Implicit GEMM on the tensor cores: M = 128 pixels of one image row, N =
+// output channels, K = input channels.  What bounds it is the tensor core's
+// operand reads from shared memory, so an input row is read once for all
+// three output rows it enters: with the weights of dy = 2, 1, 0 side by side
+// (N = 3 cout), input row y adds to output rows y-1, y and y+1 in one MMA per
+// dx and 16 channels, their accumulators lying in adjacent column blocks of a
+// ring in tensor memory: 9 MMAs of N = 144 per row at 48 -> 48 channels
+// instead of 27 of N = 48.  (The ring's end splits an MMA in two, and the new
+// row's block takes its first MMA apart, to start from zero.)
+//
+// The weights stay in shared memory for the CTA's lifetime.  A staged input
+// row keeps each 8-channel group of its pixels 16 bytes apart, so the operand
+// of tap dx is the row started dx pixels (16 * dx bytes) later: a descriptor
+// offset, no per-tap copies.  Warp-specialised and persistent: a CTA takes an
+// equal, contiguous share of the rows of all 128-pixel columns.  Roles:
 //   warps 0-3  epilogue: TMEM -> bias, ReLU -> BF16 / FP32 stores
-//   warp 4     one thread issues the MMAs of an output row once its three
-//              input rows are staged and its TMEM buffer is free
-//   warps 5-7  stage input rows into the ring
+//   warp 4     one thread issues the MMAs of an input row once it is staged
+//              and the new output row's accumulator block is free
+//   warps 5-7  stage input rows into a ring of slots by cp.async
 // Hand-offs are mbarriers: full[slot] (stagers -> MMA), empty[slot] (MMA
-// completion -> stagers), done[buf] (MMA completion -> epilogue),
-// drained[buf] (epilogue -> MMA).  Every wait is bounded (kMaxWaitCycles);
+// completion -> stagers), done[block] (MMA completion -> epilogue),
+// drained[block] (epilogue -> MMA).  Every wait is bounded (kMaxWaitCycles);
 // one that runs out sets the error flag and a shared abort flag that ends
 // every role's loop, and the MMA thread waits for its last commit before the
 // tensor memory is freed.
-constexpr int kStripRows = 8;
-constexpr int kConvSlots = 5;  // the convolution's input ring: 3 rows read, 2 in flight
+constexpr int kConvSlots = 5;  // the input ring
+constexpr int kConvDepth = 2;  // rows in flight (four: 68.2 us, two: 66.3)
+constexpr int kConvMaxBlocks = 8;
 constexpr int kPipeThreads = 256;
 constexpr int kEpiWarps = 4;
 constexpr int kStageThreads = 96;  // warps 5-7
-constexpr int kPipeTmemCols = 128;  // two accumulators of up to 64 columns
+constexpr uint32_t kLboX = kRowPix * 16 + 16;  // next 8 input channels (padded: banks)
+
+// Accumulator blocks of cout columns (at least four: three being summed, one
+// being drained) and the tensor memory they take: two CTAs share an SM's 512
+// columns.
+__host__ __device__ constexpr int conv_blocks(int cout) {
+  return 256 / cout < kConvMaxBlocks ? 256 / cout : kConvMaxBlocks;
+}
+__host__ __device__ constexpr int conv_tmem(int cout) {
+  return conv_blocks(cout) * cout <= 128 ? 128 : 256;
+}
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
@@ -102,10 +119,24 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
                    smem_u32(bar))
                : "memory");
 }
+// The MMAs and commits below are executed by a whole, converged warp of which
+// one elected lane (always the same) issues them: the operands then stay in
+// uniform registers (the convolution 72.1 -> 68.2 us against issuing them from
+// a branch of one lane).
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(
           smem_u32(bar))
+      : "memory");
+}
+// [dcol] (+)= A B with M = 128, BF16 operands from shared memory.
+__device__ __forceinline__ void tc_mma(uint32_t dcol, uint64_t ad, uint64_t bd, uint32_t idesc,
+                                       uint32_t acc) {
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nelect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dcol),
+      "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
       : "memory");
 }
 // 16 FP32 columns of 32 tensor-memory lanes; the values are there after
@@ -118,6 +149,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t (&r)[16], uint32_t ta) {
         "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
         "=r"(r[14]), "=r"(r[15])
       : "r"(ta));
+}
+// 32 bytes to p: one store where p is 32-byte aligned (`whole`: a whole
+// sector per lane), else two.
+__device__ __forceinline__ void store_32b(void* p, const uint32_t (&v)[8], int whole) {
+  if (whole)
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]),
+                 "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+  else {
+    reinterpret_cast<uint4*>(p)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<uint4*>(p)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+  }
 }
 // Waits for the phase with the given parity to complete; false if the wait
 // ran out after max_cycles (flag and error set) or another role aborted.
@@ -158,17 +201,25 @@ __global__ void k_selftest_wait(long long max_cycles, int* err) {
   if (threadIdx.x == 0 && mbar_wait(&bar, 0, &abort_flag, err, max_cycles)) atomicExch(err, 2);
 }
 
-struct StripWalk {  // work unit u -> (image, first row, rows, column segment)
-  int img, y0, rows, x0;
-  __device__ StripWalk(long long u, int H, int segs) {
-    const int strips = (H + kStripRows - 1) / kStripRows;
-    const int seg = (int)(u % segs);
-    const long long r = u / segs;
-    const int st = (int)(r % strips);
-    img = (int)(r / strips);
-    y0 = st * kStripRows;
-    rows = min(kStripRows, H - y0);
-    x0 = seg * kTileM;
+// A CTA's share of the rows: rows [g, end) of the list of all columns' rows,
+// cut into segments of one column each.
+struct RowSegments {
+  long long g, end;
+  int H, segs;
+  __device__ RowSegments(int batch, int H_, int segs_) : H(H_), segs(segs_) {
+    const long long total = (long long)batch * segs * H;
+    g = total * blockIdx.x / gridDim.x;
+    end = total * (blockIdx.x + 1) / gridDim.x;
+  }
+  __device__ bool next(int& img, int& x0, int& y0, int& rows) {
+    if (g >= end) return false;
+    const long long col = g / H;
+    img = (int)(col / segs);
+    x0 = (int)(col - (long long)img * segs) * kTileM;
+    y0 = (int)(g - col * H);
+    rows = (int)(end - g < H - y0 ? end - g : H - y0);
+    g += rows;
+    return true;
   }
 };
 
@@ -176,36 +227,40 @@ __global__ void __launch_bounds__(kPipeThreads)
     k_conv3x3_pipe(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const float* __restrict__ bias, __nv_bfloat16* __restrict__ y,
                    float* __restrict__ y32, int batch, int H, int W, int cin, int cout,
-                   int relu, int* __restrict__ err) {
+                   int relu, int wide_store, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t full_bar[kConvSlots], empty_bar[kConvSlots];
-  __shared__ __align__(8) uint64_t done_bar[2], drained_bar[2], last_bar;
+  __shared__ __align__(8) uint64_t done_bar[kConvMaxBlocks], drained_bar[kConvMaxBlocks], last_bar;
+  __shared__ __align__(16) float bias_s[64];
   __shared__ uint32_t taddr_slot;
   __shared__ int abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int kc = cin >> 3;
-  const uint32_t lbo_a = kRowPix * 16;
-  const uint32_t row_bytes = (uint32_t)kc * lbo_a;
-  const uint32_t b_bytes = (uint32_t)cout * cin * 2;
+  const int blocks = conv_blocks(cout);
+  const uint32_t row_bytes = (uint32_t)kc * kLboX;
+  const uint32_t b_bytes = 3u * (uint32_t)cout * cin * 2;  // one dx: [dy = 2, 1, 0][cout][cin]
   unsigned char* b_s = smem;
-  unsigned char* ring = smem + ((9 * b_bytes + 1023) & ~1023u);
+  unsigned char* ring = smem + ((3 * b_bytes + 1023) & ~1023u);
   volatile int* abort_v = &abort_flag;
 
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&taddr_slot)),
-                 "r"(kPipeTmemCols));
+    if (conv_tmem(cout) == 128)
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(
+          smem_u32(&taddr_slot)));
+    else
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(
+          smem_u32(&taddr_slot)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
     for (int q = 0; q < kConvSlots; q++) {
-      mbar_init(&full_bar[q], kStageThreads);
+      mbar_init(&full_bar[q], kStageThreads / 32);
       mbar_init(&empty_bar[q], 1);
     }
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < blocks; q++) {
       mbar_init(&done_bar[q], 1);
-      mbar_init(&drained_bar[q], kEpiWarps * 32);
+      mbar_init(&drained_bar[q], kEpiWarps);
     }
     mbar_init(&last_bar, 1);
     abort_flag = 0;
@@ -214,125 +269,147 @@ __global__ void __launch_bounds__(kPipeThreads)
   for (int t = tid; t < 9 * cout * kc; t += kPipeThreads) {
     const int tap = t / (cout * kc), rem = t - tap * cout * kc;
     const int n = rem / kc, ch = rem - n * kc;
+    const int dy = tap / 3, dx = tap - 3 * dy;
     const uint4 v =
         *reinterpret_cast<const uint4*>(w + ((size_t)tap * cout + n) * cin + ch * 8);
-    *reinterpret_cast<uint4*>(b_s + tap * b_bytes + core_off(n, ch * 8, cin)) = v;
+    *reinterpret_cast<uint4*>(b_s + dx * b_bytes + core_off((2 - dy) * cout + n, ch * 8, cin)) = v;
   }
+  if (tid < cout) bias_s[tid] = bias ? bias[tid] : 0.f;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t taddr = taddr_slot;
   const int segs = W / kTileM;
-  const long long units = (long long)batch * ((H + kStripRows - 1) / kStripRows) * segs;
+  RowSegments rs(batch, H, segs);
+  int img, x0, y0, rows;
+  // Positions in the rings of slots and blocks: the index, and the parity of
+  // the phase to wait for.
+  struct Pos {
+    int at;
+    uint32_t par;
+  };
+  auto next = [](Pos p, int n) {
+    const bool wrap = p.at + 1 == n;
+    return Pos{wrap ? 0 : p.at + 1, p.par ^ (wrap ? 1u : 0u)};
+  };
 
   if (warp >= 5) {
-    // ---- stagers: input rows y0-1 .. y0+rows of every strip, in order.
+    // ---- stagers: input rows y0-1 .. y0+rows of every segment, in order.
     // cp.async copies each 16-byte group of 8 channels straight into its
-    // ring slot (zero-filled outside the image), so a stager does not hold
-    // a row in registers: it starts row q, then waits for its own copies of
-    // row q-1, makes them visible to the tensor core's (async) proxy and
-    // marks that slot full.  Two rows are in flight per CTA (the ring's
-    // other three slots hold the rows the MMAs read), where register
-    // staging kept one.
+    // ring slot (zero-filled outside the image); consecutive threads take
+    // consecutive groups of a pixel, so a warp's copies cover whole lines,
+    // and a thread's chunks have the same offsets in every row.  A row is
+    // marked full once kConvDepth - 1 younger rows are in flight.
     const int st = tid - 5 * 32;
-    long long q = 0;      // input rows started so far (ring sequence)
-    bool pending = false;  // row q-1 started, its slot not yet marked full
-    for (long long u = blockIdx.x; u < units && !*abort_v; u += gridDim.x) {
-      const StripWalk sw(u, H, segs);
-      for (int a = 0; a < sw.rows + 2 && !*abort_v; a++, q++) {
-        const int slot = (int)(q % kConvSlots);
-        const int yy = sw.y0 - 1 + a;
-        if (q >= kConvSlots &&
-            !mbar_wait(&empty_bar[slot], (uint32_t)((q / kConvSlots - 1) & 1), abort_v, err))
-          break;
-        const uint32_t dst = smem_u32(ring + slot * row_bytes);
-        for (int t = st; t < kc * kRowPix; t += kStageThreads) {
-          const int p = t % kRowPix, ch = t / kRowPix;
-          const int xx = sw.x0 - 1 + p;
-          const bool in = yy >= 0 && yy < H && xx >= 0 && xx < W;
-          const __nv_bfloat16* src =
-              in ? x + (((size_t)sw.img * H + yy) * W + xx) * cin + ch * 8 : x;
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                           dst + (uint32_t)(ch * lbo_a + p * 16)),
-                       "l"(src), "r"(in ? 16 : 0)
-                       : "memory");
-        }
+    constexpr int kX = (8 * kRowPix + kStageThreads - 1) / kStageThreads;  // cin <= 64
+    uint32_t dst[kX];
+    int off[kX];
+    unsigned mine = 0, left = 0, right = 0;  // chunks there are; in the edge columns
+#pragma unroll
+    for (int k = 0; k < kX; k++) {
+      const int t = st + k * kStageThreads, p = t / kc, ch = t - p * kc;
+      dst[k] = (uint32_t)(ch * kLboX + p * 16);
+      off[k] = (p - 1) * cin + ch * 8;
+      if (p < kRowPix) mine |= 1u << k;
+      if (p == 0) left |= 1u << k;
+      if (p > kTileM) right |= 1u << k;  // pixel x0 + 128 and beyond (only the first is read)
+    }
+    Pos put{0, 1}, mark{0, 0};
+    int ahead = 0;  // rows started and not yet marked full
+    bool fresh = true, ok = true;  // the ring's first turn waits for nothing
+    auto finish = [&]() {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full_bar[mark.at]);
+      mark = next(mark, kConvSlots);
+      ahead--;
+    };
+    while (ok && rs.next(img, x0, y0, rows) && !*abort_v) {
+      const unsigned in = mine & ~(x0 == 0 ? left : 0u) & ~(x0 + kTileM >= W ? right : 0u);
+      const __nv_bfloat16* seg = x + (((size_t)img * H + y0) * W + x0) * cin;
+      for (int a = 0; a < rows + 2; a++) {
+        const int yy = y0 - 1 + a;
+        if (!fresh) ok = mbar_wait(&empty_bar[put.at], put.par, abort_v, err);
+        if (!ok) break;
+        const unsigned take = yy >= 0 && yy < H ? in : 0u;
+        const __nv_bfloat16* src = seg + (long long)(a - 1) * W * cin;
+        const uint32_t d0 = smem_u32(ring + put.at * row_bytes);
+#pragma unroll
+        for (int k = 0; k < kX; k++)
+          if (mine >> k & 1u) {
+            const bool t = take >> k & 1u;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d0 + dst[k]),
+                         "l"(t ? src + off[k] : x), "r"(t ? 16 : 0)
+                         : "memory");
+          }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (pending) {  // row q-1 has landed once at most one group is open
-          asm volatile("cp.async.wait_group 1;" ::: "memory");
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          mbar_arrive(&full_bar[(q - 1) % kConvSlots]);
+        put = next(put, kConvSlots);
+        if (put.at == 0) fresh = false;
+        if (++ahead == kConvDepth) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(kConvDepth - 1) : "memory");
+          finish();
         }
-        pending = true;
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    if (pending && !*abort_v) {  // the last row started
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_arrive(&full_bar[(q - 1) % kConvSlots]);
-    }
+    while (ahead > 0 && !*abort_v) finish();
   } else if (warp == 4) {
-    // ---- MMA issuer ----
-    if (lane == 0) {
-      const uint32_t idesc = idesc_bf16(cout);
+    // ---- MMA issuer: the whole warp walks, one lane issues ----
+    {
       const uint64_t b_desc0 = smem_desc(smem_u32(b_s), 128, (uint32_t)cin * 16);
-      const uint32_t a_kstep = (2 * lbo_a) >> 4;
+      const uint64_t a_desc0 = smem_desc(smem_u32(ring), kLboX, 128);
+      const uint32_t a_kstep = (2 * kLboX) >> 4;
+      const uint32_t b_block = ((uint32_t)cout * cin * 2) >> 4;  // one dy's weights
       const int kcq = cin / 16;
-      long long q = 0, p = 0;  // input rows consumed (sequence base), output rows issued
-      bool issued = false;
-      for (long long u = blockIdx.x; u < units && !*abort_v; u += gridDim.x) {
-        const StripWalk sw(u, H, segs);
-        const long long qb = q;  // sequence number of this strip's first input row
-        // its first two input rows
-        bool ok = mbar_wait(&full_bar[qb % kConvSlots], (uint32_t)((qb / kConvSlots) & 1),
-                            abort_v, err) &&
-                  mbar_wait(&full_bar[(qb + 1) % kConvSlots],
-                            (uint32_t)(((qb + 1) / kConvSlots) & 1), abort_v, err);
-        for (int o = 0; o < sw.rows && ok; o++, p++) {
-          const long long qn = qb + o + 2;  // the new input row this output needs
-          const int buf = (int)(p & 1);
-          ok = mbar_wait(&full_bar[qn % kConvSlots], (uint32_t)((qn / kConvSlots) & 1), abort_v,
-                         err);
-          if (ok && p >= 2)
-            ok = mbar_wait(&drained_bar[buf], (uint32_t)((p / 2 - 1) & 1), abort_v, err);
+      const uint32_t idesc[3] = {idesc_bf16(cout), idesc_bf16(2 * cout), idesc_bf16(3 * cout)};
+      // n blocks from column block `at`, weights from dy block `from`
+      auto mma = [&](int at, int from, int n, uint64_t ad, uint64_t bd, uint32_t acc) {
+        tc_mma(taddr + (uint32_t)(at * cout), ad, bd + (uint64_t)((uint32_t)from * b_block),
+               n == 1 ? idesc[0] : (n == 2 ? idesc[1] : idesc[2]), acc);
+      };
+      Pos in{0, 0};            // the input row's slot
+      Pos fresh{0, 1};         // the new output row's block
+      Pos oldest{0, 0};        // the block of the oldest output row being summed
+      bool first_turn = true, issued = false, ok = true;
+      while (ok && rs.next(img, x0, y0, rows) && __all_sync(0xffffffffu, !*abort_v)) {
+        for (int a = 0; a < rows + 2 && ok; a++) {
+          // output rows (of the segment) max(0, a-2) .. min(rows-1, a)
+          const int lo = a > 2 ? a - 2 : 0, hi = a < rows ? a : rows - 1;
+          const int n = hi - lo + 1, from = lo - (a - 2);
+          const bool opens = a < rows;
+          ok = mbar_wait(&full_bar[in.at], in.par, abort_v, err);
+          if (ok && opens && !first_turn)
+            ok = mbar_wait(&drained_bar[fresh.at], fresh.par, abort_v, err);
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t dcol = taddr + (uint32_t)(buf * 64);
-          // Operand descriptors: built once per input row and for tap 0, then
-          // advanced by adding byte offsets / 16 to their address field
-          // (shared addresses stay below 256 KB, so the field never carries
-          // into the others): + dx for the tap's pixel shift, + 2 lbo / 16
-          // per A K-step, + 256 / 16 per B K-step, + b_bytes / 16 per tap.
-          uint64_t arow[3];
+          const int to_end = blocks - oldest.at;  // blocks before the ring's end
+          uint64_t arow = a_desc0 + (uint64_t)((uint32_t)in.at * (row_bytes >> 4));
+          uint64_t bdx = b_desc0;
 #pragma unroll
-          for (int dy = 0; dy < 3; dy++)
-            arow[dy] = smem_desc(smem_u32(ring + (int)((qb + o + dy) % kConvSlots) * row_bytes),
-                                 lbo_a, 128);
-          uint64_t btap = b_desc0;
-          uint32_t acc = 0u;
-#pragma unroll
-          for (int tap = 0; tap < 9; tap++, btap += b_bytes >> 4) {
-            uint64_t ad = arow[tap / 3] + (uint64_t)(tap % 3), bd = btap;
+          for (int dx = 0; dx < 3; dx++, arow += 1, bdx += b_bytes >> 4) {
+            uint64_t ad = arow, bd = bdx;
             for (int kq = 0; kq < kcq; kq++, ad += a_kstep, bd += 256 >> 4) {
-              asm volatile(
-                  "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dcol),
-                  "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-              acc = 1u;
+              // the new row's block starts from zero: its first MMA apart
+              const bool apart = opens && dx == 0 && kq == 0;
+              const int m = apart ? n - 1 : n, m1 = m < to_end ? m : to_end;
+              if (m1 > 0) mma(oldest.at, from, m1, ad, bd, 1u);
+              if (m > m1) mma(0, from + m1, m - m1, ad, bd, 1u);
+              if (apart) mma(fresh.at, from + m, 1, ad, bd, 0u);
             }
           }
           issued = true;
-          tc_commit(&done_bar[buf]);
-          // input row o is not read by later outputs of this strip
-          tc_commit(&empty_bar[(qb + o) % kConvSlots]);
-        }
-        q = qb + sw.rows + 2;
-        if (ok) {  // the strip's last two input rows are free too
-          tc_commit(&empty_bar[(q - 2) % kConvSlots]);
-          tc_commit(&empty_bar[(q - 1) % kConvSlots]);
-        } else {
-          break;
+          tc_commit(&empty_bar[in.at]);
+          in = next(in, kConvSlots);
+          if (opens) {
+            fresh = next(fresh, blocks);
+            if (fresh.at == 0) first_turn = false;
+          }
+          if (a >= 2) {  // output row a - 2 is complete
+            tc_commit(&done_bar[oldest.at]);
+            oldest = next(oldest, blocks);
+          }
         }
       }
       if (issued) {  // nothing may be in flight when the tensor memory is freed
@@ -343,60 +420,74 @@ __global__ void __launch_bounds__(kPipeThreads)
     }
   } else {
     // ---- epilogue: warp w owns accumulator lanes (pixels) 32w .. 32w+31 ----
-    long long p = 0;
-    for (long long u = blockIdx.x; u < units && !*abort_v; u += gridDim.x) {
-      const StripWalk sw(u, H, segs);
-      for (int o = 0; o < sw.rows; o++, p++) {
-        const int buf = (int)(p & 1);
+    Pos blk{0, 0};
+    bool ok = true;
+    while (ok && rs.next(img, x0, y0, rows) && !*abort_v) {
+      size_t pix = ((size_t)img * H + y0) * W + x0 + warp * 32 + lane;
+      for (int o = 0; o < rows; o++, pix += W) {
         // warp-uniform outcome: tcgen05.ld below needs the whole warp
-        const bool ok = mbar_wait(&done_bar[buf], (uint32_t)((p / 2) & 1), abort_v, err);
-        if (!__all_sync(0xffffffffu, ok)) break;
+        ok = mbar_wait(&done_bar[blk.at], blk.par, abort_v, err);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int m = warp * 32 + lane;
-        const size_t pix = ((size_t)sw.img * H + sw.y0 + o) * W + sw.x0 + m;
-        for (int n0 = 0; n0 < cout; n0 += 16) {
-          uint32_t r[16];
-          const uint32_t ta =
-              taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * 64 + n0);
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,"
-              "%12,%13,%14,%15}, [%16];"
-              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-                "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-                "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-              : "r"(ta));
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          __align__(16) __nv_bfloat16 out[16];
+        const uint32_t ta =
+            taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(blk.at * cout);
+        uint32_t r[4][16];
+        const int nq = cout >> 4;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          if (q < nq) tmem_ld16(r[q], ta + 16 * q);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&drained_bar[blk.at]);  // the values are in registers
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          if (q >= nq) break;
           float v[16];
 #pragma unroll
-          for (int k = 0; k < 16; k++) {
-            v[k] = __uint_as_float(r[k]) + (bias ? bias[n0 + k] : 0.f);
-            if (relu) v[k] = fmaxf(v[k], 0.f);
-            out[k] = __float2bfloat16(v[k]);
+          for (int k = 0; k < 16; k += 4) {
+            const float4 b4 = *reinterpret_cast<const float4*>(bias_s + 16 * q + k);
+            v[k] = __uint_as_float(r[q][k]) + b4.x;
+            v[k + 1] = __uint_as_float(r[q][k + 1]) + b4.y;
+            v[k + 2] = __uint_as_float(r[q][k + 2]) + b4.z;
+            v[k + 3] = __uint_as_float(r[q][k + 3]) + b4.w;
           }
+          if (relu)
+#pragma unroll
+            for (int k = 0; k < 16; k++) v[k] = fmaxf(v[k], 0.f);
           if (y) {
-            uint4* dst = reinterpret_cast<uint4*>(y + pix * cout + n0);
-            dst[0] = reinterpret_cast<const uint4*>(out)[0];
-            dst[1] = reinterpret_cast<const uint4*>(out)[1];
+            uint32_t o2[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+              o2[k] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            store_32b(y + pix * cout + 16 * q, o2, wide_store & 1);
           }
           if (y32) {
-            float4* dst = reinterpret_cast<float4*>(y32 + pix * cout + n0);
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-              dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+            for (int h = 0; h < 2; h++) {
+              uint32_t o4[8];
+#pragma unroll
+              for (int k = 0; k < 8; k++) o4[k] = __float_as_uint(v[8 * h + k]);
+              store_32b(y32 + pix * cout + 16 * q + 8 * h, o4, wide_store & 2);
+            }
           }
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        mbar_arrive(&drained_bar[buf]);
+        blk = next(blk, blocks);
       }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr),
-                 "r"(kPipeTmemCols));
+  if (warp == 0) {
+    if (conv_tmem(cout) == 128)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(taddr));
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(taddr));
+  }
 }
 
 // Tap-flipped, channel-transposed weights for the input gradient:
@@ -443,14 +534,11 @@ __global__ void k_flip_transpose(const __nv_bfloat16* __restrict__ w,
 // 48 -> 48 channels at 16 x 256^2: 193 us (9 x N = 48 per row, one row in
 // flight in registers) plus 24 us for a separate bias pass before.
 constexpr int kWgTmemCols = 512;
-#ifndef WGW
-#define WGW 8
-#endif
-constexpr int kWgThreads = 32 * WGW, kWgStagers = kWgThreads - 32;  // the last warp issues
-constexpr int kWgDepth = 3;      // rows in flight per CTA (fewer where slots are scarce)
+constexpr int kWgThreads = 256, kWgStagers = kWgThreads - 32;  // the last warp issues
+constexpr int kWgDepth = 2;  // rows in flight per CTA (1: 118 us, 2: 99, 3: 101, 4: 104)
 constexpr int kWgMaxSlots = 8;
 constexpr uint32_t kWgLboY = kTileM * 16 + 16;   // next 8 output channels (padded: banks)
-constexpr uint32_t kWgLboX = kRowPix * 16 + 16;  // next 8 input channels
+constexpr uint32_t kWgLboX = kLboX;
 constexpr size_t kWgMaxSmem = 216 * 1024;
 
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int n) {
@@ -474,28 +562,6 @@ __host__ __device__ constexpr int wg_depth(int cout, int slots) {
   const int d = slots - (cout <= 64 ? 1 : 2);
   return d < kWgDepth ? d : kWgDepth;
 }
-
-// A CTA's share of the rows: rows [g, end) of the list of all columns' rows,
-// cut into segments of one column each.
-struct RowSegments {
-  long long g, end;
-  int H, segs;
-  __device__ RowSegments(int batch, int H_, int segs_) : H(H_), segs(segs_) {
-    const long long total = (long long)batch * segs * H;
-    g = total * blockIdx.x / gridDim.x;
-    end = total * (blockIdx.x + 1) / gridDim.x;
-  }
-  __device__ bool next(int& img, int& x0, int& y0, int& rows) {
-    if (g >= end) return false;
-    const long long col = g / H;
-    img = (int)(col / segs);
-    x0 = (int)(col - (long long)img * segs) * kTileM;
-    y0 = (int)(g - col * H);
-    rows = (int)(end - g < H - y0 ? end - g : H - y0);
-    g += rows;
-    return true;
-  }
-};
 
 __global__ void __launch_bounds__(kWgThreads)
     k_conv_wgrad_pipe(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
@@ -540,8 +606,8 @@ __global__ void __launch_bounds__(kWgThreads)
   float* mine = part + (size_t)blockIdx.x * (nel + cout);
 
   if (tid >= kWgStagers) {
-    // ---- MMA issuer ----
-    if (lane == 0) {
+    // ---- MMA issuer: the whole warp walks, one lane issues ----
+    {
       const uint32_t idesc = idesc_bf16_mn(pair ? 2 * cin : cin);
       RowSegments rs(batch, H, segs);
       bool issued = false, ok = true;
@@ -557,25 +623,25 @@ __global__ void __launch_bounds__(kWgThreads)
         const bool wrap = p.slot + 1 == slots;
         return Pos{wrap ? 0 : p.slot + 1, p.par ^ (wrap ? 1u : 0u)};
       };
-      auto full = [&](Pos p) { return mbar_wait(&full_bar[p.slot], p.par, abort_v, err); };
+      auto full = [&](Pos p) {
+        return (bool)__all_sync(0xffffffffu, mbar_wait(&full_bar[p.slot], p.par, abort_v, err));
+      };
       const uint64_t yd0 = smem_desc(smem_u32(yring), 128, kWgLboY);
       const uint64_t xd0 = smem_desc(smem_u32(xring), 128, kWgLboX);
-      auto mma = [&](uint32_t dcol, uint64_t ad, uint64_t bd) {
-        // MN-major, no swizzle: LBO steps along K (8 pixels = 128 B), SBO
-        // along M / N (the next 8 channels); + 256 / 16 per K-step of 16
-        // pixels (the address field never carries: shared addresses stay
-        // below 256 KB)
+      // One K-step (16 pixels) of a row after the other, its accumulators in
+      // turn.  MN-major, no swizzle: LBO steps along K (8 pixels = 128
+      // B), SBO along M / N (the next 8 channels); + 256 / 16 per K-step (the
+      // address field never carries: shared addresses stay below 256 KB).
+      auto mmas = [&](auto count, uint64_t yd, auto xdesc, uint32_t cols) {
 #pragma unroll
-        for (int kq = 0; kq < kTileM / 16; kq++, ad += 256 >> 4, bd += 256 >> 4) {
-          const uint32_t acc = (issued || kq > 0) ? 1u : 0u;
-          asm volatile(
-              "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dcol),
-              "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-        }
+        for (int kq = 0; kq < kTileM / 16; kq++)
+#pragma unroll
+          for (int b = 0; b < decltype(count)::value; b++)
+            tc_mma(taddr + (uint32_t)b * cols, yd + (uint64_t)(kq * (256 >> 4)),
+                   xdesc(b) + (uint64_t)(kq * (256 >> 4)), idesc, issued || kq > 0 ? 1u : 0u);
       };
       Pos cur{0, 0};  // the ring row of the segment's row y0 - 1, then of each row
-      while (ok && rs.next(img, x0, y0, rows) && !*abort_v) {
+      while (ok && rs.next(img, x0, y0, rows) && __all_sync(0xffffffffu, !*abort_v)) {
         ok = full(cur);
         if (pair) {
           for (int o = 0; o <= rows && ok; o++) {  // rows (cur, nxt)
@@ -585,9 +651,8 @@ __global__ void __launch_bounds__(kWgThreads)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t yd = yd0 + (uint64_t)((uint32_t)cur.slot * (ybytes >> 4));
             const uint64_t xd = xd0 + (uint64_t)((uint32_t)cur.slot * (xbytes >> 4));
-#pragma unroll
-            for (int dx = 0; dx < 3; dx++)
-              mma(taddr + (uint32_t)(dx * 2 * cin), yd, xd + (uint64_t)dx);
+            mmas(std::integral_constant<int, 3>{}, yd,
+                 [&](int dx) { return xd + (uint64_t)dx; }, (uint32_t)(2 * cin));
             issued = true;
             tc_commit(&empty_bar[cur.slot]);  // no later step of this segment reads cur
             cur = nxt;
@@ -601,11 +666,11 @@ __global__ void __launch_bounds__(kWgThreads)
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t yd = yd0 + (uint64_t)((uint32_t)mid.slot * (ybytes >> 4));
-            const int xs[3] = {cur.slot, mid.slot, nxt.slot};
-#pragma unroll
-            for (int tap = 0; tap < 9; tap++)
-              mma(taddr + (uint32_t)(tap * cin), yd,
-                  xd0 + (uint64_t)((uint32_t)xs[tap / 3] * (xbytes >> 4)) + (uint64_t)(tap % 3));
+            const uint64_t xs[3] = {xd0 + (uint64_t)((uint32_t)cur.slot * (xbytes >> 4)),
+                                    xd0 + (uint64_t)((uint32_t)mid.slot * (xbytes >> 4)),
+                                    xd0 + (uint64_t)((uint32_t)nxt.slot * (xbytes >> 4))};
+            mmas(std::integral_constant<int, 9>{}, yd,
+                 [&](int tap) { return xs[tap / 3] + (uint64_t)(tap % 3); }, (uint32_t)cin);
             issued = true;
             tc_commit(&empty_bar[cur.slot]);
             cur = mid;
@@ -617,11 +682,12 @@ __global__ void __launch_bounds__(kWgThreads)
         if (ok) tc_commit(&empty_bar[cur.slot]);
         cur = next(cur);
       }
-      s_issued = (issued && ok) ? 1 : 0;
+      if (lane == 0) s_issued = (issued && ok) ? 1 : 0;
       __threadfence_block();
+      __syncwarp();
       if (issued)
         tc_commit(&last_bar);  // arrives once every MMA above has completed
-      else
+      else if (lane == 0)
         mbar_arrive(&last_bar);
     }
   } else {
@@ -714,12 +780,10 @@ __global__ void __launch_bounds__(kWgThreads)
           qphase ^= 1u;
         }
         if (q - done >= depth) {  // all but the newest depth - 1 rows must have landed
-          switch (depth) {
-            case 1: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-            case 2: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-            case 3: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-            default: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-          }
+          if (depth == 1)
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+          else
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
           finish();
         }
       }
@@ -1051,7 +1115,7 @@ int nl2d_emu_conv3x3(const void* x, const void* w, const float* bias, void* y, f
       batch < 1 || !x || !w || !err || (!y && !y32))
     return NL2D_ERR_ARGS;
   const size_t wbytes = ((9 * (size_t)cout * cin * 2) + 1023) & ~(size_t)1023;
-  const size_t smem = wbytes + kConvSlots * (size_t)(cin / 8) * kRowPix * 16;
+  const size_t smem = wbytes + kConvSlots * (size_t)(cin / 8) * kLboX;
   constexpr int kMaxSmem = 200 * 1024;
   static bool attr = false;
   if (!attr) {
@@ -1064,15 +1128,13 @@ int nl2d_emu_conv3x3(const void* x, const void* w, const float* bias, void* y, f
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long units =
-      (long long)batch * ((H + kStripRows - 1) / kStripRows) * (W / kTileM);
-  // Persistent CTAs: as many as are resident at once.  Counted from the
-  // kernel's registers (allocated per warp in units of 256) and shared
-  // memory (dynamic + static + the driver's reserve per block), as the
-  // hardware limits them; each CTA also holds kPipeTmemCols of the SM's 512
-  // TMEM columns.  (cudaOccupancyMaxActiveBlocksPerMultiprocessor answered 1
-  // here where 2 are resident, and the forward pass took 0.78 instead of
-  // 0.51 ms.)
+  const long long rows = (long long)batch * H * (W / kTileM);
+  // Persistent CTAs: as many as are resident at once, with two rows or more
+  // each.  Counted from the kernel's registers (allocated per warp in units of
+  // 256) and shared memory (dynamic + static + the driver's reserve per
+  // block), as the hardware limits them; each CTA also holds conv_tmem() of
+  // the SM's 512 TMEM columns.  (cudaOccupancyMaxActiveBlocksPerMultiprocessor
+  // answered 1 where 2 are resident.)
   static cudaFuncAttributes fa;
   static bool fa_ok = false;
   if (!fa_ok) {
@@ -1087,12 +1149,16 @@ int nl2d_emu_conv3x3(const void* x, const void* w, const float* bias, void* y, f
   const int by_regs = regs_sm / (warp_regs * (kPipeThreads / 32));
   const int by_smem = smem_sm / (int)(smem + fa.sharedSizeBytes + smem_rsv);
   int per_sm = by_regs < by_smem ? by_regs : by_smem;
-  per_sm = per_sm < 512 / kPipeTmemCols ? per_sm : 512 / kPipeTmemCols;
+  per_sm = per_sm < 512 / conv_tmem(cout) ? per_sm : 512 / conv_tmem(cout);
   per_sm = per_sm < 1 ? 1 : per_sm;
-  const int grid = (int)(units < (long long)per_sm * sms ? units : (long long)per_sm * sms);
+  const int grid =
+      (int)std::max<long long>(1, std::min<long long>(rows / 2, (long long)per_sm * sms));
+  // 32-byte stores where an output starts on a 32-byte boundary (every pixel
+  // then does: cout is a multiple of 16)
+  const int wide = ((uintptr_t)y % 32 == 0 ? 1 : 0) | ((uintptr_t)y32 % 32 == 0 ? 2 : 0);
   k_conv3x3_pipe<<<grid, kPipeThreads, smem, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, bias, (__nv_bfloat16*)y, y32, batch, H,
-      W, cin, cout, relu, err);
+      W, cin, cout, relu, wide, err);
   return cudaGetLastError() == cudaSuccess ? NL2D_OK : NL2D_ERR_CUDA;
 }
 
