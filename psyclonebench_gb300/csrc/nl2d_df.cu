@@ -31,7 +31,6 @@ using namespace dfk;
 namespace {
 
 using namespace dfm;
-constexpr int MR = 32;
 
 // One step.  Of the grid's blocks, nring take the exact cells' parts (all
 // cells' v, then u, then ssh; 128 each, one per thread; block b is one when floor((b+1) nring / grid) >
@@ -181,10 +180,8 @@ void launch_df_step(const Fields& f, const FusedState& fs, const Dims& d, const 
                     const double* tide_table, int tide_index, cudaStream_t st) {
   const int nx = d.xe - d.xs + 3, ny = d.ye - d.ys + 2;
   const int ncol = (nx + MW - 1) / MW;
-  // strips of MR rows, halved (down to 8) until the grid holds about two
-  // waves of warps
-  int mr = MR;
-  while (mr > 8 && (long long)ncol * ((ny + mr - 1) / mr) < 2 * 152 * 2 * WARPS) mr /= 2;
+  int mr = kMaxStrip;
+  while (mr > 8 && (long long)ncol * ((ny + mr - 1) / mr) < kStripWarps) mr /= 2;
   const int nrow = (ny + mr - 1) / mr, nwarps = ncol * nrow;
   const int nring = (kParts * ff.n_ring + 32 * WARPS - 1) / (32 * WARPS);
   k_df_step<<<(nwarps + WARPS - 1) / WARPS + nring, 32 * WARPS, 0, st>>>(

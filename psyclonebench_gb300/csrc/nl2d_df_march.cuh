@@ -13,6 +13,14 @@ using namespace dfk;
 
 constexpr int MW = kDfMarchCols;
 constexpr int WARPS = 4;
+// Strips start at kMaxStrip rows and are halved (down to 8) until the grid
+// holds kStripWarps warps, four waves of three blocks per SM.  The march
+// issues at the FP32 pipe's rate, so what costs is a last wave that is
+// partly empty, more than a strip's three extra rows: 1501 x 1103 in strips
+// of 8 rows 93.7 us, of 16 (two waves) 98.2, of 32 (one) 111; 2048^2 in 16
+// 182, in 32 188; 16 domains of 64 to 1024 in 8 114.6, in 32 133.7.
+constexpr int kMaxStrip = 32;
+constexpr long long kStripWarps = 4LL * 152 * 3 * WARPS;
 constexpr unsigned FULL = 0xffffffffu;
 
 __device__ __forceinline__ df shd(df x) {

@@ -168,8 +168,8 @@ __global__ void __launch_bounds__(32 * dfm::WARPS, 3)
   }
 }
 
-// The column marches' strip height until the autotuner chooses one (8, 16,
-// 32 or 64 rows).
+// The mixed march's strip height until the autotuner or the caller chooses one
+// (8, 16, 32 or 64 rows).  96 domains of 256^2: 16 rows 113 us, 32 110, 64 119.
 constexpr int kDefaultMarchRows = 32;
 
 // The tile shapes the ensemble's FP64 kernel is built for (the autotuner's
@@ -345,7 +345,7 @@ struct Ens {
   bool built = false;
   bool int_mul = false;  // every domain's constants have the integer form
   int shape = kDefaultShape;  // index into kShapes: the FP64 kernel's tile
-  int march_rows = kDefaultMarchRows;  // strip height of the column marches
+  int march_rows = 0;  // strip height of the column marches (0: none chosen)
   // mixed-precision form
   int precision = 0;
   float2* msn[2] = {};
@@ -377,6 +377,21 @@ struct Ens {
 };
 
 Ens g_ens;
+
+// The strip heights in use: the one chosen, or each form's own.  The
+// double-float march's is chosen as a single domain's is (kStripWarps).
+int mixed_rows() { return g_ens.march_rows ? g_ens.march_rows : kDefaultMarchRows; }
+int df_rows() {
+  if (g_ens.march_rows) return g_ens.march_rows;
+  for (int mr = dfm::kMaxStrip;; mr /= 2) {
+    long long warps = 0;
+    for (const DomainHost& D : g_ens.dom) {
+      const int nx = D.xe - D.xs + 3, ny = D.ye - D.ys + 2;
+      warps += (long long)((nx + kDfMarchCols - 1) / kDfMarchCols) * ((ny + mr - 1) / mr);
+    }
+    if (mr == 8 || warps >= dfm::kStripWarps) return mr;
+  }
+}
 
 bool ck(cudaError_t e) { return e == cudaSuccess; }
 
@@ -457,7 +472,7 @@ void ens_free() {
   e.ndom = 0;
   e.dom.clear();
   e.shape = kDefaultShape;
-  e.march_rows = kDefaultMarchRows;
+  e.march_rows = 0;
 }
 
 // Flather chains or reads outside the array exclude a domain (the one-launch
@@ -681,7 +696,7 @@ bool build_march(const std::vector<EnsMixDomain>& desc) {
   for (const EnsMixDomain& x : desc) {
     const int nx = x.d.xe - x.d.xs + 3, ny = x.d.ye - x.d.ys + 2;
     const int dom = (int)(&x - desc.data());
-    const int mr = e.march_rows;
+    const int mr = mixed_rows();
     for (int gy = 0; gy < (ny + mr - 1) / mr; gy++)
       for (int gx = 0; gx < (nx + mixk::MW - 1) / mixk::MW; gx++)
         units.push_back(make_int4(dom, x.d.xs - 1 + gx * mixk::MW, x.d.ys - 1 + gy * mr, 0));
@@ -784,6 +799,7 @@ bool build_df() {
   if (!ck(cudaMemsetAsync(e.dfreg, 0, n, st))) return false;
   std::vector<EnsDfDomain> desc(e.ndom);
   std::vector<int4> units;
+  const int mr = df_rows();
   std::vector<int2> ring;
   for (int k = 0; k < e.ndom; k++) {
     const DomainHost& D = e.dom[k];
@@ -803,7 +819,7 @@ bool build_df() {
     x.ff.rhv = pr[4] + o;
     x.ff.reg = e.dfreg + o;
     x.d = d;
-    const int nx = D.xe - D.xs + 3, ny = D.ye - D.ys + 2, mr = e.march_rows;
+    const int nx = D.xe - D.xs + 3, ny = D.ye - D.ys + 2;
     for (int gy = 0; gy < (ny + mr - 1) / mr; gy++)
       for (int gx = 0; gx < (nx + kDfMarchCols - 1) / kDfMarchCols; gx++)
         units.push_back(make_int4(k, D.xs - 1 + gx * kDfMarchCols, D.ys - 1 + gy * mr, 0));
@@ -1120,7 +1136,7 @@ int nl2d_ens_run(int istep0, int nsteps, int checksum_every, double* checksums_o
         launch_ens_mixed_general(e.d_mdesc, e.mglist, e.mgn, par,
                                  e.d_tides + (size_t)q * e.ndom, e.side);
         launch_ens_mixed_march(e.d_mdesc, e.d_units, e.nunits, mf, ms, &e.mk, e.d_mks,
-                               e.march_rows, e.stream);
+                               mixed_rows(), e.stream);
         cudaEventRecord(e.join, e.side);
         cudaStreamWaitEvent(e.stream, e.join, 0);
         par = 1 - par;
@@ -1129,17 +1145,18 @@ int nl2d_ens_run(int istep0, int nsteps, int checksum_every, double* checksums_o
                                                                             sums);
       } else if (e.precision == 2) {
         constexpr int B = 32 * dfm::WARPS;
+        const int strip = df_rows();
         const int nring = (kParts * e.ndfring + B - 1) / B;
         const int nmarch = (e.ndfunits + dfm::WARPS - 1) / dfm::WARPS;
         const double* tq = e.d_tides + (size_t)q * e.ndom;
         if (e.d_dks)
           k_ensemble_df_step<true><<<nring + nmarch, B, 0, e.stream>>>(
               e.d_dfdesc, e.d_dfunits, e.ndfunits, e.d_desc, e.dfring, e.ndfring, nring, par,
-              e.dk, e.d_dks, e.march_rows, tq);
+              e.dk, e.d_dks, strip, tq);
         else
           k_ensemble_df_step<false><<<nring + nmarch, B, 0, e.stream>>>(
               e.d_dfdesc, e.d_dfunits, e.ndfunits, e.d_desc, e.dfring, e.ndfring, nring, par,
-              e.dk, nullptr, e.march_rows, tq);
+              e.dk, nullptr, strip, tq);
         par = 1 - par;
         if (want_sums)
           k_ensemble_checksums<<<dim3(e.ndom, 3), 256, 0, e.stream>>>(e.d_desc, par, e.ndom,

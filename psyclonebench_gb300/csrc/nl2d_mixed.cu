@@ -28,7 +28,7 @@ namespace nl2d {
 using namespace mixk;
 namespace {
 
-// The regular cells: one warp per MW columns x MR rows of the copy region.
+// The regular cells: one warp per MW columns x mr rows of the copy region.
 // Both march kernels are held to 96 registers, 5 blocks of 4 warps per SM.
 __global__ void __launch_bounds__(32 * MARCH_WARPS, 5)
     k_mixed_march(MixedFields mf, MixedState ms, Dims d, MarchConst k, int ncol, int nwarps,
@@ -175,17 +175,36 @@ __global__ void k_from_mixed(const float2* __restrict__ sn2, const float* __rest
 
 }  // namespace
 
+namespace {
+// The march's strip height: one wave of at most four blocks per SM where the
+// strips are then no taller than 128 rows (and no shorter than 8), else MR.
+// The march lives on the L1: neighbouring warps share the 128-byte lines at
+// their columns' edges and the rows in flight are held there, and a fifth
+// block per SM costs more in lines evicted than its loads in flight give
+// (2048^2: 35 strips of 59 rows, four blocks per SM, 46.6 us; 47 rows, five
+// per SM, 62; 16 rows, three waves, 59.5; the same four blocks with 3/4 of
+// the L1 taken as shared memory 63).  One wave also leaves no strip's first
+// rows to load behind another strip.  us at the heights of this rule and
+// of the one before it (halving from 64 until two waves of five blocks):
+// 2048^2 45.9 / 59.5, 3001 x 2003 63 / 75, 4096 x 2048 89 / 96, 1024^2 18.1
+// / 18.2.  Above 128 rows a wave's blocks drift apart (4096^2:
+// 64 rows 172 us, 257 rows 226).
+int strip_rows(int ncol, int ny) {
+  const int fit = 4 * 152 * MARCH_WARPS / ncol;  // strips that one such wave holds
+  if (fit < 1) return MR;
+  const int mr = (ny + fit - 1) / fit;
+  return mr > 2 * MR ? MR : (mr < 8 ? 8 : mr);
+}
+}  // namespace
+
 void launch_mixed_step(const MixedFields& mf, const MixedState& ms, const Fields& f,
                        const Dims& d, const Scalars& s, const UniformMetrics& um, double tide,
                        const double* tide_table, int tide_index, cudaStream_t st,
                        cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
   const MixConst k = make_mix_const(s, um);
   const int nx = d.xe - d.xs + 3, ny = d.ye - d.ys + 2;
-  // Strips of MR rows, halved (down to 8) until the grid holds about two
-  // waves of warps: a smaller domain trades halo rows for parallelism.
   const int ncol = (nx + MW - 1) / MW;
-  int mr = MR;
-  while (mr > 8 && (long long)ncol * ((ny + mr - 1) / mr) < 2 * 152 * 5 * MARCH_WARPS) mr /= 2;
+  const int mr = strip_rows(ncol, ny);
   const int nrow = (ny + mr - 1) / mr, nwarps = ncol * nrow;
   // The general cells (a list of a few thousand, each a long chain of
   // global loads) and the march read the same buffers and write disjoint

@@ -2,11 +2,11 @@
 // domain's and the ensemble's kernels).
 //
 // One warp owns MW = 30 consecutive columns (one lane per column, plus one
-// halo lane on each side) and marches down a strip of MR rows.  Each lane
+// halo lane on each side) and marches down a strip of mr rows.  Each lane
 // keeps rows j-1, j, j+1 of its column in registers, takes its x neighbours
 // by warp shuffles, and forms every term that two neighbouring updates
 // share once per position.  No shared memory, no block barrier; the
-// redundancy is 32/30 in x and (MR+3)/MR in loads along y.  (A shared-memory
+// redundancy is 32/30 in x and (mr+3)/mr in loads along y.  (A shared-memory
 // tile form staging a 2-cell halo of every field took 1.7x the cells in
 // loads, index arithmetic and terms, ~930 instructions per cell.)
 //
@@ -28,7 +28,7 @@ namespace mixk {
 namespace {
 
 constexpr int MW = 30;  // output columns per warp
-constexpr int MR = 64;  // output rows per warp (at most; smaller domains take shorter strips)
+constexpr int MR = 64;  // output rows per warp where a domain takes several waves
 constexpr int MARCH_WARPS = 4;
 constexpr int PF = 2;  // rows between an L2 prefetch and the row's loads
 constexpr unsigned FULL = 0xffffffffu;
