@@ -236,6 +236,21 @@ __global__ void k_selftest_exact(long long n, unsigned long long seed, IntDiviso
         if (bits(xr) != bits(div_depth(cand[c], d, v.rc))) nd++;
       }
     }
+    // Quotients at and beside the midpoints of the subnormals: (2c + 1)
+    // 2^-1075 d for c of every length, and its neighbours.
+    {
+      const unsigned long long y = mix64(z + 4);
+      const unsigned long long c = (y >> 12) >> (y & 63);
+      const long long nudge = (long long)((y >> 6) & 7) - 3;
+      const double xm = ((double)(2 * c + 1) * 0x1p-600) * d * 0x1p-475;
+      const double cand[3] = {xm, -xm, from_bits(bits(xm) + nudge)};
+      for (int i = 0; i < 3; i++) {
+        const double xr = cand[i] / d;
+        const bool nan = xr != xr;
+        if (!nan && bits(xr) != bits(div_const(cand[i], v))) nd++;
+        if (!nan && bits(xr) != bits(div_depth(cand[i], d, v.rc))) nd++;
+      }
+    }
     const double h_ref = 0.5 * x, h = half(x);
     if (bits(h_ref) != bits(h) && !(h_ref != h_ref && h != h)) nh++;
     const double p = sample(mix64(z + 1)), w = sample(mix64(z + 2));
