@@ -536,14 +536,25 @@ bool build_schedule(int TXv, int TYv) {
     const DomainHost& D = e.dom[k];
     const Dims d{D.xs, D.xe, D.ys, D.ye, D.W, D.H};
     const int nr = kParts * ring_count(d, D.ys - 1, D.ye + 1);
-    for (int g = 0; g < nr; g += kRingUnit)
-      tiles.push_back(
-          {k, 0, 0, g, (1.0 + e.boundary_weight) * std::min(kRingUnit, nr - g) / kParts});
+    const int units = (nr + kRingUnit - 1) / kRingUnit;
     const int nx = D.xe - D.xs - 1, ny = D.ye - D.ys - 1;
-    if (nx < 1 || ny < 1) continue;
-    const int ntx = (nx + TXv - 1) / TXv, nty = (ny + TYv - 1) / TYv;
+    const bool inner = nx >= 1 && ny >= 1;
+    const int ntx = inner ? (nx + TXv - 1) / TXv : 0, nty = inner ? (ny + TYv - 1) / TYv : 0;
+    // Contiguous chunks take the ring units spread among the tiles: together
+    // they had fallen to few CTAs where their weight was off (16 domains in
+    // 32 x 32 tiles, weight 16: 0.90 ms per step against 0.72 so).
+    const long long every = e.policy == 0 && inner ? (long long)ntx * nty : 0;
+    int u = 0;
+    auto ring_until = [&](long long tile) {
+      for (; u < units && (every == 0 || u * every / units <= tile); u++)
+        tiles.push_back({k, 0, 0, u * kRingUnit,
+                         (1.0 + e.boundary_weight) * std::min(kRingUnit, nr - u * kRingUnit) /
+                             kParts});
+    };
+    ring_until(0);
     for (int by = 0; by < nty; by++)
       for (int bx = 0; bx < ntx; bx++) {
+        ring_until((long long)by * ntx + bx);
         const int cx = std::min(TXv, nx - bx * TXv), cy = std::min(TYv, ny - by * TYv);
         tiles.push_back({k, D.xs + 1 + bx * TXv, D.ys + 1 + by * TYv, -1, (double)(cx * cy)});
       }
