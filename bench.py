@@ -684,7 +684,7 @@ def run_tra_adv(lib, jpi=512, jpj=512, jpk=75, iters=500, cpu_iters=10):
         "roofline": {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s",
                      "frac": ach / hbm, "peak_kind": peak_kind,
                      "alg_bytes_per_point": 72,
-                     "kernels": ["k_tra_horizontal_tiled", "k_tra_vertical"]},
+                     "kernels": ["k_tra_horizontal", "k_tra_vertical"]},
         "cpu_baseline": {"value": points * cpu_iters / cpu_s / 1e6,
                          "unit": "Mpoint-iterations/s",
                          "cores": int(os.environ["OMP_NUM_THREADS"]), "kind": "port",
