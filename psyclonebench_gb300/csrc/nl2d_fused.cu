@@ -37,9 +37,11 @@ namespace {
 // per thread (2048^2: 32 x 16 and two CTAs 597 us, 16 x 16 and three 540,
 // 32 x 12 and two CTAs of 384 threads 565, 32 x 8 and two 620, three 537).
 using T = Tile<32, 8, 256, 3>;
-// Domains too small to give every SM a few of those take 16 x 8 cells and 128
+// Domains too small to give every SM two of those take 16 x 8 cells and 128
 // threads: twice the tiles, the same bits (the arithmetic does not depend on
-// the shape; 256^2: 19.4 us with 16 x 16, 16.3 with 16 x 8).
+// the shape).  32 x 8 and 16 x 8, us per step: 256^2 (256 tiles of 32 x 8) 17.7 /
+// 15.0, 384 x 256 (384) 19.1 / 21.5, 512 x 256 (512) 24.9 / 25.1, 1024 x 512
+// (2048) 75.4 / 87.3.
 using SmallTile = Tile<16, 8, 128, 4>;
 
 // One step of copy-region rows [ja, jb).  The first nring blocks take the
@@ -77,7 +79,7 @@ int interior_y(const Dims& d) { return d.ye - d.ys - 1; }
 
 bool small_tiles(const Dims& d) {
   return (long long)tiles_over(interior_x(d), T::TX) * tiles_over(interior_y(d), T::TY) <
-         4LL * 152;
+         2LL * 152;
 }
 int tile_height(const Dims& d) { return small_tiles(d) ? SmallTile::TY : T::TY; }
 
