@@ -1135,6 +1135,7 @@ int nl2d_ens_run(int istep0, int nsteps, int checksum_every, double* checksums_o
     if (!ck(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal)))
       return NL2D_ERR_CUDA;
     int par = e.parity;
+    const int strip = e.precision == 2 ? df_rows() : mixed_rows();
     for (int q = 0; q < nsteps; q++) {
       double* sums = e.d_sums + (size_t)((q + 1) / std::max(checksum_every, 1) - 1) * e.ndom * 3;
       const bool want_sums = checksum_every > 0 && (q + 1) % checksum_every == 0;
@@ -1150,7 +1151,7 @@ int nl2d_ens_run(int istep0, int nsteps, int checksum_every, double* checksums_o
         launch_ens_mixed_general(e.d_mdesc, e.mglist, e.mgn, par,
                                  e.d_tides + (size_t)q * e.ndom, e.side);
         launch_ens_mixed_march(e.d_mdesc, e.d_units, e.nunits, mf, ms, &e.mk, e.d_mks,
-                               mixed_rows(), e.stream);
+                               strip, e.stream);
         cudaEventRecord(e.join, e.side);
         cudaStreamWaitEvent(e.stream, e.join, 0);
         par = 1 - par;
@@ -1159,7 +1160,6 @@ int nl2d_ens_run(int istep0, int nsteps, int checksum_every, double* checksums_o
                                                                             sums);
       } else if (e.precision == 2) {
         constexpr int B = 32 * dfm::WARPS;
-        const int strip = df_rows();
         const int nring = (kParts * e.ndfring + B - 1) / B;
         const int nmarch = (e.ndfunits + dfm::WARPS - 1) / dfm::WARPS;
         const double* tq = e.d_tides + (size_t)q * e.ndom;
