@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cstdint>
+#include <mutex>
 #include <type_traits>
 
 #include "../../include/nl2d_gpu.h"
@@ -875,17 +876,34 @@ __global__ void __launch_bounds__(kSumWays * kSumElems)
   }
 }
 
-// Scratch for the per-CTA partial gradients (grown on demand, kept).
-float* g_parts = nullptr;
-size_t g_parts_cap = 0;
-bool ensure_parts(size_t n) {
-  if (n <= g_parts_cap) return true;
-  cudaFree(g_parts);
-  g_parts = nullptr;
-  g_parts_cap = 0;
-  if (cudaMalloc(&g_parts, n * sizeof(float)) != cudaSuccess) return false;
-  g_parts_cap = n;
-  return true;
+// Scratch for the per-CTA partial gradients: allocated and freed in the
+// caller's stream's order from a pool of the device, so that calls on other
+// streams and threads get memory of their own.  The pool keeps kPartsKept
+// bytes (the widest gradient's partials are 34 MB) from one call to the next
+// and gives back what is beyond them when a stream is synchronised.  Null if
+// there is none to be had.
+constexpr unsigned long long kPartsKept = 64ull << 20;
+constexpr int kMaxDevices = 64;
+cudaMemPool_t parts_pool(int dev) {
+  static cudaMemPool_t pools[kMaxDevices] = {};
+  static std::mutex lock;
+  if (dev < 0 || dev >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> hold(lock);
+  if (!pools[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
+    uint64_t kept = kPartsKept;
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept) != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return nullptr;
+    }
+    pools[dev] = pool;
+  }
+  return pools[dev];
 }
 
 // dx = (y > 0) ? g : 0 for a ReLU output y (BF16), g FP32 -> BF16.
@@ -1196,14 +1214,20 @@ int nl2d_emu_conv_wgrad(const void* x, const void* dy, float* dw, float* db, int
   const long long rows = (long long)batch * H * (W / kTileM);
   const int grid = (int)std::max<long long>(1, std::min<long long>(rows / 4, sms));
   const long long nel = 9LL * cout * cin;
-  if (!ensure_parts((size_t)(grid * (nel + cout)))) return NL2D_ERR_CUDA;
   const cudaStream_t st = (cudaStream_t)stream;
+  const cudaMemPool_t pool = parts_pool(dev);
+  float* parts = nullptr;
+  if (!pool || cudaMallocFromPoolAsync(&parts, grid * (nel + cout) * sizeof(float), pool, st) !=
+                   cudaSuccess)
+    return NL2D_ERR_CUDA;
   k_conv_wgrad_pipe<<<grid, kWgThreads, smem, st>>>((const __nv_bfloat16*)x,
-                                                      (const __nv_bfloat16*)dy, g_parts, batch,
-                                                      H, W, cin, cout, slots, err);
+                                                      (const __nv_bfloat16*)dy, parts, batch, H,
+                                                      W, cin, cout, slots, err);
   k_sum_parts<<<(int)((nel + cout + kSumElems - 1) / kSumElems), kSumWays * kSumElems, 0, st>>>(
-      g_parts, grid, nel, cout, dw, db);
-  return cudaGetLastError() == cudaSuccess ? NL2D_OK : NL2D_ERR_CUDA;
+      parts, grid, nel, cout, dw, db);
+  const cudaError_t launched = cudaGetLastError();
+  return cudaFreeAsync(parts, st) == cudaSuccess && launched == cudaSuccess ? NL2D_OK
+                                                                             : NL2D_ERR_CUDA;
 }
 
 int nl2d_emu_relu_bwd(const float* g, const void* y, void* out, long long n, void* stream) {
