@@ -377,6 +377,16 @@ int nl2d_selftest_df(const double *x, long long n, float *hi, float *lo,
  * 0 that the flag was not set).  The context stays usable. */
 int nl2d_selftest_wait(long long max_cycles, int *status);
 
+/* Test hook (no reference counterpart): nl2d_emu_conv3x3 without bias and
+ * ReLU into FP32 (wgrad = 0: b the weights, out y32, db unused) or
+ * nl2d_emu_conv_wgrad (b the output's gradient, out dw), on the default
+ * stream, with the roles' waits for one another limited to max_cycles (0 ..
+ * 2^31 clocks).  A launch in which a wait runs out sets *err and ends; what it
+ * wrote is not valid then. */
+int nl2d_selftest_emu_wait(int wgrad, const void *x, const void *b, float *out,
+                           float *db, int batch, int H, int W, int cin, int cout,
+                           long long max_cycles, int *err);
+
 /* Checkpoint / resume (no reference counterpart; the reference keeps no
  * restart files).  nl2d_checkpoint_write stores the registered problem's 13
  * fields exactly as c_read_from_device returns them (FP64, row-major

@@ -85,6 +85,8 @@ EXPORTS = {
     "nl2d_ens_export_interior": (ctypes.c_int, [_VP]),
     "nl2d_ens_uses_march": (ctypes.c_int, []),
     "nl2d_selftest_wait": (ctypes.c_int, [ctypes.c_longlong, _IP]),
+    "nl2d_selftest_emu_wait": (ctypes.c_int, [ctypes.c_int, _VP, _VP, _VP, _VP] +
+                               [ctypes.c_int] * 5 + [ctypes.c_longlong, _VP]),
     "nl2d_selftest_df": (ctypes.c_int, [_DP, ctypes.c_longlong, _VP, _VP, _DP, _DP]),
     "nl2d_checkpoint_write": (ctypes.c_int, [ctypes.c_char_p, ctypes.c_int]),
     "nl2d_checkpoint_read": (ctypes.c_int, [ctypes.c_char_p, _IP]),

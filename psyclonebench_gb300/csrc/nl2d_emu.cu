@@ -92,8 +92,8 @@ constexpr int kRowPix = 136;
 // completion -> stagers), done[block] (MMA completion -> epilogue),
 // drained[block] (epilogue -> MMA).  Every wait is bounded (kMaxWaitCycles);
 // one that runs out sets the error flag and a shared abort flag that ends
-// every role's loop, and the MMA thread waits for its last commit before the
-// tensor memory is freed.
+// every role's loop, a whole warp at a time (warp_wait), and the MMA thread
+// waits for its last commit before the tensor memory is freed.
 constexpr int kConvSlots = 5;  // the input ring
 constexpr int kConvDepth = 2;  // rows in flight (four: 68.2 us, two: 66.3)
 constexpr int kConvMaxBlocks = 8;
@@ -164,19 +164,30 @@ __device__ __forceinline__ void store_32b(void* p, const uint32_t (&v)[8], int w
   }
 }
 // Waits for the phase with the given parity to complete; false if the wait
-// ran out after max_cycles (flag and error set) or another role aborted.
+// ran out after max_cycles (flag and error set) or another role aborted.  The
+// lanes of a warp may be answered differently: see warp_wait.  POLL: without
+// the hardware's own wait in each try, so that short limits hold (tests).
+template <bool POLL>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
                                           volatile int* abort_flag, int* err,
-                                          long long max_cycles = kMaxWaitCycles) {
+                                          long long max_cycles) {
   const long long t0 = clock64();
   for (;;) {
     uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
+    if constexpr (POLL)
+      asm volatile(
+          "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+          "selp.u32 %0, 1, 0, p;\n}"
+          : "=r"(ok)
+          : "r"(smem_u32(bar)), "r"(parity)
+          : "memory");
+    else
+      asm volatile(
+          "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+          "selp.u32 %0, 1, 0, p;\n}"
+          : "=r"(ok)
+          : "r"(smem_u32(bar)), "r"(parity)
+          : "memory");
     if (ok) return true;
     if (*abort_flag) return false;
     if (clock64() - t0 > max_cycles) {
@@ -185,6 +196,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
       return false;
     }
   }
+}
+
+// The waits and tests of the abort flag by which the roles' loops go on, for
+// a whole converged warp: one answer for all its lanes.  (The loops' bodies
+// hold warp-wide operations, __syncwarp and tcgen05.ld among them; a lane
+// that left a loop by itself would leave the others waiting there for ever.)
+template <bool POLL>
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                          int* err, long long max_cycles) {
+  return __all_sync(0xffffffffu, mbar_wait<POLL>(bar, parity, abort_flag, err, max_cycles));
+}
+__device__ __forceinline__ bool warp_goes_on(volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, !*abort_flag);
 }
 
 // The failure path of the bounded waits, exercised on purpose: one thread
@@ -199,7 +223,7 @@ __global__ void k_selftest_wait(long long max_cycles, int* err) {
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   __syncthreads();
-  if (threadIdx.x == 0 && mbar_wait(&bar, 0, &abort_flag, err, max_cycles)) atomicExch(err, 2);
+  if (threadIdx.x == 0 && mbar_wait<false>(&bar, 0, &abort_flag, err, max_cycles)) atomicExch(err, 2);
 }
 
 // A CTA's share of the rows: rows [g, end) of the list of all columns' rows,
@@ -224,11 +248,13 @@ struct RowSegments {
   }
 };
 
+// (max_cycles: the limit of the roles' waits for each other in the POLL form.)
+template <bool POLL>
 __global__ void __launch_bounds__(kPipeThreads)
     k_conv3x3_pipe(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const float* __restrict__ bias, __nv_bfloat16* __restrict__ y,
                    float* __restrict__ y32, int batch, int H, int W, int cin, int cout,
-                   int relu, int wide_store, int* __restrict__ err) {
+                   int relu, int wide_store, long long max_cycles, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t full_bar[kConvSlots], empty_bar[kConvSlots];
   __shared__ __align__(8) uint64_t done_bar[kConvMaxBlocks], drained_bar[kConvMaxBlocks], last_bar;
@@ -244,6 +270,7 @@ __global__ void __launch_bounds__(kPipeThreads)
   unsigned char* b_s = smem;
   unsigned char* ring = smem + ((3 * b_bytes + 1023) & ~1023u);
   volatile int* abort_v = &abort_flag;
+  const long long max_wait = POLL ? max_cycles : kMaxWaitCycles;
 
   if (warp == 0) {
     if (conv_tmem(cout) == 128)
@@ -326,12 +353,12 @@ __global__ void __launch_bounds__(kPipeThreads)
       mark = next(mark, kConvSlots);
       ahead--;
     };
-    while (ok && rs.next(img, x0, y0, rows) && !*abort_v) {
+    while (ok && rs.next(img, x0, y0, rows) && warp_goes_on(abort_v)) {
       const unsigned in = mine & ~(x0 == 0 ? left : 0u) & ~(x0 + kTileM >= W ? right : 0u);
       const __nv_bfloat16* seg = x + (((size_t)img * H + y0) * W + x0) * cin;
       for (int a = 0; a < rows + 2; a++) {
         const int yy = y0 - 1 + a;
-        if (!fresh) ok = mbar_wait(&empty_bar[put.at], put.par, abort_v, err);
+        if (!fresh) ok = warp_wait<POLL>(&empty_bar[put.at], put.par, abort_v, err, max_wait);
         if (!ok) break;
         const unsigned take = yy >= 0 && yy < H ? in : 0u;
         const __nv_bfloat16* src = seg + (long long)(a - 1) * W * cin;
@@ -354,7 +381,7 @@ __global__ void __launch_bounds__(kPipeThreads)
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    while (ahead > 0 && !*abort_v) finish();
+    while (ahead > 0 && warp_goes_on(abort_v)) finish();
   } else if (warp == 4) {
     // ---- MMA issuer: the whole warp walks, one lane issues ----
     {
@@ -373,15 +400,15 @@ __global__ void __launch_bounds__(kPipeThreads)
       Pos fresh{0, 1};         // the new output row's block
       Pos oldest{0, 0};        // the block of the oldest output row being summed
       bool first_turn = true, issued = false, ok = true;
-      while (ok && rs.next(img, x0, y0, rows) && __all_sync(0xffffffffu, !*abort_v)) {
+      while (ok && rs.next(img, x0, y0, rows) && warp_goes_on(abort_v)) {
         for (int a = 0; a < rows + 2 && ok; a++) {
           // output rows (of the segment) max(0, a-2) .. min(rows-1, a)
           const int lo = a > 2 ? a - 2 : 0, hi = a < rows ? a : rows - 1;
           const int n = hi - lo + 1, from = lo - (a - 2);
           const bool opens = a < rows;
-          ok = mbar_wait(&full_bar[in.at], in.par, abort_v, err);
+          ok = mbar_wait<POLL>(&full_bar[in.at], in.par, abort_v, err, max_wait);
           if (ok && opens && !first_turn)
-            ok = mbar_wait(&drained_bar[fresh.at], fresh.par, abort_v, err);
+            ok = mbar_wait<POLL>(&drained_bar[fresh.at], fresh.par, abort_v, err, max_wait);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -416,19 +443,17 @@ __global__ void __launch_bounds__(kPipeThreads)
       if (issued) {  // nothing may be in flight when the tensor memory is freed
         tc_commit(&last_bar);
         volatile int never = 0;
-        if (!mbar_wait(&last_bar, 0, &never, err)) atomicExch(err, 1);
+        if (!mbar_wait<false>(&last_bar, 0, &never, err, kMaxWaitCycles)) atomicExch(err, 1);
       }
     }
   } else {
     // ---- epilogue: warp w owns accumulator lanes (pixels) 32w .. 32w+31 ----
     Pos blk{0, 0};
     bool ok = true;
-    while (ok && rs.next(img, x0, y0, rows) && !*abort_v) {
+    while (ok && rs.next(img, x0, y0, rows) && warp_goes_on(abort_v)) {
       size_t pix = ((size_t)img * H + y0) * W + x0 + warp * 32 + lane;
       for (int o = 0; o < rows; o++, pix += W) {
-        // warp-uniform outcome: tcgen05.ld below needs the whole warp
-        ok = mbar_wait(&done_bar[blk.at], blk.par, abort_v, err);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = warp_wait<POLL>(&done_bar[blk.at], blk.par, abort_v, err, max_wait);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t ta =
@@ -564,10 +589,11 @@ __host__ __device__ constexpr int wg_depth(int cout, int slots) {
   return d < kWgDepth ? d : kWgDepth;
 }
 
+template <bool POLL>
 __global__ void __launch_bounds__(kWgThreads)
     k_conv_wgrad_pipe(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                       float* __restrict__ part, int batch, int H, int W, int cin, int cout,
-                      int slots, int* __restrict__ err) {
+                      int slots, long long max_cycles, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t full_bar[kWgMaxSlots], empty_bar[kWgMaxSlots], last_bar;
   __shared__ uint32_t taddr_slot;
@@ -581,6 +607,7 @@ __global__ void __launch_bounds__(kWgThreads)
   unsigned char* xring = smem + (size_t)(slots + (pair ? 1 : 0)) * ybytes;
   const int depth = wg_depth(cout, slots);
   volatile int* abort_v = &abort_flag;
+  const long long max_wait = POLL ? max_cycles : kMaxWaitCycles;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -625,7 +652,7 @@ __global__ void __launch_bounds__(kWgThreads)
         return Pos{wrap ? 0 : p.slot + 1, p.par ^ (wrap ? 1u : 0u)};
       };
       auto full = [&](Pos p) {
-        return (bool)__all_sync(0xffffffffu, mbar_wait(&full_bar[p.slot], p.par, abort_v, err));
+        return warp_wait<POLL>(&full_bar[p.slot], p.par, abort_v, err, max_wait);
       };
       const uint64_t yd0 = smem_desc(smem_u32(yring), 128, kWgLboY);
       const uint64_t xd0 = smem_desc(smem_u32(xring), 128, kWgLboX);
@@ -642,7 +669,7 @@ __global__ void __launch_bounds__(kWgThreads)
                    xdesc(b) + (uint64_t)(kq * (256 >> 4)), idesc, issued || kq > 0 ? 1u : 0u);
       };
       Pos cur{0, 0};  // the ring row of the segment's row y0 - 1, then of each row
-      while (ok && rs.next(img, x0, y0, rows) && __all_sync(0xffffffffu, !*abort_v)) {
+      while (ok && rs.next(img, x0, y0, rows) && warp_goes_on(abort_v)) {
         ok = full(cur);
         if (pair) {
           for (int o = 0; o <= rows && ok; o++) {  // rows (cur, nxt)
@@ -738,8 +765,8 @@ __global__ void __launch_bounds__(kWgThreads)
     };
     RowSegments rs(batch, H, segs);
     int img, x0, y0, rows;
-    bool ok = true;
-    while (ok && rs.next(img, x0, y0, rows) && !*abort_v) {
+    bool ok = true;  // this lane's waits; see below
+    while (rs.next(img, x0, y0, rows)) {
       unsigned xin = 0;  // bit k: chunk k lies inside the image's columns
 #pragma unroll
       for (int k = 0; k < kX; k++)
@@ -749,13 +776,16 @@ __global__ void __launch_bounds__(kWgThreads)
       const __nv_bfloat16* xrow_p = x + row0 * cin;
       for (int a = 0; a < rows + 2; a++) {
         const long long dr = a - 1;
-        if (q >= slots) ok = mbar_wait(&empty_bar[qslot], qphase, abort_v, err);
-        if (!ok) break;
+        // A lane whose wait ran out goes through its remaining rows without
+        // waits or copies, so that its warp stays whole for finish() without a
+        // vote per row (which cost 4 us of 100); the results are not valid then.
+        if (q >= slots && ok)
+          ok = mbar_wait<POLL>(&empty_bar[qslot], qphase, abort_v, err, max_wait);
         const bool yrow = a >= 1 && a <= rows, xrow = y0 + dr >= 0 && y0 + dr < H;
         const __nv_bfloat16* ys = yrow ? yrow_p + dr * W * cout : dy;
         const __nv_bfloat16* xs = xrow_p + dr * W * cin;
         const int ystep = yrow ? yL * cout : 0;
-        for (int copy = qslot; copy <= slots; copy += slots) {  // slot 0: twice, paired
+        for (int copy = qslot; ok && copy <= slots; copy += slots) {  // slot 0: twice, paired
           uint32_t yd = smem_u32(yring + copy * ybytes) + ydst;
           const __nv_bfloat16* yp = ys;
           for (int k = 0; k < yn; k++, yd += yL * 16, yp += ystep)
@@ -790,11 +820,11 @@ __global__ void __launch_bounds__(kWgThreads)
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    while (done < q && !*abort_v) finish();
+    while (done < q) finish();
     // the accumulators: rows 32w .. 32w+31 of M
     volatile int never = 0;
-    const bool mmas = mbar_wait(&last_bar, 0, &never, err);
-    if (warp < 4 && __all_sync(0xffffffffu, mmas) && s_issued && !*abort_v) {
+    const bool mmas = warp_wait<false>(&last_bar, 0, &never, err, kMaxWaitCycles);
+    if (warp < 4 && mmas && s_issued && warp_goes_on(abort_v)) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int m = warp * 32 + lane;
       const bool second = pair && m >= cout;  // dY row r+1: the tap dy = 0
@@ -1100,6 +1130,106 @@ __global__ void k_advance(float* __restrict__ state, const float* __restrict__ i
   }
 }
 
+// The launches of the two kernels (POLL with its limit: the test hook's form).
+template <bool POLL>
+int conv3x3(const void* x, const void* w, const float* bias, void* y, float* y32, int batch, int H,
+            int W, int cin, int cout, int relu, long long max_cycles, int* err, void* stream) {
+  if (cin % 16 || cout % 16 || cout > 64 || cin < 16 || cin > 64 || W % kTileM || H < 1 ||
+      batch < 1 || !x || !w || !err || (!y && !y32))
+    return NL2D_ERR_ARGS;
+  const size_t wbytes = ((9 * (size_t)cout * cin * 2) + 1023) & ~(size_t)1023;
+  const size_t smem = wbytes + kConvSlots * (size_t)(cin / 8) * kLboX;
+  constexpr int kMaxSmem = 200 * 1024;
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(k_conv3x3_pipe<POLL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kMaxSmem) != cudaSuccess)
+      return NL2D_ERR_CUDA;
+    attr = true;
+  }
+  if (smem > kMaxSmem) return NL2D_ERR_ARGS;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long rows = (long long)batch * H * (W / kTileM);
+  // Persistent CTAs: as many as are resident at once, with two rows or more
+  // each.  Counted from the kernel's registers (allocated per warp in units of
+  // 256) and shared memory (dynamic + static + the driver's reserve per
+  // block), as the hardware limits them; each CTA also holds conv_tmem() of
+  // the SM's 512 TMEM columns.  (cudaOccupancyMaxActiveBlocksPerMultiprocessor
+  // answered 1 where 2 are resident.)
+  static cudaFuncAttributes fa;
+  static bool fa_ok = false;
+  if (!fa_ok) {
+    if (cudaFuncGetAttributes(&fa, k_conv3x3_pipe<POLL>) != cudaSuccess) return NL2D_ERR_CUDA;
+    fa_ok = true;
+  }
+  int regs_sm = 0, smem_sm = 0, smem_rsv = 0;
+  cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
+  cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  cudaDeviceGetAttribute(&smem_rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+  const int warp_regs = (fa.numRegs * 32 + 255) / 256 * 256;
+  const int by_regs = regs_sm / (warp_regs * (kPipeThreads / 32));
+  const int by_smem = smem_sm / (int)(smem + fa.sharedSizeBytes + smem_rsv);
+  int per_sm = by_regs < by_smem ? by_regs : by_smem;
+  per_sm = per_sm < 512 / conv_tmem(cout) ? per_sm : 512 / conv_tmem(cout);
+  per_sm = per_sm < 1 ? 1 : per_sm;
+  const int grid =
+      (int)std::max<long long>(1, std::min<long long>(rows / 2, (long long)per_sm * sms));
+  // 32-byte stores where an output starts on a 32-byte boundary (every pixel
+  // then does: cout is a multiple of 16)
+  const int wide = ((uintptr_t)y % 32 == 0 ? 1 : 0) | ((uintptr_t)y32 % 32 == 0 ? 2 : 0);
+  k_conv3x3_pipe<POLL><<<grid, kPipeThreads, smem, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, bias, (__nv_bfloat16*)y, y32, batch, H,
+      W, cin, cout, relu, wide, max_cycles, err);
+  return cudaGetLastError() == cudaSuccess ? NL2D_OK : NL2D_ERR_CUDA;
+}
+
+template <bool POLL>
+int conv_wgrad(const void* x, const void* dy, float* dw, float* db, int batch, int H, int W,
+               int cin, int cout, long long max_cycles, int* err, void* stream) {
+  if (!x || !dy || !dw || !db || !err || cin % 16 || cin < 16 || 9 * cin > kWgTmemCols ||
+      cout % 8 || cout < 8 || cout > 128 || W % kTileM || H < 1 || batch < 1)
+    return NL2D_ERR_ARGS;
+  // As many ring slots as fit (at least one row in flight: wg_depth).
+  // The kernel holds all 512 TMEM columns, so it must be alone on its SM:
+  // asking for more than half an SM's shared memory guarantees that.
+  int slots = kWgMaxSlots;
+  while (slots > 3 && wg_smem(cin, cout, slots) > kWgMaxSmem) slots--;
+  const size_t need = wg_smem(cin, cout, slots);
+  const size_t smem = need > 120 * 1024 ? need : 120 * 1024;
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(k_conv_wgrad_pipe<POLL>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kWgMaxSmem) != cudaSuccess)
+      return NL2D_ERR_CUDA;
+    attr = true;
+  }
+  if (smem > kWgMaxSmem) return NL2D_ERR_ARGS;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // one CTA per SM (512 TMEM columns), with four rows or more each
+  const long long rows = (long long)batch * H * (W / kTileM);
+  const int grid = (int)std::max<long long>(1, std::min<long long>(rows / 4, sms));
+  const long long nel = 9LL * cout * cin;
+  const cudaStream_t st = (cudaStream_t)stream;
+  const cudaMemPool_t pool = parts_pool(dev);
+  float* parts = nullptr;
+  if (!pool || cudaMallocFromPoolAsync(&parts, grid * (nel + cout) * sizeof(float), pool, st) !=
+                   cudaSuccess)
+    return NL2D_ERR_CUDA;
+  k_conv_wgrad_pipe<POLL><<<grid, kWgThreads, smem, st>>>(
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, parts, batch, H, W, cin, cout, slots,
+      max_cycles, err);
+  k_sum_parts<<<(int)((nel + cout + kSumElems - 1) / kSumElems), kSumWays * kSumElems, 0, st>>>(
+      parts, grid, nel, cout, dw, db);
+  const cudaError_t launched = cudaGetLastError();
+  return cudaFreeAsync(parts, st) == cudaSuccess && launched == cudaSuccess ? NL2D_OK
+                                                                             : NL2D_ERR_CUDA;
+}
+
 }  // namespace
 }  // namespace emu
 }  // namespace nl2d
@@ -1129,55 +1259,7 @@ int nl2d_selftest_wait(long long max_cycles, int* status) {
 int nl2d_emu_conv3x3(const void* x, const void* w, const float* bias, void* y, float* y32,
                      int batch, int H, int W, int cin, int cout, int relu, int* err,
                      void* stream) {
-  if (cin % 16 || cout % 16 || cout > 64 || cin < 16 || cin > 64 || W % kTileM || H < 1 ||
-      batch < 1 || !x || !w || !err || (!y && !y32))
-    return NL2D_ERR_ARGS;
-  const size_t wbytes = ((9 * (size_t)cout * cin * 2) + 1023) & ~(size_t)1023;
-  const size_t smem = wbytes + kConvSlots * (size_t)(cin / 8) * kLboX;
-  constexpr int kMaxSmem = 200 * 1024;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_conv3x3_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kMaxSmem) != cudaSuccess)
-      return NL2D_ERR_CUDA;
-    attr = true;
-  }
-  if (smem > kMaxSmem) return NL2D_ERR_ARGS;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long rows = (long long)batch * H * (W / kTileM);
-  // Persistent CTAs: as many as are resident at once, with two rows or more
-  // each.  Counted from the kernel's registers (allocated per warp in units of
-  // 256) and shared memory (dynamic + static + the driver's reserve per
-  // block), as the hardware limits them; each CTA also holds conv_tmem() of
-  // the SM's 512 TMEM columns.  (cudaOccupancyMaxActiveBlocksPerMultiprocessor
-  // answered 1 where 2 are resident.)
-  static cudaFuncAttributes fa;
-  static bool fa_ok = false;
-  if (!fa_ok) {
-    if (cudaFuncGetAttributes(&fa, k_conv3x3_pipe) != cudaSuccess) return NL2D_ERR_CUDA;
-    fa_ok = true;
-  }
-  int regs_sm = 0, smem_sm = 0, smem_rsv = 0;
-  cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
-  cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-  cudaDeviceGetAttribute(&smem_rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-  const int warp_regs = (fa.numRegs * 32 + 255) / 256 * 256;
-  const int by_regs = regs_sm / (warp_regs * (kPipeThreads / 32));
-  const int by_smem = smem_sm / (int)(smem + fa.sharedSizeBytes + smem_rsv);
-  int per_sm = by_regs < by_smem ? by_regs : by_smem;
-  per_sm = per_sm < 512 / conv_tmem(cout) ? per_sm : 512 / conv_tmem(cout);
-  per_sm = per_sm < 1 ? 1 : per_sm;
-  const int grid =
-      (int)std::max<long long>(1, std::min<long long>(rows / 2, (long long)per_sm * sms));
-  // 32-byte stores where an output starts on a 32-byte boundary (every pixel
-  // then does: cout is a multiple of 16)
-  const int wide = ((uintptr_t)y % 32 == 0 ? 1 : 0) | ((uintptr_t)y32 % 32 == 0 ? 2 : 0);
-  k_conv3x3_pipe<<<grid, kPipeThreads, smem, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, bias, (__nv_bfloat16*)y, y32, batch, H,
-      W, cin, cout, relu, wide, err);
-  return cudaGetLastError() == cudaSuccess ? NL2D_OK : NL2D_ERR_CUDA;
+  return conv3x3<false>(x, w, bias, y, y32, batch, H, W, cin, cout, relu, 0, err, stream);
 }
 
 int nl2d_emu_flip_transpose(const void* w, void* wt, int cout, int cin, void* stream) {
@@ -1189,45 +1271,19 @@ int nl2d_emu_flip_transpose(const void* w, void* wt, int cout, int cin, void* st
 
 int nl2d_emu_conv_wgrad(const void* x, const void* dy, float* dw, float* db, int batch, int H,
                         int W, int cin, int cout, int* err, void* stream) {
-  if (!x || !dy || !dw || !db || !err || cin % 16 || cin < 16 || 9 * cin > kWgTmemCols ||
-      cout % 8 || cout < 8 || cout > 128 || W % kTileM || H < 1 || batch < 1)
-    return NL2D_ERR_ARGS;
-  // As many ring slots as fit (at least one row in flight: wg_depth).
-  // The kernel holds all 512 TMEM columns, so it must be alone on its SM:
-  // asking for more than half an SM's shared memory guarantees that.
-  int slots = kWgMaxSlots;
-  while (slots > 3 && wg_smem(cin, cout, slots) > kWgMaxSmem) slots--;
-  const size_t need = wg_smem(cin, cout, slots);
-  const size_t smem = need > 120 * 1024 ? need : 120 * 1024;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_conv_wgrad_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kWgMaxSmem) != cudaSuccess)
-      return NL2D_ERR_CUDA;
-    attr = true;
-  }
-  if (smem > kWgMaxSmem) return NL2D_ERR_ARGS;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // one CTA per SM (512 TMEM columns), with four rows or more each
-  const long long rows = (long long)batch * H * (W / kTileM);
-  const int grid = (int)std::max<long long>(1, std::min<long long>(rows / 4, sms));
-  const long long nel = 9LL * cout * cin;
-  const cudaStream_t st = (cudaStream_t)stream;
-  const cudaMemPool_t pool = parts_pool(dev);
-  float* parts = nullptr;
-  if (!pool || cudaMallocFromPoolAsync(&parts, grid * (nel + cout) * sizeof(float), pool, st) !=
-                   cudaSuccess)
-    return NL2D_ERR_CUDA;
-  k_conv_wgrad_pipe<<<grid, kWgThreads, smem, st>>>((const __nv_bfloat16*)x,
-                                                      (const __nv_bfloat16*)dy, parts, batch, H,
-                                                      W, cin, cout, slots, err);
-  k_sum_parts<<<(int)((nel + cout + kSumElems - 1) / kSumElems), kSumWays * kSumElems, 0, st>>>(
-      parts, grid, nel, cout, dw, db);
-  const cudaError_t launched = cudaGetLastError();
-  return cudaFreeAsync(parts, st) == cudaSuccess && launched == cudaSuccess ? NL2D_OK
-                                                                             : NL2D_ERR_CUDA;
+  return conv_wgrad<false>(x, dy, dw, db, batch, H, W, cin, cout, 0, err, stream);
+}
+
+// Test hook (no reference counterpart): the convolution (wgrad = 0; b the
+// weights, out FP32 values, db unused) or the weight gradient (b the output's
+// gradient, out dw) with another limit on the roles' waits for each other.
+int nl2d_selftest_emu_wait(int wgrad, const void* x, const void* b, float* out, float* db,
+                           int batch, int H, int W, int cin, int cout, long long max_cycles,
+                           int* err) {
+  if (max_cycles < 0 || max_cycles > kMaxWaitCycles) return NL2D_ERR_ARGS;
+  return wgrad ? conv_wgrad<true>(x, b, out, db, batch, H, W, cin, cout, max_cycles, err, nullptr)
+               : conv3x3<true>(x, b, nullptr, nullptr, out, batch, H, W, cin, cout, 0, max_cycles,
+                               err, nullptr);
 }
 
 int nl2d_emu_relu_bwd(const float* g, const void* y, void* out, long long n, void* stream) {
