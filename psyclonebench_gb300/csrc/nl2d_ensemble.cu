@@ -180,6 +180,9 @@ constexpr int kDefaultMarchRows = 32;
 constexpr int kNumShapes = 5;
 constexpr int kShapes[kNumShapes][2] = {{32, 16}, {32, 8}, {16, 16}, {64, 8}, {32, 32}};
 constexpr int kDefaultShape = 1;
+// The schedule until the caller or the autotuner chooses one (nl2d_ens_schedule).
+constexpr int kDefaultCtas = 2, kDefaultPolicy = 2;
+constexpr double kDefaultWeight = 4.0;
 
 template <class T>
 bool set_ens_attr() {
@@ -328,8 +331,8 @@ struct Ens {
   EnsDomain* d_desc = nullptr;
   int4* d_tiles = nullptr;
   int* d_first = nullptr;
-  int ntiles = 0, nctas = 0, ctas_per_sm = 2, policy = 2;
-  double boundary_weight = 4.0;
+  int ntiles = 0, nctas = 0, ctas_per_sm = kDefaultCtas, policy = kDefaultPolicy;
+  double boundary_weight = kDefaultWeight;
   double* d_tides = nullptr;
   size_t tides_cap = 0;
   double* d_sums = nullptr;
@@ -471,6 +474,9 @@ void ens_free() {
   e.built = false;
   e.ndom = 0;
   e.dom.clear();
+  e.ctas_per_sm = kDefaultCtas;
+  e.policy = kDefaultPolicy;
+  e.boundary_weight = kDefaultWeight;
   e.shape = kDefaultShape;
   e.march_rows = 0;
 }
