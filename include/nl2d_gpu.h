@@ -238,9 +238,9 @@ int nl2d_ens_schedule(int ctas_per_sm, int policy, double boundary_weight);
  * psykal_omp/time_step_mod.f90:587-1182, fixes its tile size per run): the
  * FP64 kernel's tile shape tx x ty, one of 32 x 16, 32 x 8 (the default),
  * 16 x 16, 64 x 8 and 32 x 32, and the column marches' strip height (the
- * mixed and FP64-equivalent forms), 8, 16, 32 or 64 rows (until a height is
- * given the mixed form takes 32 and the FP64-equivalent one as many of 32, 16
- * and 8 as leave the SMs evenly loaded).  Results do not depend on either.  A
+ * mixed and FP64-equivalent forms), 8, 16, 32 or 64 rows, or 0 (the default):
+ * the mixed form then takes 32 and the FP64-equivalent one as many of 32, 16
+ * and 8 as leave the SMs evenly loaded.  Results do not depend on either.  A
  * new ensemble starts with the defaults.  Returns NL2D_ERR_ARGS for other
  * values. */
 int nl2d_ens_tile(int tx, int ty, int march_rows);

@@ -1071,8 +1071,8 @@ int nl2d_ens_tile(int tx, int ty, int march_rows) {
   int shape = -1;
   for (int k = 0; k < kNumShapes; k++)
     if (kShapes[k][0] == tx && kShapes[k][1] == ty) shape = k;
-  if (shape < 0 ||
-      (march_rows != 8 && march_rows != 16 && march_rows != 32 && march_rows != 64))
+  if (shape < 0 || (march_rows != 0 && march_rows != 8 && march_rows != 16 && march_rows != 32 &&
+                    march_rows != 64))
     return NL2D_ERR_ARGS;
   e.shape = shape;
   e.march_rows = march_rows;

@@ -21,6 +21,12 @@ G = 9.80665
 OMEGA = 7.292116e-05
 D2R = PI / 180.0
 
+# The knobs a new ensemble starts with (the library's own defaults, see
+# nl2d_ens_schedule and nl2d_ens_tile): one tile per CTA, each march's own rule
+# for its strip height (march_rows 0).
+DEFAULT_KNOBS = {"ctas_per_sm": 2, "policy": 2, "boundary_weight": 4.0, "tile": (32, 8),
+                 "march_rows": 0}
+
 _DP = ctypes.POINTER(ctypes.c_double)
 _IP = ctypes.POINTER(ctypes.c_int)
 
@@ -131,11 +137,14 @@ class Ensemble:
         differ)."""
         return bool(self.lib.nl2d_ens_uses_march())
 
-    def schedule(self, ctas_per_sm=2, policy=0, boundary_weight=4.0, tile=(32, 16),
-                 march_rows=32):
+    def schedule(self, ctas_per_sm=DEFAULT_KNOBS["ctas_per_sm"],
+                 policy=DEFAULT_KNOBS["policy"],
+                 boundary_weight=DEFAULT_KNOBS["boundary_weight"],
+                 tile=DEFAULT_KNOBS["tile"], march_rows=DEFAULT_KNOBS["march_rows"]):
         """Schedule and tile knobs (nl2d_ens_schedule, nl2d_ens_tile): CTAs
         per SM, tile assignment policy, ring-cell cost weight, the FP64
-        tile shape and the mixed form's march strip height."""
+        tile shape and the column marches' strip height.  Without arguments:
+        the knobs a new ensemble starts with."""
         self._check(self.lib.nl2d_ens_schedule(ctas_per_sm, policy, boundary_weight),
                     "nl2d_ens_schedule")
         self._check(self.lib.nl2d_ens_tile(int(tile[0]), int(tile[1]), march_rows),

@@ -25,9 +25,27 @@ def test_a_new_ensemble_starts_with_the_default_schedule(gpulib, domains):
     ens = Ensemble(domains, lib=gpulib)
     cells, tiles, ctas = layout(ens)
     ens.close()
-    assert ctas == tiles and other[2] < other[1]  # one unit per CTA, not a grid over chunks
+    assert ctas == tiles and other[2] != other[1]  # one unit per CTA, not a grid per SM
     ens = Ensemble(domains, lib=gpulib)  # without a close between: the same
     ens.schedule(1, 0, 0.0, (32, 32))
     ens = Ensemble(domains, lib=gpulib)
     assert layout(ens) == (cells, tiles, ctas)
+    ens.close()
+
+
+@pytest.mark.parametrize("precision", [1, 2])
+def test_the_strip_rule_can_be_had_back(gpulib, domains, precision):
+    import numpy as np
+    from psyclonebench_gb300.ensemble import Ensemble
+    ens = Ensemble(domains, lib=gpulib)
+    ens.set_precision(precision)
+    ens.run(1, 20)
+    want = ens.read(1)
+    for rows in (16, 0):
+        assert gpulib.nl2d_ens_tile(32, 8, rows) == 0
+        ens.reset()
+        ens.run(1, 20)
+        assert all(np.array_equal(a, b) for a, b in zip(ens.read(1), want))
+    for rows in (-1, 1, 7, 24, 128):
+        assert gpulib.nl2d_ens_tile(32, 8, rows) != 0
     ens.close()
