@@ -251,7 +251,6 @@ enum : unsigned {
   kScanOutside = 1u << 13,
   kScanSshaT = 1u << 14,
   kScanCopies = 1u << 15,
-  kScanLand = 1u << 17,  // land in the internal region (only a hint: where cells run)
   kScanNextSsh = 1u << 16,
 };
 
@@ -332,7 +331,6 @@ __global__ void k_register_scan(ScanIn in, unsigned* __restrict__ flags) {
       if (bits(in.ua[c]) != bits(in.un[c]) || bits(in.va[c]) != bits(in.vn[c])) f |= kScanCopies;
     }
     if (j >= in.ys && j <= in.ye && i >= in.xs && i <= in.xe) {
-      if (m[c] <= 0) f |= kScanLand;
       double v;
       if (i <= in.xe - 1 && next_ssh_value(m, in.sn, c, 1, at, au, zu, v) &&
           bits(v) != bits(in.snu[c]))
@@ -902,8 +900,7 @@ void fused_launch(const double* tide_table, int tide_index, double tide) {
   } else if (s.bands_pending) {  // (never inside a graph: prepare_graph finishes them)
     banded_first_step(fs, tide);
   } else {
-    launch_fused_step(s.dev, fs, dims(), s.sc, s.um, tide, tide_table, tide_index,
-                      (s.scan_flags & kScanLand) != 0, s.stream);
+    launch_fused_step(s.dev, fs, dims(), s.sc, s.um, tide, tide_table, tide_index, s.stream);
   }
   s.cur = nxt;
 }

@@ -46,16 +46,15 @@ using SmallTile = Tile<16, 8, 128, 4>;
 
 // One step of copy-region rows [ja, jb).  The first nring blocks take the
 // ring's cells in those rows, rc parts of them each (one per thread: their
-// long FP64 chains start first and run beside the tiles), the next nland (as
-// many as tiles, or none) a tile's cells beside land; the others one tile each
-// of the ntx per row of tiles, from tile row row0.
+// long FP64 chains start first and run beside the tiles); the others one tile
+// each of the ntx per row of tiles, from tile row row0.
 template <class TT, bool IC>
 __global__ void __launch_bounds__(TT::NTHREADS, TT::kMinBlocks)
     k_fused_step(const __grid_constant__ Fields f, const __grid_constant__ FusedState fs,
                  const __grid_constant__ Dims d, const __grid_constant__ Scalars p,
                  const __grid_constant__ FastConst k, const double* __restrict__ tide_table,
                  int tide_index, double tide, int row0, int ntx, int ja, int jb, int nring,
-                 int rc, int nland) {
+                 int rc) {
   extern __shared__ double smem[];
   const double td = tide_table ? tide_table[tide_index] : tide;
   if ((int)blockIdx.x < nring) {
@@ -69,13 +68,9 @@ __global__ void __launch_bounds__(TT::NTHREADS, TT::kMinBlocks)
     }
     return;
   }
-  const int b = blockIdx.x - nring, t = b < nland ? b : b - nland;
-  const int by = t / ntx, bx = t - by * ntx;
-  const int i0 = d.xs + 1 + bx * TT::TX, j0 = d.ys + 1 + (row0 + by) * TT::TY;
-  if (b < nland)
-    land_cells<TT>(f, fs, d, p, k, td, i0, j0, smem);
-  else
-    fused_tile<TT, IC>(f, fs, d, p, k, td, i0, j0, smem, nland > 0);
+  const int t = blockIdx.x - nring, by = t / ntx, bx = t - by * ntx;
+  fused_tile<TT, IC>(f, fs, d, p, k, td, d.xs + 1 + bx * TT::TX, d.ys + 1 + (row0 + by) * TT::TY,
+                 smem);
 }
 
 int tiles_over(int n, int t) { return n > 0 ? (n + t - 1) / t : 0; }
@@ -91,7 +86,7 @@ int tile_height(const Dims& d) { return small_tiles(d) ? SmallTile::TY : T::TY; 
 template <class TT>
 void launch_rows(const Fields& f, const FusedState& fs, const Dims& d, const Scalars& s,
                  const UniformMetrics& um, double tide, const double* tide_table, int tide_index,
-                 int row0, int row1, bool land, cudaStream_t st) {
+                 int row0, int row1, cudaStream_t st) {
   if (row1 <= row0) return;
   const int ja = fused_step_first_row(d, row0), jb = fused_step_first_row(d, row1);
   const int ntx = tiles_over(interior_x(d), TT::TX);
@@ -104,9 +99,8 @@ void launch_rows(const Fields& f, const FusedState& fs, const Dims& d, const Sca
   const int nring = (nr + rc - 1) / rc;
   const FastConst k = make_fast_const(s, um);
   auto step = k.int_mul ? k_fused_step<TT, true> : k_fused_step<TT, false>;
-  const int nland = land ? ntx * nty : 0;
-  step<<<nring + nland + ntx * nty, dim3(TT::TX, TT::RPP), TT::kSmemBytes, st>>>(
-      f, fs, d, s, k, tide_table, tide_index, tide, row0, ntx, ja, jb, nring, rc, nland);
+  step<<<nring + ntx * nty, dim3(TT::TX, TT::RPP), TT::kSmemBytes, st>>>(
+      f, fs, d, s, k, tide_table, tide_index, tide, row0, ntx, ja, jb, nring, rc);
 }
 
 void set_step_attrs() {
@@ -139,20 +133,20 @@ void launch_fused_step_rows(const Fields& f, const FusedState& fs, const Dims& d
                             int row1, cudaStream_t st) {
   set_step_attrs();
   if (small_tiles(d))
-    launch_rows<SmallTile>(f, fs, d, s, um, tide, nullptr, 0, row0, row1, false, st);
+    launch_rows<SmallTile>(f, fs, d, s, um, tide, nullptr, 0, row0, row1, st);
   else
-    launch_rows<T>(f, fs, d, s, um, tide, nullptr, 0, row0, row1, false, st);
+    launch_rows<T>(f, fs, d, s, um, tide, nullptr, 0, row0, row1, st);
 }
 
 void launch_fused_step(const Fields& f, const FusedState& fs, const Dims& d,
                        const Scalars& s, const UniformMetrics& um, double tide,
-                       const double* tide_table, int tide_index, bool land, cudaStream_t st) {
+                       const double* tide_table, int tide_index, cudaStream_t st) {
   set_step_attrs();
   const int rows = fused_step_tile_rows(d);
   if (small_tiles(d))
-    launch_rows<SmallTile>(f, fs, d, s, um, tide, tide_table, tide_index, 0, rows, land, st);
+    launch_rows<SmallTile>(f, fs, d, s, um, tide, tide_table, tide_index, 0, rows, st);
   else
-    launch_rows<T>(f, fs, d, s, um, tide, tide_table, tide_index, 0, rows, false, st);
+    launch_rows<T>(f, fs, d, s, um, tide, tide_table, tide_index, 0, rows, st);
 }
 
 namespace {

@@ -858,7 +858,7 @@ __device__ __forceinline__ bool tile_faces(const Fields& f, const Dims& d, const
 // the tile's list.
 template <class T, bool IC, bool WIDE>
 __device__ __forceinline__ void tile_update(const Fields& f, const FusedState& fs, const Dims& d,
-                                            const FastConst& k, int i0, int j0, double* smem, bool apart) {
+                                            const FastConst& k, int i0, int j0, double* smem) {
   constexpr int TX = T::TX, TY = T::TY, SX = T::SX, S0 = T::S0, NTHREADS = T::NTHREADS;
   constexpr int RX = T::RX, RY = T::RY;
   const TileSmem<T> sm(smem);
@@ -920,7 +920,7 @@ __device__ __forceinline__ void tile_update(const Fields& f, const FusedState& f
   for (int pb = 0; pb < T::RPT; pb += 2) {
     constexpr int NP = T::RPT >= 2 ? 2 : 1;  // rows taken together
     int c[NP], q[NP];
-    bool live[NP], reg[NP], sea[NP];
+    bool live[NP], reg[NP];
     bool any = false;
 #pragma unroll
     for (int e = 0; e < NP; e++) {
@@ -933,7 +933,7 @@ __device__ __forceinline__ void tile_update(const Fields& f, const FusedState& f
       for (int dj = -1; dj <= 1; dj++)
 #pragma unroll
         for (int di = -1; di <= 1; di++) regular &= mk[q[e] + dj * SX + di] > 0;
-      reg[e] = sea[e] = regular;
+      reg[e] = regular;
       any |= regular;
     }
     if (any) {
@@ -964,15 +964,14 @@ __device__ __forceinline__ void tile_update(const Fields& f, const FusedState& f
     }
 #pragma unroll
     for (int e = 0; e < NP; e++)
-      if (live[e] && !reg[e] && (T::NTHREADS > 128 || sea[e] || !apart))
+      if (live[e] && !reg[e])
         glist[atomicAdd(gcount, 1)] = (threadIdx.y + (pb + e) * T::RPP) * TX + threadIdx.x;
   }
   __syncthreads();
 }
 
 // One tile of the fused step: interior cells [i0, i0+TX) x [j0, j0+TY) of one
-// domain.  `tide` is this step's bc_ssh value (general cells).  apart: the
-// cells beside land are another block's (land_cells).
+// domain.  `tide` is this step's bc_ssh value (general cells).
 //
 // The FP64 pipe bounds the step (about 1.7 instructions per clock per SM;
 // each holds a scheduler's share of it for 64 issue slots), so every phase
@@ -986,7 +985,7 @@ __device__ __forceinline__ void tile_update(const Fields& f, const FusedState& f
 template <class T, bool IC>
 __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs, const Dims& d,
                                            const Scalars& p, const FastConst& k, double tide,
-                                           int i0, int j0, double* smem, bool apart = false) {
+                                           int i0, int j0, double* smem) {
   constexpr int TX = T::TX, TY = T::TY, SX = T::SX, S0 = T::S0;
   constexpr int NTHREADS = T::NTHREADS;
   const TileSmem<T> sm(smem);
@@ -1031,13 +1030,13 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
   bool any_wide = __syncthreads_or(wide);
   if (!any_wide) any_wide = __syncthreads_or(tile_faces<T, false>(f, d, k, i0, j0, smem));
   if (!any_wide) {
-    tile_update<T, IC, false>(f, fs, d, k, i0, j0, smem, apart);
+    tile_update<T, IC, false>(f, fs, d, k, i0, j0, smem);
   } else {
     for (int t = tid; t < S0; t += NTHREADS) B(B_AREA_SSH, t) = k.area_t * A(A_SN, t);
     __syncthreads();
     tile_faces<T, true>(f, d, k, i0, j0, smem);
     __syncthreads();
-    tile_update<T, IC, true>(f, fs, d, k, i0, j0, smem, apart);
+    tile_update<T, IC, true>(f, fs, d, k, i0, j0, smem);
   }
 
   // ---- general cells: the reference's per-point code, in its order ----
@@ -1049,39 +1048,6 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
   }
 #undef A
 #undef B
-}
-
-// The cells of tile (i0, j0) that have land beside them, by the general code,
-// in a block of their own: their chains of dependent operations then run
-// beside the tile's update instead of after it.  Taken with the small tiles
-// (128 threads) where the registration scan saw land: 500 steps and the rest of
-// a run, 130 x 109 with islands 17.3 -> 13.9 ms, 538 x 127 17.9 -> 15.2.
-template <class T>
-__device__ __forceinline__ void land_cells(const Fields& f, const FusedState& fs, const Dims& d,
-                                           const Scalars& p, const FastConst& k, double tide,
-                                           int i0, int j0, double* smem) {
-  constexpr int TX = T::TX, TY = T::TY;
-  int* list = reinterpret_cast<int*>(smem);
-  int* count = list + TX * TY;
-  const int tid = threadIdx.y * TX + threadIdx.x;
-  if (tid == 0) *count = 0;
-  __syncthreads();
-  for (int t = tid; t < TX * TY; t += T::NTHREADS) {
-    const int i = i0 + t % TX, j = j0 + t / TX;
-    if (i > d.xe - 1 || j > d.ye - 1) continue;
-    bool sea = true;
-#pragma unroll
-    for (int dj = -1; dj <= 1; dj++)
-#pragma unroll
-      for (int di = -1; di <= 1; di++) sea &= f.tmask[(j + dj) * d.width + i + di] > 0;
-    if (!sea) list[atomicAdd(count, 1)] = t;
-  }
-  __syncthreads();
-  const int n = *count;
-  for (int g = tid; g < kParts * n; g += T::NTHREADS) {
-    const int part = g / n, t = list[g - part * n];
-    general_at(f, fs, d, p, k, tide, part, i0 + t % TX, j0 + t / TX);
-  }
 }
 
 bool in_fast_range(double d) {

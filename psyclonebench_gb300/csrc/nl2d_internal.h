@@ -83,12 +83,10 @@ struct FusedState {
 };
 // `tide` is the bc_ssh value of this step, or, when `tide_table` is not
 // null, tide_table[tide_index] (a device table; used by captured graphs).
-// land: whether the internal region may hold land (a hint: the result does
-// not depend on it).
 void launch_fused_step(const Fields& f, const FusedState& fs, const Dims& d,
                        const Scalars& s, const UniformMetrics& um, double tide,
                        const double* tide_table, int tide_index,
-                       bool land, cudaStream_t st);
+                       cudaStream_t st);
 // The rows of tiles the fused step's grid has for this domain, and the first
 // copy-region row that tile row `row` updates (0 .. the number of rows).
 int fused_step_tile_rows(const Dims& d);
