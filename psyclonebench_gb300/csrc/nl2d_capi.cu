@@ -541,6 +541,10 @@ bool upload_rows(void* const* ptrs, int k, int r0, int r1, cudaStream_t st) {
 
 // speculate: the caller is c_invoke_time_step, which can take fused steps
 // before the scan has answered (see State::spec_pending).
+// Registrations above kAskRoom bytes look how much memory there is; the mixed
+// form's arrays take kFormBytes per point, the others' less.
+constexpr size_t kAskRoom = (size_t)1 << 30, kFormBytes = 64;
+
 bool do_register(void* const* ptrs, int xs, int xe, int ys, int ye, int width, int height,
                  const Scalars& sc, bool speculate = false) {
   State& s = g_state;
@@ -566,12 +570,25 @@ bool do_register(void* const* ptrs, int xs, int xe, int ys, int ye, int width, i
   s.registered = true;  // so free_device releases partial allocations
   s.h2d_bytes = s.d2h_bytes = 0;
   // One allocation carved into the registration's 34 arrays (256-byte
-  // aligned): 34 separate cudaMalloc calls took 1.7-2.9 ms on the GB300
-  // box, one of the same total 0.18 ms, and the first call waits for them
-  // before its first copy.
+  // aligned): 34 separate cudaMalloc calls took 1.7-2.9 ms, one of the same
+  // total 0.18 ms, and the first call waits for them before its first copy.
+  // Without the two depth sums (Fields::depth_sums) where they would not leave
+  // room for the other forms' arrays, or do not fit themselves; small
+  // registrations always have them.
   const size_t a8 = (n * 8 + 255) & ~(size_t)255, a4 = (n * 4 + 255) & ~(size_t)255;
-  if (!CK(cudaMalloc(&s.slab, (size_t)(kNumFields + kNumGrid - 1 + 6 + 3) * a8 + a4)))
-    return false;
+  const size_t need = (size_t)(kNumFields + kNumGrid - 1 + 4 + 3) * a8 + a4;
+  bool sums = true;
+  if (need > kAskRoom) {
+    size_t room = 0, all = 0;
+    if (!CK(cudaMemGetInfo(&room, &all))) return false;
+    sums = room >= need + 2 * a8 + kFormBytes * n;
+  }
+  if (sums && need > kAskRoom && cudaMalloc(&s.slab, need + 2 * a8) != cudaSuccess) {
+    cudaGetLastError();  // not an error yet
+    s.slab = nullptr;
+    sums = false;
+  }
+  if (!s.slab && !CK(cudaMalloc(&s.slab, need + (sums ? 2 * a8 : 0)))) return false;
   char* cut = static_cast<char*>(s.slab);
   auto take = [&cut](size_t bytes) {
     char* p = cut;
@@ -583,8 +600,8 @@ bool do_register(void* const* ptrs, int xs, int xe, int ys, int ye, int width, i
   for (int k = 1; k < kNumGrid; k++) *grid_slot(s.dev, k) = (double*)take(a8);
   s.dev.sin_u = (double*)take(a8);
   s.dev.sin_v = (double*)take(a8);
-  s.dev.d_hu = (double*)take(a8);
-  s.dev.d_hv = (double*)take(a8);
+  s.dev.d_hu = sums ? (double*)take(a8) : s.dev.ssha_u;
+  s.dev.d_hv = sums ? (double*)take(a8) : s.dev.ssha_v;
   s.dev.r_hu = (unsigned long long*)take(a8);
   s.dev.r_hv = (unsigned long long*)take(a8);
   for (double*& p : s.shadow) p = (double*)take(a8);

@@ -64,13 +64,16 @@ __global__ void __launch_bounds__(32 * WARPS, 3)
   df_march(fs, ff, d, k, d.xs - 1 + gx * MW, d.ys - 1 + gy * mr, mr);
 }
 
-// FP64 arrays, or their elements' reciprocals (0 for depths outside the range
-// in which the step takes reciprocals), split into pairs once per set-up.
+// FP64 arrays, or the reciprocals of their elements (plus those of `add`, if
+// given; 0 for depths outside the range in which the step takes reciprocals),
+// split into pairs once per set-up.
 template <bool RECIPROCAL>
-__global__ void k_split(const double* __restrict__ a, float2* __restrict__ out, long long n) {
+__global__ void k_split(const double* __restrict__ a, const double* __restrict__ add,
+                        float2* __restrict__ out, long long n) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     double x = a[t];
+    if (RECIPROCAL && add) x += add[t];
     if (RECIPROCAL) x = (x >= 0x1p-100 && x <= 0x1p100) ? 1.0 / x : 0.0;
     const df p = from_double(x);
     out[t] = make_float2(p.hi, p.lo);
@@ -162,11 +165,11 @@ DfConst make_df_const(const Scalars& s, const UniformMetrics& um) {
 
 void launch_df_setup(const Fields& f, const Dims& d, const DfFields& ff, cudaStream_t st) {
   const long long n = (long long)d.width * d.height;
-  k_split<false><<<152 * 8, 256, 0, st>>>(f.ht, ff.ht, n);
-  k_split<false><<<152 * 8, 256, 0, st>>>(f.hu, ff.hu, n);
-  k_split<false><<<152 * 8, 256, 0, st>>>(f.hv, ff.hv, n);
-  k_split<true><<<152 * 8, 256, 0, st>>>(f.d_hu, ff.rhu, n);
-  k_split<true><<<152 * 8, 256, 0, st>>>(f.d_hv, ff.rhv, n);
+  k_split<false><<<152 * 8, 256, 0, st>>>(f.ht, nullptr, ff.ht, n);
+  k_split<false><<<152 * 8, 256, 0, st>>>(f.hu, nullptr, ff.hu, n);
+  k_split<false><<<152 * 8, 256, 0, st>>>(f.hv, nullptr, ff.hv, n);
+  k_split<true><<<152 * 8, 256, 0, st>>>(f.d_hu, f.depth_sums() ? nullptr : f.hu, ff.rhu, n);
+  k_split<true><<<152 * 8, 256, 0, st>>>(f.d_hv, f.depth_sums() ? nullptr : f.hv, ff.rhv, n);
   k_df_flags<<<152 * 8, 256, 0, st>>>(f.tmask, d, ff.reg);
 }
 
@@ -222,7 +225,7 @@ namespace nl2d {
 void launch_df_split(const double* a, float2* out, long long n, bool reciprocal,
                      cudaStream_t st) {
   auto split = reciprocal ? k_split<true> : k_split<false>;
-  split<<<152 * 8, 256, 0, st>>>(a, out, n);
+  split<<<152 * 8, 256, 0, st>>>(a, nullptr, out, n);
 }
 
 void launch_df_flags(const int* tmask, const Dims& d, unsigned char* reg, cudaStream_t st) {

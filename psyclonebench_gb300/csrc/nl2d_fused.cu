@@ -48,7 +48,7 @@ using SmallTile = Tile<16, 8, 128, 4>;
 // ring's cells in those rows, rc parts of them each (one per thread: their
 // long FP64 chains start first and run beside the tiles); the others one tile
 // each of the ntx per row of tiles, from tile row row0.
-template <class TT, bool IC>
+template <class TT, bool IC, bool SUMS>
 __global__ void __launch_bounds__(TT::NTHREADS, TT::kMinBlocks)
     k_fused_step(const __grid_constant__ Fields f, const __grid_constant__ FusedState fs,
                  const __grid_constant__ Dims d, const __grid_constant__ Scalars p,
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(TT::NTHREADS, TT::kMinBlocks)
     return;
   }
   const int t = blockIdx.x - nring, by = t / ntx, bx = t - by * ntx;
-  fused_tile<TT, IC>(f, fs, d, p, k, td, d.xs + 1 + bx * TT::TX, d.ys + 1 + (row0 + by) * TT::TY,
+  fused_tile<TT, IC, SUMS>(f, fs, d, p, k, td, d.xs + 1 + bx * TT::TX, d.ys + 1 + (row0 + by) * TT::TY,
                  smem);
 }
 
@@ -98,7 +98,10 @@ void launch_rows(const Fields& f, const FusedState& fs, const Dims& d, const Sca
   while (rc < TT::NTHREADS && nr > rc * 152) rc *= 2;
   const int nring = (nr + rc - 1) / rc;
   const FastConst k = make_fast_const(s, um);
-  auto step = k.int_mul ? k_fused_step<TT, true> : k_fused_step<TT, false>;
+  auto step = k.int_mul ? k_fused_step<TT, true, true> : k_fused_step<TT, false, true>;
+  // (one form without the depth sums must do: it is for the few registrations
+  // that fill the memory; a branch in the others would cost all 1 %)
+  if (!f.depth_sums()) step = k_fused_step<TT, false, false>;
   step<<<nring + ntx * nty, dim3(TT::TX, TT::RPP), TT::kSmemBytes, st>>>(
       f, fs, d, s, k, tide_table, tide_index, tide, row0, ntx, ja, jb, nring, rc);
 }
@@ -106,9 +109,11 @@ void launch_rows(const Fields& f, const FusedState& fs, const Dims& d, const Sca
 void set_step_attrs() {
   static bool attr_set = false;
   if (!attr_set) {
-    for (auto* fn : {k_fused_step<T, false>, k_fused_step<T, true>})
+    for (auto* fn : {k_fused_step<T, false, true>, k_fused_step<T, true, true>,
+                     k_fused_step<T, false, false>})
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmemBytes);
-    for (auto* fn : {k_fused_step<SmallTile, false>, k_fused_step<SmallTile, true>})
+    for (auto* fn : {k_fused_step<SmallTile, false, true>, k_fused_step<SmallTile, true, true>,
+                     k_fused_step<SmallTile, false, false>})
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)SmallTile::kSmemBytes);
     attr_set = true;
@@ -151,15 +156,16 @@ void launch_fused_step(const Fields& f, const FusedState& fs, const Dims& d,
 
 namespace {
 
-// The momentum denominators h + ssha and their 64-bit reciprocals, 0 where
-// the depth lies outside [2^-100, 2^100] (the kernel then divides).
+// The momentum denominators h + ssha (not stored where dh is null) and their
+// 64-bit reciprocals, 0 where the depth lies outside [2^-100, 2^100] (the
+// kernel then divides).
 __global__ void k_depth_reciprocal(const double* __restrict__ h,
                                    const double* __restrict__ ssha, double* __restrict__ dh,
                                    unsigned long long* __restrict__ r, long long n) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     const double dd = h[t] + ssha[t];
-    dh[t] = dd;
+    if (dh) dh[t] = dd;
     r[t] = recip64_of(dd);
   }
 }
@@ -172,8 +178,10 @@ void launch_depth_reciprocals(const Fields& f, const Dims& d, cudaStream_t st, i
   const size_t o = (size_t)row0 * d.width;
   const long long n = (long long)(row1 - row0) * d.width;
   if (n <= 0) return;
-  k_depth_reciprocal<<<152 * 8, 256, 0, st>>>(f.hu + o, f.ssha_u + o, f.d_hu + o, f.r_hu + o, n);
-  k_depth_reciprocal<<<152 * 8, 256, 0, st>>>(f.hv + o, f.ssha_v + o, f.d_hv + o, f.r_hv + o, n);
+  double* du = f.depth_sums() ? f.d_hu + o : nullptr;
+  double* dv = f.depth_sums() ? f.d_hv + o : nullptr;
+  k_depth_reciprocal<<<152 * 8, 256, 0, st>>>(f.hu + o, f.ssha_u + o, du, f.r_hu + o, n);
+  k_depth_reciprocal<<<152 * 8, 256, 0, st>>>(f.hv + o, f.ssha_v + o, dv, f.r_hv + o, n);
 }
 
 }  // namespace nl2d

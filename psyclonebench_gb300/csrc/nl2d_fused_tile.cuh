@@ -855,8 +855,8 @@ __device__ __forceinline__ bool tile_faces(const Fields& f, const Dims& d, const
 }
 
 // The shared terms and the regular cells' update; the other cells go to
-// the tile's list.
-template <class T, bool IC, bool WIDE>
+// the tile's list.  SUMS: Fields::depth_sums.
+template <class T, bool IC, bool WIDE, bool SUMS>
 __device__ __forceinline__ void tile_update(const Fields& f, const FusedState& fs, const Dims& d,
                                             const FastConst& k, int i0, int j0, double* smem) {
   constexpr int TX = T::TX, TY = T::TY, SX = T::SX, S0 = T::S0, NTHREADS = T::NTHREADS;
@@ -946,6 +946,10 @@ __device__ __forceinline__ void tile_update(const Fields& f, const FusedState& f
         rhu[e] = f.r_hu[cc];
         dhv[e] = f.d_hv[cc];
         rhv[e] = f.r_hv[cc];
+        if (!SUMS) {
+          dhu[e] += f.hu[cc];
+          dhv[e] += f.hv[cc];
+        }
       }
       RegOut o[NP];
 #pragma unroll
@@ -982,7 +986,7 @@ __device__ __forceinline__ void tile_update(const Fields& f, const FusedState& f
 // cell of the form that used it for everything on 2- and 1-cell halos.  The
 // integer forms pay only as straight-line code: with a range branch each,
 // the same products made the step slower.
-template <class T, bool IC>
+template <class T, bool IC, bool SUMS = true>
 __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs, const Dims& d,
                                            const Scalars& p, const FastConst& k, double tide,
                                            int i0, int j0, double* smem) {
@@ -1030,13 +1034,13 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
   bool any_wide = __syncthreads_or(wide);
   if (!any_wide) any_wide = __syncthreads_or(tile_faces<T, false>(f, d, k, i0, j0, smem));
   if (!any_wide) {
-    tile_update<T, IC, false>(f, fs, d, k, i0, j0, smem);
+    tile_update<T, IC, false, SUMS>(f, fs, d, k, i0, j0, smem);
   } else {
     for (int t = tid; t < S0; t += NTHREADS) B(B_AREA_SSH, t) = k.area_t * A(A_SN, t);
     __syncthreads();
     tile_faces<T, true>(f, d, k, i0, j0, smem);
     __syncthreads();
-    tile_update<T, IC, true>(f, fs, d, k, i0, j0, smem);
+    tile_update<T, IC, true, SUMS>(f, fs, d, k, i0, j0, smem);
   }
 
   // ---- general cells: the reference's per-point code, in its order ----

@@ -38,6 +38,9 @@ struct Fields {
   // outside [2^-100, 2^100]), for the fused step.
   double *d_hu, *d_hv;
   unsigned long long *r_hu, *r_hv;
+  // (In a registration that leaves no room for the sums, d_hu and d_hv are
+  // ssha_u and ssha_v themselves, and hu and hv are added where they are read.)
+  bool depth_sums() const { return d_hu != ssha_u; }
 };
 
 struct Dims {
