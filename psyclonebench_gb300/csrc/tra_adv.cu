@@ -176,7 +176,10 @@ __device__ __forceinline__ double upstream_b(double vel, double zu, double f1, d
 
 struct TraDev {
   const double *pun, *pvn, *pwn, *umask, *vmask, *tmask, *zind;
-  const double *cun, *cvn, *cwn;  // the velocities' Courant factors zu
+  // the velocities' Courant factors zu (the velocities themselves where there
+  // is no room for them: every kernel then takes the wide forms, which make
+  // their own)
+  const double *cun, *cvn, *cwn;
   int I, J, K;
 };
 
@@ -199,9 +202,11 @@ __global__ void k_tra_zind(const double* __restrict__ tsn, const double* __restr
     double z = max2(max2(rnfmsk[p2] * rnfmsk_z[k], upsmsk[p2]), zice) * tm;
     zind[t] = 1 - z;
     const double u = d.pun[t], v = d.pvn[t], w = d.pwn[t];
-    cun[t] = courant(half_sign(u), u);
-    cvn[t] = courant(half_sign(v), v);
-    cwn[t] = courant(half_sign(w), w);
+    if (cun) {
+      cun[t] = courant(half_sign(u), u);
+      cvn[t] = courant(half_sign(v), v);
+      cwn[t] = courant(half_sign(w), w);
+    }
     out |= vel_out(u) | vel_out(v) | vel_out(w) | mask_out(d.umask[t]) | mask_out(d.vmask[t]) |
            mask_out(tm) | mask_out(1 - z);
   }
@@ -476,8 +481,20 @@ void tra_release() {
 
 TraDev tra_dev() {
   const TraState& s = g_tra;
-  return TraDev{s.pun,  s.pvn, s.pwn, s.umask, s.vmask, s.tmask, s.zind,
-                s.cun,  s.cvn, s.cwn, s.I,     s.J,     s.K};
+  const bool f = s.cun != nullptr;
+  return TraDev{s.pun,
+                s.pvn,
+                s.pwn,
+                s.umask,
+                s.vmask,
+                s.tmask,
+                s.zind,
+                f ? s.cun : s.pun,
+                f ? s.cvn : s.pvn,
+                f ? s.cwn : s.pwn,
+                s.I,
+                s.J,
+                s.K};
 }
 
 // One iteration's two launches on the library's stream.
@@ -513,7 +530,7 @@ bool tra_register(const double* ztfreez, const double* pun, const double* pvn, c
   const size_t n3 = (size_t)I * J * K, b3 = n3 * sizeof(double);
   const size_t b2 = (size_t)I * J * sizeof(double);
   for (double** p : {&s.m[0], &s.m[1], &s.pun, &s.pvn, &s.pwn, &s.umask, &s.vmask, &s.tmask,
-                     &s.zind, &s.cun, &s.cvn, &s.cwn})
+                     &s.zind})
     if (!tra_ck(cudaMalloc(p, b3), "cudaMalloc")) return false;
   double *d_tsn = nullptr, *d2[3] = {nullptr, nullptr, nullptr}, *d_rz = nullptr;
   int* d_wide = nullptr;
@@ -521,6 +538,16 @@ bool tra_register(const double* ztfreez, const double* pun, const double* pvn, c
             tra_ck(cudaMalloc(&d_wide, sizeof(int)), "cudaMalloc") &&
             tra_ck(cudaMalloc(&d_rz, K * sizeof(double)), "cudaMalloc");
   for (int q = 0; q < 3 && ok; q++) ok = tra_ck(cudaMalloc(&d2[q], b2), "cudaMalloc");
+  // the Courant factors, where there is room for all three
+  bool room = ok;
+  for (double** p : {&s.cun, &s.cvn, &s.cwn}) room = room && cudaMalloc(p, b3) == cudaSuccess;
+  if (!room) {
+    cudaGetLastError();  // not an error
+    for (double** p : {&s.cun, &s.cvn, &s.cwn}) {
+      cudaFree(*p);
+      *p = nullptr;
+    }
+  }
   const struct {
     double* dst;
     const double* src;
@@ -545,6 +572,7 @@ bool tra_register(const double* ztfreez, const double* pun, const double* pvn, c
          tra_ck(cudaMemcpyAsync(&s.wide, d_wide, sizeof(int), cudaMemcpyDeviceToHost, s.stream),
                 "registration") &&
          tra_ck(cudaStreamSynchronize(s.stream), "registration");
+    if (!room) s.wide = 1;
   }
   cudaFree(d_tsn);
   cudaFree(d_rz);

@@ -78,3 +78,27 @@ def test_registration_without_room_for_the_depth_sums(gpulib, oracle, precision,
     if precision == 0:
         T.run(oracle.oracle_invoke_time_step, start, 3)
         assert all(bits_equal(got.f[k], start.f[k]) for k in ("sshn_t", "un", "vn"))
+
+
+def test_tracer_without_room_for_the_courant_factors(gpulib, oracle):
+    import torch
+    from test_gpu_tra_adv import gpu_compute, gpu_field, oracle_field
+    from test_tra_oracle import random_inputs
+    f = random_inputs(300, 200, 40, seed=5)
+    size = f["mydomain"].nbytes
+
+    def go():
+        free = torch.cuda.mem_get_info()[0]
+        gpu_compute(gpulib, f, 3)
+        taken = free - torch.cuda.mem_get_info()[0]
+        got = gpu_field(gpulib, f["mydomain"].shape)
+        gpulib.tra_adv_finalize()
+        return got, taken
+
+    want, taken = go()
+    assert taken > 11 * size
+    with Filled(11 * size + 16 * MB):  # nine fields and what the registration needs for a while
+        got, taken = go()
+    assert taken < 10 * size
+    np.testing.assert_array_equal(got.view(np.int64), want.view(np.int64))
+    np.testing.assert_array_equal(got.view(np.int64), oracle_field(f, 3).view(np.int64))
