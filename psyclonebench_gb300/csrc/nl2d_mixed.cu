@@ -177,7 +177,7 @@ __global__ void k_from_mixed(const float2* __restrict__ sn2, const float* __rest
 
 namespace {
 // The march's strip height: one wave of at most four blocks per SM where the
-// strips are then no taller than 128 rows (and no shorter than 8), else MR.
+// strips are then no taller than kWaveRows (and no shorter than 8), else MR.
 // The march lives on the L1: neighbouring warps share the 128-byte lines at
 // their columns' edges and the rows in flight are held there, and a fifth
 // block per SM costs more in lines evicted than its loads in flight give
@@ -187,13 +187,17 @@ namespace {
 // rows to load behind another strip.  us at the heights of this rule and
 // of the one before it (halving from 64 until two waves of five blocks):
 // 2048^2 45.9 / 59.5, 3001 x 2003 63 / 75, 4096 x 2048 89 / 96, 1024^2 18.1
-// / 18.2.  Above 128 rows a wave's blocks drift apart (4096^2:
-// 64 rows 172 us, 257 rows 226).
+// / 18.2.  In taller strips a wave's blocks drift apart: 64 rows against the
+// wave's, 4096^2 172 us against 226 (257 rows), 3000^2 101.8 / 105.5 (126), 2100
+// x 4096 99.6 / 104.6 (121); there are exceptions up to 124 rows (2950^2 96.3 /
+// 93.8), and shorter strips gain (2700 x 3000, 113 rows, 86.7 against 90.9 by
+// the rule before).
+constexpr int kWaveRows = 120;
 int strip_rows(int ncol, int ny) {
   const int fit = 4 * 152 * MARCH_WARPS / ncol;  // strips that one such wave holds
   if (fit < 1) return MR;
   const int mr = (ny + fit - 1) / fit;
-  return mr > 2 * MR ? MR : (mr < 8 ? 8 : mr);
+  return mr > kWaveRows ? MR : (mr < 8 ? 8 : mr);
 }
 }  // namespace
 
