@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(T::NTHREADS, T::kMinBlocks)
       const int tid = threadIdx.y * T::TX + threadIdx.x, g = tl.w + tid;
       const int ja = D.d.ys - 1, jb = D.d.ye + 1, n = ring_count(D.d, ja, jb);
       const int part = g / n;
-      if (part < kParts) {
+      if (tid < kRingUnit && part < kParts) {
         int i, j;
         ring_pos(D.d, ja, jb, g - part * n, i, j);
         general_at(D.f, D.fs[parity], D.d, D.p, D.k, tides[tl.x], part, i, j);
@@ -177,6 +177,9 @@ constexpr int kDefaultMarchRows = 32;
 // (the fastest or within 5 % of it from rest and in motion: 8 domains of 256^2
 // in motion 85.6 us per step, 32 x 16 in contiguous chunks 103.8; from rest
 // 159 and 265).
+// (32 x 32 takes the SM's shared memory for one CTA, so 512 threads: with 256,
+// long chains on eight warps, 16 domains in contiguous chunks with a boundary
+// weight of 16 took 866 us per step, 655 so; 64 in one-tile CTAs 2396 and 1618.)
 constexpr int kNumShapes = 5;
 constexpr int kShapes[kNumShapes][2] = {{32, 16}, {32, 8}, {16, 16}, {64, 8}, {32, 32}};
 constexpr int kDefaultShape = 1;
@@ -204,7 +207,7 @@ bool prepare_ens_step(int shape) {
     case 1: return set_ens_attr<Tile<32, 8, 256, 3>>();
     case 2: return set_ens_attr<Tile<16, 16, 256, 3>>();
     case 3: return set_ens_attr<Tile<64, 8>>();
-    case 4: return set_ens_attr<Tile<32, 32>>();
+    case 4: return set_ens_attr<Tile<32, 32, 512>>();
     default: return set_ens_attr<DefaultTile>();
   }
 }
@@ -225,7 +228,7 @@ void launch_ens_step(int shape, bool int_mul, int nctas, const EnsDomain* doms,
     case 1: launch = launch_ens_step_shape<Tile<32, 8, 256, 3>>; break;
     case 2: launch = launch_ens_step_shape<Tile<16, 16, 256, 3>>; break;
     case 3: launch = launch_ens_step_shape<Tile<64, 8>>; break;
-    case 4: launch = launch_ens_step_shape<Tile<32, 32>>; break;
+    case 4: launch = launch_ens_step_shape<Tile<32, 32, 512>>; break;
     default: break;
   }
   launch(int_mul, nctas, doms, tiles, first, parity, tides, st);
