@@ -906,35 +906,76 @@ __global__ void __launch_bounds__(kSumWays * kSumElems)
   }
 }
 
-// Scratch for the per-CTA partial gradients: allocated and freed in the
-// caller's stream's order from a pool of the device, so that calls on other
-// streams and threads get memory of their own.  The pool keeps kPartsKept
-// bytes (the widest gradient's partials are 34 MB) from one call to the next
-// and gives back what is beyond them when a stream is synchronised.  Null if
-// there is none to be had.
-constexpr unsigned long long kPartsKept = 64ull << 20;
-constexpr int kMaxDevices = 64;
-cudaMemPool_t parts_pool(int dev) {
-  static cudaMemPool_t pools[kMaxDevices] = {};
-  static std::mutex lock;
-  if (dev < 0 || dev >= kMaxDevices) return nullptr;
-  std::lock_guard<std::mutex> hold(lock);
-  if (!pools[dev]) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t pool = nullptr;
-    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
-    uint64_t kept = kPartsKept;
-    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept) != cudaSuccess) {
-      cudaMemPoolDestroy(pool);
-      return nullptr;
+// Scratch for one call's per-CTA partial gradients, which no other call may
+// touch until the reduction has read them.  A stream (by its id: handles are
+// used again) keeps a buffer of its own, in which its calls follow each other;
+// `lock` is held until the call's launches are made, so that two threads'
+// launches on one stream do not mix.  The first kPartsStreams streams of a
+// device get one (at most 34 MB each); others, and calls under capture, whose
+// graphs may run beside their stream, allocate and free in stream order (3 us
+// per call) from a pool that keeps kPartsKept bytes.
+constexpr int kPartsStreams = 4, kMaxDevices = 64;
+constexpr uint64_t kPartsKept = 64ull << 20;
+class Parts {
+ public:
+  Parts(int dev, size_t n, cudaStream_t st) : st_(st) {
+    static struct {
+      std::mutex lock;
+      cudaMemPool_t pool;
+      struct {
+        unsigned long long id;
+        float* p;
+        size_t cap;
+      } of[kPartsStreams];
+    } all[kMaxDevices];
+    if (dev < 0 || dev >= kMaxDevices) return;
+    auto& d = all[dev];
+    hold_ = std::unique_lock<std::mutex>(d.lock);
+    unsigned long long id = 0;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess ||
+        (capture == cudaStreamCaptureStatusNone && cudaStreamGetId(st, &id) != cudaSuccess))
+      return;
+    if (capture == cudaStreamCaptureStatusNone)
+      for (auto& e : d.of) {
+        if (e.p && e.id != id) continue;
+        e.id = id;
+        if (e.cap < n) {
+          cudaFree(e.p);  // (waits for the stream's calls)
+          e.p = nullptr;
+          e.cap = 0;
+          if (cudaMalloc(&e.p, n * sizeof(float)) != cudaSuccess) return;
+          e.cap = n;
+        }
+        p = e.p;
+        return;
+      }
+    if (!d.pool) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      uint64_t kept = kPartsKept;
+      if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) {
+        d.pool = nullptr;
+        return;
+      }
+      cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &kept);
     }
-    pools[dev] = pool;
+    if (cudaMallocFromPoolAsync(&p, n * sizeof(float), d.pool, st) == cudaSuccess)
+      ordered_ = true;
+    else
+      p = nullptr;
   }
-  return pools[dev];
-}
+  // After the last launch that reads p; false on a CUDA error.
+  bool done() { return !ordered_ || cudaFreeAsync(p, st_) == cudaSuccess; }
+  float* p = nullptr;  // null: none to be had
+
+ private:
+  std::unique_lock<std::mutex> hold_;
+  cudaStream_t st_;
+  bool ordered_ = false;
+};
 
 // dx = (y > 0) ? g : 0 for a ReLU output y (BF16), g FP32 -> BF16.
 __global__ void k_relu_bwd(const float* __restrict__ g, const __nv_bfloat16* __restrict__ y,
@@ -1215,19 +1256,15 @@ int conv_wgrad(const void* x, const void* dy, float* dw, float* db, int batch, i
   const int grid = (int)std::max<long long>(1, std::min<long long>(rows / 4, sms));
   const long long nel = 9LL * cout * cin;
   const cudaStream_t st = (cudaStream_t)stream;
-  const cudaMemPool_t pool = parts_pool(dev);
-  float* parts = nullptr;
-  if (!pool || cudaMallocFromPoolAsync(&parts, grid * (nel + cout) * sizeof(float), pool, st) !=
-                   cudaSuccess)
-    return NL2D_ERR_CUDA;
+  Parts parts(dev, (size_t)(grid * (nel + cout)), st);
+  if (!parts.p) return NL2D_ERR_CUDA;
   k_conv_wgrad_pipe<POLL><<<grid, kWgThreads, smem, st>>>(
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, parts, batch, H, W, cin, cout, slots,
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, parts.p, batch, H, W, cin, cout, slots,
       max_cycles, err);
   k_sum_parts<<<(int)((nel + cout + kSumElems - 1) / kSumElems), kSumWays * kSumElems, 0, st>>>(
-      parts, grid, nel, cout, dw, db);
+      parts.p, grid, nel, cout, dw, db);
   const cudaError_t launched = cudaGetLastError();
-  return cudaFreeAsync(parts, st) == cudaSuccess && launched == cudaSuccess ? NL2D_OK
-                                                                             : NL2D_ERR_CUDA;
+  return parts.done() && launched == cudaSuccess ? NL2D_OK : NL2D_ERR_CUDA;
 }
 
 }  // namespace

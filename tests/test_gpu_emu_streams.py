@@ -6,7 +6,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(2, 96, 128, 48, 48), (3, 40, 256, 16, 64), (2, 30, 128, 48, 128)]
+# more streams than keep a buffer of their own
+SHAPES = [(2, 96, 128, 48, 48), (3, 40, 256, 16, 64), (2, 30, 128, 48, 128)] * 2
 
 
 def _inputs(shape):
