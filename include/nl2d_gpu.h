@@ -260,7 +260,8 @@ int nl2d_ens_read(int dom, double *sshn_t, double *un, double *vn);
 int nl2d_ens_set_precision(int precision);
 /* Puts every domain back at rest (step 0). */
 int nl2d_ens_reset(void);
-/* Interior cells over all domains, tiles, persistent CTAs. */
+/* Interior cells over all domains, the FP64 form's work units (tiles, and runs
+ * of boundary cells) and its CTAs; the last two as of the last run. */
 int nl2d_ens_info(long long *cells, int *ntiles, int *nctas);
 void nl2d_ens_destroy(void);
 
@@ -287,7 +288,8 @@ int nl2d_emu_flip_transpose(const void *w, void *wt, int cout, int cin,
  * FP32.  Runs on the tensor cores (tcgen05, FP32 accumulation in tensor
  * memory, one persistent CTA per SM).  cin a multiple of 16 with 9*cin <=
  * 512, cout a multiple of 8 up to 128, W a multiple of 128; err (device
- * int) is set to 1 if a bounded MMA wait ran out. */
+ * int) is set to 1 if a bounded wait ran out.  Calls on several streams and
+ * threads, and under capture, keep their partial sums apart. */
 int nl2d_emu_conv_wgrad(const void *x, const void *dy, float *dw, float *db,
                         int batch, int H, int W, int cin, int cout, int *err,
                         void *stream);

@@ -15,12 +15,12 @@
 //
 // The backward pass reuses the same kernel: the input gradient is the
 // convolution of the output gradient with the tap-flipped, channel-
-// transposed weights.  The weight gradient is a reduction over pixels done
-// on the CUDA cores in FP32.
+// transposed weights.  The weight gradient is a GEMM over pixels, on the
+// tensor cores too (k_conv_wgrad_pipe).
 //
-// Every wait on the MMA completion barrier is bounded; on timeout the
-// kernel records an error flag, skips its epilogue, frees its tensor memory
-// and returns.
+// Every wait on an mbarrier is bounded; on timeout the kernel records an
+// error flag, ends its roles' loops, waits for the MMAs in flight, frees its
+// tensor memory and returns.
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cstdint>
@@ -70,14 +70,18 @@ constexpr int kRowPix = 136;
 // ---- 3x3 convolution ------------------------------------------------------
 //
 // Implicit GEMM on the tensor cores: M = 128 pixels of one image row, N =
-// output channels, K = input channels.  What bounds it is the tensor core's
-// operand reads from shared memory, so an input row is read once for all
-// three output rows it enters: with the weights of dy = 2, 1, 0 side by side
+// output channels, K = input channels.  With one MMA per tap the tensor core's
+// operand reads from shared memory were the largest item (62 % of its data
+// path's time), so an input row is read once for all three output rows it
+// enters: with the weights of dy = 2, 1, 0 side by side
 // (N = 3 cout), input row y adds to output rows y-1, y and y+1 in one MMA per
 // dx and 16 channels, their accumulators lying in adjacent column blocks of a
 // ring in tensor memory: 9 MMAs of N = 144 per row at 48 -> 48 channels
 // instead of 27 of N = 48.  (The ring's end splits an MMA in two, and the new
-// row's block takes its first MMA apart, to start from zero.)
+// row's block takes its first MMA apart, to start from zero.)  16 x 256^2: 88.1
+// -> 67.3 us.  Of an SM's active clocks the operand reads now take 37 %, the
+// tensor core's data path 58 %, its arithmetic 32 %, DRAM 37 %: nothing is full;
+// which hand-off between the roles the rest waits on has not been told apart.
 //
 // The weights stay in shared memory for the CTA's lifetime.  A staged input
 // row keeps each 8-channel group of its pixels 16 bytes apart, so the operand
@@ -535,9 +539,9 @@ __global__ void k_flip_transpose(const __nv_bfloat16* __restrict__ w,
 // convolution, so the tap (dy, dx) operand is again a row block started 16 *
 // dx bytes later.
 //
-// What bounds it is the tensor core's operand reads from shared memory: an M
-// = 128, N = 48 MMA reads 5.6 KB for 48 of its 128 rows' worth of products.
-// So two adjacent rows are stacked on each side (cout <= 64): A = dY rows (r,
+// One MMA per tap is mostly operand reads from shared memory: an M = 128, N =
+// 48 MMA reads 5.6 KB for 48 of its 128 rows' worth of products.  So two
+// adjacent rows are stacked on each side (cout <= 64): A = dY rows (r,
 // r+1), B = X rows (r, r+1), and the four quadrants of one accumulator are
 // dY(r) X(r): dy = 1, dY(r) X(r+1): dy = 2, dY(r+1) X(r): dy = 0, and dY(r+1)
 // X(r+1), which is not used (every row meets itself in the first).  As r runs
@@ -558,7 +562,11 @@ __global__ void k_flip_transpose(const __nv_bfloat16* __restrict__ w,
 //              warps 0-3 move the accumulators out of TMEM
 //   warp 7     one thread issues the MMAs
 // 48 -> 48 channels at 16 x 256^2: 193 us (9 x N = 48 per row, one row in
-// flight in registers) plus 24 us for a separate bias pass before.
+// flight in registers) plus 100 us for a separate bias pass and the sums before,
+// 98 us with everything now.  Of an SM's active clocks the operand reads take 49
+// %, the tensor core's data path 52 %, its arithmetic (an unused quadrant in
+// four) 42 %, DRAM 32 %; about 15 us are the launch's start and the accumulators'
+// way out, which nothing runs beside.
 constexpr int kWgTmemCols = 512;
 constexpr int kWgThreads = 256, kWgStagers = kWgThreads - 32;  // the last warp issues
 constexpr int kWgDepth = 2;  // rows in flight per CTA (1: 118 us, 2: 99, 3: 101, 4: 104)

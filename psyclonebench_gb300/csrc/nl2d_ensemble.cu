@@ -208,7 +208,7 @@ bool prepare_ens_step(int shape) {
     case 2: return set_ens_attr<Tile<16, 16, 256, 3>>();
     case 3: return set_ens_attr<Tile<64, 8>>();
     case 4: return set_ens_attr<Tile<32, 32, 512>>();
-    default: return set_ens_attr<DefaultTile>();
+    default: return set_ens_attr<Tile<32, 16>>();
   }
 }
 
@@ -223,7 +223,7 @@ void launch_ens_step_shape(bool int_mul, int nctas, const EnsDomain* doms, const
 void launch_ens_step(int shape, bool int_mul, int nctas, const EnsDomain* doms,
                      const int4* tiles, const int* first, int parity, const double* tides,
                      cudaStream_t st) {
-  auto launch = launch_ens_step_shape<DefaultTile>;
+  auto launch = launch_ens_step_shape<Tile<32, 16>>;
   switch (shape) {
     case 1: launch = launch_ens_step_shape<Tile<32, 8, 256, 3>>; break;
     case 2: launch = launch_ens_step_shape<Tile<16, 16, 256, 3>>; break;
@@ -530,9 +530,9 @@ double tide_at(const DomainHost& D, int istep, double rdt) {
   return D.amp * std::sin(omega_tide * rtime);
 }
 
-// Tile list and static schedule.  A domain's ring units come before its
-// tiles; a ring cell's general code is worth boundary_weight regular cells
-// beside the one it is (with weight 0, 512 domains longest first, all ring units
+// Tile list and static schedule.  A domain's ring units come before its tiles,
+// in contiguous chunks between them; a ring cell's general code is worth
+// boundary_weight regular cells beside the one it is (with weight 0, 512 domains longest first, all ring units
 // had gone to the emptiest CTA: 136-146 ms per step).
 bool build_schedule(int TXv, int TYv) {
   Ens& e = g_ens;

@@ -15,8 +15,8 @@ namespace {
 
 // The copy region splits into interior cells, [xs+1, xe-1] x [ys+1, ye-1],
 // and the ring around them (ring_pos).  A tile is TX x TY interior cells,
-// worked on by 256 threads laid out TX x (256 / TX); each thread updates TY /
-// (256 / TX) cells of one column.  Tile<TX, TY> holds a shape's constants;
+// worked on by NT threads laid out TX x (NT / TX); each thread updates TY / (NT
+// / TX) cells of one column.  Tile<TX, TY, NT> holds a shape's constants;
 // the ensemble instantiates several shapes (its autotuner picks one), the
 // single-domain kernel picks by domain size.  Ring cells need the general
 // per-cell code, a long FP64 chain, and are taken one per thread by blocks of
@@ -426,9 +426,8 @@ __device__ __forceinline__ void general_part(const Fields& f, const FusedState& 
   }
 }
 
-// general_part out of line: the tiles' registers are sized by the regular
-// update, and the few land-side cells of a tile and the ring's cells share
-// one copy of the code.
+// general_part out of line, for the ring's cells and the tiles' Flather faces:
+// the tiles' registers are sized by the regular update.
 static __device__ __noinline__ void general_at(const Fields& f, const FusedState& fs,
                                                const Dims& d, const Scalars& p,
                                                const FastConst& k, double tide, int part, int i,
@@ -501,7 +500,6 @@ struct Tile {
   static constexpr int RX = (TX + 31) / 32 * 32, RY = (TY + 31) / 32 * 32,
                        RY1 = (TY + 32) / 32 * 32;
 };
-using DefaultTile = Tile<32, 16>;
 
 template <class T>
 struct TileSmem {
@@ -1058,7 +1056,7 @@ bool in_fast_range(double d) {
   return d > 0.0 && d >= 0x1p-100 && d <= 0x1p100;
 }
 
-// c as mul_core's factor (host side).
+// c as mul_bounded's factor (host side).
 inline IntFactor int_factor(double c) {
   if (!in_fast_range(c)) return IntFactor{0, 0};
   unsigned long long b;
