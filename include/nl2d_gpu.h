@@ -289,7 +289,8 @@ int nl2d_emu_flip_transpose(const void *w, void *wt, int cout, int cin,
  * memory, one persistent CTA per SM).  cin a multiple of 16 with 9*cin <=
  * 512, cout a multiple of 8 up to 128, W a multiple of 128; err (device
  * int) is set to 1 if a bounded wait ran out.  Calls on several streams and
- * threads, and under capture, keep their partial sums apart. */
+ * threads, and under capture, keep their partial sums apart (in up to 200 MB
+ * per device, kept until nl2d_finalize). */
 int nl2d_emu_conv_wgrad(const void *x, const void *dy, float *dw, float *db,
                         int batch, int H, int W, int cin, int cout, int *err,
                         void *stream);

@@ -1483,6 +1483,7 @@ void nl2d_finalize(void) {
   if (s.spec_out) cudaFreeHost(s.spec_out);
   s.spec_out = nullptr;
   noalloc_forget();
+  emu_release();
 }
 
 int nl2d_set_mode(int mode) {

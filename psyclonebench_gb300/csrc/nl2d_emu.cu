@@ -921,23 +921,25 @@ __global__ void __launch_bounds__(kSumWays * kSumElems)
 // launches on one stream do not mix.  The first kPartsStreams streams of a
 // device get one (at most 34 MB each); others, and calls under capture, whose
 // graphs may run beside their stream, allocate and free in stream order (3 us
-// per call) from a pool that keeps kPartsKept bytes.
+// per call) from a pool that keeps kPartsKept bytes.  nl2d_finalize gives all
+// of it back.
 constexpr int kPartsStreams = 4, kMaxDevices = 64;
 constexpr uint64_t kPartsKept = 64ull << 20;
+struct PartsKept {
+  std::mutex lock;
+  cudaMemPool_t pool;
+  struct {
+    unsigned long long id;
+    float* p;
+    size_t cap;
+  } of[kPartsStreams];
+} g_parts[kMaxDevices];
+
 class Parts {
  public:
   Parts(int dev, size_t n, cudaStream_t st) : st_(st) {
-    static struct {
-      std::mutex lock;
-      cudaMemPool_t pool;
-      struct {
-        unsigned long long id;
-        float* p;
-        size_t cap;
-      } of[kPartsStreams];
-    } all[kMaxDevices];
     if (dev < 0 || dev >= kMaxDevices) return;
-    auto& d = all[dev];
+    PartsKept& d = g_parts[dev];
     hold_ = std::unique_lock<std::mutex>(d.lock);
     unsigned long long id = 0;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -1277,6 +1279,18 @@ int conv_wgrad(const void* x, const void* dy, float* dw, float* db, int batch, i
 
 }  // namespace
 }  // namespace emu
+
+void emu_release() {
+  for (emu::PartsKept& d : emu::g_parts) {
+    std::lock_guard<std::mutex> hold(d.lock);
+    for (auto& e : d.of) {
+      cudaFree(e.p);  // (waits for the calls in flight)
+      e = {};
+    }
+    if (d.pool) cudaMemPoolDestroy(d.pool);
+    d.pool = nullptr;
+  }
+}
 }  // namespace nl2d
 
 using namespace nl2d::emu;

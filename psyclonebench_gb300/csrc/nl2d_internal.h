@@ -208,6 +208,9 @@ int checksum_partials_needed();
 // scratch array (nl2d_finalize calls it: after a device reset the next call
 // looks the address up again).
 void noalloc_forget();
+// Gives back the memory the weight gradients keep between calls (nl2d_emu.cu;
+// nl2d_finalize calls it).
+void emu_release();
 void launch_checksum(const double* f, int width, int x0, int x1, int y0,
                      int y1, double* partials, double* out, cudaStream_t st);
 // The same sums over FP32 fields and over (hi, lo) pairs (hi + lo in FP64).
