@@ -922,7 +922,9 @@ __global__ void __launch_bounds__(kSumWays * kSumElems)
 // device get one (at most 34 MB each); others, and calls under capture, whose
 // graphs may run beside their stream, allocate and free in stream order (3 us
 // per call) from a pool that keeps kPartsKept bytes.  nl2d_finalize gives all
-// of it back.
+// of it back.  Memory and pool are made in the relaxed capture mode: in the
+// others making them would invalidate a capture, this thread's (a program that
+// has called on its own streams so far has no pool yet) or another's.
 constexpr int kPartsStreams = 4, kMaxDevices = 64;
 constexpr uint64_t kPartsKept = 64ull << 20;
 struct PartsKept {
@@ -939,12 +941,22 @@ class Parts {
  public:
   Parts(int dev, size_t n, cudaStream_t st) : st_(st) {
     if (dev < 0 || dev >= kMaxDevices) return;
-    PartsKept& d = g_parts[dev];
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return;
+    take(g_parts[dev], dev, n);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  // After the last launch that reads p; false on a CUDA error.
+  bool done() { return !ordered_ || cudaFreeAsync(p, st_) == cudaSuccess; }
+  float* p = nullptr;  // null: none to be had
+
+ private:
+  void take(PartsKept& d, int dev, size_t n) {
     hold_ = std::unique_lock<std::mutex>(d.lock);
     unsigned long long id = 0;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess ||
-        (capture == cudaStreamCaptureStatusNone && cudaStreamGetId(st, &id) != cudaSuccess))
+    if (cudaStreamIsCapturing(st_, &capture) != cudaSuccess ||
+        (capture == cudaStreamCaptureStatusNone && cudaStreamGetId(st_, &id) != cudaSuccess))
       return;
     if (capture == cudaStreamCaptureStatusNone)
       for (auto& e : d.of) {
@@ -972,16 +984,11 @@ class Parts {
       }
       cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &kept);
     }
-    if (cudaMallocFromPoolAsync(&p, n * sizeof(float), d.pool, st) == cudaSuccess)
+    if (cudaMallocFromPoolAsync(&p, n * sizeof(float), d.pool, st_) == cudaSuccess)
       ordered_ = true;
     else
       p = nullptr;
   }
-  // After the last launch that reads p; false on a CUDA error.
-  bool done() { return !ordered_ || cudaFreeAsync(p, st_) == cudaSuccess; }
-  float* p = nullptr;  // null: none to be had
-
- private:
   std::unique_lock<std::mutex> hold_;
   cudaStream_t st_;
   bool ordered_ = false;

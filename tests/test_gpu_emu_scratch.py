@@ -48,3 +48,43 @@ def test_finalize_gives_the_scratch_back(gpulib):
     assert before - free() > 100e6
     gpulib.nl2d_finalize()
     assert before - free() < 8e6
+
+
+@pytest.mark.parametrize("other", [False, True])
+def test_scratch_made_during_a_capture(gpulib, other):
+    """After calls on one stream: the first captured one, or (other) one on a
+    new stream while another captures."""
+    import torch
+    batch, h, w, cin, cout = 2, 96, 128, 48, 48
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randint(-2, 3, (batch, h, w, cin), generator=g, device="cuda").to(torch.bfloat16)
+    dy = torch.randint(-2, 3, (batch, h, w, cout), generator=g, device="cuda").to(torch.bfloat16)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    sums = [(torch.zeros(9, cout, cin, device="cuda"), torch.zeros(cout, device="cuda"))
+            for _ in range(3)]
+    here, beside = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def gradient(k, stream):
+        assert gpulib.nl2d_emu_conv_wgrad(x.data_ptr(), dy.data_ptr(), sums[k][0].data_ptr(),
+                                          sums[k][1].data_ptr(), batch, h, w, cin, cout,
+                                          err.data_ptr(), stream.cuda_stream) == 0
+
+    torch.cuda.synchronize()
+    gpulib.nl2d_finalize()
+    gradient(0, here)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        if other:
+            gradient(2, beside)
+            sums[1][0].add_(1.0)
+        else:
+            gradient(1, torch.cuda.current_stream())
+    gpulib.nl2d_finalize()  # a graph's memory is its own
+    graph.replay()
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0 and float(sums[0][0].abs().max()) > 0
+    if other:
+        assert torch.equal(sums[1][0], torch.ones_like(sums[1][0]))
+    for a, b in zip(sums[0], sums[2 if other else 1]):
+        assert torch.equal(a, b)
