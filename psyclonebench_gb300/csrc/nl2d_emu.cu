@@ -889,9 +889,49 @@ __global__ void __launch_bounds__(kWgThreads)
 // their sums are added in order.  (One thread per element made the 1216 bias
 // parts of a separate pass 100 us of dependent loads, the 152 weight parts 17.)
 constexpr int kSumWays = 8, kSumElems = 32;
-__global__ void __launch_bounds__(kSumWays * kSumElems)
+
+// The call's inputs, for k_sum_parts.
+struct WgradInputs {
+  const __nv_bfloat16 *x, *dy;
+  int batch, H, W, cin, cout;
+};
+// Element e of dw over image rows [r0, r1), by itself: per 128 pixels in FP32,
+// these in FP64.  Ends at a NaN.
+__device__ __noinline__ double wgrad_element(const WgradInputs& in, long long e, long long r0,
+                                             long long r1) {
+  const int ci = (int)(e % in.cin), co = (int)(e / in.cin % in.cout),
+            tap = (int)(e / ((long long)in.cin * in.cout));
+  const int oy = tap / 3 - 1, ox = tap % 3 - 1;
+  double sum = 0.0;
+  for (long long r = r0; r < r1 && sum == sum; r++) {
+    const int y = (int)(r % in.H);
+    const bool yin = y + oy >= 0 && y + oy < in.H;
+    const __nv_bfloat16* d = in.dy + (size_t)r * in.W * in.cout + co;
+    for (int x0 = 0; x0 < in.W; x0 += kTileM) {
+      float acc = 0.f;
+#pragma unroll 4
+      for (int px = x0; px < x0 + kTileM; px++) {
+        const bool xin = yin && px + ox >= 0 && px + ox < in.W;
+        const float xv =
+            xin ? __bfloat162float(in.x[((r + oy) * in.W + px + ox) * in.cin + ci]) : 0.f;
+        acc = fmaf(__bfloat162float(d[(size_t)px * in.cout]), xv, acc);
+      }
+      sum += acc;
+    }
+  }
+  return sum;
+}
+
+// direct: the rows were stacked in pairs.  At the ends of a CTA's rows the pair
+// holds a zero row of dY, whose products with an infinity or a NaN of X are NaN
+// where the gradient has none, so sums that are NaN are formed again without it.
+// (Finite inputs: never; the vote takes 1 us of a call's 99.5 at 16 x 256^2.  Six
+// blocks per SM, so that 648 run at once: at the 64 registers that
+// wgrad_element asks for the call took 1 us more.)
+__global__ void __launch_bounds__(kSumWays * kSumElems, 6)
     k_sum_parts(const float* __restrict__ part, int nparts, long long nel, int cout,
-                float* __restrict__ dw, float* __restrict__ db) {
+                float* __restrict__ dw, float* __restrict__ db,
+                const __grid_constant__ WgradInputs in, int direct) {
   __shared__ float sums[kSumWays][kSumElems];
   const int lane = threadIdx.x % kSumElems, way = threadIdx.x / kSumElems;
   const long long n = nel + cout, e = (long long)blockIdx.x * kSumElems + lane;
@@ -904,13 +944,28 @@ __global__ void __launch_bounds__(kSumWays * kSumElems)
   }
   sums[way][lane] = acc;
   __syncthreads();
-  if (way == 0 && e < n) {
+  float total = sums[0][lane];
 #pragma unroll
-    for (int w = 1; w < kSumWays; w++) acc += sums[w][lane];
+  for (int w = 1; w < kSumWays; w++) total += sums[w][lane];
+  const bool again = direct && e < nel && total != total;
+  if (__syncthreads_or(again)) {
+    __shared__ double exact[kSumWays][kSumElems];
+    const long long rows = (long long)in.batch * in.H;
+    exact[way][lane] = again ? wgrad_element(in, e, rows * way / kSumWays,
+                                             rows * (way + 1) / kSumWays)
+                             : 0.0;
+    __syncthreads();
+    if (again) {
+      double t = exact[0][lane];
+      for (int w = 1; w < kSumWays; w++) t += exact[w][lane];
+      total = (float)t;
+    }
+  }
+  if (way == 0 && e < n) {
     if (e < nel)
-      dw[e] += acc;
+      dw[e] += total;
     else
-      db[e - nel] += acc;
+      db[e - nel] += total;
   }
 }
 
@@ -1279,7 +1334,9 @@ int conv_wgrad(const void* x, const void* dy, float* dw, float* db, int batch, i
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, parts.p, batch, H, W, cin, cout, slots,
       max_cycles, err);
   k_sum_parts<<<(int)((nel + cout + kSumElems - 1) / kSumElems), kSumWays * kSumElems, 0, st>>>(
-      parts.p, grid, nel, cout, dw, db);
+      parts.p, grid, nel, cout, dw, db,
+      WgradInputs{(const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, batch, H, W, cin, cout},
+      cout <= 64);
   const cudaError_t launched = cudaGetLastError();
   return parts.done() && launched == cudaSuccess ? NL2D_OK : NL2D_ERR_CUDA;
 }
