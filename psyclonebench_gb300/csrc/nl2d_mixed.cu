@@ -177,7 +177,9 @@ __global__ void k_from_mixed(const float2* __restrict__ sn2, const float* __rest
 
 namespace {
 // The march's strip height: one wave of at most four blocks per SM where the
-// strips are then no taller than kWaveRows (and no shorter than 8), else MR.
+// strips are then no taller than kWaveRows (and no shorter than 8) and the wave
+// has the SMs to itself, else MR, halved (down to 8) until the grid holds about
+// two waves of five blocks: a smaller domain trades halo rows for parallelism.
 // The march lives on the L1: neighbouring warps share the 128-byte lines at
 // their columns' edges and the rows in flight are held there, and a fifth
 // block per SM costs more in lines evicted than its loads in flight give
@@ -185,19 +187,31 @@ namespace {
 // per SM, 62; 16 rows, three waves, 59.5; the same four blocks with 3/4 of
 // the L1 taken as shared memory 63).  One wave also leaves no strip's first
 // rows to load behind another strip.  us at the heights of this rule and
-// of the one before it (halving from 64 until two waves of five blocks):
-// 2048^2 45.9 / 59.5, 3001 x 2003 63 / 75, 4096 x 2048 89 / 96, 1024^2 18.1
-// / 18.2.  In taller strips a wave's blocks drift apart: 64 rows against the
-// wave's, 4096^2 172 us against 226 (257 rows), 3000^2 101.8 / 105.5 (126), 2100
-// x 4096 99.6 / 104.6 (121); there are exceptions up to 124 rows (2950^2 96.3 /
-// 93.8), and shorter strips gain (2700 x 3000, 113 rows, 86.7 against 90.9 by
-// the rule before).
-constexpr int kWaveRows = 120;
-int strip_rows(int ncol, int ny) {
+// of the halved ones: 2048^2 45.9 / 59.5, 3001 x 2003 63 / 75, 4096 x 2048 95 /
+// 96, 1024^2 17.6 / 18.0.  In taller strips a wave's blocks drift apart: 64 rows
+// against the wave's, 4096^2 172 us against 226 (257 rows), 3000^2 101.8 / 105.5
+// (126), 2100 x 4096 99.6 / 104.6 (121); there are exceptions up to 124 rows
+// (2950^2 96.3 / 93.8), and shorter strips gain (2700 x 3000, 113 rows, 86.7
+// against 90.9).
+// The general cells' blocks run beside the march, first come: up to three for
+// every four SMs find room beside the wave's four, more keep some of its blocks
+// out until they end, and a wave's block is the whole step long.  us, the wave's
+// strips and the halved ones, by general blocks: 2900 x 2500 84 blocks 72.8 /
+// 82.5, 123 (a coast) 94.1 / 83.8, 187 100.8 / 87.8, 1710 (a coast and an island)
+// 109.6 / 99.6; 3000 x 2000 109 blocks 71.4 / 76.3, 160 81.7 / 77.2, 1423 92.9 /
+// 86; 1500 x 1100 62 blocks 22.1 / 25.7, 271 32.2 / 31.4; 1024^2 282 blocks 20.8
+// / 20.1, 735 30.9 / 28.2.  (Exceptions: 2048^2 122 blocks 52.7 / 60, 4000 x 1000
+// 133 53.4 / 55.7.)
+constexpr int kWaveRows = 120, kGeneralThreads = 128, kWaveGeneral = 152 * 3 / 4;
+int strip_rows(int ncol, int ny, int general_blocks) {
   const int fit = 4 * 152 * MARCH_WARPS / ncol;  // strips that one such wave holds
-  if (fit < 1) return MR;
-  const int mr = (ny + fit - 1) / fit;
-  return mr > kWaveRows ? MR : (mr < 8 ? 8 : mr);
+  if (fit >= 1 && general_blocks <= kWaveGeneral) {
+    const int mr = (ny + fit - 1) / fit;
+    if (mr <= kWaveRows) return mr < 8 ? 8 : mr;
+  }
+  int mr = MR;
+  while (mr > 8 && (long long)ncol * ((ny + mr - 1) / mr) < 2 * 152 * 5 * MARCH_WARPS) mr /= 2;
+  return mr;
 }
 }  // namespace
 
@@ -208,7 +222,8 @@ void launch_mixed_step(const MixedFields& mf, const MixedState& ms, const Fields
   const MixConst k = make_mix_const(s, um);
   const int nx = d.xe - d.xs + 3, ny = d.ye - d.ys + 2;
   const int ncol = (nx + MW - 1) / MW;
-  const int mr = strip_rows(ncol, ny);
+  const int general_blocks = (mf.gcount + kGeneralThreads - 1) / kGeneralThreads;
+  const int mr = strip_rows(ncol, ny, general_blocks);
   const int nrow = (ny + mr - 1) / mr, nwarps = ncol * nrow;
   // The general cells (a list of a few thousand, each a long chain of
   // global loads) and the march read the same buffers and write disjoint
@@ -218,8 +233,8 @@ void launch_mixed_step(const MixedFields& mf, const MixedState& ms, const Fields
   if (beside) {
     cudaEventRecord(fork, st);
     cudaStreamWaitEvent(side, fork, 0);
-    k_mixed_general<<<(mf.gcount + 127) / 128, 128, 0, side>>>(mf, ms, f, d, k, tide_table,
-                                                               tide_index, tide);
+    k_mixed_general<<<general_blocks, kGeneralThreads, 0, side>>>(mf, ms, f, d, k, tide_table,
+                                                                  tide_index, tide);
   }
   k_mixed_march<<<(nwarps + MARCH_WARPS - 1) / MARCH_WARPS, 32 * MARCH_WARPS, 0, st>>>(
       mf, ms, d, make_march_const(k), ncol, nwarps, mr);
@@ -227,8 +242,8 @@ void launch_mixed_step(const MixedFields& mf, const MixedState& ms, const Fields
     cudaEventRecord(join, side);
     cudaStreamWaitEvent(st, join, 0);
   } else if (mf.gcount > 0) {
-    k_mixed_general<<<(mf.gcount + 127) / 128, 128, 0, st>>>(mf, ms, f, d, k, tide_table,
-                                                             tide_index, tide);
+    k_mixed_general<<<general_blocks, kGeneralThreads, 0, st>>>(mf, ms, f, d, k, tide_table,
+                                                                tide_index, tide);
   }
 }
 
