@@ -26,6 +26,8 @@
 //
 // Built with -fmad=false, as the reference oracle is with
 // -ffp-contract=off: results are bit-identical to the reference serial build.
+#include <type_traits>
+
 #include "nl2d_fused_tile.cuh"
 #include "nl2d_intfp.cuh"
 
@@ -69,8 +71,11 @@ __global__ void __launch_bounds__(TT::NTHREADS, TT::kMinBlocks)
     return;
   }
   const int t = blockIdx.x - nring, by = t / ntx, bx = t - by * ntx;
-  fused_tile<TT, IC, SUMS>(f, fs, d, p, k, td, d.xs + 1 + bx * TT::TX, d.ys + 1 + (row0 + by) * TT::TY,
-                 smem);
+  // (in line, the general cells' code made large domains without land slower:
+  // 1024^2 146.7 -> 151.9 us, 2048^2 560 -> 572; with 10 % of the cells dry faster,
+  // 371 -> 361; small domains 13.4 -> 13.1, with land 22.8 -> 22.1)
+  fused_tile<TT, IC, SUMS, std::is_same<TT, T>::value>(f, fs, d, p, k, td, d.xs + 1 + bx * TT::TX,
+                                                       d.ys + 1 + (row0 + by) * TT::TY, smem);
 }
 
 int tiles_over(int n, int t) { return n > 0 ? (n + t - 1) / t : 0; }

@@ -548,33 +548,42 @@ struct TileCtx {
   __device__ __forceinline__ double sv(int i, int j) const { return sv_at[at(i, j)]; }
 };
 
-// general_part for a cell of the tile staged in shared memory: the same
-// operations on the staged values, whose faces are formed once per tile.  By
-// general_at, which reads global memory and forms each part's seven faces anew
-// (FP64 products, the pipe that bounds the step), us per step: 2048^2 with 3 %
-// of the cells dry 2820, so 1320; 1024^2 with half of them dry 695 and 409; 601
-// x 413 with a coast and an island 61.2 and 49.6.  A Flather face reads two
-// cells on and goes there.
+// A cell of the tile staged in shared memory, by the general code: the same
+// operations as general_part's on the staged values, whose faces are formed once
+// per tile.  By general_at, which reads global memory and forms each part's seven
+// faces anew (FP64 products, the pipe that bounds the step), us per step: 2048^2
+// with 3 % of the cells dry 2820, with the staged values 1320; 601 x 413 with a
+// coast and an island 61.2 and 49.6.  A Flather face reads two cells on and goes
+// there.  One thread takes a cell's three parts, as independent chains: a thread
+// for each part kept three times as many warps on the FP64 and integer pipes for
+// it (10 % of the cells dry: 601 x 413 110.1 us, so 102.2; 1024^2 412 and 371; 16
+// domains of 256^2 537 and 466; 200 of 60^2 on static schedules in 32 x 8 tiles
+// 589 and 459).
 template <class T>
-__device__ __noinline__ void general_in_tile(const Fields& f, const FusedState& fs, const Dims& d,
-                                             const Scalars& p, const FastConst& k, double tide,
-                                             int part, int i, int j, int i0, int j0) {
+__device__ __forceinline__ void general_in_tile(const Fields& f, const FusedState& fs,
+                                                const Dims& d, const Scalars& p,
+                                                const FastConst& k, double tide, int i, int j,
+                                                int i0, int j0) {
   extern __shared__ double smem[];
   const TileCtx<T> x(smem, f, d, k, i0, j0);
   const int c = x.at(i, j), g = x.global(i, j);
-  if (part == kPartSsh) {
-    fs.sshn_out[g] = general_ssh(x, k, tide, i, j);
-  } else if (part == kPartU) {
-    if (flather_face(x.m[c], x.m[c + 1], i) == i)
-      fs.un_out[g] = ua_pre_flather(x, f.ua, i, j);
-    else
-      general_at(f, fs, d, p, k, tide, part, i, j);
-  } else {
-    if (flather_face(x.m[c], x.m[c + x.W], j) == j)
-      fs.vn_out[g] = va_pre_flather(x, f.va, i, j);
-    else
-      general_at(f, fs, d, p, k, tide, part, i, j);
-  }
+  if (flather_face(x.m[c], x.m[c + x.W], j) == j)
+    fs.vn_out[g] = va_pre_flather(x, f.va, i, j);
+  else
+    general_at(f, fs, d, p, k, tide, kPartV, i, j);
+  if (flather_face(x.m[c], x.m[c + 1], i) == i)
+    fs.un_out[g] = ua_pre_flather(x, f.ua, i, j);
+  else
+    general_at(f, fs, d, p, k, tide, kPartU, i, j);
+  fs.sshn_out[g] = general_ssh(x, k, tide, i, j);
+}
+// The same out of line, for kernels whose regular update it would slow down.
+template <class T>
+__device__ __noinline__ void general_in_tile_apart(const Fields& f, const FusedState& fs,
+                                                   const Dims& d, const Scalars& p,
+                                                   const FastConst& k, double tide, int i, int j,
+                                                   int i0, int j0) {
+  general_in_tile<T>(f, fs, d, p, k, tide, i, j, i0, j0);
 }
 
 // A regular cell's new (sshn_t, un, vn) from the tile's staged fields (a0)
@@ -973,7 +982,8 @@ __device__ __forceinline__ void tile_update(const Fields& f, const FusedState& f
 }
 
 // One tile of the fused step: interior cells [i0, i0+TX) x [j0, j0+TY) of one
-// domain.  `tide` is this step's bc_ssh value (general cells).
+// domain.  `tide` is this step's bc_ssh value (general cells).  APART: the general
+// cells' code out of line.
 //
 // The FP64 pipe bounds the step (about 1.7 instructions per clock per SM;
 // each holds a scheduler's share of it for 64 issue slots), so every phase
@@ -984,7 +994,7 @@ __device__ __forceinline__ void tile_update(const Fields& f, const FusedState& f
 // cell of the form that used it for everything on 2- and 1-cell halos.  The
 // integer forms pay only as straight-line code: with a range branch each,
 // the same products made the step slower.
-template <class T, bool IC, bool SUMS = true>
+template <class T, bool IC, bool SUMS = true, bool APART = false>
 __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs, const Dims& d,
                                            const Scalars& p, const FastConst& k, double tide,
                                            int i0, int j0, double* smem) {
@@ -1043,10 +1053,12 @@ __device__ __forceinline__ void fused_tile(const Fields& f, const FusedState& fs
 
   // ---- general cells: the reference's per-point code, in its order ----
   const int ngen = *gcount;
-  for (int g = tid; g < kParts * ngen; g += NTHREADS) {
-    const int part = g / ngen, cell = glist[g - part * ngen];
-    const int row = cell / TX, col = cell - row * TX;
-    general_in_tile<T>(f, fs, d, p, k, tide, part, i0 + col, j0 + row, i0, j0);
+  for (int g = tid; g < ngen; g += NTHREADS) {
+    const int row = glist[g] / TX, col = glist[g] - row * TX;
+    if (APART)
+      general_in_tile_apart<T>(f, fs, d, p, k, tide, i0 + col, j0 + row, i0, j0);
+    else
+      general_in_tile<T>(f, fs, d, p, k, tide, i0 + col, j0 + row, i0, j0);
   }
 #undef A
 #undef B
