@@ -231,8 +231,9 @@ int nl2d_ens_set_domain(int dom, const int *tmask, const double *ht,
  * time first, 2 one tile per CTA with as many CTAs as tiles, balanced by the
  * hardware block scheduler, the default; the CTA count then does not apply)
  * and the cost weight of a ring cell (a cell of the domain's boundary rows and
- * columns, which takes the general per-cell code) against a regular one (4).  A
- * new ensemble starts with the defaults (2 CTAs). */
+ * columns, which takes the general per-cell code) against a regular one (4; 85
+ * of them count half a tile at most).  A new ensemble starts with the defaults
+ * (2 CTAs). */
 int nl2d_ens_schedule(int ctas_per_sm, int policy, double boundary_weight);
 /* Tile knobs the autotuner searches (the reference's tiled OpenMP layer,
  * psykal_omp/time_step_mod.f90:587-1182, fixes its tile size per run): the

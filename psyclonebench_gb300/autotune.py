@@ -33,7 +33,7 @@ from .ensemble import DEFAULT_KNOBS
 
 # Raised whenever the kernels or the meaning of a knob change what a choice
 # costs: entries stored under another version are not used.
-COSTS_VERSION = 2
+COSTS_VERSION = 3
 
 # (CTAs per SM, policy, boundary weight); policy 2 (one tile per CTA)
 # ignores the CTAs per SM and the edge weight

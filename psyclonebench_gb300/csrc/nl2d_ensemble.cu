@@ -201,11 +201,13 @@ bool set_ens_attr() {
 }
 
 // Opts the chosen shape's kernel into its dynamic shared memory (before any
-// stream capture).
-bool prepare_ens_step(int shape) {
+// stream capture).  shared: three CTAs per SM (policy 2).  The static schedules
+// start two at most, and get the registers of two (128 for 80: 1 % on average over
+// 960 schedules, up to 14).
+bool prepare_ens_step(int shape, bool shared) {
   switch (shape) {
-    case 1: return set_ens_attr<Tile<32, 8, 256, 3>>();
-    case 2: return set_ens_attr<Tile<16, 16, 256, 3>>();
+    case 1: return shared ? set_ens_attr<Tile<32, 8, 256, 3>>() : set_ens_attr<Tile<32, 8>>();
+    case 2: return shared ? set_ens_attr<Tile<16, 16, 256, 3>>() : set_ens_attr<Tile<16, 16>>();
     case 3: return set_ens_attr<Tile<64, 8>>();
     case 4: return set_ens_attr<Tile<32, 32, 512>>();
     default: return set_ens_attr<Tile<32, 16>>();
@@ -220,13 +222,19 @@ void launch_ens_step_shape(bool int_mul, int nctas, const EnsDomain* doms, const
 }
 
 // int_mul: every domain's constants have the integer form (FastConst).
-void launch_ens_step(int shape, bool int_mul, int nctas, const EnsDomain* doms,
+void launch_ens_step(int shape, bool shared, bool int_mul, int nctas, const EnsDomain* doms,
                      const int4* tiles, const int* first, int parity, const double* tides,
                      cudaStream_t st) {
   auto launch = launch_ens_step_shape<Tile<32, 16>>;
   switch (shape) {
-    case 1: launch = launch_ens_step_shape<Tile<32, 8, 256, 3>>; break;
-    case 2: launch = launch_ens_step_shape<Tile<16, 16, 256, 3>>; break;
+    case 1:
+      launch = shared ? launch_ens_step_shape<Tile<32, 8, 256, 3>>
+                      : launch_ens_step_shape<Tile<32, 8>>;
+      break;
+    case 2:
+      launch = shared ? launch_ens_step_shape<Tile<16, 16, 256, 3>>
+                      : launch_ens_step_shape<Tile<16, 16>>;
+      break;
     case 3: launch = launch_ens_step_shape<Tile<64, 8>>; break;
     case 4: launch = launch_ens_step_shape<Tile<32, 32, 512>>; break;
     default: break;
@@ -531,9 +539,15 @@ double tide_at(const DomainHost& D, int istep, double rdt) {
 }
 
 // Tile list and static schedule.  A domain's ring units come before its tiles,
-// in contiguous chunks between them; a ring cell's general code is worth
-// boundary_weight regular cells beside the one it is (with weight 0, 512 domains longest first, all ring units
-// had gone to the emptiest CTA: 136-146 ms per step).
+// in contiguous chunks between them.  A tile cut off by the domain's end counts as
+// a whole one: its threads' chains are as long.  A ring cell counts boundary_weight
+// regular cells beside the one it is, a unit of them at most half a tile: its three
+// parts run as a warp's threads beside each other, shorter than a tile's chain (with
+// weight 0, 512 domains longest first, all ring units had gone to the emptiest CTA:
+// 136-146 ms per step; at its full weight a unit of weight 4 and more kept a CTA
+// from tiles).  us per step, the cells and full weights counted, and so: 8 domains
+// of 100^2 longest first, one CTA per SM, 32 x 32 tiles 134 and 46, in contiguous
+// chunks, two CTAs, 16 x 16 94 and 42.
 bool build_schedule(int TXv, int TYv) {
   Ens& e = g_ens;
   struct T {
@@ -557,15 +571,16 @@ bool build_schedule(int TXv, int TYv) {
     auto ring_until = [&](long long tile) {
       for (; u < units && (every == 0 || u * every / units <= tile); u++)
         tiles.push_back({k, 0, 0, u * kRingUnit,
-                         (1.0 + e.boundary_weight) * std::min(kRingUnit, nr - u * kRingUnit) /
-                             kParts});
+                         std::min((1.0 + e.boundary_weight) *
+                                      std::min(kRingUnit, nr - u * kRingUnit) / kParts,
+                                  0.5 * (TXv * TYv))});
     };
     ring_until(0);
     for (int by = 0; by < nty; by++)
       for (int bx = 0; bx < ntx; bx++) {
         ring_until((long long)by * ntx + bx);
-        const int cx = std::min(TXv, nx - bx * TXv), cy = std::min(TYv, ny - by * TYv);
-        tiles.push_back({k, D.xs + 1 + bx * TXv, D.ys + 1 + by * TYv, -1, (double)(cx * cy)});
+        tiles.push_back(
+            {k, D.xs + 1 + bx * TXv, D.ys + 1 + by * TYv, -1, (double)(TXv * TYv)});
       }
   }
   int dev = 0, sms = 0;
@@ -1140,7 +1155,7 @@ int nl2d_ens_run(int istep0, int nsteps, int checksum_every, double* checksums_o
     if (e.graph) cudaGraphExecDestroy(e.graph);
     e.graph = nullptr;
     cudaGraph_t g = nullptr;
-    if (e.precision == 0 && !prepare_ens_step(e.shape)) return NL2D_ERR_CUDA;
+    if (e.precision == 0 && !prepare_ens_step(e.shape, e.policy == 2)) return NL2D_ERR_CUDA;
     if (!ck(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal)))
       return NL2D_ERR_CUDA;
     int par = e.parity;
@@ -1185,7 +1200,8 @@ int nl2d_ens_run(int istep0, int nsteps, int checksum_every, double* checksums_o
           k_ensemble_checksums<<<dim3(e.ndom, 3), 256, 0, e.stream>>>(e.d_desc, par, e.ndom,
                                                                       sums);
       } else {
-        launch_ens_step(e.shape, e.int_mul, e.nctas, e.d_desc, e.d_tiles, e.d_first, par,
+        launch_ens_step(e.shape, e.policy == 2, e.int_mul, e.nctas, e.d_desc, e.d_tiles,
+                        e.d_first, par,
                         e.d_tides + (size_t)q * e.ndom, e.stream);
         par = 1 - par;
         if (want_sums)
