@@ -124,9 +124,10 @@ __device__ __forceinline__ void ring_cell(const EnsDomain* __restrict__ doms, in
 // One launch per step of the FP64-equivalent form.  A block takes one of two
 // roles: a march block runs four warps' (domain, i0, j0) units of the
 // double-float column march (nl2d_df_march.cuh); a ring block runs 128 parts
-// of exact cells (all cells' v, then u, then ssh), one per thread.  The nring
-// ring blocks are spread evenly through the
-// grid (block b is one when floor((b+1) nring / grid) > floor(b nring /
+// of exact cells (all cells' v, then u, then ssh), one per thread.  The first
+// `lead` blocks march (kDfLead: all, or none); behind them the nring ring blocks
+// are spread evenly through the
+// grid (block b of it is one when floor((b+1) nring / grid) > floor(b nring /
 // grid)), so both kinds share every SM: the march issues on the FP32 and
 // integer pipes while the exact cells wait on the FP64 pipe.  Both read the
 // state buffers of this parity and write disjoint cells.
@@ -138,20 +139,21 @@ template <bool EACH>
 __global__ void __launch_bounds__(32 * dfm::WARPS, 3)
     k_ensemble_df_step(const EnsDfDomain* __restrict__ ddoms, const int4* __restrict__ units,
                        int nunits, const EnsDomain* __restrict__ doms,
-                       const int2* __restrict__ cells, int ncells, int nring, int parity,
-                       DfConst k, const DfConst* __restrict__ dks, int mr,
+                       const int2* __restrict__ cells, int ncells, int nring, int lead,
+                       int parity, DfConst k, const DfConst* __restrict__ dks, int mr,
                        const double* __restrict__ tides) {
-  const long long grid = gridDim.x, b = blockIdx.x;
-  const int q0 = (int)(b * nring / grid), q1 = (int)((b + 1) * nring / grid);
+  const long long grid = gridDim.x - lead, b = (long long)blockIdx.x - lead;
+  const int q0 = b < 0 ? 0 : (int)(b * nring / grid),
+            q1 = b < 0 ? 0 : (int)((b + 1) * nring / grid);
   if (q1 > q0) {  // ring block q0
     const int g = q0 * (32 * dfm::WARPS) + (int)threadIdx.x;
     const int part = g / ncells;
     if (part < kParts) ring_cell(doms, cells[g - part * ncells], part, parity, tides);
     return;
   }
-  // march block b - q0: q0 ring blocks precede it
+  // q0 ring blocks precede this march block
   const int wib = (int)(threadIdx.x >> 5);
-  const int w = (int)(b - q0) * dfm::WARPS + wib;
+  const int w = ((int)blockIdx.x - q0) * dfm::WARPS + wib;
   if (w >= nunits) return;  // the whole warp leaves together
   const int4 u = units[w];
   const EnsDfDomain& D = ddoms[u.x];
@@ -171,6 +173,16 @@ __global__ void __launch_bounds__(32 * dfm::WARPS, 3)
 // The mixed march's strip height until the autotuner or the caller chooses one
 // (8, 16, 32 or 64 rows).  96 domains of 256^2: 16 rows 113 us, 32 110, 64 119.
 constexpr int kDefaultMarchRows = 32;
+
+// March blocks of the FP64-equivalent form up to which they come first in the
+// grid: two of each SM's three.  A march block there is long beside a ring
+// block, and behind the ring blocks before it (three times as many since an exact
+// cell has three threads) it ended the step late.  us per step, spread evenly with
+// a thread per cell, with three, and first: 16 domains of 128^2 in strips of 64
+// rows 110, 141 and 79; of 1000 x 20 48.3, 54.3 and 34.4; 4 of 256^2 in strips of 32
+// rows 43.0, 55.4 and 41.2; 8 of 100^2 by the rule 47.6, 18.5 and 14.3.  (Above, the
+// march fills the SMs by itself: 32 domains of 256^2 the same either way.)
+constexpr int kDfLead = 2 * 152;
 
 // The tile shapes the ensemble's FP64 kernel is built for (the autotuner's
 // search space).  Until it or the caller chooses, 32 x 8 with one tile per CTA
@@ -1186,15 +1198,16 @@ int nl2d_ens_run(int istep0, int nsteps, int checksum_every, double* checksums_o
         constexpr int B = 32 * dfm::WARPS;
         const int nring = (kParts * e.ndfring + B - 1) / B;
         const int nmarch = (e.ndfunits + dfm::WARPS - 1) / dfm::WARPS;
+        const int lead = nmarch <= kDfLead ? nmarch : 0;
         const double* tq = e.d_tides + (size_t)q * e.ndom;
         if (e.d_dks)
           k_ensemble_df_step<true><<<nring + nmarch, B, 0, e.stream>>>(
-              e.d_dfdesc, e.d_dfunits, e.ndfunits, e.d_desc, e.dfring, e.ndfring, nring, par,
-              e.dk, e.d_dks, strip, tq);
+              e.d_dfdesc, e.d_dfunits, e.ndfunits, e.d_desc, e.dfring, e.ndfring, nring, lead,
+              par, e.dk, e.d_dks, strip, tq);
         else
           k_ensemble_df_step<false><<<nring + nmarch, B, 0, e.stream>>>(
-              e.d_dfdesc, e.d_dfunits, e.ndfunits, e.d_desc, e.dfring, e.ndfring, nring, par,
-              e.dk, nullptr, strip, tq);
+              e.d_dfdesc, e.d_dfunits, e.ndfunits, e.d_desc, e.dfring, e.ndfring, nring, lead,
+              par, e.dk, nullptr, strip, tq);
         par = 1 - par;
         if (want_sums)
           k_ensemble_checksums<<<dim3(e.ndom, 3), 256, 0, e.stream>>>(e.d_desc, par, e.ndom,
