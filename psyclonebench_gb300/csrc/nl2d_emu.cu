@@ -563,7 +563,7 @@ __global__ void k_flip_transpose(const __nv_bfloat16* __restrict__ w,
 //   warp 7     one thread issues the MMAs
 // 48 -> 48 channels at 16 x 256^2: 193 us (9 x N = 48 per row, one row in
 // flight in registers) plus 100 us for a separate bias pass and the sums before,
-// 98 us with everything now.  Of an SM's active clocks the operand reads take 49
+// 100 us with everything now.  Of an SM's active clocks the operand reads take 49
 // %, the tensor core's data path 52 %, its arithmetic (an unused quadrant in
 // four) 42 %, DRAM 32 %; about 15 us are the launch's start and the accumulators'
 // way out, which nothing runs beside.

@@ -558,7 +558,8 @@ struct TileCtx {
 // for each part kept three times as many warps on the FP64 and integer pipes for
 // it (10 % of the cells dry: 601 x 413 110.1 us, so 102.2; 1024^2 412 and 371; 16
 // domains of 256^2 537 and 466; 200 of 60^2 on static schedules in 32 x 8 tiles
-// 589 and 459).
+// 589 and 459; where such cells are few the chain is longer: 601 x 413 with the
+// coast 50.8 and 51.9).
 template <class T>
 __device__ __forceinline__ void general_in_tile(const Fields& f, const FusedState& fs,
                                                 const Dims& d, const Scalars& p,
